@@ -239,9 +239,9 @@ void compute_certificates(gprm_space* h, const int* from, const int* to)
          * certificates go through pair_certified). */
         float4 fr = make_float4(0.0f, 0.0f, 0.0f, INFINITY);
         float4 sbv = make_float4(0.0f, 0.0f, 0.0f, Rf);
-        int usable = 0;
+        int usable = SCAN_GENERAL;
         if (T2 < INFINITY && (sa >= 0 || sb >= 0)) {
-            usable = 1;
+            usable = SCAN_USABLE;
             if (sa < 0 || sb < 0) {
                 const int blk = sa < 0 ? h->pairs[j].x : h->pairs[j].y;
                 const float4 c = h->tab[blk], v = h->tab[blk + 1];
@@ -940,6 +940,8 @@ int gprm_init(gprm_space* h, int rank, int size)
     s.nslots = (int)h->slot_sys.size();
     for (int i = 0; i < s.nslots; ++i) { s.slot_sys[i] = h->slot_sys[i]; s.slot_block[i] = h->slot_block[i]; }
 
+    CUDA_TRY(h, launch_static_pairs(s, cudaStreamLegacy));   /* after the uploads, on their stream */
+    CUDA_TRY(h, cudaStreamSynchronize(cudaStreamLegacy));
     CUDA_TRY(h, plan_launch(s, 1, 128, &h->cfg_v));
     CUDA_TRY(h, plan_launch(s, 0, 128, &h->cfg_e));
     CUDA_TRY(h, dev_malloc((void**)&h->d_total, sizeof(Control)));
@@ -1017,6 +1019,8 @@ int gprm_set_band(gprm_space* h, float band_m)
         if (pb) CUDA_TRY(h, cudaMemcpy((char*)h->d_scene + tb + 4 * pb, h->scan_b.data(), pb, cudaMemcpyHostToDevice));
         h->dsc.thr_dir = h->thr_dir;
         h->dsc.eps_dir = h->eps_dir;
+        CUDA_TRY(h, launch_static_pairs(h->dsc, cudaStreamLegacy));
+        CUDA_TRY(h, cudaStreamSynchronize(cudaStreamLegacy));
     }
     return GPRM_OK;
 }

@@ -41,6 +41,10 @@
 #ifndef GPRM_CLIMB_CHUNK
 #define GPRM_CLIMB_CHUNK 1
 #endif
+/* how the certificate scan treats a pair (scan_c.w) */
+#define SCAN_GENERAL 0      /* through pair_certified (no slot, or two static polytopes) */
+#define SCAN_USABLE  1      /* by the scan's own tests */
+#define SCAN_SETTLED 2      /* two static polytopes whose certificate holds: always free */
 #define GPRM_MAX_ITERS 10   /* max_for_loop, max_for_loop_whole (collision4.h:17-18) */
 
 namespace gprm {
@@ -61,8 +65,7 @@ struct DevScene {
     const float4* pairs_b;
     /* certificate scan per pair: far = (static partner's ball centre, T2);
        scan_c = (slot of P, slot of Q (-1: in frame 0), sqrt(T2) rounded up
-       (float bits), usable by the scan); scan_b = (static partner's vertex
-       0, R) */
+       (float bits), SCAN_*); scan_b = (static partner's vertex 0, R) */
     const float4* far;
     const int4* scan_c;
     const float4* scan_b;

@@ -132,6 +132,10 @@ size_t frame_smem_bytes(const DevScene& sc, int threads, bool vertex_kernel);
 cudaError_t configure_launch(const DevScene& sc, int vertex_kernel, int threads, int scene_in_smem,
                              LaunchCfg* cfg, int blocks_cap = 0);
 
+/* Settles the pairs between polytopes of frame 0 in sc.scan_c (once per
+ * upload of the certificate tables). */
+cudaError_t launch_static_pairs(const DevScene& sc, cudaStream_t st);
+
 /* Vertex checks: res[i] = code of configuration q[i + offset*j]. */
 cudaError_t launch_check_configs(const DevScene& sc, const LaunchCfg& cfg, const float* q,
                                  long long n, long long offset, int* res, int band_on, float band,
