@@ -217,6 +217,7 @@ void compute_certificates(gprm_space* h, const int* from, const int* to)
     h->far.resize(h->npairs);
     h->scan_c.resize(h->npairs);
     h->scan_b.resize(h->npairs);
+    h->swp.resize(h->npairs);
     for (int j = 0; j < h->npairs; ++j) {
         int a = h->pair_poly[2 * j], b = h->pair_poly[2 * j + 1];
         bool ok = (h->pair_sys[2 * j] == 0 || h->slot[a] >= 0) && (h->pair_sys[2 * j + 1] == 0 || h->slot[b] >= 0);
@@ -257,6 +258,18 @@ void compute_certificates(gprm_space* h, const int* from, const int* to)
         h->far[j] = fr;
         h->scan_c[j] = make_int4(sa, sb, sqb, usable);
         h->scan_b[j] = sbv;
+        /* two slots need 8 bits; a pair of one slot with itself has no
+           second one and stays out of the sweep stage */
+        float4 sw = make_float4(NAN, NAN, NAN, NAN);
+        if (usable == SCAN_USABLE && sa != sb) {
+            static_assert(GPRM_MAX_SLOTS <= 16, "a slot takes 4 bits of the record");
+            const int s0 = sa >= 0 ? sa : sb, s1 = sa >= 0 && sb >= 0 ? sb : s0;
+            const int bits = (sqb & ~255) + 256;   /* rounded up to a multiple of 256 ulp */
+            const int word = (bits & ~255) | s0 | (s1 << 4);
+            memcpy(&sw.w, &word, 4);
+            sw.x = fr.x; sw.y = fr.y; sw.z = fr.z;
+        }
+        h->swp[j] = sw;
     }
     h->thr_dir = (float)thr;
     h->eps_dir = (float)(7.0 * eps_pos);
@@ -882,10 +895,10 @@ int gprm_init(gprm_space* h, int rank, int size)
         }
     }
 
-    /* d_scene: tab | pairs | pairs_b | far | scan_c | scan_b | ppoly | box | vtab | vinfo | ctab | ccnt */
+    /* d_scene: tab | pairs | pairs_b | far | scan_c | scan_b | swp | ppoly | box | vtab | vinfo | ctab | ccnt */
     size_t tb = h->tab.size() * sizeof(float4), pb = (size_t)h->npairs * sizeof(int4);
     size_t fsb = (size_t)h->npairs * sizeof(int2);
-    size_t bxo = tb + 5 * pb + fsb, bxb = h->box.size() * sizeof(float4);
+    size_t bxo = tb + 6 * pb + fsb, bxb = h->box.size() * sizeof(float4);
     bxo = (bxo + 15) & ~(size_t)15;
     const size_t vto = (bxo + bxb + 15) & ~(size_t)15, vtb = h->vtab.size() * sizeof(float4);
     const size_t vio = vto + vtb, vib = h->vinfo.size() * sizeof(int4);
@@ -899,7 +912,8 @@ int gprm_init(gprm_space* h, int rank, int size)
     if (pb) CUDA_TRY(h, cudaMemcpy(base + tb + 2 * pb, h->far.data(), pb, cudaMemcpyHostToDevice));
     if (pb) CUDA_TRY(h, cudaMemcpy(base + tb + 3 * pb, h->scan_c.data(), pb, cudaMemcpyHostToDevice));
     if (pb) CUDA_TRY(h, cudaMemcpy(base + tb + 4 * pb, h->scan_b.data(), pb, cudaMemcpyHostToDevice));
-    if (pb) CUDA_TRY(h, cudaMemcpy(base + tb + 5 * pb, h->pair_poly.data(), fsb, cudaMemcpyHostToDevice));
+    if (pb) CUDA_TRY(h, cudaMemcpy(base + tb + 5 * pb, h->swp.data(), pb, cudaMemcpyHostToDevice));
+    if (pb) CUDA_TRY(h, cudaMemcpy(base + tb + 6 * pb, h->pair_poly.data(), fsb, cudaMemcpyHostToDevice));
     if (bxb) CUDA_TRY(h, cudaMemcpy(base + bxo, h->box.data(), bxb, cudaMemcpyHostToDevice));
     if (vtb) CUDA_TRY(h, cudaMemcpy(base + vto, h->vtab.data(), vtb, cudaMemcpyHostToDevice));
     if (vib) CUDA_TRY(h, cudaMemcpy(base + vio, h->vinfo.data(), vib, cudaMemcpyHostToDevice));
@@ -927,7 +941,8 @@ int gprm_init(gprm_space* h, int rank, int size)
     s.far = (const float4*)(base + tb + 2 * pb);
     s.scan_c = (const int4*)(base + tb + 3 * pb);
     s.scan_b = (const float4*)(base + tb + 4 * pb);
-    s.ppoly = (const int2*)(base + tb + 5 * pb);
+    s.swp = (const float4*)(base + tb + 5 * pb);
+    s.ppoly = (const int2*)(base + tb + 6 * pb);
     s.box = bxb ? (const float4*)(base + bxo) : nullptr;
     s.vtab = (const float4*)(base + vto);
     s.vinfo = (const int4*)(base + vio);
@@ -1017,6 +1032,7 @@ int gprm_set_band(gprm_space* h, float band_m)
         if (pb) CUDA_TRY(h, cudaMemcpy((char*)h->d_scene + tb + 2 * pb, h->far.data(), pb, cudaMemcpyHostToDevice));
         if (pb) CUDA_TRY(h, cudaMemcpy((char*)h->d_scene + tb + 3 * pb, h->scan_c.data(), pb, cudaMemcpyHostToDevice));
         if (pb) CUDA_TRY(h, cudaMemcpy((char*)h->d_scene + tb + 4 * pb, h->scan_b.data(), pb, cudaMemcpyHostToDevice));
+        if (pb) CUDA_TRY(h, cudaMemcpy((char*)h->d_scene + tb + 5 * pb, h->swp.data(), pb, cudaMemcpyHostToDevice));
         h->dsc.thr_dir = h->thr_dir;
         h->dsc.eps_dir = h->eps_dir;
         CUDA_TRY(h, launch_static_pairs(h->dsc, cudaStreamLegacy));
@@ -1041,7 +1057,7 @@ int gprm_get_stats(const gprm_space* hc, gprm_stats* out)
     out->edge_steps_executed = (int64_t)tot.steps_exec;
     out->band_rechecks = (int64_t)tot.band_checks;
     out->band_flips = (int64_t)tot.band_flips;
-    out->pairs_certified = (int64_t)(tot.cert_far + tot.cert_dir);
+    out->pairs_certified = (int64_t)tot.certified;
     out->pairs_tested = (int64_t)tot.full_tests;
     out->band_overflow_items = (int64_t)tot.ovf_count;
     if (tot.flags & GPRM_DEVFLAG_BAD_EDGE)

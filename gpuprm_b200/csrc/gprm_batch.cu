@@ -716,7 +716,7 @@ int gprm_batch_get_stats(const gprm_batch* bc, gprm_stats* out)
     out->edge_steps_executed = (int64_t)tot.steps_exec;
     out->band_rechecks = (int64_t)tot.band_checks;
     out->band_flips = (int64_t)tot.band_flips;
-    out->pairs_certified = (int64_t)(tot.cert_far + tot.cert_dir);
+    out->pairs_certified = (int64_t)tot.certified;
     out->pairs_tested = (int64_t)tot.full_tests;
     out->band_overflow_items = (int64_t)tot.ovf_count;
     if (tot.flags & GPRM_DEVFLAG_BAD_EDGE)

@@ -69,6 +69,12 @@ struct DevScene {
     const float4* far;
     const int4* scan_c;
     const float4* scan_b;
+    /* sweep stage of the edge checks per pair: the static partner's ball
+       centre (unused between two moving polytopes), and sqrt(T2) rounded up
+       with, in its low 8 bits, the slot of a moving polytope and (equal, or
+       the other moving polytope's) a second slot; negative: SCAN_SETTLED;
+       NaN: SCAN_GENERAL */
+    const float4* swp;
     /* certificates: a pair whose guaranteed separation along the first
        search direction exceeds thr_dir is reported free without the test;
        eps_dir bounds the direction error of the approximate first direction

@@ -21,8 +21,7 @@ struct Control {
     unsigned long long band_checks;   /* checks recomputed in FP64 */
     unsigned long long band_flips;    /* FP64 verdict differs from FP32 verdict */
     unsigned long long configs_exec;  /* vertex checks that ran the pair loop */
-    unsigned long long cert_far;      /* pair tests settled by the distance certificate */
-    unsigned long long cert_dir;      /* ... by the first-direction certificate */
+    unsigned long long certified;     /* pair tests settled by a certificate */
     unsigned long long full_tests;    /* pair tests that ran the Chung-Wang iteration */
     unsigned long long ovf_count;     /* items recorded in the overflow list (BandQueue) */
 };
@@ -132,8 +131,8 @@ size_t frame_smem_bytes(const DevScene& sc, int threads, bool vertex_kernel);
 cudaError_t configure_launch(const DevScene& sc, int vertex_kernel, int threads, int scene_in_smem,
                              LaunchCfg* cfg, int blocks_cap = 0);
 
-/* Settles the pairs between polytopes of frame 0 in sc.scan_c (once per
- * upload of the certificate tables). */
+/* Settles the pairs between polytopes of frame 0 in sc.scan_c and sc.swp (once
+ * per upload of the certificate tables). */
 cudaError_t launch_static_pairs(const DevScene& sc, cudaStream_t st);
 
 /* Vertex checks: res[i] = code of configuration q[i + offset*j]. */

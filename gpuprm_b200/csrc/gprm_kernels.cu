@@ -46,8 +46,8 @@ namespace gprm {
 
 size_t scene_smem_bytes(const DevScene& sc)
 {
-    /* tab | pairs | pairs_b | far | scan_c | scan_b, padded to 16 bytes */
-    return ((size_t)sc.ntab * 16 + (size_t)sc.npairs * 80 + 15) & ~(size_t)15;
+    /* tab | pairs | pairs_b | far | scan_c | scan_b | swp, padded to 16 bytes */
+    return ((size_t)sc.ntab * 16 + (size_t)sc.npairs * 96 + 15) & ~(size_t)15;
 }
 
 size_t frame_smem_bytes(const DevScene& sc, int threads, bool vertex_kernel)
@@ -62,6 +62,7 @@ struct SceneView {
     const float4* far;
     const int4* scan_c;
     const float4* scan_b;
+    const float4* swp;
     float* frames;   /* this lane's frames (lane-interleaved, stride 32) */
     float* cen;      /* this lane's slot ball centres, then the slots' world vertex 0 */
     float4* sweep;   /* the warp's per-slot sweep balls (GPRM_MAX_SLOTS) */
@@ -103,6 +104,7 @@ __device__ __forceinline__ SceneView stage_scene(const DevScene& sc, unsigned ch
         float4* fr = reinterpret_cast<float4*>(smem + (size_t)sc.ntab * 16 + np * 32);
         int4* scc = reinterpret_cast<int4*>(smem + (size_t)sc.ntab * 16 + np * 48);
         float4* scb = reinterpret_cast<float4*>(smem + (size_t)sc.ntab * 16 + np * 64);
+        float4* sw = reinterpret_cast<float4*>(smem + (size_t)sc.ntab * 16 + np * 80);
         for (int i = threadIdx.x; i < sc.ntab; i += blockDim.x) t[i] = sc.tab[i];
         for (int i = threadIdx.x; i < sc.npairs; i += blockDim.x) {
             p[i] = sc.pairs[i];
@@ -110,6 +112,7 @@ __device__ __forceinline__ SceneView stage_scene(const DevScene& sc, unsigned ch
             fr[i] = sc.far[i];
             scc[i] = sc.scan_c[i];
             scb[i] = sc.scan_b[i];
+            sw[i] = sc.swp[i];
         }
         s.tab = t;
         s.pairs = p;
@@ -117,7 +120,8 @@ __device__ __forceinline__ SceneView stage_scene(const DevScene& sc, unsigned ch
         s.far = fr;
         s.scan_c = scc;
         s.scan_b = scb;
-        off = ((size_t)sc.ntab * 16 + np * 80 + 15) & ~(size_t)15;   /* frames stay 16-byte aligned */
+        s.swp = sw;
+        off = ((size_t)sc.ntab * 16 + np * 96 + 15) & ~(size_t)15;   /* frames stay 16-byte aligned */
     } else {
         s.tab = sc.tab;
         s.pairs = sc.pairs;
@@ -125,6 +129,7 @@ __device__ __forceinline__ SceneView stage_scene(const DevScene& sc, unsigned ch
         s.far = sc.far;
         s.scan_c = sc.scan_c;
         s.scan_b = sc.scan_b;
+        s.swp = sc.swp;
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     s.frames = reinterpret_cast<float*>(smem + off) + (size_t)warp * lane_floats(sc, VERTEX) * 32 + lane;
@@ -135,52 +140,80 @@ __device__ __forceinline__ SceneView stage_scene(const DevScene& sc, unsigned ch
     return s;
 }
 
-/* Per slot, a ball holding that slot's ball centre in every lane of `mask`
- * (lanes whose frames are current): centre m = the midpoint of the lanes'
+/* min / max of three, NaN if any is NaN */
+__device__ __forceinline__ float min3_nan(float a, float b, float c)
+{
+    float d;
+    asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+__device__ __forceinline__ float max3_nan(float a, float b, float c)
+{
+    float d;
+    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
+/* Per slot, a ball holding that slot's ball centre in every lane (every
+ * lane's frames are current): centre m = the midpoint of the lanes'
  * bounding box, radius rho >= max |c_lane - m| (the box half-diagonal from
- * m, rounded up).  Lanes with a non-finite centre make rho infinite, which
- * disables the sweep tests for the slot.  Lanes 0.. nslots-1 bound the
- * slots' ball centres (sweep[slot]); with at most SWEEP_V0_SLOTS slots,
- * lanes 16.. bound the slots' vertex 0 the same way (sweep[SWEEP_V0_SLOTS
- * + slot]), for the swept direction test of cert_scan. */
+ * m, rounded up).  A non-finite centre makes rho infinite, which disables
+ * the sweep tests for the slot.  sweep[slot] bounds the slots' ball
+ * centres; with at most SWEEP_V0_SLOTS slots, sweep[SWEEP_V0_SLOTS + slot]
+ * bounds the slots' vertex 0 the same way, for the swept direction test.
+ *
+ * A row of 32 lane values per coordinate (6 rows a slot): lane r reduces
+ * row r on its own, eight 16-byte loads whose order is rotated by the lane
+ * (the rows alias in the banks), two three-input min/max a load; the three
+ * rows of a point then meet by shuffles.  One lane per point, one value at
+ * a time with 12 lanes on the same bank, took 5,800 cycles of a hull6 round
+ * (8 %); this takes about a third. */
 constexpr int SWEEP_V0_SLOTS = GPRM_MAX_SLOTS / 2;
-__device__ __forceinline__ void sweep_bounds(const DevScene& sc, const SceneView& S, unsigned mask)
+__device__ __forceinline__ void sweep_bounds(const DevScene& sc, const SceneView& S)
 {
     const int lane = threadIdx.x & 31;
     __syncwarp();   /* the lanes' centres are written */
-    const bool v0 = lane >= 16 && lane - 16 < sc.nslots && sc.nslots <= SWEEP_V0_SLOTS;
-    if (lane < sc.nslots || v0) {
-        const int sl = v0 ? lane - 16 : lane;
-        /* lane 0's points of slot sl; lane i at +i */
-        const float* c0 = S.cen - lane + (v0 ? sc.nslots * 3 * 32 : 0) + sl * 3 * 32;
-        float lo[3], hi[3];
-        bool bad = false;
-        for (int c = 0; c < 3; ++c) { lo[c] = PF32::inf(); hi[c] = -PF32::inf(); }
-        for (unsigned m = mask; m; m &= m - 1u) {
-            const int i = __ffs(m) - 1;
-            for (int c = 0; c < 3; ++c) {
-                const float v = c0[c * 32 + i];
-                bad |= !isfinite(v);
-                lo[c] = fminf(lo[c], v);
-                hi[c] = fmaxf(hi[c], v);
+    const int n3 = sc.nslots * 3;
+    const int rows = sc.nslots <= SWEEP_V0_SLOTS ? 2 * n3 : n3;
+    const float* base = S.cen - lane;   /* row r: base[r * 32 ..] */
+    float* out = reinterpret_cast<float*>(S.sweep);
+#pragma unroll 1
+    for (int r0 = 0; r0 < rows; r0 += 30) {       /* whole points per pass */
+        const int r = r0 + lane;
+        const bool mine = lane < 30 && r < rows;
+        const float4* row = reinterpret_cast<const float4*>(base + (mine ? r : 0) * 32);
+        float4 v = row[lane & 7];
+        float lo = min3_nan(v.x, v.y, v.z), hi = max3_nan(v.x, v.y, v.z);
+        lo = min3_nan(lo, v.w, v.w);
+        hi = max3_nan(hi, v.w, v.w);
+#pragma unroll
+        for (int i = 1; i < 8; ++i) {
+            v = row[(lane + i) & 7];
+            lo = min3_nan(min3_nan(lo, v.x, v.y), v.z, v.w);
+            hi = max3_nan(max3_nan(hi, v.x, v.y), v.z, v.w);
+        }
+        const float mid = 0.5f * (lo + hi);
+        const float e = fmaxf(hi - mid, mid - lo);
+        const float bad = mid - mid + (hi - lo) * 0.0f;      /* NaN unless both ends are finite */
+        const float e2 = __fmaf_rn(e, e, bad);
+        const float s2 = e2 + __shfl_down_sync(FULL_MASK, e2, 1) + __shfl_down_sync(FULL_MASK, e2, 2);
+        if (mine) {
+            const int pt = r / 3, c = r - 3 * pt;
+            float* o = out + 4 * (pt < sc.nslots ? pt : SWEEP_V0_SLOTS + pt - sc.nslots);
+            o[c] = mid;
+            if (c == 0) {
+                const float rho = __fsqrt_ru(s2) * (1.0f + 5e-6f) + 1e-30f;
+                o[3] = rho < PF32::inf() ? rho : PF32::inf();
             }
         }
-        float mc[3], e2 = 0.0f;
-        for (int c = 0; c < 3; ++c) {
-            mc[c] = 0.5f * (lo[c] + hi[c]);
-            const float e = fmaxf(hi[c] - mc[c], mc[c] - lo[c]);
-            e2 = __fmaf_rn(e, e, e2);
-        }
-        float rho = __fsqrt_ru(e2) * (1.0f + 4e-6f) + 1e-30f;
-        if (bad || !mask || !isfinite(rho)) rho = PF32::inf();
-        S.sweep[v0 ? SWEEP_V0_SLOTS + sl : sl] = make_float4(mc[0], mc[1], mc[2], rho);
     }
     __syncwarp();
 }
 
-/* Per-lane counts of how pair tests were settled. */
+/* Counts of how pair tests were settled: by a certificate (a lane's own
+ * and, in lane 0, those settled for the whole warp), by the exact test. */
 struct PairCounts {
-    unsigned long long far, dir, full;
+    unsigned long long cert, full;
 };
 
 /* The ball-distance test of pair_certified for a usable pair (scan_c.w)
@@ -226,91 +259,92 @@ __device__ __forceinline__ bool cert_dir(const DevScene& sc, const SceneView& S,
 }
 
 /* The direction test of pair_certified_dir for every lane of the warp at
- * once, for a pair with one moving polytope (slot balls bc: its ball
- * centre, bv: its vertex 0, over the lanes; f: the static partner's ball
- * centre; b: its vertex 0 and R).  With s = b_Q - a_P (vertex 0 of Q minus
- * that of P) = sbar - alpha, |alpha| <= rho_v, and D = c_Q - c_P = Dbar -
- * gamma, |gamma| <= rho_c, every lane has
- *     <s, D> >= <sbar, Dbar> - |sbar| rho_c - rho_v |Dbar| - rho_v rho_c = N
- *     |s| in [|sbar| - rho_v, |sbar| + rho_v],  |D| <= |Dbar| + rho_c,
- * so when N > 0, its G - err of the per-lane test is at least
- *     N / (|sbar| + rho_v) - R - (|Dbar| + rho_c + R)(eps_dir / (|sbar| - rho_v) + 1e-6),
+ * once.  Each polytope's ball centre lies in a ball over the lanes, and so
+ * does its vertex 0 (the slot's sweep balls; radius 0 for a polytope of
+ * frame 0): s = the difference of the vertex-0 ball centres, D = that of
+ * the centres' (both from the same polytope to the other; the sign cancels
+ * in <s, D>), rv and rc the sums of the two radii.  Every lane's s' = s -
+ * alpha, |alpha| <= rv, and D' = D - gamma, |gamma| <= rc, have
+ *     <s', D'> >= <s, D> - |s| rc - rv |D| - rv rc = N
+ *     |s'| in [|s| - rv, |s| + rv],  |D'| <= |D| + rc,
+ * so when N > 0, the G - err of the per-lane test is at least
+ *     N / (|s| + rv) - R - (|D| + rc + R)(eps_dir / (|s| - rv) + 1e-6),
  * which must exceed thr_dir (with 1e-5 relative allowances for the
- * rounding of this bound).  True when every lane's test would certify. */
-__device__ __forceinline__ bool swept_direction(const DevScene& sc, bool moving_p, float4 bc, float4 bv, float4 f,
-                                                float4 b)
+ * rounding of this bound, which cover the approximate root and quotient:
+ * a settled pair is one that every lane's own test would certify). */
+__device__ __forceinline__ bool swept_direction(const DevScene& sc, float sx, float sy, float sz, float rv, float dx,
+                                                float dy, float dz, float rc, float R)
 {
-    float sx, sy, sz, dx, dy, dz;
-    if (moving_p) {
-        sx = b.x - bv.x; sy = b.y - bv.y; sz = b.z - bv.z;
-        dx = f.x - bc.x; dy = f.y - bc.y; dz = f.z - bc.z;
-    } else {
-        sx = bv.x - b.x; sy = bv.y - b.y; sz = bv.z - b.z;
-        dx = bc.x - f.x; dy = bc.y - f.y; dz = bc.z - f.z;
-    }
-    const float sn = sqrtf(__fmaf_rn(sx, sx, __fmaf_rn(sy, sy, sz * sz)));
-    const float dn = sqrtf(__fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz)));
-    const float rv = bv.w, rc = bc.w;
+    const float n2 = __fmaf_rn(sx, sx, __fmaf_rn(sy, sy, sz * sz));
+    const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
+    const float sn = n2 * rsqrtf(n2), dn = d2 * rsqrtf(d2);   /* NaN for 0: not settled */
     const float N = __fmaf_rn(sx, dx, __fmaf_rn(sy, dy, sz * dz)) * (1.0f - 1e-5f) -
-                    (sn * rc + rv * dn + rv * rc) * (1.0f + 1e-5f);
-    const float slo = (sn - rv) * (1.0f - 1e-5f), sup = (sn + rv) * (1.0f + 1e-5f);
-    if (!(N > 0.0f) || !(slo > 1e-3f)) return false;
-    const float err = (dn + rc + b.w) * (sc.eps_dir / slo + 1e-6f) * (1.0f + 1e-5f);
-    return (N / sup) * (1.0f - 1e-5f) - b.w * (1.0f + 1e-5f) - err > sc.thr_dir;
+                    __fmaf_rn(sn, rc, __fmaf_rn(rv, dn, rv * rc)) * (1.0f + 1e-5f);
+    const float slo = sn * (1.0f - 1e-5f) - rv * (1.0f + 1e-5f), sup = (sn + rv) * (1.0f + 1e-5f);
+    const float err = (dn + rc + R) * (__fdividef(sc.eps_dir, slo) + 1e-6f) * (1.0f + 2e-5f);
+    return N > 0.0f && slo > 1e-3f && N * (1.0f - 1e-5f) > sup * (__fmaf_rn(R, 1.0f + 1e-5f, err) + sc.thr_dir);
 }
 
-/* Certificates of pairs j0 .. j0+jn-1 (jn <= 32) for this lane, all
- * order-free (a certified pair is free with its margin above the band, so
- * it changes neither a code nor a band decision), in three stages:
- *   sweep     (SWEPT, lanes holding nearby configurations) lane k tests pair
- *             j0+k against the sweep ball of its moving slot: a pair whose
- *             static partner lies farther than rho + sqrt(T2) from the sweep
- *             centre is settled for every lane at once (each lane's exact
- *             distance then exceeds sqrt(T2)); else the direction test is
- *             bounded over every lane at once (swept_direction) from the
- *             balls of the slot's centre and vertex 0;
- *   per lane  the other pairs, two at a time: the ball-distance and
- *             direction tests (cert_dist_dir), then for the few pairs both
- *             miss the box test of pair_certified_dir; pairs the scan cannot
- *             use go through pair_certified.
- * Pairs with both polytopes in frame 0 whose certificate holds
- * (SCAN_SETTLED, decided once per scene by k_static_pairs) drop out first.
- * Returns the pairs that need the exact test (bit k: pair j0+k); 0 for an
- * inactive lane.  Every lane of the warp must call it (it votes). */
-template <bool SWEPT>
-__device__ __forceinline__ unsigned cert_scan(const DevScene& sc, const SceneView& S, int j0, int jn, bool active,
-                                              PairCounts& pc)
+/* The sweep stage of an edge round for the pairs of up to 32 chunks from
+ * j0 (lane k of chunk c: pair j0 + 32 c + k), against the warp's sweep
+ * balls: a pair whose ball centres are farther apart in every lane than
+ * rho_P + rho_Q + sqrt(T2) is settled for all lanes at once (each lane's
+ * exact distance then exceeds sqrt(T2)); else the direction test is bounded
+ * over all lanes at once (swept_direction).  Returns, in lane c, the pairs
+ * of chunk c left for the lanes' own tests (bit k).
+ *
+ * One 16-byte record a pair (swp: the static partner's ball centre and
+ * sqrt(T2) with the two slots in its low bits), chunks independent of each
+ * other and of the lanes' state, so that their loads overlap; the second
+ * record (scan_b) is read only where the distance leaves the pair open.
+ * With three records a pair and a vote, a scan and a branch after every
+ * chunk this stage took 17,000 cycles of a hull6 round (13 chunks). */
+__device__ __forceinline__ unsigned sweep_stage(const DevScene& sc, const SceneView& S, int j0, int chunks)
 {
     const int lane = threadIdx.x & 31;
-    const unsigned all = jn >= 32 ? FULL_MASK : ((1u << jn) - 1u);
-    unsigned cand = all, swept_dir = 0u;
-    if constexpr (SWEPT) {
-        bool maybe = false, by_dir = false;
-        if (lane < jn) {
-            const int4 c = S.scan_c[j0 + lane];
-            maybe = c.w != SCAN_SETTLED;
-            if (c.w == SCAN_USABLE && ((c.x < 0) != (c.y < 0))) {
-                const int ms = c.x >= 0 ? c.x : c.y;
-                const float4 f = S.far[j0 + lane];
-                const float4 b = S.sweep[ms];
-                const float dx = f.x - b.x, dy = f.y - b.y, dz = f.z - b.z;
-                const float dd2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
-                const float A = (__int_as_float(c.z) + b.w) * (1.0f + 1e-6f);
-                /* |m - c|^2 >= dd2 (1 - 1e-6) > A^2 >= (rho + sqrt(T2))^2 */
-                if (dd2 * (1.0f - 1e-6f) > A * A) maybe = false;
-                else if (sc.nslots <= SWEEP_V0_SLOTS &&
-                         swept_direction(sc, c.x >= 0, b, S.sweep[SWEEP_V0_SLOTS + ms], f, S.scan_b[j0 + lane]))
-                    maybe = false, by_dir = true;
+    const bool dir_on = sc.nslots <= SWEEP_V0_SLOTS;
+    unsigned mine = 0u;
+#pragma unroll 2
+    for (int c = 0; c < chunks; ++c) {
+        const int j = j0 + c * 32 + lane;
+        bool open = false;
+        if (j < sc.npairs) {
+            const float4 r = S.swp[j];
+            const int w = __float_as_int(r.w);
+            const int a = w & 15, b = (w >> 4) & 15;   /* a: a moving polytope's slot; b != a: the other's */
+            const float4 m = S.sweep[a];
+            float4 o = make_float4(r.x, r.y, r.z, 0.0f);
+            if (b != a) o = S.sweep[b];
+            const float dx = o.x - m.x, dy = o.y - m.y, dz = o.z - m.z, rc = o.w + m.w;
+            const float dd2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
+            const float root = __int_as_float(w | 255);   /* the slot bits round it up */
+            const float A = (root + rc) * (1.0f + 1e-6f);
+            /* |m - o|^2 >= dd2 (1 - 1e-6) > A^2; a negative root: settled
+               for every configuration; NaN: not for the sweep tests */
+            open = !(dd2 * (1.0f - 1e-6f) > A * A) && !(root < 0.0f);
+            if (open && dir_on) {
+                const float4 v = S.sweep[SWEEP_V0_SLOTS + a];
+                const float4 sb = S.scan_b[j];
+                float4 u = make_float4(sb.x, sb.y, sb.z, 0.0f);
+                if (b != a) u = S.sweep[SWEEP_V0_SLOTS + b];
+                open = !swept_direction(sc, u.x - v.x, u.y - v.y, u.z - v.z, u.w + v.w, dx, dy, dz, rc, sb.w);
             }
         }
-        cand = __ballot_sync(FULL_MASK, maybe);
-        swept_dir = __ballot_sync(FULL_MASK, by_dir);
-    } else {
-        cand = __ballot_sync(FULL_MASK, lane < jn && S.scan_c[j0 + lane].w != SCAN_SETTLED);
+        const unsigned left = __ballot_sync(FULL_MASK, open);
+        if (lane == c) mine = left;
     }
-    if (!active) return 0u;
-    pc.far += (unsigned)__popc(all & ~cand & ~swept_dir);
-    pc.dir += (unsigned)__popc(swept_dir);
+    return mine;
+}
+
+/* This lane's certificates of the pairs j0 + k, k in cand (warp-uniform),
+ * all order-free (a certified pair is free with its margin above the band,
+ * so it changes neither a code nor a band decision): two pairs at a time
+ * the ball-distance and direction tests, then for the few pairs both miss
+ * the box test of pair_certified_dir; pairs the scan cannot use go through
+ * pair_certified.  Returns the pairs that need the exact test (bit k). */
+__device__ __forceinline__ unsigned lane_scan(const DevScene& sc, const SceneView& S, int j0, unsigned cand,
+                                              PairCounts& pc)
+{
     unsigned need = 0;
 #pragma unroll 1
     while (cand) {
@@ -346,28 +380,39 @@ __device__ __forceinline__ unsigned cert_scan(const DevScene& sc, const SceneVie
             const int r = h ? rb : ra;
             const int j = h ? jb : ja;
             const int k = h ? k1 : k0;
-            if (r == 1) { ++pc.far; continue; }
-            if (r == 2) { ++pc.dir; continue; }
+            if (r > 0) { ++pc.cert; continue; }
             bool ok;
             if (r == 0) {
                 /* the box test (pair_certified_dir's last stage) */
                 const float3 D = h ? Db : Da;
                 ok = pair_certified_dir(sc, S.tab, S.pairs[j], S.pairs_b[j], S.cen, S.frames, j, D.x, D.y, D.z,
                                         h ? d2b : d2a, true);
-                if (ok) ++pc.dir;
             } else {
                 bool used_dir;
                 ok = pair_certified(sc, S.tab, S.pairs[j], S.pairs_b[j], S.cen, S.frames, &used_dir, j);
-                if (ok) { if (used_dir) ++pc.dir; else ++pc.far; }
             }
-            if (!ok) need |= 1u << k;
+            if (ok) ++pc.cert;
+            else need |= 1u << k;
         }
     }
     return need;
 }
 
-/* The exact test of pair j for this lane (its certificates failed in
- * cert_scan): the pair's code, and its margin in *margin. */
+/* lane_scan over the chunk j0 .. j0+jn-1 (jn <= 32) of a vertex check, whose
+ * lanes hold unrelated configurations: every pair but those settled for
+ * every configuration (SCAN_SETTLED).  0 for an inactive lane; every lane
+ * of the warp must call it (it votes). */
+__device__ __forceinline__ unsigned config_scan(const DevScene& sc, const SceneView& S, int j0, int jn, bool active,
+                                                PairCounts& pc)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned cand = __ballot_sync(FULL_MASK, lane < jn && S.scan_c[j0 + lane].w != SCAN_SETTLED);
+    if (!active) return 0u;
+    pc.cert += (unsigned)(jn - __popc(cand));
+    return lane_scan(sc, S, j0, cand, pc);
+}
+
+/* The exact test of pair j for this lane (its certificates failed): the pair's code, and its margin in *margin. */
 template <bool FAST>
 __device__ __forceinline__ int eval_pair(const DevScene& sc, const SceneView& S, int j, float* margin,
                                          PairCounts& pc);
@@ -403,13 +448,11 @@ __device__ __forceinline__ void lane_fk(const DevScene& sc, const SceneView& S, 
 __device__ __forceinline__ void flush_counts(PairCounts pc, Control* ctl)
 {
     for (int o = 16; o > 0; o >>= 1) {
-        pc.far += __shfl_xor_sync(0xffffffffu, pc.far, o);
-        pc.dir += __shfl_xor_sync(0xffffffffu, pc.dir, o);
+        pc.cert += __shfl_xor_sync(0xffffffffu, pc.cert, o);
         pc.full += __shfl_xor_sync(0xffffffffu, pc.full, o);
     }
     if ((threadIdx.x & 31) == 0) {
-        if (pc.far) atomicAdd(&ctl->cert_far, pc.far);
-        if (pc.dir) atomicAdd(&ctl->cert_dir, pc.dir);
+        if (pc.cert) atomicAdd(&ctl->certified, pc.cert);
         if (pc.full) atomicAdd(&ctl->full_tests, pc.full);
     }
 }
@@ -600,7 +643,7 @@ __device__ __forceinline__ void check_config_chunk(const DevScene& sc, const Sce
     for (int j0 = 0; j0 < sc.npairs; j0 += 32) {
         if (!__any_sync(FULL_MASK, st.active)) break;
         const int jn = min(32, sc.npairs - j0);
-        const unsigned need = cert_scan<false>(sc, S, j0, jn, st.active, pc);
+        const unsigned need = config_scan(sc, S, j0, jn, st.active, pc);
         const unsigned todo = __reduce_or_sync(FULL_MASK, need);
         defer_chunk<FAST>(sc, S, j0, need, todo, st, pc, band);
     }
@@ -626,7 +669,7 @@ __global__ void GPRM_BOUNDS k_check_configs(DevScene sc, const float* __restrict
     const SceneView S = stage_scene<SMEM, true>(sc, smem);
     const int lane = threadIdx.x & 31;
     unsigned long long exec = 0;
-    PairCounts pc = {0, 0, 0};
+    PairCounts pc = {0, 0};
     for (;;) {
         unsigned long long base = 0;
         if (lane == 0) base = atomicAdd(&ctl->next, 32ull);
@@ -702,27 +745,28 @@ __device__ __forceinline__ void check_edge(const DevScene& sc, const SceneView& 
                 : (kv != 0u && (int)(kv >> 4) - 1 > tn - 1 - r * 32);
             if (__any_sync(FULL_MASK, beaten)) break;
         }
+        /* lanes past the round's last step repeat it: every lane's frames
+           then belong to the round and the sweep balls need no mask */
         int t;
         unsigned order;
         bool valid;
         if (POLICY == EDGE_EARLY_EXIT) {
-            t = lane * R + r;
-            valid = t < tn;
+            const int last = (tn - 1 - r) / R;     /* lanes 0 .. last hold steps */
+            valid = lane <= last;
+            t = (valid ? lane : last) * R + r;
             order = (unsigned)(r * 32 + lane);
         } else {
-            int idx = r * 32 + lane;
-            t = tn - 1 - idx;
-            valid = idx < tn;
+            t = tn - 1 - (r * 32 + lane);
+            valid = t >= 0;
+            if (!valid) t = 0;
             order = 0;
         }
         float qi[GPRM_MAX_FRAMES];
-        if (valid) {
-            edge_step_config(qs, qe, e, offset, sc.ndof, t, tn, qi);
-            lane_fk<FAST>(sc, S, qi);
-        }
+        edge_step_config(qs, qe, e, offset, sc.ndof, t, tn, qi);
+        lane_fk<FAST>(sc, S, qi);
         const unsigned valid_mask = __ballot_sync(FULL_MASK, valid);
         if (lane == 0) exec += __popc(valid_mask);
-        sweep_bounds(sc, S, valid_mask);
+        sweep_bounds(sc, S);
         bool active = valid;
         int code = 0;
         float mmin = PF32::inf(), mdec = 0.0f;
@@ -730,38 +774,55 @@ __device__ __forceinline__ void check_edge(const DevScene& sc, const SceneView& 
         int jend = 0;   /* pairs processed by the warp */
         int jrec = 0x7fffffff, jlast = -1;   /* first and last pair decided within the band */
         bool stop = false;
-        /* pairs in chunks of 32: the order-free certificate scan, then the
-           pairs left for the exact test in the reference's order; a code can
-           only change at such a pair, so the vote runs only there */
+        /* groups of 32 chunks of 32 pairs: the sweep stage for the whole
+           group, then per chunk with a pair left the lanes' own certificates
+           and the exact tests in the reference's order; a code can only
+           change at such a test, so the vote runs only there */
 #pragma unroll 1
-        for (int j0 = 0; j0 < sc.npairs && !stop; j0 += 32) {
-            if (!__any_sync(FULL_MASK, active)) break;
-            const int jn = min(32, sc.npairs - j0);
-            const unsigned need = cert_scan<true>(sc, S, j0, jn, active, pc);
-            unsigned todo = __reduce_or_sync(FULL_MASK, need);
-            while (todo) {
-                const int k = __ffs(todo) - 1;
-                todo &= todo - 1u;
-                if (active && ((need >> k) & 1u)) {
-                    float m;
-                    const int rr = eval_pair<FAST>(sc, S, j0 + k, &m, pc);
-                    if (rr != 0) { code = rr; mdec = m; active = false; jrec = min(jrec, j0 + k); }
-                    else {
-                        mmin = min_nan(mmin, m);
-                        if (!(m >= band)) { jrec = min(jrec, j0 + k); jlast = j0 + k; }
+        for (int g0 = 0; g0 < sc.npairs && !stop; g0 += 1024) {
+            const int gend = min(sc.npairs, g0 + 1024);
+            unsigned nact = __ballot_sync(FULL_MASK, active);
+            if (!nact) break;
+            const unsigned open = sweep_stage(sc, S, g0, (gend - g0 + 31) >> 5);
+            unsigned left = __ballot_sync(FULL_MASK, open != 0u);
+            int pos = g0;   /* pairs before it are counted */
+            while (left) {
+                const int c = __ffs(left) - 1;
+                left &= left - 1u;
+                const unsigned cand = __shfl_sync(FULL_MASK, open, c);
+                const int j0 = g0 + 32 * c, j1 = min(gend, j0 + 32);
+                if (lane == 0) pc.cert += (unsigned)((j1 - pos - __popc(cand)) * __popc(nact));
+                pos = j1;
+                const unsigned need = active ? lane_scan(sc, S, j0, cand, pc) : 0u;
+                unsigned todo = __reduce_or_sync(FULL_MASK, need);
+                while (todo) {
+                    const int k = __ffs(todo) - 1;
+                    todo &= todo - 1u;
+                    if (active && ((need >> k) & 1u)) {
+                        float m;
+                        const int rr = eval_pair<FAST>(sc, S, j0 + k, &m, pc);
+                        if (rr != 0) { code = rr; mdec = m; active = false; jrec = min(jrec, j0 + k); }
+                        else {
+                            mmin = min_nan(mmin, m);
+                            if (!(m >= band)) { jrec = min(jrec, j0 + k); jlast = j0 + k; }
+                        }
+                    }
+                    jend = j0 + k + 1;
+                    bool oobj = code != 0 && !(band_on && in_band(code, mdec, band));
+                    unsigned hits = __ballot_sync(FULL_MASK, oobj);
+                    if (hits) {
+                        int Lj = __ffs(hits) - 1;
+                        if (Lj < cut) cut = Lj;
+                        if (POLICY == EDGE_EARLY_EXIT) { stop = true; break; }
+                        if (lane > cut) active = false;
                     }
                 }
-                jend = j0 + k + 1;
-                bool oobj = code != 0 && !(band_on && in_band(code, mdec, band));
-                unsigned hits = __ballot_sync(FULL_MASK, oobj);
-                if (hits) {
-                    int Lj = __ffs(hits) - 1;
-                    if (Lj < cut) cut = Lj;
-                    if (POLICY == EDGE_EARLY_EXIT) { stop = true; break; }
-                    if (lane > cut) active = false;
-                }
+                nact = __ballot_sync(FULL_MASK, active);
+                if (stop || !nact) break;
             }
-            if (!stop) jend = j0 + jn;
+            if (stop || !nact) break;
+            if (lane == 0) pc.cert += (unsigned)((gend - pos) * __popc(nact));
+            jend = gend;
         }
         /* settle the round */
         const bool oob = code != 0 && !(band_on && in_band(code, mdec, band));
@@ -813,7 +874,7 @@ __global__ void GPRM_BOUNDS k_check_edges(DevScene sc, const float* __restrict__
     const SceneView S = stage_scene<SMEM, false>(sc, smem);
     const int lane = threadIdx.x & 31;
     unsigned long long exec = 0, nominal = 0;
-    PairCounts pc = {0, 0, 0};
+    PairCounts pc = {0, 0};
     if constexpr (!SPLIT) {
         for (;;) {
             unsigned long long eu = 0;
@@ -1277,7 +1338,7 @@ __global__ void k_fk_probe(DevScene sc, const float* q, float* out)
  * 72 % of an edge round there (570,000 of 790,000 cycles): 70,001 roadmap
  * edges 135.0 -> 43.0 ms, a vertex check of 100,003 configurations 8.8 ->
  * 8.2 ms. */
-__global__ void k_static_pairs(DevScene sc, int4* __restrict__ scan_c)
+__global__ void k_static_pairs(DevScene sc, int4* __restrict__ scan_c, float4* __restrict__ swp)
 {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= sc.npairs) return;
@@ -1287,7 +1348,10 @@ __global__ void k_static_pairs(DevScene sc, int4* __restrict__ scan_c)
     /* no slot and no frame is read: both polytopes are untransformed */
     __shared__ float none[1];
     bool used_dir;
-    if (pair_certified(sc, sc.tab, pr, sc.pairs_b[j], none, none, &used_dir, j)) scan_c[j].w = SCAN_SETTLED;
+    if (pair_certified(sc, sc.tab, pr, sc.pairs_b[j], none, none, &used_dir, j)) {
+        scan_c[j].w = SCAN_SETTLED;
+        swp[j].w = -1.0f;
+    }
 }
 
 /* ------------------------------------------------------------------ */
@@ -1297,7 +1361,8 @@ __global__ void k_static_pairs(DevScene sc, int4* __restrict__ scan_c)
 cudaError_t launch_static_pairs(const DevScene& sc, cudaStream_t st)
 {
     if (sc.npairs < 1) return cudaSuccess;
-    k_static_pairs<<<(sc.npairs + 127) / 128, 128, 0, st>>>(sc, const_cast<int4*>(sc.scan_c));
+    k_static_pairs<<<(sc.npairs + 127) / 128, 128, 0, st>>>(sc, const_cast<int4*>(sc.scan_c),
+                                                            const_cast<float4*>(sc.swp));
     return cudaGetLastError();
 }
 
@@ -1582,6 +1647,7 @@ __device__ __forceinline__ void switch_scene(const BatchView& B, int p, DevScene
     S.far = wsc->far;
     S.scan_c = wsc->scan_c;
     S.scan_b = wsc->scan_b;
+    S.swp = wsc->swp;
     S.frames = frames;
     S.cen = frames + (size_t)wsc->ndof * 12 * 32;
     S.sweep = sweep_area<VERTEX>(*wsc, frames);
@@ -1600,7 +1666,7 @@ __global__ void GPRM_BOUNDS k_check_configs_multi(BatchView B, const float* __re
     SceneView S;
     int cur = -1;
     unsigned long long exec = 0;
-    PairCounts pc = {0, 0, 0};
+    PairCounts pc = {0, 0};
     for (;;) {
         unsigned long long c = 0;
         if (lane == 0) c = atomicAdd(&ctl->next, 1ull);
@@ -1628,7 +1694,7 @@ __global__ void GPRM_BOUNDS k_check_edges_multi(BatchView B, const float* __rest
     SceneView S;
     int cur = -1;
     unsigned long long exec = 0, nominal = 0;
-    PairCounts pc = {0, 0, 0};
+    PairCounts pc = {0, 0};
     for (;;) {
         unsigned long long eu = 0;
         if (lane == 0) eu = atomicAdd(&ctl->next, 1ull);
@@ -1810,8 +1876,7 @@ __global__ void k_accumulate(const Control* c, Control* total)
     atomicAdd(&total->band_checks, c->band_checks);
     atomicAdd(&total->band_flips, c->band_flips);
     atomicAdd(&total->configs_exec, c->configs_exec);
-    atomicAdd(&total->cert_far, c->cert_far);
-    atomicAdd(&total->cert_dir, c->cert_dir);
+    atomicAdd(&total->certified, c->certified);
     atomicAdd(&total->full_tests, c->full_tests);
     atomicAdd(&total->ovf_count, c->ovf_count);
     atomicOr(&total->flags, c->flags);
