@@ -234,10 +234,9 @@ void compute_certificates(gprm_space* h, const int* from, const int* to)
         h->pairs_b[j] = make_float4(Rf, T2, fa, fb);
         /* certificate-scan records: the static partner's ball centre and
          * vertex 0 inline (a polytope in frame 0 is used untransformed), the
-         * slots of the moving ones, T2 and sqrt(T2) rounded up (for the
-         * sweep test), R.  A pair without a slot for each moving polytope,
-         * or with two static polytopes, is not usable by the scan (its
-         * certificates go through pair_certified). */
+         * slots of the moving ones, T2, R.  A pair without a slot for each
+         * moving polytope, or with two static polytopes, is not usable by
+         * the scan. */
         float4 fr = make_float4(0.0f, 0.0f, 0.0f, INFINITY);
         float4 sbv = make_float4(0.0f, 0.0f, 0.0f, Rf);
         int usable = SCAN_GENERAL;
@@ -256,7 +255,7 @@ void compute_certificates(gprm_space* h, const int* from, const int* to)
         int sqb;
         memcpy(&sqb, &sq, 4);
         h->far[j] = fr;
-        h->scan_c[j] = make_int4(sa, sb, sqb, usable);
+        h->scan_c[j] = make_int4(SCAN_PACK(sa, sb, h->pair_sys[2 * j], h->pair_sys[2 * j + 1]), a, b, usable);
         h->scan_b[j] = sbv;
         /* two slots need 8 bits; a pair of one slot with itself has no
            second one and stays out of the sweep stage */

@@ -42,9 +42,17 @@
 #define GPRM_CLIMB_CHUNK 1
 #endif
 /* how the certificate scan treats a pair (scan_c.w) */
-#define SCAN_GENERAL 0      /* through pair_certified (no slot, or two static polytopes) */
+#define SCAN_GENERAL 0      /* never certified (a moving polytope without a slot, or two static
+                               ones whose certificate fails) */
 #define SCAN_USABLE  1      /* by the scan's own tests */
 #define SCAN_SETTLED 2      /* two static polytopes whose certificate holds: always free */
+/* slots (-1: none) and frames of a pair's polytopes in one word (scan_c.x) */
+#define SCAN_PACK(slot_p, slot_q, sys_p, sys_q) \
+    (((slot_p) & 255) | (((slot_q) & 255) << 8) | ((sys_p) << 16) | ((sys_q) << 24))
+#define SCAN_SLOT_P(x) ((int)(signed char)((x) & 255))
+#define SCAN_SLOT_Q(x) ((int)(signed char)(((x) >> 8) & 255))
+#define SCAN_SYS_P(x) (((x) >> 16) & 255)
+#define SCAN_SYS_Q(x) (((x) >> 24) & 255)
 #define GPRM_MAX_ITERS 10   /* max_for_loop, max_for_loop_whole (collision4.h:17-18) */
 
 namespace gprm {
@@ -64,8 +72,8 @@ struct DevScene {
     const int4* pairs;
     const float4* pairs_b;
     /* certificate scan per pair: far = (static partner's ball centre, T2);
-       scan_c = (slot of P, slot of Q (-1: in frame 0), sqrt(T2) rounded up
-       (float bits), SCAN_*); scan_b = (static partner's vertex 0, R) */
+       scan_c = (SCAN_PACK of the slots and frames of P and Q, polytopes P
+       and Q, SCAN_*); scan_b = (static partner's vertex 0, R) */
     const float4* far;
     const int4* scan_c;
     const float4* scan_b;
@@ -541,7 +549,7 @@ __device__ __forceinline__ float box_support(const float4* __restrict__ B, const
  * infinity: nothing can be certified. */
 __device__ __forceinline__ bool pair_certified_dir(const DevScene& sc, const float4* __restrict__ tab, int4 pr,
                                                    float4 pb, const float* cen, const float* frames, int j,
-                                                   float dx, float dy, float dz, float d2, bool box_only = false)
+                                                   float dx, float dy, float dz, float d2)
 {
     if (!(pb.x < PF32::inf())) return false;
     const int sa = __float_as_int(pb.z), sb = __float_as_int(pb.w);
@@ -560,7 +568,7 @@ __device__ __forceinline__ bool pair_certified_dir(const DevScene& sc, const flo
     const float dn = d2 * rsqrtf(d2) * (1.0f + 2e-6f);
     /* direction error <= eps_dir*inv (+ rsqrt and rounding, 1e-6) */
     const float err = (dn + pb.x) * __fmaf_rn(sc.eps_dir, inv, 1e-6f);
-    if (!box_only && G - err > sc.thr_dir) return true;
+    if (G - err > sc.thr_dir) return true;
     /* box test: the same bound with each polytope's support along S taken
        from its bounding box instead of its ball (every vertex v of X has
        <S, v - c_X> <= sum_a e_a |<a_a, R_X^T S>|), tighter for elongated

@@ -77,7 +77,7 @@ struct gprm_space {
     std::vector<int4> pairs;
     std::vector<float4> pairs_b;   /* certificate data per pair */
     std::vector<float4> far;       /* distance test: static ball centre, T2 */
-    std::vector<int4> scan_c;      /* certificate scan: slots of P and Q (-1 static), sqrt(T2) up, SCAN_* */
+    std::vector<int4> scan_c;      /* certificate scan: slots and frames, polytopes, SCAN_* */
     std::vector<float4> scan_b;    /* certificate scan: static polytope's vertex 0, R */
     std::vector<float4> swp;       /* sweep stage record (DevScene::swp) */
     std::vector<double> rad;       /* inflated ball radius per polytope */

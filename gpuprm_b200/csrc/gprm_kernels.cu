@@ -216,48 +216,6 @@ struct PairCounts {
     unsigned long long cert, full;
 };
 
-/* The ball-distance test of pair_certified for a usable pair (scan_c.w)
- * and this lane: true when it certifies; *d2o and *Do get |D|^2 and D =
- * c_Q - c_P (the moving ball centres from the slots, a static one from
- * far). */
-__device__ __forceinline__ bool cert_dist(const SceneView& S, int4 c, float4 f, float* d2o, float3* Do)
-{
-    const float* cen = S.cen;
-    float px = f.x, py = f.y, pz = f.z, qx = f.x, qy = f.y, qz = f.z;
-    if (c.x >= 0) { px = cen[(c.x * 3) * 32]; py = cen[(c.x * 3 + 1) * 32]; pz = cen[(c.x * 3 + 2) * 32]; }
-    if (c.y >= 0) { qx = cen[(c.y * 3) * 32]; qy = cen[(c.y * 3 + 1) * 32]; qz = cen[(c.y * 3 + 2) * 32]; }
-    const float dx = qx - px, dy = qy - py, dz = qz - pz;
-    const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
-    *d2o = d2;
-    *Do = make_float3(dx, dy, dz);
-    return d2 > f.w;
-}
-
-/* The direction test of pair_certified for a usable pair whose distance
- * test failed (D, d2 from cert_dist), the world vertex 0 of a moving
- * polytope from its slot (the FK pass wrote it with the FMA chain T*v0)
- * and that of a static one from scan_b; branch-free, so that two pairs can
- * be evaluated side by side. */
-__device__ __forceinline__ bool cert_dir(const DevScene& sc, const SceneView& S, int4 c, float4 b, float d2,
-                                         float3 D)
-{
-    const float* v0w = S.cen + sc.nslots * 3 * 32;
-    float ax = b.x, ay = b.y, az = b.z, bx = b.x, by = b.y, bz = b.z;
-    if (c.x >= 0) { ax = v0w[(c.x * 3) * 32]; ay = v0w[(c.x * 3 + 1) * 32]; az = v0w[(c.x * 3 + 2) * 32]; }
-    if (c.y >= 0) { bx = v0w[(c.y * 3) * 32]; by = v0w[(c.y * 3 + 1) * 32]; bz = v0w[(c.y * 3 + 2) * 32]; }
-    const float dx = D.x, dy = D.y, dz = D.z;
-    const float sx = bx - ax, sy = by - ay, sz = bz - az;
-    const float n2 = __fmaf_rn(sx, sx, __fmaf_rn(sy, sy, sz * sz));
-    const float inv = rsqrtf(n2);
-    const float G = __fmaf_rn(sx, dx, __fmaf_rn(sy, dy, sz * dz)) * inv - b.w;
-    /* |D| from above: d2 * rsqrt(d2) is within 3 ulp of |D| (rsqrtf <= 2
-       ulp), the factor covers it; d2 = 0 gives NaN, which fails the test */
-    const float dn = d2 * rsqrtf(d2) * (1.0f + 2e-6f);
-    /* direction error <= eps_dir*inv (+ rsqrt and rounding, 1e-6) */
-    const float err = (dn + b.w) * __fmaf_rn(sc.eps_dir, inv, 1e-6f);
-    return n2 > 1e-6f && G - err > sc.thr_dir;
-}
-
 /* The direction test of pair_certified_dir for every lane of the warp at
  * once.  Each polytope's ball centre lies in a ball over the lanes, and so
  * does its vertex 0 (the slot's sweep balls; radius 0 for a polytope of
@@ -338,63 +296,79 @@ __device__ __forceinline__ unsigned sweep_stage(const DevScene& sc, const SceneV
 
 /* This lane's certificates of the pairs j0 + k, k in cand (warp-uniform),
  * all order-free (a certified pair is free with its margin above the band,
- * so it changes neither a code nor a band decision): two pairs at a time
- * the ball-distance and direction tests, then for the few pairs both miss
- * the box test of pair_certified_dir; pairs the scan cannot use go through
- * pair_certified.  Returns the pairs that need the exact test (bit k). */
+ * so it changes neither a code nor a band decision): the ball-distance and
+ * direction tests of pair_certified without a branch between them, then, on
+ * the lanes both miss, its box test.  The moving polytopes' ball centres and
+ * vertices 0 come from the lane's slots (written by the FK pass), a static
+ * one's from far and scan_b.  A pair that is not SCAN_USABLE here is never
+ * certified (no slot, or two static polytopes whose certificate failed when
+ * the tables were uploaded).  Returns the pairs that need the exact test
+ * (bit k).
+ *
+ * One copy of the code and the next pair's records loaded ahead, rather than
+ * two pairs side by side with every case inlined for each: the edge kernel
+ * waits on instruction fetches more than on anything else (2.6 of 9.5 warp
+ * cycles per instruction before). */
 __device__ __forceinline__ unsigned lane_scan(const DevScene& sc, const SceneView& S, int j0, unsigned cand,
                                               PairCounts& pc)
 {
-    unsigned need = 0;
+    if (!cand) return 0u;
+    unsigned need = 0, done = cand;
+    const float* cen = S.cen;
+    const float* v0w = cen + sc.nslots * 3 * 32;
+    int k = __ffs(cand) - 1;
+    int4 c = S.scan_c[j0 + k];
+    float4 f = S.far[j0 + k], b = S.scan_b[j0 + k];
 #pragma unroll 1
-    while (cand) {
-        const int k0 = __ffs(cand) - 1;
+    for (;;) {
         cand &= cand - 1u;
-        int k1 = k0;
-        const bool two = cand != 0;
-        if (two) {
-            k1 = __ffs(cand) - 1;
-            cand &= cand - 1u;
-        }
-        const int ja = j0 + k0, jb = j0 + k1;
-        const int4 ca = S.scan_c[ja], cb = S.scan_c[jb];
-        const float4 fa = S.far[ja], fb = S.far[jb];
-        const float4 ba = S.scan_b[ja], bb = S.scan_b[jb];
-        float d2a = 0.0f, d2b = 0.0f;
-        float3 Da = make_float3(0.0f, 0.0f, 0.0f), Db = Da;
-        /* 1: distance, 2: direction, 0: neither, -1: not usable by the scan */
-        int ra = ca.w ? (cert_dist(S, ca, fa, &d2a, &Da) ? 1 : 0) : -1;
-        int rb = (two && cb.w) ? (cert_dist(S, cb, fb, &d2b, &Db) ? 1 : 0) : -1;
-        if (ra == 0 && rb == 0) {
-            /* both need the direction test: side by side */
-            const bool oa = cert_dir(sc, S, ca, ba, d2a, Da), ob = cert_dir(sc, S, cb, bb, d2b, Db);
-            ra = oa ? 2 : 0;
-            rb = ob ? 2 : 0;
-        } else {
-            if (ra == 0 && cert_dir(sc, S, ca, ba, d2a, Da)) ra = 2;
-            if (rb == 0 && cert_dir(sc, S, cb, bb, d2b, Db)) rb = 2;
-        }
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            if (h == 1 && !two) break;
-            const int r = h ? rb : ra;
-            const int j = h ? jb : ja;
-            const int k = h ? k1 : k0;
-            if (r > 0) { ++pc.cert; continue; }
-            bool ok;
-            if (r == 0) {
-                /* the box test (pair_certified_dir's last stage) */
-                const float3 D = h ? Db : Da;
-                ok = pair_certified_dir(sc, S.tab, S.pairs[j], S.pairs_b[j], S.cen, S.frames, j, D.x, D.y, D.z,
-                                        h ? d2b : d2a, true);
-            } else {
-                bool used_dir;
-                ok = pair_certified(sc, S.tab, S.pairs[j], S.pairs_b[j], S.cen, S.frames, &used_dir, j);
+        const int kn = cand ? __ffs(cand) - 1 : k;
+        const int4 cn = S.scan_c[j0 + kn];
+        const float4 fn = S.far[j0 + kn], bn = S.scan_b[j0 + kn];
+        bool ok = false;
+        if (c.w == SCAN_USABLE) {
+            float px = f.x, py = f.y, pz = f.z, qx = f.x, qy = f.y, qz = f.z;
+            float ax = b.x, ay = b.y, az = b.z, bx = b.x, by = b.y, bz = b.z;
+            const int sp = SCAN_SLOT_P(c.x), sq = SCAN_SLOT_Q(c.x);
+            if (sp >= 0) {
+                const float* u = cen + sp * 3 * 32;
+                const float* v = v0w + sp * 3 * 32;
+                px = u[0]; py = u[32]; pz = u[64];
+                ax = v[0]; ay = v[32]; az = v[64];
             }
-            if (ok) ++pc.cert;
-            else need |= 1u << k;
+            if (sq >= 0) {
+                const float* u = cen + sq * 3 * 32;
+                const float* v = v0w + sq * 3 * 32;
+                qx = u[0]; qy = u[32]; qz = u[64];
+                bx = v[0]; by = v[32]; bz = v[64];
+            }
+            const float dx = qx - px, dy = qy - py, dz = qz - pz;
+            const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
+            float sx = bx - ax, sy = by - ay, sz = bz - az;
+            const float n2 = __fmaf_rn(sx, sx, __fmaf_rn(sy, sy, sz * sz));
+            const float inv = rsqrtf(n2);
+            const float G = __fmaf_rn(sx, dx, __fmaf_rn(sy, dy, sz * dz)) * inv - b.w;
+            /* |D| from above: d2 * rsqrt(d2) is within 3 ulp of |D| (rsqrtf
+               <= 2 ulp), the factor covers it; d2 = 0 gives NaN, which fails
+               the tests */
+            const float dn = d2 * rsqrtf(d2) * (1.0f + 2e-6f);
+            /* direction error <= eps_dir*inv (+ rsqrt and rounding, 1e-6) */
+            const float err = (dn + b.w) * __fmaf_rn(sc.eps_dir, inv, 1e-6f);
+            const bool dir = n2 > 1e-6f;   /* |s| < 1e-3: leave it to the test */
+            ok = d2 > f.w || (dir && G - err > sc.thr_dir);
+            if (!ok && dir) {
+                sx = sx * inv; sy = sy * inv; sz = sz * inv;
+                const float hp = box_support(sc.box + 3 * c.y, S.frames, SCAN_SYS_P(c.x), sx, sy, sz);
+                const float hq = box_support(sc.box + 3 * c.z, S.frames, SCAN_SYS_Q(c.x), sx, sy, sz);
+                const float Gb = __fmaf_rn(sx, dx, __fmaf_rn(sy, dy, sz * dz)) - (hp + hq) * (1.0f + 1e-5f);
+                ok = Gb - err > sc.thr_dir;
+            }
         }
+        if (!ok) need |= 1u << k;
+        if (!cand) break;
+        k = kn; c = cn; f = fn; b = bn;
     }
+    pc.cert += (unsigned)__popc(done & ~need);
     return need;
 }
 
