@@ -217,64 +217,6 @@ __device__ __forceinline__ void forward_kinematics(const DevScene& sc, const flo
     }
 }
 
-/* The same chain for the FP32 kernels, storing frames 1..ndof to a
- * lane-interleaved shared-memory array: entry e of frame f at
- * out[((f-1)*12 + e) * 32] (out already offset by the lane).  The world
- * centre of every slot's bounding ball follows at
- * cen[(slot*3 + c) * 32], then the world position of the slot polytope's
- * vertex 0 at cen[((nslots + slot)*3 + c) * 32] (both with FMA: they only
- * feed the certificates, whose slack covers their rounding). */
-__device__ __forceinline__ void slot_points(const DevScene& sc, const float4* __restrict__ tab, const Frame<float>& O,
-                                            int slot, float* cen)
-{
-    const float4 b = tab[sc.slot_block[slot]];
-    cen[(slot * 3 + 0) * 32] = __fmaf_rn(O.m[0], b.x, __fmaf_rn(O.m[3], b.y, __fmaf_rn(O.m[6], b.z, O.m[9])));
-    cen[(slot * 3 + 1) * 32] = __fmaf_rn(O.m[1], b.x, __fmaf_rn(O.m[4], b.y, __fmaf_rn(O.m[7], b.z, O.m[10])));
-    cen[(slot * 3 + 2) * 32] = __fmaf_rn(O.m[2], b.x, __fmaf_rn(O.m[5], b.y, __fmaf_rn(O.m[8], b.z, O.m[11])));
-    const float4 v = tab[sc.slot_block[slot] + 1];
-    float* w = cen + sc.nslots * 3 * 32;
-    w[(slot * 3 + 0) * 32] = __fmaf_rn(O.m[0], v.x, __fmaf_rn(O.m[3], v.y, __fmaf_rn(O.m[6], v.z, O.m[9])));
-    w[(slot * 3 + 1) * 32] = __fmaf_rn(O.m[1], v.x, __fmaf_rn(O.m[4], v.y, __fmaf_rn(O.m[7], v.z, O.m[10])));
-    w[(slot * 3 + 2) * 32] = __fmaf_rn(O.m[2], v.x, __fmaf_rn(O.m[5], v.y, __fmaf_rn(O.m[8], v.z, O.m[11])));
-}
-
-__device__ __forceinline__ void forward_kinematics_smem(const DevScene& sc, const float4* __restrict__ tab,
-                                                        const float* q, float* out, float* cen)
-{
-    Frame<float> T;
-    {
-        float c0, s0;
-        PF32::trig(0.0f, c0, s0);
-        dh_frame<PF32>(T, c0, s0, c0, s0, 0.0f, 0.0f);
-    }
-    int slot = 0;
-#pragma unroll 1
-    for (int i = 0; i < sc.ndof; ++i) {
-        float th = sc.q0[i], d = sc.d0[i];
-        if (sc.types[i] == 0) th = q[i];
-        else d = q[i];
-        float cq, sq, ca, sa;
-        PF32::trig(th, cq, sq);
-        PF32::trig_alpha(sc, i, ca, sa);
-        Frame<float> L;
-        dh_frame<PF32>(L, cq, sq, ca, sa, sc.a[i], d);
-        Frame<float> O;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            float ux = L.m[3 * c], uy = L.m[3 * c + 1], uz = L.m[3 * c + 2];
-            float ox = T.m[0] * ux + T.m[3] * uy + T.m[6] * uz;
-            float oy = T.m[1] * ux + T.m[4] * uy + T.m[7] * uz;
-            float oz = T.m[2] * ux + T.m[5] * uy + T.m[8] * uz;
-            if (c == 3) { ox = ox + T.m[9]; oy = oy + T.m[10]; oz = oz + T.m[11]; }
-            O.m[3 * c] = ox; O.m[3 * c + 1] = oy; O.m[3 * c + 2] = oz;
-        }
-#pragma unroll
-        for (int e = 0; e < 12; ++e) out[(i * 12 + e) * 32] = O.m[e];
-        for (; slot < sc.nslots && sc.slot_sys[slot] == i + 1; ++slot) slot_points(sc, tab, O, slot, cen);
-        T = O;
-    }
-}
-
 /* Loads frame f (1..ndof) of the lane from the array written above. */
 __device__ __forceinline__ void load_frame(const float* fr, int f, Frame<float>& T)
 {
@@ -919,11 +861,11 @@ __device__ __forceinline__ int pair_test_fast(const DevScene& sc, const float4* 
 /* Frame i+1 of the fast path from frame i (T): sincosf of the joint angle
  * and FMA products.  Shared by the shared-memory and register versions so
  * that both give the same bits. */
-__device__ __forceinline__ Frame<float> fast_link(const DevScene& sc, const Frame<float>& T, const float* q, int i)
+__device__ __forceinline__ Frame<float> fast_link(const DevScene& sc, const Frame<float>& T, float q, int i)
 {
     float th = sc.q0[i], d = sc.d0[i];
-    if (sc.types[i] == 0) th = q[i];
-    else d = q[i];
+    if (sc.types[i] == 0) th = q;
+    else d = q;
     float cq, sq;
     sincosf(th, &sq, &cq);
     const float ca = sc.ca[i], sa = sc.sa[i];
@@ -952,23 +894,80 @@ __device__ __forceinline__ void forward_kinematics_fast(const DevScene& sc, cons
 {
     identity_frame(F[0]);
 #pragma unroll 1
-    for (int i = 0; i < sc.ndof; ++i) F[i + 1] = fast_link(sc, F[i], q, i);
+    for (int i = 0; i < sc.ndof; ++i) F[i + 1] = fast_link(sc, F[i], q[i], i);
 }
 
-/* Forward kinematics of the fast path into the lane's shared-memory frames
- * (same layout as forward_kinematics_smem). */
-__device__ __forceinline__ void forward_kinematics_smem_fast(const DevScene& sc, const float4* __restrict__ tab,
-                                                             const float* q, float* out, float* cen)
+/* Forward kinematics of the FP32 kernels, in the arithmetic of the variant
+ * (FAST: fast_link; else the reference's operations as in
+ * forward_kinematics): frames 1..ndof go to a lane-interleaved
+ * shared-memory array, entry e of frame f at out[((f-1)*12 + e) * 32] (out
+ * already offset by the lane).  The world centre of every slot's bounding
+ * ball goes to cen[(slot*3 + c) * 32], the world position of the slot
+ * polytope's vertex 0 to cen[((nslots + slot)*3 + c) * 32] (both with FMA:
+ * they only feed the certificates, whose slack covers their rounding).
+ * joint(i): the lane's value of joint i.  One loop body for every joint (the
+ * kernels wait on instruction fetches), its slot's table entries loaded
+ * before the trigonometry. */
+template <bool FAST, class Joint>
+__device__ __forceinline__ void forward_kinematics_smem(const DevScene& sc, const float4* __restrict__ tab,
+                                                        Joint joint, float* out, float* cen)
 {
     Frame<float> T;
     identity_frame(T);
+    if constexpr (!FAST) T.m[3] = T.m[7] = T.m[10] = -0.0f;   /* set(0, 0, 0, 0), signs included */
     int slot = 0;
 #pragma unroll 1
     for (int i = 0; i < sc.ndof; ++i) {
-        const Frame<float> O = fast_link(sc, T, q, i);
+        bool has = slot < sc.nslots && sc.slot_sys[slot] == i + 1;
+        float4 b = make_float4(0.0f, 0.0f, 0.0f, 0.0f), v = b;
+        if (has) {
+            const float4* blk = tab + sc.slot_block[slot];
+            b = blk[0];
+            v = blk[1];
+        }
+        const float q = joint(i);
+        Frame<float> O;
+        if constexpr (FAST) {
+            O = fast_link(sc, T, q, i);
+        } else {
+            float th = sc.q0[i], d = sc.d0[i];
+            if (sc.types[i] == 0) th = q;
+            else d = q;
+            float cq, sq, ca, sa;
+            PF32::trig(th, cq, sq);
+            PF32::trig_alpha(sc, i, ca, sa);
+            Frame<float> L;
+            dh_frame<PF32>(L, cq, sq, ca, sa, sc.a[i], d);
 #pragma unroll
-        for (int e = 0; e < 12; ++e) out[(i * 12 + e) * 32] = O.m[e];
-        for (; slot < sc.nslots && sc.slot_sys[slot] == i + 1; ++slot) slot_points(sc, tab, O, slot, cen);
+            for (int c = 0; c < 4; ++c) {
+                float ux = L.m[3 * c], uy = L.m[3 * c + 1], uz = L.m[3 * c + 2];
+                float ox = T.m[0] * ux + T.m[3] * uy + T.m[6] * uz;
+                float oy = T.m[1] * ux + T.m[4] * uy + T.m[7] * uz;
+                float oz = T.m[2] * ux + T.m[5] * uy + T.m[8] * uz;
+                if (c == 3) { ox = ox + T.m[9]; oy = oy + T.m[10]; oz = oz + T.m[11]; }
+                O.m[3 * c] = ox; O.m[3 * c + 1] = oy; O.m[3 * c + 2] = oz;
+            }
+        }
+        float* fr = out + i * 12 * 32;
+#pragma unroll
+        for (int e = 0; e < 12; ++e) fr[e * 32] = O.m[e];
+#pragma unroll 1
+        while (has) {
+            float* u = cen + slot * 3 * 32;
+            float* w = u + sc.nslots * 3 * 32;
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                u[c * 32] = __fmaf_rn(O.m[c], b.x, __fmaf_rn(O.m[3 + c], b.y, __fmaf_rn(O.m[6 + c], b.z, O.m[9 + c])));
+                w[c * 32] = __fmaf_rn(O.m[c], v.x, __fmaf_rn(O.m[3 + c], v.y, __fmaf_rn(O.m[6 + c], v.z, O.m[9 + c])));
+            }
+            ++slot;
+            has = slot < sc.nslots && sc.slot_sys[slot] == i + 1;
+            if (has) {
+                const float4* blk = tab + sc.slot_block[slot];
+                b = blk[0];
+                v = blk[1];
+            }
+        }
         T = O;
     }
 }
@@ -996,6 +995,7 @@ __device__ __forceinline__ void edge_step_config(const float* __restrict__ qs, c
 {
     float c1 = (float)t / (float)(tn - 1);
     float c2 = 1.0f - c1;
+#pragma unroll 1
     for (int j = 0; j < ndof; ++j)
         q[j] = c1 * qs[e + offset * j] + c2 * qe[e + offset * j];
 }

@@ -412,11 +412,10 @@ __device__ __forceinline__ int eval_pair(const DevScene& sc, const SceneView& S,
 
 /* Forward kinematics of a lane into its shared-memory frames, in the
  * arithmetic of the kernel variant. */
-template <bool FAST>
-__device__ __forceinline__ void lane_fk(const DevScene& sc, const SceneView& S, const float* q)
+template <bool FAST, class Joint>
+__device__ __forceinline__ void lane_fk(const DevScene& sc, const SceneView& S, Joint joint)
 {
-    if constexpr (FAST) forward_kinematics_smem_fast(sc, S.tab, q, S.frames, S.cen);
-    else forward_kinematics_smem(sc, S.tab, q, S.frames, S.cen);
+    forward_kinematics_smem<FAST>(sc, S.tab, joint, S.frames, S.cen);
 }
 
 __device__ __forceinline__ void flush_counts(PairCounts pc, Control* ctl)
@@ -599,16 +598,17 @@ __device__ __forceinline__ void check_config_chunk(const DevScene& sc, const Sce
     const int lane = threadIdx.x & 31;
     const long long i = i0 + lane;
     const bool valid = lane < count;
-    float qi[GPRM_MAX_FRAMES];
     int code = 0;
     bool active = valid;
     if (valid) {
-        for (int j = 0; j < sc.ndof; ++j) qi[j] = q[i + offset * j];
         /* check_boundaries(q) (robotconfigspace.cpp:795-802) */
-        for (int j = 0; j < sc.ndof; ++j)
-            if (qi[j] < sc.mins[j] || qi[j] > sc.maxs[j]) { code = 1; active = false; break; }
+#pragma unroll 1
+        for (int j = 0; j < sc.ndof; ++j) {
+            const float x = q[i + offset * j];
+            if (x < sc.mins[j] || x > sc.maxs[j]) { code = 1; active = false; }
+        }
     }
-    if (active) lane_fk<FAST>(sc, S, qi);
+    if (active) lane_fk<FAST>(sc, S, [&](int j) { return q[i + offset * j]; });
     LaneState st{code, 0.0f, PF32::inf(), active, DEFER_NONE, 0x7fffffff, -1};
     /* pairs in chunks of 32: the order-free certificate scan, then the
        pairs left for the exact test in the reference's order, their exact
@@ -701,6 +701,10 @@ __device__ __forceinline__ void check_edge(const DevScene& sc, const SceneView& 
         return;
     }
     if (lane == 0 && seg == 0) nominal += tn;
+    /* the edge's ends, spread over the lanes for every round: lane j holds
+       joint j of qs, lane 16 + j that of qe */
+    float ends = 0.0f;
+    if ((lane & 15) < sc.ndof) ends = (lane < 16 ? qs : qe)[e + offset * (lane & 15)];
     const int R = (tn + 31) >> 5;
     int r_begin = 0, r_end = R;
     if constexpr (SPLIT) {
@@ -735,9 +739,11 @@ __device__ __forceinline__ void check_edge(const DevScene& sc, const SceneView& 
             if (!valid) t = 0;
             order = 0;
         }
-        float qi[GPRM_MAX_FRAMES];
-        edge_step_config(qs, qe, e, offset, sc.ndof, t, tn, qi);
-        lane_fk<FAST>(sc, S, qi);
+        /* the step's configuration as edge_step_config */
+        const float c1 = (float)t / (float)(tn - 1), c2 = 1.0f - c1;
+        lane_fk<FAST>(sc, S, [&](int j) {
+            return c1 * __shfl_sync(FULL_MASK, ends, j) + c2 * __shfl_sync(FULL_MASK, ends, 16 + j);
+        });
         const unsigned valid_mask = __ballot_sync(FULL_MASK, valid);
         if (lane == 0) exec += __popc(valid_mask);
         sweep_bounds(sc, S);
