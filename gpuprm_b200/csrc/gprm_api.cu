@@ -217,7 +217,6 @@ void compute_certificates(gprm_space* h, const int* from, const int* to)
     h->far.resize(h->npairs);
     h->scan_c.resize(h->npairs);
     h->scan_b.resize(h->npairs);
-    h->swp.resize(h->npairs);
     for (int j = 0; j < h->npairs; ++j) {
         int a = h->pair_poly[2 * j], b = h->pair_poly[2 * j + 1];
         bool ok = (h->pair_sys[2 * j] == 0 || h->slot[a] >= 0) && (h->pair_sys[2 * j + 1] == 0 || h->slot[b] >= 0);
@@ -251,24 +250,9 @@ void compute_certificates(gprm_space* h, const int* from, const int* to)
                 fr.w = T2;
             }
         }
-        float sq = nextafterf((float)sqrt((double)T2), INFINITY);
-        int sqb;
-        memcpy(&sqb, &sq, 4);
         h->far[j] = fr;
         h->scan_c[j] = make_int4(SCAN_PACK(sa, sb, h->pair_sys[2 * j], h->pair_sys[2 * j + 1]), a, b, usable);
         h->scan_b[j] = sbv;
-        /* two slots need 8 bits; a pair of one slot with itself has no
-           second one and stays out of the sweep stage */
-        float4 sw = make_float4(NAN, NAN, NAN, NAN);
-        if (usable == SCAN_USABLE && sa != sb) {
-            static_assert(GPRM_MAX_SLOTS <= 16, "a slot takes 4 bits of the record");
-            const int s0 = sa >= 0 ? sa : sb, s1 = sa >= 0 && sb >= 0 ? sb : s0;
-            const int bits = (sqb & ~255) + 256;   /* rounded up to a multiple of 256 ulp */
-            const int word = (bits & ~255) | s0 | (s1 << 4);
-            memcpy(&sw.w, &word, 4);
-            sw.x = fr.x; sw.y = fr.y; sw.z = fr.z;
-        }
-        h->swp[j] = sw;
     }
     h->thr_dir = (float)thr;
     h->eps_dir = (float)(7.0 * eps_pos);
@@ -283,6 +267,165 @@ void compute_certificates(gprm_space* h, const int* from, const int* to)
             h->box[3 * k + a] = make_float4((float)h->box_ax[9 * k + 3 * a], (float)h->box_ax[9 * k + 3 * a + 1],
                                             (float)h->box_ax[9 * k + 3 * a + 2], nextafterf((float)e, INFINITY));
         }
+}
+
+/* Entry and leaf records of the sweep stage (DevScene::swp .. swg). */
+struct SweepLists {
+    std::vector<float4> leaf, rec, v0;
+    std::vector<int> pair, group;
+};
+
+/* x rounded up to a float whose low `bits` bits are clear, with `code` in
+ * them: whatever the code, the value with those bits set is >= x. */
+float up_with_code(double x, int bits, int code)
+{
+    float f = nextafterf((float)x, INFINITY);
+    unsigned w;
+    memcpy(&w, &f, 4);
+    w = (w & ~((1u << bits) - 1u)) + (1u << bits);
+    w |= (unsigned)code;
+    memcpy(&f, &w, 4);
+    return f;
+}
+
+/* Splits the pairs idx (static partners' centres h->far) into leaves of at
+ * most 32 that lie close together: halves by whole leaves along the widest
+ * axis. */
+void sweep_leaves(const gprm_space* h, std::vector<int>& idx, size_t lo, size_t hi, std::vector<size_t>& ends)
+{
+    if (hi - lo <= 32) {
+        if (hi > lo) ends.push_back(hi);
+        return;
+    }
+    float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (size_t i = lo; i < hi; ++i) {
+        const float4 f = h->far[idx[i]];
+        const float c[3] = {f.x, f.y, f.z};
+        for (int k = 0; k < 3; ++k) { mn[k] = fminf(mn[k], c[k]); mx[k] = fmaxf(mx[k], c[k]); }
+    }
+    int ax = 0;
+    for (int k = 1; k < 3; ++k) if (mx[k] - mn[k] > mx[ax] - mn[ax]) ax = k;
+    const size_t leaves = (hi - lo + 31) / 32, mid = lo + 32 * ((leaves + 1) / 2);
+    std::nth_element(idx.begin() + lo, idx.begin() + mid, idx.begin() + hi, [&](int a, int b) {
+        const float4 fa = h->far[a], fb = h->far[b];
+        const float ca = ax == 0 ? fa.x : ax == 1 ? fa.y : fa.z, cb = ax == 0 ? fb.x : ax == 1 ? fb.y : fb.z;
+        return ca < cb || (ca == cb && a < b);
+    });
+    sweep_leaves(h, idx, lo, mid, ends);
+    sweep_leaves(h, idx, mid, hi, ends);
+}
+
+/* The sweep lists of the scene's pairs, but those settled for every
+ * configuration (scan_c as launch_static_pairs left it). */
+void build_sweep(const gprm_space* h, const std::vector<int4>& scan_c, SweepLists& L)
+{
+    static_assert(GPRM_MAX_SLOTS <= 16, "a slot takes 4 bits of a record");
+    L = SweepLists();
+    const float4 nan4 = make_float4(NAN, NAN, NAN, NAN);
+    auto leaf = [&](const int* idx, size_t n, int slot) {
+        double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300}, rad = 0;
+        for (size_t i = 0; i < 32; ++i) {
+            if (i >= n) {   /* empty */
+                L.rec.push_back(make_float4(0.0f, 0.0f, 0.0f, -1.0f));
+                L.v0.push_back(make_float4(0.0f, 0.0f, 0.0f, 0.0f));
+                L.pair.push_back(0);
+                continue;
+            }
+            const int j = idx[i];
+            const int4 c = scan_c[j];
+            const float4 f = h->far[j];
+            const int sa = SCAN_SLOT_P(c.x), sb = SCAN_SLOT_Q(c.x);
+            float4 r = nan4;
+            if (c.w == SCAN_USABLE && sa != sb) {   /* a pair of one slot with itself has no second one */
+                const int s0 = sa >= 0 ? sa : sb, s1 = sa >= 0 && sb >= 0 ? sb : s0;
+                r = make_float4(f.x, f.y, f.z, up_with_code(sqrt((double)h->pairs_b[j].y), 8, s0 | (s1 << 4)));
+            } else {
+                const unsigned w = 0x7fc00000u;     /* NaN, slots 0 and 0 */
+                memcpy(&r.w, &w, 4);
+            }
+            L.rec.push_back(r);
+            L.v0.push_back(h->scan_b[j]);
+            L.pair.push_back(j);
+            const float cc[3] = {f.x, f.y, f.z};
+            for (int k = 0; k < 3; ++k) { lo[k] = fmin(lo[k], cc[k]); hi[k] = fmax(hi[k], cc[k]); }
+        }
+        float4 b = nan4;
+        const unsigned nanw = 0x7fc00000u;
+        memcpy(&b.w, &nanw, 4);
+        if (slot >= 0) {
+            b = make_float4((float)(0.5 * (lo[0] + hi[0])), (float)(0.5 * (lo[1] + hi[1])),
+                            (float)(0.5 * (lo[2] + hi[2])), 0.0f);
+            for (size_t i = 0; i < n; ++i) {
+                const float4 f = h->far[idx[i]];
+                const double dx = (double)f.x - b.x, dy = (double)f.y - b.y, dz = (double)f.z - b.z;
+                rad = fmax(rad, sqrt(dx * dx + dy * dy + dz * dz) + sqrt((double)h->pairs_b[idx[i]].y));
+            }
+            b.w = up_with_code(rad * (1 + 1e-6), 4, slot);
+        }
+        L.leaf.push_back(b);
+    };
+    for (int g0 = 0; g0 < h->npairs; g0 += SWEEP_GROUP) {
+        const int g1 = std::min(h->npairs, g0 + SWEEP_GROUP);
+        L.group.push_back((int)L.leaf.size());
+        std::vector<std::vector<int>> by_slot(GPRM_MAX_SLOTS);
+        std::vector<int> other;
+        for (int j = g0; j < g1; ++j) {
+            const int4 c = scan_c[j];
+            if (c.w == SCAN_SETTLED) continue;
+            const int sa = SCAN_SLOT_P(c.x), sb = SCAN_SLOT_Q(c.x);
+            if (c.w == SCAN_USABLE && (sa < 0) != (sb < 0)) by_slot[sa >= 0 ? sa : sb].push_back(j);
+            else other.push_back(j);
+        }
+        std::vector<size_t> ends;
+        for (int s = 0; s < GPRM_MAX_SLOTS; ++s) {
+            ends.clear();
+            sweep_leaves(h, by_slot[s], 0, by_slot[s].size(), ends);
+            size_t at = 0;
+            for (size_t e : ends) { leaf(by_slot[s].data() + at, e - at, s); at = e; }
+        }
+        for (size_t at = 0; at < other.size(); at += 32)
+            leaf(other.data() + at, std::min<size_t>(32, other.size() - at), -1);
+    }
+    L.group.push_back((int)L.leaf.size());
+}
+
+/* Leaves that the sweep lists can take, whatever pairs are settled: each
+ * group wastes at most one partly filled leaf per slot and one of the rest. */
+size_t sweep_leaf_cap(const gprm_space* h)
+{
+    const size_t groups = ((size_t)h->npairs + SWEEP_GROUP - 1) / SWEEP_GROUP;
+    return (size_t)h->npairs / 32 + groups * (GPRM_MAX_SLOTS + 2) + 1;
+}
+
+/* Uploads the certificate tables (compute_certificates) to the handle's
+ * scene memory, settles the static pairs there and uploads the sweep lists
+ * of the others.  Synchronises. */
+int upload_certificates(gprm_space* h)
+{
+    DevScene& s = h->dsc;
+    const size_t n = (size_t)h->npairs, pb = n * sizeof(float4);
+    s.thr_dir = h->thr_dir;
+    s.eps_dir = h->eps_dir;
+    std::vector<int4> settled(h->scan_c);
+    if (n) {
+        CUDA_TRY(h, cudaMemcpy((void*)s.pairs_b, h->pairs_b.data(), pb, cudaMemcpyHostToDevice));
+        CUDA_TRY(h, cudaMemcpy((void*)s.far, h->far.data(), pb, cudaMemcpyHostToDevice));
+        CUDA_TRY(h, cudaMemcpy((void*)s.scan_c, h->scan_c.data(), pb, cudaMemcpyHostToDevice));
+        CUDA_TRY(h, cudaMemcpy((void*)s.scan_b, h->scan_b.data(), pb, cudaMemcpyHostToDevice));
+        CUDA_TRY(h, launch_static_pairs(s, cudaStreamLegacy));   /* after the copies, on their stream */
+        CUDA_TRY(h, cudaMemcpy(settled.data(), s.scan_c, pb, cudaMemcpyDeviceToHost));
+    }
+    SweepLists L;
+    build_sweep(h, settled, L);
+    if (L.leaf.size() > sweep_leaf_cap(h)) return fail(h, GPRM_ERR_STATE, "sweep lists exceed their buffer");
+    if (!L.leaf.empty()) {
+        CUDA_TRY(h, cudaMemcpy((void*)s.swl, L.leaf.data(), L.leaf.size() * 16, cudaMemcpyHostToDevice));
+        CUDA_TRY(h, cudaMemcpy((void*)s.swp, L.rec.data(), L.rec.size() * 16, cudaMemcpyHostToDevice));
+        CUDA_TRY(h, cudaMemcpy((void*)s.swb, L.v0.data(), L.v0.size() * 16, cudaMemcpyHostToDevice));
+        CUDA_TRY(h, cudaMemcpy((void*)s.swj, L.pair.data(), L.pair.size() * 4, cudaMemcpyHostToDevice));
+    }
+    CUDA_TRY(h, cudaMemcpy((void*)s.swg, L.group.data(), L.group.size() * 4, cudaMemcpyHostToDevice));
+    return GPRM_OK;
 }
 
 int build_space(const gprm_scene_desc* d, float dq, int nbuf, gprm_space** out)
@@ -894,25 +1037,24 @@ int gprm_init(gprm_space* h, int rank, int size)
         }
     }
 
-    /* d_scene: tab | pairs | pairs_b | far | scan_c | scan_b | swp | ppoly | box | vtab | vinfo | ctab | ccnt */
+    /* d_scene: tab | pairs | pairs_b | far | scan_c | scan_b | ppoly | box | vtab | vinfo | ctab | ccnt |
+       the sweep lists swl | swp | swb | swj | swg */
     size_t tb = h->tab.size() * sizeof(float4), pb = (size_t)h->npairs * sizeof(int4);
     size_t fsb = (size_t)h->npairs * sizeof(int2);
-    size_t bxo = tb + 6 * pb + fsb, bxb = h->box.size() * sizeof(float4);
+    size_t bxo = tb + 5 * pb + fsb, bxb = h->box.size() * sizeof(float4);
     bxo = (bxo + 15) & ~(size_t)15;
     const size_t vto = (bxo + bxb + 15) & ~(size_t)15, vtb = h->vtab.size() * sizeof(float4);
     const size_t vio = vto + vtb, vib = h->vinfo.size() * sizeof(int4);
     const size_t cbo = (vio + vib + 15) & ~(size_t)15, cbb = h->ctab.size() * sizeof(float4);
     const size_t cio = cbo + cbb, cib = h->ccnt.size();
-    CUDA_TRY(h, dev_malloc((void**)&h->d_scene, cio + cib + 64));
+    const size_t leaves = sweep_leaf_cap(h);
+    const size_t swo = (cio + cib + 127) & ~(size_t)127;
+    const size_t groups = ((size_t)h->npairs + SWEEP_GROUP - 1) / SWEEP_GROUP + 1;
+    CUDA_TRY(h, dev_malloc((void**)&h->d_scene, swo + leaves * (16 + 32 * 36) + groups * 4));
     char* base = (char*)h->d_scene;
     CUDA_TRY(h, cudaMemcpy(base, h->tab.data(), tb, cudaMemcpyHostToDevice));
     if (pb) CUDA_TRY(h, cudaMemcpy(base + tb, h->pairs.data(), pb, cudaMemcpyHostToDevice));
-    if (pb) CUDA_TRY(h, cudaMemcpy(base + tb + pb, h->pairs_b.data(), pb, cudaMemcpyHostToDevice));
-    if (pb) CUDA_TRY(h, cudaMemcpy(base + tb + 2 * pb, h->far.data(), pb, cudaMemcpyHostToDevice));
-    if (pb) CUDA_TRY(h, cudaMemcpy(base + tb + 3 * pb, h->scan_c.data(), pb, cudaMemcpyHostToDevice));
-    if (pb) CUDA_TRY(h, cudaMemcpy(base + tb + 4 * pb, h->scan_b.data(), pb, cudaMemcpyHostToDevice));
-    if (pb) CUDA_TRY(h, cudaMemcpy(base + tb + 5 * pb, h->swp.data(), pb, cudaMemcpyHostToDevice));
-    if (pb) CUDA_TRY(h, cudaMemcpy(base + tb + 6 * pb, h->pair_poly.data(), fsb, cudaMemcpyHostToDevice));
+    if (pb) CUDA_TRY(h, cudaMemcpy(base + tb + 5 * pb, h->pair_poly.data(), fsb, cudaMemcpyHostToDevice));
     if (bxb) CUDA_TRY(h, cudaMemcpy(base + bxo, h->box.data(), bxb, cudaMemcpyHostToDevice));
     if (vtb) CUDA_TRY(h, cudaMemcpy(base + vto, h->vtab.data(), vtb, cudaMemcpyHostToDevice));
     if (vib) CUDA_TRY(h, cudaMemcpy(base + vio, h->vinfo.data(), vib, cudaMemcpyHostToDevice));
@@ -940,22 +1082,26 @@ int gprm_init(gprm_space* h, int rank, int size)
     s.far = (const float4*)(base + tb + 2 * pb);
     s.scan_c = (const int4*)(base + tb + 3 * pb);
     s.scan_b = (const float4*)(base + tb + 4 * pb);
-    s.swp = (const float4*)(base + tb + 5 * pb);
-    s.ppoly = (const int2*)(base + tb + 6 * pb);
+    s.ppoly = (const int2*)(base + tb + 5 * pb);
     s.box = bxb ? (const float4*)(base + bxo) : nullptr;
     s.vtab = (const float4*)(base + vto);
     s.vinfo = (const int4*)(base + vio);
     s.ctab = cbb ? (const float4*)(base + cbo) : nullptr;
     s.ccnt = (const unsigned char*)(base + cio);
     s.cslots = h->cslots;
+    s.swl = (const float4*)(base + swo);
+    s.swp = s.swl + leaves;
+    s.swb = s.swp + leaves * 32;
+    s.swj = (const int*)(s.swb + leaves * 32);
+    s.swg = s.swj + leaves * 32;
     s.fast = (h->mode & GPRM_MODE_FAST) != 0;
-    s.thr_dir = h->thr_dir;
-    s.eps_dir = h->eps_dir;
     s.nslots = (int)h->slot_sys.size();
     for (int i = 0; i < s.nslots; ++i) { s.slot_sys[i] = h->slot_sys[i]; s.slot_block[i] = h->slot_block[i]; }
 
-    CUDA_TRY(h, launch_static_pairs(s, cudaStreamLegacy));   /* after the uploads, on their stream */
-    CUDA_TRY(h, cudaStreamSynchronize(cudaStreamLegacy));
+    {
+        const int rc = upload_certificates(h);
+        if (rc) return rc;
+    }
     CUDA_TRY(h, plan_launch(s, 1, 128, &h->cfg_v));
     CUDA_TRY(h, plan_launch(s, 0, 128, &h->cfg_e));
     CUDA_TRY(h, dev_malloc((void**)&h->d_total, sizeof(Control)));
@@ -1026,16 +1172,7 @@ int gprm_set_band(gprm_space* h, float band_m)
     if (h->inited) {
         CUDA_TRY(h, cudaSetDevice(h->device));
         CUDA_TRY(h, cudaDeviceSynchronize());
-        size_t tb = h->tab.size() * sizeof(float4), pb = (size_t)h->npairs * sizeof(int4);
-        if (pb) CUDA_TRY(h, cudaMemcpy((char*)h->d_scene + tb + pb, h->pairs_b.data(), pb, cudaMemcpyHostToDevice));
-        if (pb) CUDA_TRY(h, cudaMemcpy((char*)h->d_scene + tb + 2 * pb, h->far.data(), pb, cudaMemcpyHostToDevice));
-        if (pb) CUDA_TRY(h, cudaMemcpy((char*)h->d_scene + tb + 3 * pb, h->scan_c.data(), pb, cudaMemcpyHostToDevice));
-        if (pb) CUDA_TRY(h, cudaMemcpy((char*)h->d_scene + tb + 4 * pb, h->scan_b.data(), pb, cudaMemcpyHostToDevice));
-        if (pb) CUDA_TRY(h, cudaMemcpy((char*)h->d_scene + tb + 5 * pb, h->swp.data(), pb, cudaMemcpyHostToDevice));
-        h->dsc.thr_dir = h->thr_dir;
-        h->dsc.eps_dir = h->eps_dir;
-        CUDA_TRY(h, launch_static_pairs(h->dsc, cudaStreamLegacy));
-        CUDA_TRY(h, cudaStreamSynchronize(cudaStreamLegacy));
+        return upload_certificates(h);
     }
     return GPRM_OK;
 }

@@ -46,6 +46,7 @@
                                ones whose certificate fails) */
 #define SCAN_USABLE  1      /* by the scan's own tests */
 #define SCAN_SETTLED 2      /* two static polytopes whose certificate holds: always free */
+#define SWEEP_GROUP 4096    /* pairs of one sweep group */
 /* slots (-1: none) and frames of a pair's polytopes in one word (scan_c.x) */
 #define SCAN_PACK(slot_p, slot_q, sys_p, sys_q) \
     (((slot_p) & 255) | (((slot_q) & 255) << 8) | ((sys_p) << 16) | ((sys_q) << 24))
@@ -77,11 +78,21 @@ struct DevScene {
     const float4* far;
     const int4* scan_c;
     const float4* scan_b;
-    /* sweep stage of the edge checks per pair: the static partner's ball
-       centre (unused between two moving polytopes), and sqrt(T2) rounded up
-       with, in its low 8 bits, the slot of a moving polytope and (equal, or
-       the other moving polytope's) a second slot; negative: SCAN_SETTLED;
-       NaN: SCAN_GENERAL */
+    /* sweep stage of the edge checks (sweep_stage): the pairs regrouped
+       into leaves of 32 entries, leaf l holding entries 32 l .. 32 l + 31;
+       group g (SWEEP_GROUP consecutive pairs) owns the leaves swg[g] ..
+       swg[g+1]-1.  Per entry swp = the static partner's ball centre (unused
+       between two moving polytopes), and sqrt(T2) rounded up with, in its
+       low 8 bits, the slot of a moving polytope and (equal, or the other
+       moving polytope's) a second slot; negative: an empty entry; NaN:
+       SCAN_GENERAL; swb = (static partner's vertex 0, R); swj = the pair.
+       Per leaf swl = a ball over its entries' centres, grown by their
+       sqrt(T2), with the leaf's slot in the radius' low 4 bits; NaN: no
+       common slot. */
+    const float4* swl;
+    const float4* swb;
+    const int* swj;
+    const int* swg;
     const float4* swp;
     /* certificates: a pair whose guaranteed separation along the first
        search direction exceeds thr_dir is reported free without the test;

@@ -79,7 +79,6 @@ struct gprm_space {
     std::vector<float4> far;       /* distance test: static ball centre, T2 */
     std::vector<int4> scan_c;      /* certificate scan: slots and frames, polytopes, SCAN_* */
     std::vector<float4> scan_b;    /* certificate scan: static polytope's vertex 0, R */
-    std::vector<float4> swp;       /* sweep stage record (DevScene::swp) */
     std::vector<double> rad;       /* inflated ball radius per polytope */
     /* bounding box per polytope about its ball centre: PCA axes (FP32
        values), half extents (exact), and the device records (axis, inflated

@@ -108,16 +108,23 @@ cudaError_t launch_recheck_multi(const BatchView& B, int blocks, int kind, const
 /* Per-lane shared floats of a warp's block: frames 1..ndof (12 floats
  * each), the world ball centres of the slots (3 floats each), the world
  * vertex 0 of the slots' polytopes (3 floats each), lane-interleaved; then,
- * in the vertex kernels only, DEFER_LANE_FLOATS per lane, together the
- * warp's queue of deferred exact pair tests (64 items) and one batch's
- * results (32 codes, 32 margins); then SWEEP_LANE_FLOATS per lane,
- * together the warp's per-slot sweep balls (GPRM_MAX_SLOTS float4). */
+ * in the vertex kernels, DEFER_LANE_FLOATS per lane, together the warp's
+ * queue of deferred exact pair tests (64 items) and one batch's results (32
+ * codes, 32 margins), in the edge kernels one float per lane and 1024 pairs
+ * of a sweep group, together the bits of the pairs that the sweep stage
+ * leaves open; then SWEEP_LANE_FLOATS per lane, together the warp's
+ * per-slot sweep balls (GPRM_MAX_SLOTS float4). */
 #define SWEEP_LANE_FLOATS 2
 static_assert(SWEEP_LANE_FLOATS * 32 >= GPRM_MAX_SLOTS * 4, "sweep area too small");
 #define DEFER_LANE_FLOATS 4
+__host__ __device__ __forceinline__ int open_lane_floats(const DevScene& sc)
+{
+    const int pairs = sc.npairs < SWEEP_GROUP ? sc.npairs : SWEEP_GROUP;
+    return (pairs + 1023) / 1024;
+}
 __host__ __device__ __forceinline__ size_t lane_floats(const DevScene& sc, bool vertex_kernel)
 {
-    return (size_t)sc.ndof * 12 + (size_t)sc.nslots * 6 + (vertex_kernel ? DEFER_LANE_FLOATS : 0) +
+    return (size_t)sc.ndof * 12 + (size_t)sc.nslots * 6 + (vertex_kernel ? DEFER_LANE_FLOATS : open_lane_floats(sc)) +
            SWEEP_LANE_FLOATS;
 }
 
@@ -131,8 +138,8 @@ size_t frame_smem_bytes(const DevScene& sc, int threads, bool vertex_kernel);
 cudaError_t configure_launch(const DevScene& sc, int vertex_kernel, int threads, int scene_in_smem,
                              LaunchCfg* cfg, int blocks_cap = 0);
 
-/* Settles the pairs between polytopes of frame 0 in sc.scan_c and sc.swp (once
- * per upload of the certificate tables). */
+/* Settles the pairs between polytopes of frame 0 in sc.scan_c (once per
+ * upload of the certificate tables). */
 cudaError_t launch_static_pairs(const DevScene& sc, cudaStream_t st);
 
 /* Vertex checks: res[i] = code of configuration q[i + offset*j]. */

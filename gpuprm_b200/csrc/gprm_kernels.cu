@@ -46,8 +46,8 @@ namespace gprm {
 
 size_t scene_smem_bytes(const DevScene& sc)
 {
-    /* tab | pairs | pairs_b | far | scan_c | scan_b | swp, padded to 16 bytes */
-    return ((size_t)sc.ntab * 16 + (size_t)sc.npairs * 96 + 15) & ~(size_t)15;
+    /* tab | pairs | pairs_b | far | scan_c | scan_b, padded to 16 bytes */
+    return ((size_t)sc.ntab * 16 + (size_t)sc.npairs * 80 + 15) & ~(size_t)15;
 }
 
 size_t frame_smem_bytes(const DevScene& sc, int threads, bool vertex_kernel)
@@ -62,11 +62,11 @@ struct SceneView {
     const float4* far;
     const int4* scan_c;
     const float4* scan_b;
-    const float4* swp;
     float* frames;   /* this lane's frames (lane-interleaved, stride 32) */
     float* cen;      /* this lane's slot ball centres, then the slots' world vertex 0 */
     float4* sweep;   /* the warp's per-slot sweep balls (GPRM_MAX_SLOTS) */
-    unsigned* defer; /* the warp's deferred-test queue (64) and batch results (32 + 32) */
+    unsigned* defer; /* vertex checks: the warp's deferred-test queue (64) and batch results (32 + 32);
+                        edge checks: the pairs of the sweep group left open (one bit each) */
 };
 
 /* The warp's sweep area: the last SWEEP_LANE_FLOATS entries of its block. */
@@ -77,15 +77,14 @@ __device__ __forceinline__ float4* sweep_area(const DevScene& sc, float* lane_fr
     return reinterpret_cast<float4*>(lane_frames - lane + (lane_floats(sc, VERTEX) - SWEEP_LANE_FLOATS) * 32);
 }
 
-/* The warp's deferred-test area (vertex kernels): the DEFER_LANE_FLOATS
- * entries before the sweep area; null in the edge kernels. */
+/* The warp's area before the sweep area: the deferred tests of a vertex
+ * kernel, the open pairs of an edge kernel. */
 template <bool VERTEX>
 __device__ __forceinline__ unsigned* defer_area(const DevScene& sc, float* lane_frames)
 {
-    if constexpr (!VERTEX) return nullptr;
     const int lane = threadIdx.x & 31;
     return reinterpret_cast<unsigned*>(lane_frames - lane +
-                                       (lane_floats(sc, true) - SWEEP_LANE_FLOATS - DEFER_LANE_FLOATS) * 32);
+                                       ((size_t)sc.ndof * 12 + (size_t)sc.nslots * 6) * 32);
 }
 
 /* Copies the scene into shared memory (SMEM) and returns the pointers the
@@ -104,7 +103,6 @@ __device__ __forceinline__ SceneView stage_scene(const DevScene& sc, unsigned ch
         float4* fr = reinterpret_cast<float4*>(smem + (size_t)sc.ntab * 16 + np * 32);
         int4* scc = reinterpret_cast<int4*>(smem + (size_t)sc.ntab * 16 + np * 48);
         float4* scb = reinterpret_cast<float4*>(smem + (size_t)sc.ntab * 16 + np * 64);
-        float4* sw = reinterpret_cast<float4*>(smem + (size_t)sc.ntab * 16 + np * 80);
         for (int i = threadIdx.x; i < sc.ntab; i += blockDim.x) t[i] = sc.tab[i];
         for (int i = threadIdx.x; i < sc.npairs; i += blockDim.x) {
             p[i] = sc.pairs[i];
@@ -112,7 +110,6 @@ __device__ __forceinline__ SceneView stage_scene(const DevScene& sc, unsigned ch
             fr[i] = sc.far[i];
             scc[i] = sc.scan_c[i];
             scb[i] = sc.scan_b[i];
-            sw[i] = sc.swp[i];
         }
         s.tab = t;
         s.pairs = p;
@@ -120,8 +117,7 @@ __device__ __forceinline__ SceneView stage_scene(const DevScene& sc, unsigned ch
         s.far = fr;
         s.scan_c = scc;
         s.scan_b = scb;
-        s.swp = sw;
-        off = ((size_t)sc.ntab * 16 + np * 96 + 15) & ~(size_t)15;   /* frames stay 16-byte aligned */
+        off = ((size_t)sc.ntab * 16 + np * 80 + 15) & ~(size_t)15;   /* frames stay 16-byte aligned */
     } else {
         s.tab = sc.tab;
         s.pairs = sc.pairs;
@@ -129,7 +125,6 @@ __device__ __forceinline__ SceneView stage_scene(const DevScene& sc, unsigned ch
         s.far = sc.far;
         s.scan_c = sc.scan_c;
         s.scan_b = sc.scan_b;
-        s.swp = sc.swp;
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     s.frames = reinterpret_cast<float*>(smem + off) + (size_t)warp * lane_floats(sc, VERTEX) * 32 + lane;
@@ -230,8 +225,8 @@ struct PairCounts {
  * which must exceed thr_dir (with 1e-5 relative allowances for the
  * rounding of this bound, which cover the approximate root and quotient:
  * a settled pair is one that every lane's own test would certify). */
-__device__ __forceinline__ bool swept_direction(const DevScene& sc, float sx, float sy, float sz, float rv, float dx,
-                                                float dy, float dz, float rc, float R)
+__device__ __forceinline__ bool swept_direction(float eps_dir, float thr_dir, float sx, float sy, float sz, float rv,
+                                                float dx, float dy, float dz, float rc, float R)
 {
     const float n2 = __fmaf_rn(sx, sx, __fmaf_rn(sy, sy, sz * sz));
     const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
@@ -239,59 +234,115 @@ __device__ __forceinline__ bool swept_direction(const DevScene& sc, float sx, fl
     const float N = __fmaf_rn(sx, dx, __fmaf_rn(sy, dy, sz * dz)) * (1.0f - 1e-5f) -
                     __fmaf_rn(sn, rc, __fmaf_rn(rv, dn, rv * rc)) * (1.0f + 1e-5f);
     const float slo = sn * (1.0f - 1e-5f) - rv * (1.0f + 1e-5f), sup = (sn + rv) * (1.0f + 1e-5f);
-    const float err = (dn + rc + R) * (__fdividef(sc.eps_dir, slo) + 1e-6f) * (1.0f + 2e-5f);
-    return N > 0.0f && slo > 1e-3f && N * (1.0f - 1e-5f) > sup * (__fmaf_rn(R, 1.0f + 1e-5f, err) + sc.thr_dir);
+    const float err = (dn + rc + R) * (__fdividef(eps_dir, slo) + 1e-6f) * (1.0f + 2e-5f);
+    return N > 0.0f && slo > 1e-3f && N * (1.0f - 1e-5f) > sup * (__fmaf_rn(R, 1.0f + 1e-5f, err) + thr_dir);
 }
 
-/* The sweep stage of an edge round for the pairs of up to 32 chunks from
- * j0 (lane k of chunk c: pair j0 + 32 c + k), against the warp's sweep
- * balls: a pair whose ball centres are farther apart in every lane than
- * rho_P + rho_Q + sqrt(T2) is settled for all lanes at once (each lane's
- * exact distance then exceeds sqrt(T2)); else the direction test is bounded
- * over all lanes at once (swept_direction).  Returns, in lane c, the pairs
- * of chunk c left for the lanes' own tests (bit k).
+/* Distance test of a sweep record against the warp's sweep balls: false
+ * when the balls are farther apart in every lane than rc (the radii) +
+ * root, with D from the moving slot's ball to the other's. */
+__device__ __forceinline__ bool swept_near(float4 o, float4 m, float root, float& dx, float& dy, float& dz, float& rc)
+{
+    dx = o.x - m.x; dy = o.y - m.y; dz = o.z - m.z;
+    rc = o.w + m.w;
+    const float dd2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
+    const float A = (root + rc) * (1.0f + 1e-6f);
+    /* |m - o|^2 >= dd2 (1 - 1e-6) > A^2 settles; NaN does not */
+    return !(dd2 * (1.0f - 1e-6f) > A * A);
+}
+
+/* A sweep entry (r: swp, v: swb) against the warp's sweep balls: true when
+ * neither the distance nor the direction settles its pair for every lane.
+ * Branch-free, so that two entries go side by side. */
+__device__ __forceinline__ bool swept_open(const float4* sweep, bool dir_on, float eps_dir, float thr_dir, float4 r,
+                                           float4 v)
+{
+    const int w = __float_as_int(r.w);
+    const int a = w & 15, b = (w >> 4) & 15;   /* a: a moving polytope's slot; b != a: the other's */
+    const float4* v0 = sweep + (dir_on ? SWEEP_V0_SLOTS : 0);
+    float4 o = make_float4(r.x, r.y, r.z, 0.0f), u = make_float4(v.x, v.y, v.z, 0.0f);
+    if (b != a) { o = sweep[b]; u = v0[b]; }
+    const float root = __int_as_float(w | 255);   /* the slot bits round it up */
+    float dx, dy, dz, rc;
+    const bool near = swept_near(o, sweep[a], root, dx, dy, dz, rc);
+    const float4 m = v0[a];
+    const bool settled = dir_on && swept_direction(eps_dir, thr_dir, u.x - m.x, u.y - m.y, u.z - m.z, u.w + m.w, dx,
+                                                   dy, dz, rc, v.w);
+    return near && !settled && !(root < 0.0f);
+}
+
+__device__ __forceinline__ void sweep_mark(const int* swj, unsigned* bits, int g, int i, bool open)
+{
+    if (open) {
+        const int j = swj[i] - g * SWEEP_GROUP;
+        atomicOr(&bits[j >> 5], 1u << (j & 31));
+    }
+}
+
+/* The sweep stage of an edge round for the pairs of group g, against the
+ * warp's sweep balls: a pair whose ball centres are farther apart in every
+ * lane than rho_P + rho_Q + sqrt(T2) is settled for all lanes at once (each
+ * lane's exact distance then exceeds sqrt(T2)); else the direction test is
+ * bounded over all lanes at once (swept_direction).  Leaves in S.defer the
+ * pairs left for the lanes' own tests (bit j - g * SWEEP_GROUP), words of
+ * them.
  *
- * One 16-byte record a pair (swp: the static partner's ball centre and
- * sqrt(T2) with the two slots in its low bits), chunks independent of each
- * other and of the lanes' state, so that their loads overlap; the second
- * record (scan_b) is read only where the distance leaves the pair open.
- * With three records a pair and a vote, a scan and a branch after every
- * chunk this stage took 17,000 cycles of a hull6 round (13 chunks). */
-__device__ __forceinline__ unsigned sweep_stage(const DevScene& sc, const SceneView& S, int j0, int chunks)
+ * Two levels: lane l tests leaf l of the next 32 (32 pairs of one slot whose
+ * static partners lie close together) by its ball, then the warp goes
+ * through the leaves left, a lane per pair, two leaves side by side without
+ * branches (this stage waits on its loads: 3 % slower one leaf at a time
+ * with the next one's records loaded ahead, 7 % with swb read only where
+ * the distance leaves a pair open).  In pair order, with every pair of the
+ * list tested, it took 108,000 of 151,000 cycles of a round on the 7-DOF
+ * wall scene (129 chunks of 32 pairs; 70,001 edges 27.7 -> 15.9 ms with the
+ * leaves); on 64 obstacles (two leaves a slot) the leaf level costs what it
+ * saves (62.1 -> 61.7 ms). */
+__device__ __forceinline__ void sweep_stage(const DevScene& sc, const SceneView& S, int g, int words)
 {
     const int lane = threadIdx.x & 31;
+    /* the descriptor's fields in registers: a batch keeps it in shared
+       memory, where the bits are set */
     const bool dir_on = sc.nslots <= SWEEP_V0_SLOTS;
-    unsigned mine = 0u;
-#pragma unroll 2
-    for (int c = 0; c < chunks; ++c) {
-        const int j = j0 + c * 32 + lane;
+    const float eps_dir = sc.eps_dir, thr_dir = sc.thr_dir;
+    const float4 *swl = sc.swl, *swp = sc.swp, *swb = sc.swb, *sweep = S.sweep;
+    const int* swj = sc.swj;
+    unsigned* bits = S.defer;
+    for (int w = lane; w < words; w += 32) bits[w] = 0u;
+    __syncwarp();
+    const int end = sc.swg[g + 1];
+#pragma unroll 1
+    for (int l0 = sc.swg[g]; l0 < end; l0 += 32) {
         bool open = false;
-        if (j < sc.npairs) {
-            const float4 r = S.swp[j];
+        if (l0 + lane < end) {
+            const float4 r = swl[l0 + lane];
             const int w = __float_as_int(r.w);
-            const int a = w & 15, b = (w >> 4) & 15;   /* a: a moving polytope's slot; b != a: the other's */
-            const float4 m = S.sweep[a];
-            float4 o = make_float4(r.x, r.y, r.z, 0.0f);
-            if (b != a) o = S.sweep[b];
-            const float dx = o.x - m.x, dy = o.y - m.y, dz = o.z - m.z, rc = o.w + m.w;
-            const float dd2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
-            const float root = __int_as_float(w | 255);   /* the slot bits round it up */
-            const float A = (root + rc) * (1.0f + 1e-6f);
-            /* |m - o|^2 >= dd2 (1 - 1e-6) > A^2; a negative root: settled
-               for every configuration; NaN: not for the sweep tests */
-            open = !(dd2 * (1.0f - 1e-6f) > A * A) && !(root < 0.0f);
-            if (open && dir_on) {
-                const float4 v = S.sweep[SWEEP_V0_SLOTS + a];
-                const float4 sb = S.scan_b[j];
-                float4 u = make_float4(sb.x, sb.y, sb.z, 0.0f);
-                if (b != a) u = S.sweep[SWEEP_V0_SLOTS + b];
-                open = !swept_direction(sc, u.x - v.x, u.y - v.y, u.z - v.z, u.w + v.w, dx, dy, dz, rc, sb.w);
-            }
+            float dx, dy, dz, rc;
+            open = swept_near(make_float4(r.x, r.y, r.z, 0.0f), sweep[w & 15], __int_as_float(w | 15), dx, dy, dz,
+                              rc);
         }
-        const unsigned left = __ballot_sync(FULL_MASK, open);
-        if (lane == c) mine = left;
+        unsigned left = __ballot_sync(FULL_MASK, open);
+        if (!left) continue;
+        /* two leaves side by side (the last one with itself: the bits are
+           only ever set) */
+        int ia = (l0 + __ffs(left) - 1) * 32 + lane;
+        left &= left - 1u;
+        int ib = left ? (l0 + __ffs(left) - 1) * 32 + lane : ia;
+        left &= left - 1u;
+#pragma unroll 1
+        for (;;) {
+            const float4 ra = swp[ia], va = swb[ia], rb = swp[ib], vb = swb[ib];
+            const bool oa = swept_open(sweep, dir_on, eps_dir, thr_dir, ra, va);
+            const bool ob = swept_open(sweep, dir_on, eps_dir, thr_dir, rb, vb);
+            sweep_mark(swj, bits, g, ia, oa);
+            sweep_mark(swj, bits, g, ib, ob);
+            if (!left) break;
+            ia = (l0 + __ffs(left) - 1) * 32 + lane;
+            left &= left - 1u;
+            ib = left ? (l0 + __ffs(left) - 1) * 32 + lane : ia;
+            left &= left - 1u;
+        }
     }
-    return mine;
+    __syncwarp();
 }
 
 /* This lane's certificates of the pairs j0 + k, k in cand (warp-uniform),
@@ -754,16 +805,18 @@ __device__ __forceinline__ void check_edge(const DevScene& sc, const SceneView& 
         int jend = 0;   /* pairs processed by the warp */
         int jrec = 0x7fffffff, jlast = -1;   /* first and last pair decided within the band */
         bool stop = false;
-        /* groups of 32 chunks of 32 pairs: the sweep stage for the whole
-           group, then per chunk with a pair left the lanes' own certificates
-           and the exact tests in the reference's order; a code can only
-           change at such a test, so the vote runs only there */
+        /* the sweep stage for a group of pairs, then per chunk of 32 pairs
+           with one left open the lanes' own certificates and the exact tests
+           in the reference's order; a code can only change at such a test,
+           so the vote runs only there */
+        unsigned nact = __ballot_sync(FULL_MASK, active);
 #pragma unroll 1
-        for (int g0 = 0; g0 < sc.npairs && !stop; g0 += 1024) {
+        for (int g0 = 0; g0 < sc.npairs; g0 += 1024) {     /* a word per lane */
             const int gend = min(sc.npairs, g0 + 1024);
-            unsigned nact = __ballot_sync(FULL_MASK, active);
-            if (!nact) break;
-            const unsigned open = sweep_stage(sc, S, g0, (gend - g0 + 31) >> 5);
+            if (g0 % SWEEP_GROUP == 0)
+                sweep_stage(sc, S, g0 / SWEEP_GROUP, (min(sc.npairs - g0, SWEEP_GROUP) + 31) >> 5);
+            const int wi = ((g0 % SWEEP_GROUP) >> 5) + lane;
+            const unsigned open = g0 + 32 * lane < gend ? S.defer[wi] : 0u;
             unsigned left = __ballot_sync(FULL_MASK, open != 0u);
             int pos = g0;   /* pairs before it are counted */
             while (left) {
@@ -1318,7 +1371,7 @@ __global__ void k_fk_probe(DevScene sc, const float* q, float* out)
  * 72 % of an edge round there (570,000 of 790,000 cycles): 70,001 roadmap
  * edges 135.0 -> 43.0 ms, a vertex check of 100,003 configurations 8.8 ->
  * 8.2 ms. */
-__global__ void k_static_pairs(DevScene sc, int4* __restrict__ scan_c, float4* __restrict__ swp)
+__global__ void k_static_pairs(DevScene sc, int4* __restrict__ scan_c)
 {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= sc.npairs) return;
@@ -1328,10 +1381,7 @@ __global__ void k_static_pairs(DevScene sc, int4* __restrict__ scan_c, float4* _
     /* no slot and no frame is read: both polytopes are untransformed */
     __shared__ float none[1];
     bool used_dir;
-    if (pair_certified(sc, sc.tab, pr, sc.pairs_b[j], none, none, &used_dir, j)) {
-        scan_c[j].w = SCAN_SETTLED;
-        swp[j].w = -1.0f;
-    }
+    if (pair_certified(sc, sc.tab, pr, sc.pairs_b[j], none, none, &used_dir, j)) scan_c[j].w = SCAN_SETTLED;
 }
 
 /* ------------------------------------------------------------------ */
@@ -1341,8 +1391,7 @@ __global__ void k_static_pairs(DevScene sc, int4* __restrict__ scan_c, float4* _
 cudaError_t launch_static_pairs(const DevScene& sc, cudaStream_t st)
 {
     if (sc.npairs < 1) return cudaSuccess;
-    k_static_pairs<<<(sc.npairs + 127) / 128, 128, 0, st>>>(sc, const_cast<int4*>(sc.scan_c),
-                                                            const_cast<float4*>(sc.swp));
+    k_static_pairs<<<(sc.npairs + 127) / 128, 128, 0, st>>>(sc, const_cast<int4*>(sc.scan_c));
     return cudaGetLastError();
 }
 
@@ -1627,7 +1676,6 @@ __device__ __forceinline__ void switch_scene(const BatchView& B, int p, DevScene
     S.far = wsc->far;
     S.scan_c = wsc->scan_c;
     S.scan_b = wsc->scan_b;
-    S.swp = wsc->swp;
     S.frames = frames;
     S.cen = frames + (size_t)wsc->ndof * 12 * 32;
     S.sweep = sweep_area<VERTEX>(*wsc, frames);

@@ -1,5 +1,5 @@
 """The certificate scan at the sizes where it can go wrong: pair counts at
-and around whole chunks of 32 (and groups of 32 chunks), robots with a base
+and around whole chunks of 32, rows of 32 chunks and sweep groups, robots with a base
 link (pairs whose polytopes are both in frame 0), and more slots than the
 swept direction test covers.  Codes of the exact arithmetic must equal the
 oracle's, bit for bit."""
@@ -38,6 +38,8 @@ SIZES = [
     (3, 1, 11, False, 0),     # 34 pairs: one chunk and two pairs
     (6, 1, 169, False, 0),    # 1024 pairs: one whole group
     (6, 1, 170, False, 0),    # a group and a few pairs
+    (6, 1, 681, False, 0),    # 4096 pairs: one whole sweep group
+    (6, 1, 690, False, 0),    # a sweep group and a few pairs
     (4, 1, 20, True, 0),      # base link, every static pair settled
     (4, 1, 20, True, 1),      # base link, one static pair left to the exact test
     (4, 1, 20, True, 2),      # base link through an obstacle: nothing is free
@@ -49,6 +51,7 @@ SIZES = [
 def test_sizes_are_the_intended_ones():
     n = [make(*s).num_pairs for s in SIZES]
     assert n[0] == 1 and n[1] == 32 and n[2] == 34 and n[3] == 1024 and n[4] == 1030
+    assert n[5] == 4096 and n[6] == 4150
 
 
 def check(sc, cs, exact, nq=400, ne=60):
