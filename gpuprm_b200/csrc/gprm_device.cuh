@@ -37,10 +37,6 @@
 
 #define GPRM_MAX_FRAMES 8   /* ndof + 1 */
 #define GPRM_MAX_SLOTS 16   /* moving polytopes whose ball centre is tracked per lane */
-/* neighbours evaluated together by the support climb (1 or 4) */
-#ifndef GPRM_CLIMB_CHUNK
-#define GPRM_CLIMB_CHUNK 1
-#endif
 /* how the certificate scan treats a pair (scan_c.w) */
 #define SCAN_GENERAL 0      /* never certified (a moving polytope without a slot, or two static
                                ones whose certificate fails) */
@@ -269,53 +265,88 @@ __device__ __forceinline__ typename P::R normalize3(V3<typename P::R>& u)
     return norm;
 }
 
-/* support_vertex_searcher::search_support_vertex (collision4.h:66-103):
- * first-improvement climb over the vertex adjacency, starting at `cur`
- * (an entry of the polytope's block B).  The neighbours of the current
- * vertex are evaluated four at a time (independent loads and dot
- * products); the move goes to the first of them, in CRS order, whose dot
- * product exceeds the current maximum, which is the vertex the reference's
- * one-at-a-time scan moves to.  The maximum rises strictly, so there are at
- * most n-1 moves; the loop bound only guards corrupt data. */
+/* neighbours of each side evaluated together by the support climbs (two:
+ * three or four are slower in FP32, which they push past 128 registers, and
+ * no faster in FP64) */
+constexpr int CLIMB_CHUNK = 2;
+
+/* One side of climb2: the climb's vertex, its dot product, and how many of
+ * its neighbours are done. */
+template <class R> struct Climber {
+    static constexpr int CH = CLIMB_CHUNK;
+    float4 cur;
+    R best;
+    int i;
+    bool on;
+
+    __device__ __forceinline__ void start(float4 at, V3<R> d)
+    {
+        cur = at;
+        best = dot3<R>((R)cur.x, (R)cur.y, (R)cur.z, d.x, d.y, d.z);
+        i = 0;
+        on = true;
+    }
+    /* the next CH neighbours, the last one repeated past the end */
+    __device__ __forceinline__ void load(const float4* __restrict__ B, float4* u) const
+    {
+        const float4* e = B + 2 + ent_dsp(cur);
+        const int n = ent_cnt(cur) - 1;
+#pragma unroll
+        for (int k = 0; k < CH; ++k) u[k] = e[min(i + k, n)];
+    }
+    /* moves to the first of them, in order, that improves on the vertex (a
+       repeated one cannot improve anew) */
+    __device__ __forceinline__ void step(const float4* u, V3<R> d)
+    {
+        float4 t = u[CH - 1];
+        R dt = dot3<R>((R)t.x, (R)t.y, (R)t.z, d.x, d.y, d.z);
+#pragma unroll
+        for (int k = CH - 2; k >= 0; --k) {
+            const R dk = dot3<R>((R)u[k].x, (R)u[k].y, (R)u[k].z, d.x, d.y, d.z);
+            if (dk > best) { t = u[k]; dt = dk; }
+        }
+        i += CH;
+        const bool more = i < ent_cnt(cur);
+        if (on && dt > best) { best = dt; cur = t; i = 0; }
+        else on = on && more;
+    }
+};
+
+/* support_vertex_searcher::search_support_vertex (collision4.h:66-103) for
+ * both polytopes of a pair: first-improvement climbs over the vertex
+ * adjacency along p and q, starting at ep and eq (entries of the polytopes'
+ * blocks).  The move goes to the first neighbour, in CRS order, whose dot
+ * product exceeds the current maximum, the vertex the reference's
+ * one-at-a-time scan moves to.  The maximum rises strictly, so a climb makes
+ * at most n-1 moves of at most n neighbours; the loop bound only guards
+ * corrupt data.
+ *
+ * The climbs are chains of dependent loads (one exact test of a pair took
+ * 16,000 cycles inside the edge kernel, 80,000 to 180,000 on an idle GPU
+ * with cold caches): two neighbours of each side are loaded and
+ * evaluated at a time, both sides together.  150,001-sample roadmap edges
+ * (exact, host buffers) 19.1 -> 18.0 ms, 100,003 exact vertex checks of the
+ * wall scene 7.0 -> 5.9 ms, 500 short edges of the box scene 245 -> 195 us
+ * (their FP64 rechecks). */
 template <class P>
-__device__ __forceinline__ float4 climb(const float4* __restrict__ B, float4 cur, typename P::R dx,
-                                        typename P::R dy, typename P::R dz)
+__device__ __forceinline__ void climb2(const float4* __restrict__ BP, float4& ep, V3<typename P::R> p,
+                                       const float4* __restrict__ BQ, float4& eq, V3<typename P::R> q)
 {
     typedef typename P::R R;
-    R best = dot3<R>((R)cur.x, (R)cur.y, (R)cur.z, dx, dy, dz);
+    constexpr int CH = CLIMB_CHUNK;
+    Climber<R> a, b;
+    a.start(ep, p);
+    b.start(eq, q);
 #pragma unroll 1
-    for (int guard = 0; guard < 128; ++guard) {
-        const float4* e = B + 2 + ent_dsp(cur);
-        const int c = ent_cnt(cur);
-        bool moved = false;
-#if GPRM_CLIMB_CHUNK == 4
-#pragma unroll 1
-        for (int i = 0; i < c && !moved; i += 4) {
-            const int left = c - i;
-            float4 u0 = e[i], u1 = u0, u2 = u0, u3 = u0;
-            if (left > 1) u1 = e[i + 1];
-            if (left > 2) u2 = e[i + 2];
-            if (left > 3) u3 = e[i + 3];
-            R d0 = dot3<R>((R)u0.x, (R)u0.y, (R)u0.z, dx, dy, dz);
-            R d1 = dot3<R>((R)u1.x, (R)u1.y, (R)u1.z, dx, dy, dz);
-            R d2 = dot3<R>((R)u2.x, (R)u2.y, (R)u2.z, dx, dy, dz);
-            R d3 = dot3<R>((R)u3.x, (R)u3.y, (R)u3.z, dx, dy, dz);
-            if (d0 > best) { best = d0; cur = u0; moved = true; }
-            else if (left > 1 && d1 > best) { best = d1; cur = u1; moved = true; }
-            else if (left > 2 && d2 > best) { best = d2; cur = u2; moved = true; }
-            else if (left > 3 && d3 > best) { best = d3; cur = u3; moved = true; }
-        }
-#else
-#pragma unroll 1
-        for (int i = 0; i < c; ++i) {
-            float4 u = e[i];
-            R d = dot3<R>((R)u.x, (R)u.y, (R)u.z, dx, dy, dz);
-            if (d > best) { best = d; cur = u; moved = true; break; }
-        }
-#endif
-        if (!moved) break;
+    for (int guard = 0; guard < 16384 && (a.on || b.on); ++guard) {
+        float4 u[CH], v[CH];
+        a.load(BP, u);
+        b.load(BQ, v);
+        a.step(u, p);
+        b.step(v, q);
     }
-    return cur;
+    ep = a.cur;
+    eq = b.cur;
 }
 
 template <class R> struct V2 { R x, y; };
@@ -407,8 +438,7 @@ __device__ __forceinline__ int pair_test(const DevScene& sc, const float4* __res
         else Sp = rot_t<R>(tp, S.x, S.y, S.z);
         if (idQ) { Sq.x = -S.x; Sq.y = -S.y; Sq.z = -S.z; }
         else Sq = rot_t<R>(tq, -S.x, -S.y, -S.z);
-        ep = climb<P>(BP, ep, Sp.x, Sp.y, Sp.z);
-        eq = climb<P>(BQ, eq, Sq.x, Sq.y, Sq.z);
+        climb2<P>(BP, ep, Sp, BQ, eq, Sq);
         V3<R> p0, q0;
         if (idP) { p0.x = (R)ep.x; p0.y = (R)ep.y; p0.z = (R)ep.z; }
         else p0 = xform<R>(tp, (R)ep.x, (R)ep.y, (R)ep.z);
