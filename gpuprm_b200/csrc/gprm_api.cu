@@ -767,6 +767,56 @@ int event_pair(gprm_space* h, std::vector<cudaEvent_t>& pool, size_t& used, cuda
     return GPRM_OK;
 }
 
+/* Whether a request of n items goes through the small-request kernels.
+ * Measured on one B200, host buffers in and out, us a call, large path
+ * against small (box: 67 pairs, hull: 394, wall: 4117):
+ *   configurations  exact arithmetic  box        hull       wall
+ *     n = 1                           68 / 27    104 / 43   219 / 54
+ *     n = 592                         167 / 73   377 / 99   1992 / 162
+ *     n = 16384                       243 / 112  600 / 209  2536 / 603
+ *   edges (0.25 rad on average)
+ *     n = 32                          123 / 84   196 / 130  322 / 256
+ *     n = 592                         193 / 105  335 / 257  532 / 332
+ *     n = 1024                        194 / 125  283 / 372  847 / 785
+ *     n = 4096                        239 / 281  425 / 615  2493 / 1154
+ * A configuration's block has as much to do as its lanes' share of a warp
+ * elsewhere, so the small path holds far up; above 16384 the persistent
+ * kernels, which keep the FP64 rechecks apart, catch up on the smaller
+ * scenes.  An edge's block costs four warps for one: it pays while every
+ * block is resident at once, and beyond that only on large pair lists,
+ * where four warps share the sweep stage. */
+constexpr int SMALL_CONFIGS = 16384;
+constexpr int SMALL_EDGE_WAVES = 16, SMALL_EDGE_PAIRS = 2048;
+bool small_request(const gprm_space* h, int kind, long long n)
+{
+    /* the queue-capacity hook and the per-kernel profile belong to the large path */
+    if (!h->small_smem || h->profiling || h->debug_qcap || h->npairs > 65535 || n < 1) return false;
+    const int wave = h->sms * 4;     /* resident blocks */
+    if (kind == 0) return n <= SMALL_CONFIGS;
+    return n <= wave || (n <= (long long)wave * SMALL_EDGE_WAVES && h->npairs >= SMALL_EDGE_PAIRS);
+}
+
+/* Enqueues a small request: one launch (after zeroing the keys of edges
+ * that several blocks share).  status: pinned word for a rejected edge. */
+int enqueue_small(gprm_space* h, Request& r, int kind, const float* a, const float* b, int* res, int n, long long offset,
+                  cudaStream_t st, unsigned* status)
+{
+    const int band_on = (h->mode & GPRM_MODE_FP64_BAND) != 0;
+    const int wave = h->sms * 4;     /* resident blocks */
+    if (kind == 0) {
+        const int per = n <= wave ? 1 : std::min(32, (n + wave - 1) / wave);
+        CUDA_TRY(h, launch_configs_small(h->dsc, h->small_smem, a, n, offset, per, res, band_on, h->band, h->d_total, st));
+    } else {
+        int segs = 1;
+        while (segs < 16 && 2 * segs * n <= wave) segs *= 2;
+        if (segs > 1) CUDA_TRY(h, cudaMemsetAsync(r.d_ovf, 0, 2 * (size_t)n * sizeof(unsigned), st));
+        CUDA_TRY(h, launch_edges_small(h->dsc, h->small_smem, a, b, n, offset, h->dq, h->policy, segs, res, r.d_ovf,
+                                       band_on, h->band, h->d_total, status, st));
+    }
+    h->host_stats.launches += 1;
+    return GPRM_OK;
+}
+
 /* Enqueues one request on stream `st` with device inputs/outputs.
  * kind 0: q -> res.  kind 1: (qs, qe) -> res. */
 int enqueue_part(gprm_space* h, Request& r, int kind, const float* a, const float* b, int* res, long long n,
@@ -775,6 +825,7 @@ int enqueue_part(gprm_space* h, Request& r, int kind, const float* a, const floa
 int enqueue(gprm_space* h, Request& r, int kind, const float* a, const float* b, int* res, long long n,
             long long offset, cudaStream_t st)
 {
+    if (small_request(h, kind, n)) return enqueue_small(h, r, kind, a, b, res, (int)n, offset, st, nullptr);
     int rc = enqueue_part(h, r, kind, a, b, res, n, offset, st, r.ctl, r.d_key);
     if (rc || kind != 1 || !(h->mode & GPRM_MODE_FP64_BAND) || r.q_pending) return rc;
     /* read the queue demand back for the next call's sizing, unless the
@@ -878,6 +929,19 @@ int submit_host(gprm_space* h, int kind, const float* a, const float* b, int* re
     int rc = ensure_request(h, r, kind, (size_t)(n > 0 ? n : 1), true, true);
     if (rc) return rc;
     const int nd = h->ndof;
+    r.small = small_request(h, kind, n);
+    if (r.small) {
+        /* the kernel reads the pinned staging and writes the pinned results
+           itself: no copies, one launch */
+        for (int j = 0; j < nd; ++j) {
+            memcpy(r.h_a + (size_t)j * n, a + (size_t)offset * j, (size_t)n * sizeof(float));
+            if (kind == 1) memcpy(r.h_b + (size_t)j * n, b + (size_t)offset * j, (size_t)n * sizeof(float));
+        }
+        r.parts = 1;
+        r.ctl_host[0].flags = 0;
+        rc = enqueue_small(h, r, kind, r.h_a, r.h_b, r.h_res, n, n, r.st, &r.ctl_host[0].flags);
+        if (rc) return rc;
+    }
     /* parts: the host copies part p into pinned staging while the device
        transfers and checks part p-1 (same stream, so the parts' checks run
        in order and share the FP64 queue) */
@@ -886,7 +950,7 @@ int submit_host(gprm_space* h, int kind, const float* a, const float* b, int* re
     /* part boundaries (in 16ths): a small first part, whose staging is the
        only one not hidden, then three equal parts */
     static const int edge16[HOST_PARTS + 1] = {0, 1, 6, 11, 16};
-    for (int p = 0; p < parts && n > 0; ++p) {
+    for (int p = 0; p < parts && n > 0 && !r.small; ++p) {
         const size_t c0 = parts == 1 ? 0 : (size_t)n * edge16[p] / 16;
         const size_t c1 = parts == 1 ? (size_t)n : (size_t)n * edge16[p + 1] / 16, m = c1 - c0;
         for (int j = 0; j < nd; ++j) {
@@ -904,7 +968,7 @@ int submit_host(gprm_space* h, int kind, const float* a, const float* b, int* re
         if (rc) return rc;
         CUDA_TRY(h, cudaMemcpyAsync(r.h_res + c0, r.d_res + c0, m * sizeof(int), cudaMemcpyDeviceToHost, r.st));
     }
-    if (n > 0)
+    if (n > 0 && !r.small)
         CUDA_TRY(h, cudaMemcpyAsync(r.ctl_host, r.ctl, parts * sizeof(Control), cudaMemcpyDeviceToHost, r.st));
     r.busy = true;
     r.kind = kind;
@@ -930,7 +994,7 @@ int complete_host(gprm_space* h, int slot)
     }
     if (c.flags & GPRM_DEVFLAG_BAD_EDGE)
         return fail(h, GPRM_ERR_ARG, "an edge has a non-finite or oversized length (|qe-qs|/dq >= 1e8)");
-    if (r.kind == 1) {
+    if (r.kind == 1 && !r.small) {
         static const int edge16[HOST_PARTS + 1] = {0, 1, 6, 11, 16};
         for (int p = 0; p < r.parts; ++p) {
             const long long m = r.parts == 1 ? r.n
@@ -1102,6 +1166,7 @@ int gprm_init(gprm_space* h, int rank, int size)
         const int rc = upload_certificates(h);
         if (rc) return rc;
     }
+    CUDA_TRY(h, configure_small(s, &h->small_smem));
     CUDA_TRY(h, plan_launch(s, 1, 128, &h->cfg_v));
     CUDA_TRY(h, plan_launch(s, 0, 128, &h->cfg_e));
     CUDA_TRY(h, dev_malloc((void**)&h->d_total, sizeof(Control)));

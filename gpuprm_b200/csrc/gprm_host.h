@@ -32,6 +32,7 @@ struct Request {
     Control* ctl = nullptr;       /* device, HOST_PARTS blocks (one per part) */
     Control* ctl_host = nullptr;  /* pinned copies read after the request */
     int parts = 1;                /* parts of the request in flight */
+    bool small = false;           /* run by the small-request kernels: ctl_host[0].flags is its status */
     float* d_a = nullptr;         /* q or qs (contiguous SoA, offset = n) */
     float* d_b = nullptr;         /* qe */
     int* d_res = nullptr;
@@ -109,6 +110,7 @@ struct gprm_space {
     void* d_scene = nullptr;
     gprm::DevScene dsc;
     gprm::LaunchCfg cfg_v, cfg_e;
+    size_t small_smem = 0;        /* shared bytes of a small request's block (0: not available) */
 
     int mode = GPRM_MODE_FP64_BAND;
     int policy = GPRM_EDGES_ALL_STEPS;

@@ -164,6 +164,18 @@ cudaError_t launch_check_edges(const DevScene& sc, const LaunchCfg& cfg, const f
                                unsigned* key, int band_on, float band, BandQueue bq,
                                Control* ctl, cudaStream_t st, unsigned* seg_off = nullptr, int seg_rounds = 0);
 
+/* Small requests in one launch each (k_configs_small, k_edges_small):
+ * checks, FP64 rechecks, results and counters (added to `total`).  Inputs,
+ * results and status may be pinned host memory.  per: configurations per
+ * block (1..32); segs: blocks per edge, with scratch = 2 n zeroed words when
+ * it is above 1.  smem: configure_small's bytes, not 0. */
+cudaError_t configure_small(const DevScene& sc, size_t* bytes);
+cudaError_t launch_configs_small(const DevScene& sc, size_t smem, const float* q, int n, long long offset, int per,
+                                 int* res, int band_on, float band, Control* total, cudaStream_t st);
+cudaError_t launch_edges_small(const DevScene& sc, size_t smem, const float* qs, const float* qe, int n, long long offset,
+                               float dq, int policy, int segs, int* res, unsigned* scratch, int band_on, float band,
+                               Control* total, unsigned* status, cudaStream_t st);
+
 /* FP64 recheck of queued vertex (kind 0) or edge-step (kind 1) items. */
 cudaError_t launch_recheck(const DevScene& sc, int blocks, int kind, const float* q, const float* qs,
                            const float* qe, long long offset, float dq, int policy, int* res,

@@ -283,9 +283,9 @@ __device__ __forceinline__ void sweep_mark(const int* swj, unsigned* bits, int g
  * warp's sweep balls: a pair whose ball centres are farther apart in every
  * lane than rho_P + rho_Q + sqrt(T2) is settled for all lanes at once (each
  * lane's exact distance then exceeds sqrt(T2)); else the direction test is
- * bounded over all lanes at once (swept_direction).  Leaves in S.defer the
- * pairs left for the lanes' own tests (bit j - g * SWEEP_GROUP), words of
- * them.
+ * bounded over all lanes at once (swept_direction).  Sets in S.defer the
+ * bits of the pairs left for the lanes' own tests (bit j - g *
+ * SWEEP_GROUP); share: the leaves of every 32 that this warp goes through.
  *
  * Two levels: lane l tests leaf l of the next 32 (32 pairs of one slot whose
  * static partners lie close together) by its ball, then the warp goes
@@ -297,7 +297,7 @@ __device__ __forceinline__ void sweep_mark(const int* swj, unsigned* bits, int g
  * wall scene (129 chunks of 32 pairs; 70,001 edges 27.7 -> 15.9 ms with the
  * leaves); on 64 obstacles (two leaves a slot) the leaf level costs what it
  * saves (62.1 -> 61.7 ms). */
-__device__ __forceinline__ void sweep_stage(const DevScene& sc, const SceneView& S, int g, int words)
+__device__ __forceinline__ void sweep_leaves(const DevScene& sc, const SceneView& S, int g, unsigned share)
 {
     const int lane = threadIdx.x & 31;
     /* the descriptor's fields in registers: a batch keeps it in shared
@@ -307,8 +307,6 @@ __device__ __forceinline__ void sweep_stage(const DevScene& sc, const SceneView&
     const float4 *swl = sc.swl, *swp = sc.swp, *swb = sc.swb, *sweep = S.sweep;
     const int* swj = sc.swj;
     unsigned* bits = S.defer;
-    for (int w = lane; w < words; w += 32) bits[w] = 0u;
-    __syncwarp();
     const int end = sc.swg[g + 1];
 #pragma unroll 1
     for (int l0 = sc.swg[g]; l0 < end; l0 += 32) {
@@ -320,7 +318,7 @@ __device__ __forceinline__ void sweep_stage(const DevScene& sc, const SceneView&
             open = swept_near(make_float4(r.x, r.y, r.z, 0.0f), sweep[w & 15], __int_as_float(w | 15), dx, dy, dz,
                               rc);
         }
-        unsigned left = __ballot_sync(FULL_MASK, open);
+        unsigned left = __ballot_sync(FULL_MASK, open) & share;
         if (!left) continue;
         /* two leaves side by side (the last one with itself: the bits are
            only ever set) */
@@ -342,6 +340,13 @@ __device__ __forceinline__ void sweep_stage(const DevScene& sc, const SceneView&
             left &= left - 1u;
         }
     }
+}
+
+__device__ __forceinline__ void sweep_stage(const DevScene& sc, const SceneView& S, int g, int words)
+{
+    for (int w = threadIdx.x & 31; w < words; w += 32) S.defer[w] = 0u;
+    __syncwarp();
+    sweep_leaves(sc, S, g, FULL_MASK);
     __syncwarp();
 }
 
@@ -1363,6 +1368,461 @@ __global__ void k_fk_probe(DevScene sc, const float* q, float* out)
         for (int c = 0; c < 12; ++c) out[f * 12 + c] = F[f].m[c];
 }
 
+/* ------------------------------------------------------------------ */
+/* small requests: a block per configuration or edge                    */
+/* ------------------------------------------------------------------ */
+/*
+ * A request of few items is bound by the latency of its longest chain, not
+ * by throughput: with a warp per 32 configurations or per edge most of the
+ * GPU idles, the exact tests of a warp run one after the other, the FP64
+ * recheck is a second launch in which one thread goes through a check's
+ * pairs, and control words, keys and results pass through eight more stream
+ * operations.  k_check_small runs the whole request in one launch: a block
+ * of four warps per configuration (up to 32 of them, one per lane, for
+ * larger requests) or per edge, whose rounds of 32 steps `segs` blocks
+ * share.  Per round warp 0 runs the forward kinematics and the sweep balls,
+ * the warps share the sweep stage's leaves and the open pairs' words, queue
+ * the exact tests that their lanes need and run them 32 at a time whoever
+ * they belong to; a step's first colliding pair is the minimum over the
+ * pairs that collide, so the tests need no order.  Steps decided in the
+ * band get their FP64 check at once, a warp per step with its pairs over
+ * the lanes.  Codes, bands and key merges are those of the kernels above.
+ */
+constexpr int SMALL_WARPS = 4;
+
+struct SmallShared {
+    unsigned jkey[32];            /* per lane: min over colliding pairs of j << 8 | in band << 4 | code + 1 */
+    unsigned jfirst[32];          /* first free pair with a margin inside the band */
+    int jlast[32];                /* last one */
+    unsigned queue[SMALL_WARPS][64];
+    float q[GPRM_MAX_FRAMES][32]; /* configurations: joint j of lane i */
+    Frame<double> F[SMALL_WARPS][GPRM_MAX_FRAMES];
+    Frame<double> L[SMALL_WARPS][GPRM_MAX_FRAMES];
+    double cen[SMALL_WARPS][GPRM_MAX_SLOTS * 3];
+    unsigned cut;                 /* what an out-of-band collision found so far makes needless (small_run) */
+    unsigned key;                 /* the edge's merged key (all steps: max, early exit: min) */
+    unsigned beaten;
+    unsigned full, checks, flips;
+};
+
+/* check_config64 by a warp, joint j's value in lane j: joint trigonometry a
+ * lane per joint, the frame products an entry per lane, the pairs of the
+ * range over the lanes, those that no certificate settles queued (64
+ * entries) and tested 32 at a time.  Same operations as check_config64, same
+ * code. */
+__device__ __forceinline__ int warp_check64(const DevScene& sc, Frame<double>* F, Frame<double>* L, double* cen,
+                                            unsigned* queue, float q, int j_start, int j_end)
+{
+    const int lane = threadIdx.x & 31;
+    if (j_end > sc.npairs) j_end = sc.npairs;
+    if (lane < sc.ndof) {
+        float th = sc.q0[lane], d = sc.d0[lane];
+        if (sc.types[lane] == 0) th = q;
+        else d = q;
+        double cq, sq, ca, sa;
+        PF64::trig(th, cq, sq);
+        PF64::trig_alpha(sc, lane, ca, sa);
+        dh_frame<PF64>(L[lane], cq, sq, ca, sa, (double)sc.a[lane], (double)d);
+    }
+    if (lane < 12) F[0].m[lane] = lane % 4 == 0 && lane < 9 ? 1.0 : (lane == 3 || lane == 7 || lane == 10 ? -0.0 : 0.0);
+    __syncwarp();
+    const int c = lane / 3, r = lane - 3 * c;
+#pragma unroll 1
+    for (int i = 0; i < sc.ndof; ++i) {
+        if (lane < 12) {
+            const double* T = F[i].m;
+            const double* u = L[i].m + 3 * c;
+            double o = T[r] * u[0] + T[3 + r] * u[1] + T[6 + r] * u[2];
+            if (c == 3) o = o + T[9 + r];
+            F[i + 1].m[lane] = o;
+        }
+        __syncwarp();
+    }
+    if (lane < sc.nslots) {
+        const float4 b = sc.tab[sc.slot_block[lane]];
+        const V3<double> w = xform<double>(F[sc.slot_sys[lane]], (double)b.x, (double)b.y, (double)b.z);
+        cen[3 * lane] = w.x; cen[3 * lane + 1] = w.y; cen[3 * lane + 2] = w.z;
+    }
+    __syncwarp();
+    int code = 0, n = 0;
+#pragma unroll 1
+    for (int j0 = j_start; j0 < j_end || n > 0; j0 += 32) {
+        const int j = j0 + lane;
+        bool open = false;
+        if (j < j_end) open = !pair_certified64(sc, sc.tab, sc.pairs[j], sc.pairs_b[j], F, cen, j);
+        const unsigned m = __ballot_sync(FULL_MASK, open);
+        if (open) queue[n + __popc(m & ((1u << lane) - 1u))] = (unsigned)j;
+        n += __popc(m);
+        __syncwarp();
+        if (n < 32 && j0 + 32 < j_end) continue;
+        /* the first 32 open pairs side by side, in order */
+        int rr = 0;
+        if (lane < n) {
+            const int4 pr = sc.pairs[queue[lane]];
+            double mg;
+            rr = pair_test<PF64>(sc, sc.tab, pr, F[pr.z], F[pr.w], &mg);
+        }
+        const unsigned hit = __ballot_sync(FULL_MASK, rr != 0);
+        if (hit) {
+            code = __shfl_sync(FULL_MASK, rr, __ffs(hit) - 1);
+            break;
+        }
+        const unsigned mv = lane + 32 < n ? queue[32 + lane] : 0u;
+        __syncwarp();
+        if (lane + 32 < n) queue[lane] = mv;
+        n = n > 32 ? n - 32 : 0;
+        __syncwarp();
+    }
+    __syncwarp();
+    return code;
+}
+
+/* What B.cut holds of a lane's collision outside the band at pair j. */
+enum SmallCut { CUT_NONE, CUT_LANE, CUT_PAIR };
+template <int CUT>
+__device__ __forceinline__ unsigned small_cut(int lane, int j)
+{
+    return CUT == CUT_LANE ? (unsigned)lane : (unsigned)j;
+}
+
+/* Runs the first cnt (<= 32) of the warp's queued tests (lane | pair << 5),
+ * one per lane on its owner's frames, and merges their results.  Left out:
+ * pairs after one that the owner already collides at, and, with a cut (the
+ * lowest lane, or the first pair, with a collision outside the band so far),
+ * the lanes or pairs beyond it, which cannot change the round's decision as
+ * long as that collision stands (the caller checks that it does). */
+template <bool FAST, int CUT>
+__device__ __forceinline__ void small_run(const DevScene& sc, const SceneView& S, SmallShared& B, unsigned* q, int cnt,
+                                          bool cutting, int band_on, float band)
+{
+    const int lane = threadIdx.x & 31;
+    __syncwarp();
+    const unsigned it = q[lane];
+    const int owner = (int)(it & 31u), j = (int)(it >> 5);
+    bool run = lane < cnt && ((unsigned)j << 8) <= *(volatile unsigned*)&B.jkey[owner];
+    if (CUT != CUT_NONE && cutting) run = run && small_cut<CUT>(owner, j) <= *(volatile unsigned*)&B.cut;
+    if (run) {
+        const int4 pr = S.pairs[j];
+        Frame<float> tp, tq;
+        pair_frames(S.frames - lane + owner, pr, tp, tq);
+        float m;
+        int c;
+        if constexpr (FAST) c = pair_test_fast(sc, S.tab, pr, sc.ppoly[j], tp, tq, &m);
+        else c = pair_test<PF32>(sc, S.tab, pr, tp, tq, &m);
+        if (c != 0) {
+            const unsigned inb = band_on && in_band(c, m, band) ? 16u : 0u;
+            atomicMin(&B.jkey[owner], ((unsigned)j << 8) | inb | (unsigned)(c + 1));
+            if (CUT != CUT_NONE && !inb) atomicMin(&B.cut, small_cut<CUT>(owner, j));
+        } else if (!(m >= band)) {
+            atomicMin(&B.jfirst[owner], (unsigned)j);
+            atomicMax(&B.jlast[owner], j);
+        }
+    }
+    const unsigned ran = __ballot_sync(FULL_MASK, run);
+    if (lane == 0 && ran) atomicAdd(&B.full, (unsigned)__popc(ran));
+}
+
+/* Certificates and exact tests of one round for the lanes of `valid` (their
+ * frames in S, ready to read by the block): fills jkey, jfirst and jlast.
+ * Every thread of the block calls it; ends with a block barrier. */
+template <bool FAST, int CUT>
+__device__ __forceinline__ void small_pairs(const DevScene& sc, const SceneView& S, SmallShared& B, unsigned valid,
+                                            bool cutting, int band_on, float band)
+{
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool mine = (valid >> lane) & 1u;
+    unsigned* q = B.queue[warp];
+    PairCounts pc = {0, 0};
+    int n = 0;
+#pragma unroll 1
+    for (int g0 = 0; g0 < sc.npairs; g0 += SWEEP_GROUP) {
+        const int words = (min(sc.npairs - g0, SWEEP_GROUP) + 31) >> 5;
+        for (int w = threadIdx.x; w < words; w += SMALL_WARPS * 32) S.defer[w] = 0u;
+        __syncthreads();
+        sweep_leaves(sc, S, g0 / SWEEP_GROUP, 0x11111111u << warp);
+        __syncthreads();
+#pragma unroll 1
+        for (int w = warp; w < words; w += SMALL_WARPS) {
+            const unsigned cand = S.defer[w];
+            if (!cand) continue;
+            const int j0 = g0 + 32 * w;
+            bool scan = mine && ((unsigned)j0 << 8) <= *(volatile unsigned*)&B.jkey[lane];
+            if (CUT != CUT_NONE && cutting) scan = scan && small_cut<CUT>(lane, j0) <= *(volatile unsigned*)&B.cut;
+            const unsigned need = scan ? lane_scan(sc, S, j0, cand, pc) : 0u;
+            unsigned todo = __reduce_or_sync(FULL_MASK, need);
+            while (todo) {
+                const int k = __ffs(todo) - 1;
+                todo &= todo - 1u;
+                const unsigned m = __ballot_sync(FULL_MASK, (need >> k) & 1u);
+                if ((need >> k) & 1u) q[n + __popc(m & ((1u << lane) - 1u))] = (unsigned)lane | ((unsigned)(j0 + k) << 5);
+                n += __popc(m);
+                if (n >= 32) {
+                    small_run<FAST, CUT>(sc, S, B, q, 32, cutting, band_on, band);
+                    n -= 32;
+                    const unsigned mv = lane < n ? q[32 + lane] : 0u;
+                    __syncwarp();
+                    if (lane < n) q[lane] = mv;
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (n > 0) small_run<FAST, CUT>(sc, S, B, q, n, cutting, band_on, band);
+    __syncthreads();
+}
+
+/* The view of the block's one set of frames for this thread's lane. */
+__device__ __forceinline__ SceneView small_view(const DevScene& sc, unsigned char* smem)
+{
+    SceneView S;
+    S.tab = sc.tab; S.pairs = sc.pairs; S.pairs_b = sc.pairs_b;
+    S.far = sc.far; S.scan_c = sc.scan_c; S.scan_b = sc.scan_b;
+    S.frames = reinterpret_cast<float*>(smem) + (threadIdx.x & 31);
+    S.cen = S.frames + (size_t)sc.ndof * 12 * 32;
+    S.sweep = sweep_area<false>(sc, S.frames);
+    S.defer = defer_area<false>(sc, S.frames);
+    return S;
+}
+
+__device__ __forceinline__ void small_reset(SmallShared& B)
+{
+    if (threadIdx.x < 32) {
+        B.jkey[threadIdx.x] = 0xffffffffu;
+        B.jfirst[threadIdx.x] = 0x7fffffffu;
+        B.jlast[threadIdx.x] = -1;
+    }
+    if (threadIdx.x == 32) B.cut = 0xffffffffu;
+}
+
+/* Configurations: block b checks items b * per .. b * per + per - 1 (per <=
+ * 32), one per lane. */
+template <bool FAST>
+__global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_configs_small(DevScene sc, const float* __restrict__ q, int n,
+                                                                       long long offset, int per, int* __restrict__ res,
+                                                                       int band_on, float band, Control* total)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ SmallShared B;
+    const SceneView S = small_view(sc, smem);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int i0 = blockIdx.x * per, count = min(per, n - i0);
+    small_reset(B);
+    if (threadIdx.x == 0) B.full = B.checks = B.flips = 0u;
+    for (int t = threadIdx.x; t < sc.ndof * 32; t += blockDim.x) {
+        const int j = t >> 5, i = t & 31;
+        if (i < count) B.q[j][i] = q[i0 + i + offset * j];
+    }
+    __syncthreads();
+    /* check_boundaries(q) (robotconfigspace.cpp:795-802) */
+    bool in = lane < count;
+    if (in)
+#pragma unroll 1
+        for (int j = 0; j < sc.ndof; ++j) {
+            const float x = B.q[j][lane];
+            if (x < sc.mins[j] || x > sc.maxs[j]) in = false;
+        }
+    const unsigned valid = __ballot_sync(FULL_MASK, in);
+    int code = lane < count && !in ? 1 : 0;
+    bool want = false;
+    if (valid) {
+        if (warp == 0) {
+            /* the other lanes repeat a valid one, so that the sweep balls hold no more */
+            const int src = in ? lane : __ffs(valid) - 1;
+            lane_fk<FAST>(sc, S, [&](int j) { return B.q[j][src]; });
+            sweep_bounds(sc, S);
+        }
+        small_pairs<FAST, CUT_NONE>(sc, S, B, valid, false, band_on, band);
+        if (in) {
+            const unsigned jk = B.jkey[lane];
+            if (jk != 0xffffffffu) {
+                code = (int)(jk & 15u) - 1;
+                want = (jk & 16u) != 0u;
+            } else {
+                want = band_on && B.jfirst[lane] != 0x7fffffffu;
+            }
+        }
+        unsigned todo = __ballot_sync(FULL_MASK, want);
+        for (int w = 0; todo; ++w) {
+            const int i = __ffs(todo) - 1;
+            todo &= todo - 1u;
+            if (w % SMALL_WARPS != warp) continue;
+            const unsigned jk = B.jkey[i];
+            const bool coll = jk != 0xffffffffu;
+            const int lo = (int)min(B.jfirst[i], jk >> 8), hi = coll ? sc.npairs : B.jlast[i] + 1;
+            const int c64 = warp_check64(sc, B.F[warp], B.L[warp], B.cen[warp], B.queue[warp],
+                                         lane < sc.ndof ? B.q[lane][i] : 0.0f, lo, hi);
+            if (lane == i) {
+                atomicAdd(&B.checks, 1u);
+                if ((c64 != 0) != (code != 0)) atomicAdd(&B.flips, 1u);
+                res[i0 + i] = c64;
+            }
+        }
+    }
+    if (warp == 0 && lane < count && !want) res[i0 + lane] = code;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const unsigned done = (unsigned)__popc(valid);
+        atomicAdd(&total->configs_exec, (unsigned long long)done);
+        atomicAdd(&total->certified, (unsigned long long)done * (unsigned)sc.npairs - B.full);
+        if (B.full) atomicAdd(&total->full_tests, (unsigned long long)B.full);
+        if (B.checks) atomicAdd(&total->band_checks, (unsigned long long)B.checks);
+        if (B.flips) atomicAdd(&total->band_flips, (unsigned long long)B.flips);
+    }
+}
+
+/* Edges: block (e, s) of n * segs checks rounds s, s + segs, ... of edge e.
+ * With segs > 1 scratch (2 n zeroed words) holds the edges' merged keys and
+ * counts their finished blocks, the last of which writes the code.  status:
+ * gets GPRM_DEVFLAG_BAD_EDGE for a non-finite or oversized edge (or null). */
+template <int POLICY, bool FAST>
+__global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_edges_small(DevScene sc, const float* __restrict__ qs,
+                                                                     const float* __restrict__ qe, int n,
+                                                                     long long offset, float dq, int segs,
+                                                                     int* __restrict__ res, unsigned* scratch,
+                                                                     int band_on, float band, Control* total,
+                                                                     volatile unsigned* status)
+{
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ SmallShared B;
+    const SceneView S = small_view(sc, smem);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int e = blockIdx.x / segs, s = blockIdx.x - e * segs;
+    constexpr unsigned NONE = POLICY == EDGE_EARLY_EXIT ? 0xffffffffu : 0u;
+    float ends = 0.0f;
+    if ((lane & 15) < sc.ndof) ends = (lane < 16 ? qs : qe)[e + offset * (lane & 15)];
+    /* edge_testnum */
+    float norm = 0.0f;
+#pragma unroll 1
+    for (int j = 0; j < sc.ndof; ++j) {
+        const float diff = __shfl_sync(FULL_MASK, ends, 16 + j) - __shfl_sync(FULL_MASK, ends, j);
+        norm = norm + diff * diff;
+    }
+    const float x = __fsqrt_rn(norm) / dq;
+    const int tn = x < 1.0e8f ? (int)x + 1 : -1;
+    const int R = (tn + 31) >> 5;      /* no round for a rejected edge */
+    if (threadIdx.x == 0) {
+        B.key = NONE;
+        B.full = B.checks = B.flips = 0u;
+    }
+    unsigned exec = 0;
+#pragma unroll 1
+    for (int r = s; r < R; r += segs) {
+        if (segs > 1) {
+            /* a decision that no step of this round or a later one improves on */
+            if (threadIdx.x == 0) {
+                unsigned kv = *(volatile unsigned*)&scratch[e];
+                if (POLICY == EDGE_EARLY_EXIT) kv = ~kv;
+                B.beaten = kv == NONE ? 0u
+                    : (POLICY == EDGE_EARLY_EXIT) ? (kv >> 4) < (unsigned)(r * 32) : (int)(kv >> 4) - 1 > tn - 1 - r * 32;
+            }
+            __syncthreads();
+            if (B.beaten) break;
+        }
+        int t;
+        bool in;
+        if (POLICY == EDGE_EARLY_EXIT) {
+            const int last = (tn - 1 - r) / R;
+            in = lane <= last;
+            t = (in ? lane : last) * R + r;
+        } else {
+            t = tn - 1 - (r * 32 + lane);
+            in = t >= 0;
+            if (!in) t = 0;
+        }
+        const float c1 = (float)t / (float)(tn - 1), c2 = 1.0f - c1;   /* as edge_step_config */
+        const unsigned valid = __ballot_sync(FULL_MASK, in);
+        if (warp == 0) {
+            lane_fk<FAST>(sc, S, [&](int j) {
+                return c1 * __shfl_sync(FULL_MASK, ends, j) + c2 * __shfl_sync(FULL_MASK, ends, 16 + j);
+            });
+            sweep_bounds(sc, S);
+        }
+        exec += (unsigned)__popc(valid);
+        /* settle the round as check_edge does; where the collision that the
+           tests were cut by turned out to be decided by an earlier pair
+           inside the band, go through the round again without the cut */
+        unsigned jk;
+        int code, L, jstar;
+        bool oob;
+#pragma unroll 1
+        for (bool cutting = true;; cutting = false) {
+            small_reset(B);
+            small_pairs<FAST, POLICY == EDGE_EARLY_EXIT ? CUT_PAIR : CUT_LANE>(sc, S, B, valid, cutting, band_on, band);
+            jk = B.jkey[lane];
+            code = jk == 0xffffffffu ? 0 : (int)(jk & 15u) - 1;
+            oob = in && code != 0 && !(jk & 16u);
+            L = 32;
+            jstar = 0x7fffffff;
+            if (POLICY == EDGE_EARLY_EXIT)
+                jstar = (int)__reduce_min_sync(FULL_MASK, oob ? jk >> 8 : 0x7fffffffu);
+            const unsigned hits = __ballot_sync(FULL_MASK, oob && (POLICY != EDGE_EARLY_EXIT || (int)(jk >> 8) == jstar));
+            if (hits) L = __ffs(hits) - 1;
+            const unsigned stands = !hits ? 0xffffffffu : POLICY == EDGE_EARLY_EXIT ? (unsigned)jstar : (unsigned)L;
+            if (!cutting || B.cut == stands) break;
+            __syncthreads();
+        }
+        bool want = band_on && in && lane < L;
+        if (code != 0) want = want && !oob && (POLICY != EDGE_EARLY_EXIT || (int)(jk >> 8) <= jstar);
+        else want = want && B.jfirst[lane] != 0x7fffffffu &&
+                    (POLICY != EDGE_EARLY_EXIT || L == 32 || jstar == sc.npairs - 1);
+        if (warp == 0 && lane == L) {
+            if (POLICY == EDGE_EARLY_EXIT) atomicMin(&B.key, early_key((unsigned)(r * 32 + lane), code));
+            else atomicMax(&B.key, all_key(t, code));
+        }
+        unsigned todo = __ballot_sync(FULL_MASK, want);
+        for (int w = 0; todo; ++w) {
+            const int i = __ffs(todo) - 1;
+            todo &= todo - 1u;
+            if (w % SMALL_WARPS != warp) continue;
+            const unsigned ik = B.jkey[i];
+            const int lo = (int)min(B.jfirst[i], ik >> 8), hi = ik != 0xffffffffu ? sc.npairs : B.jlast[i] + 1;
+            const float d1 = __shfl_sync(FULL_MASK, c1, i), d2 = __shfl_sync(FULL_MASK, c2, i);
+            const float q = d1 * __shfl_sync(FULL_MASK, ends, lane & 15) + d2 * __shfl_sync(FULL_MASK, ends, 16 + (lane & 15));
+            const int c64 = warp_check64(sc, B.F[warp], B.L[warp], B.cen[warp], B.queue[warp], q, lo, hi);
+            if (lane == i) {
+                atomicAdd(&B.checks, 1u);
+                if ((c64 != 0) != (code != 0)) atomicAdd(&B.flips, 1u);
+                if (c64 != 0) {
+                    if (POLICY == EDGE_EARLY_EXIT) atomicMin(&B.key, early_key((unsigned)(r * 32 + i), c64));
+                    else atomicMax(&B.key, all_key(t, c64));
+                }
+            }
+        }
+        __syncthreads();
+        if (L < 32) break;
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    unsigned key = B.key;
+    bool write = true;
+    if (segs > 1) {
+        /* zeroed words: the larger is the better for both policies */
+        if (key != NONE) atomicMax(&scratch[e], POLICY == EDGE_EARLY_EXIT ? ~key : key);
+        __threadfence();
+        write = atomicAdd(&scratch[n + e], 1u) == (unsigned)segs - 1u;
+        if (write) {
+            __threadfence();
+            key = *(volatile unsigned*)&scratch[e];
+            if (POLICY == EDGE_EARLY_EXIT) key = ~key;
+        }
+    }
+    if (write) res[e] = key == NONE ? 0 : (int)(key & 15u) - 1;
+    if (s == 0) {
+        if (tn >= 0) atomicAdd(&total->steps_nominal, (unsigned long long)tn);
+        else {
+            atomicOr(&total->flags, GPRM_DEVFLAG_BAD_EDGE);
+            if (status) *status = GPRM_DEVFLAG_BAD_EDGE;
+        }
+    }
+    if (exec) {
+        atomicAdd(&total->steps_exec, (unsigned long long)exec);
+        atomicAdd(&total->certified, (unsigned long long)exec * (unsigned)sc.npairs - B.full);
+    }
+    if (B.full) atomicAdd(&total->full_tests, (unsigned long long)B.full);
+    if (B.checks) atomicAdd(&total->band_checks, (unsigned long long)B.checks);
+    if (B.flips) atomicAdd(&total->band_flips, (unsigned long long)B.flips);
+}
+
 /* Marks (SCAN_SETTLED) the pairs whose polytopes are both in frame 0 and
  * whose certificate holds: it is the same for every configuration, so the
  * checks need not evaluate it again.  A robot with a base link has one such
@@ -1628,6 +2088,56 @@ cudaError_t launch_finalize_edges(long long n, int policy, const unsigned* key, 
     return cudaGetLastError();
 }
 
+
+/* Opens the dynamic shared-memory cap of the small-request kernels for the
+ * scene's frames; *bytes gets one block's, 0 where they do not fit. */
+cudaError_t configure_small(const DevScene& sc, size_t* bytes)
+{
+    *bytes = 0;
+    int dev = 0, optin = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err != cudaSuccess) return err;
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    const size_t need = lane_floats(sc, false) * 32 * sizeof(float);
+    const void* fns[6] = {(const void*)k_configs_small<false>, (const void*)k_configs_small<true>,
+                          (const void*)k_edges_small<EDGE_ALL_STEPS, false>,
+                          (const void*)k_edges_small<EDGE_ALL_STEPS, true>,
+                          (const void*)k_edges_small<EDGE_EARLY_EXIT, false>,
+                          (const void*)k_edges_small<EDGE_EARLY_EXIT, true>};
+    for (const void* fn : fns) {
+        err = open_smem_cap(fn, optin, need);
+        if (err != cudaSuccess) {
+            cudaGetLastError();
+            return err == cudaErrorInvalidValue ? cudaSuccess : err;
+        }
+    }
+    *bytes = need;
+    return cudaSuccess;
+}
+
+cudaError_t launch_configs_small(const DevScene& sc, size_t smem, const float* q, int n, long long offset, int per,
+                                 int* res, int band_on, float band, Control* total, cudaStream_t st)
+{
+    const int blocks = (n + per - 1) / per;
+    if (sc.fast)
+        k_configs_small<true><<<blocks, SMALL_WARPS * 32, smem, st>>>(sc, q, n, offset, per, res, band_on, band, total);
+    else
+        k_configs_small<false><<<blocks, SMALL_WARPS * 32, smem, st>>>(sc, q, n, offset, per, res, band_on, band, total);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_edges_small(const DevScene& sc, size_t smem, const float* qs, const float* qe, int n, long long offset,
+                               float dq, int policy, int segs, int* res, unsigned* scratch, int band_on, float band,
+                               Control* total, unsigned* status, cudaStream_t st)
+{
+#define GPRM_SMALL_LAUNCH(POL_, FAST_)                                                                            \
+    k_edges_small<POL_, FAST_><<<n * segs, SMALL_WARPS * 32, smem, st>>>(sc, qs, qe, n, offset, dq, segs, res, scratch, \
+                                                                        band_on, band, total, status)
+    if (policy == EDGE_EARLY_EXIT) { if (sc.fast) GPRM_SMALL_LAUNCH(EDGE_EARLY_EXIT, true); else GPRM_SMALL_LAUNCH(EDGE_EARLY_EXIT, false); }
+    else { if (sc.fast) GPRM_SMALL_LAUNCH(EDGE_ALL_STEPS, true); else GPRM_SMALL_LAUNCH(EDGE_ALL_STEPS, false); }
+#undef GPRM_SMALL_LAUNCH
+    return cudaGetLastError();
+}
 
 /* ------------------------------------------------------------------ */
 /* many problems in one launch                                          */
