@@ -1290,9 +1290,93 @@ __device__ __forceinline__ void overflow_item(const DevScene& sc, int kind, unsi
     key[x] = k;
 }
 
-/* The FP64 recheck of the queued items, one thread per item.  (A warp per
- * item, the pairs spread over the lanes, ran 1.4x slower on the hull6
- * edge workload: the items' own parallelism hides the FP64 latency better.) */
+/* check_config64 by a warp, joint j's value in lane j: joint trigonometry a
+ * lane per joint, the frame products an entry per lane, the pairs of the
+ * range over the lanes, those that no certificate settles queued (64
+ * entries) and tested 32 at a time.  Same operations as check_config64, same
+ * code. */
+__device__ __forceinline__ int warp_check64(const DevScene& sc, Frame<double>* F, Frame<double>* L, double* cen,
+                                            unsigned* queue, float q, int j_start, int j_end)
+{
+    const int lane = threadIdx.x & 31;
+    if (j_end > sc.npairs) j_end = sc.npairs;
+    if (lane < sc.ndof) {
+        float th = sc.q0[lane], d = sc.d0[lane];
+        if (sc.types[lane] == 0) th = q;
+        else d = q;
+        double cq, sq, ca, sa;
+        PF64::trig(th, cq, sq);
+        PF64::trig_alpha(sc, lane, ca, sa);
+        dh_frame<PF64>(L[lane], cq, sq, ca, sa, (double)sc.a[lane], (double)d);
+    }
+    if (lane < 12) F[0].m[lane] = lane % 4 == 0 && lane < 9 ? 1.0 : (lane == 3 || lane == 7 || lane == 10 ? -0.0 : 0.0);
+    __syncwarp();
+    const int c = lane / 3, r = lane - 3 * c;
+#pragma unroll 1
+    for (int i = 0; i < sc.ndof; ++i) {
+        if (lane < 12) {
+            const double* T = F[i].m;
+            const double* u = L[i].m + 3 * c;
+            double o = T[r] * u[0] + T[3 + r] * u[1] + T[6 + r] * u[2];
+            if (c == 3) o = o + T[9 + r];
+            F[i + 1].m[lane] = o;
+        }
+        __syncwarp();
+    }
+    if (lane < sc.nslots) {
+        const float4 b = sc.tab[sc.slot_block[lane]];
+        const V3<double> w = xform<double>(F[sc.slot_sys[lane]], (double)b.x, (double)b.y, (double)b.z);
+        cen[3 * lane] = w.x; cen[3 * lane + 1] = w.y; cen[3 * lane + 2] = w.z;
+    }
+    __syncwarp();
+    int code = 0, n = 0;
+#pragma unroll 1
+    for (int j0 = j_start; j0 < j_end || n > 0; j0 += 32) {
+        const int j = j0 + lane;
+        bool open = false;
+        if (j < j_end) open = !pair_certified64(sc, sc.tab, sc.pairs[j], sc.pairs_b[j], F, cen, j);
+        const unsigned m = __ballot_sync(FULL_MASK, open);
+        if (open) queue[n + __popc(m & ((1u << lane) - 1u))] = (unsigned)j;
+        n += __popc(m);
+        __syncwarp();
+        if (n < 32 && j0 + 32 < j_end) continue;
+        /* the first 32 open pairs side by side, in order */
+        int rr = 0;
+        if (lane < n) {
+            const int4 pr = sc.pairs[queue[lane]];
+            double mg;
+            rr = pair_test<PF64>(sc, sc.tab, pr, F[pr.z], F[pr.w], &mg);
+        }
+        const unsigned hit = __ballot_sync(FULL_MASK, rr != 0);
+        if (hit) {
+            code = __shfl_sync(FULL_MASK, rr, __ffs(hit) - 1);
+            break;
+        }
+        const unsigned mv = lane + 32 < n ? queue[32 + lane] : 0u;
+        __syncwarp();
+        if (lane + 32 < n) queue[lane] = mv;
+        n = n > 32 ? n - 32 : 0;
+        __syncwarp();
+    }
+    __syncwarp();
+    return code;
+}
+
+/* The FP64 recheck of the queued items: one thread per item, or, for few
+ * items, one warp per item with its pairs over the lanes (warp_check64).
+ * With many items their own parallelism hides the FP64 latency better; with
+ * few, the longest item's chain of pairs is the kernel's time, so what
+ * counts as few grows with the pair list.  Measured (thread per item ->
+ * warp per item): 1 item per resident warp, 4117 pairs (vertex checks of
+ * the wall scene) 1.7 -> 0.35 ms; 59 per warp, 4117 pairs (its edges) 3.0 ->
+ * 1.8 ms; 10 per warp, 394 pairs (hull6 vertices) 0.34 -> 0.54 ms; 27 per
+ * warp, 394 pairs (exact hull6 edges) 1.1 -> 3.0 ms. */
+constexpr unsigned RECHECK_FEW = 4;
+__device__ __forceinline__ bool recheck_by_warp(unsigned items, unsigned warps, int npairs)
+{
+    const unsigned few = RECHECK_FEW * (npairs > 512 ? (unsigned)npairs >> 8 : 1u);
+    return (unsigned long long)items <= (unsigned long long)few * warps;
+}
 constexpr int RECHECK_THREADS = 128;
 
 __device__ __forceinline__ void recheck_item(const DevScene& sc, int kind, uint2 it, const float* __restrict__ q,
@@ -1310,6 +1394,41 @@ __device__ __forceinline__ void recheck_item(const DevScene& sc, int kind, uint2
     recheck_store(kind, it, code, t, tn, policy, res, key);
 }
 
+/* Shared memory of a warp's item (warp_check64). */
+struct Warp64 {
+    Frame<double> F[GPRM_MAX_FRAMES], L[GPRM_MAX_FRAMES];
+    double cen[GPRM_MAX_SLOTS * 3];
+    unsigned queue[64];
+};
+
+/* recheck_item by a warp; lane 0 counts and stores. */
+__device__ __forceinline__ void recheck_item_warp(const DevScene& sc, int kind, uint2 it, const float* __restrict__ q,
+                                                  const float* __restrict__ qs, const float* __restrict__ qe,
+                                                  long long offset, float dq, int policy, int* __restrict__ res,
+                                                  unsigned* __restrict__ key, unsigned long long& checks,
+                                                  unsigned long long& flips, unsigned range, Warp64& W)
+{
+    const int lane = threadIdx.x & 31;
+    int t = 0, tn = 0;
+    float x = 0.0f;
+    if (kind == 0) {
+        if (lane < sc.ndof) x = q[(long long)it.x + offset * lane];
+    } else {
+        /* as recheck_config: joint j in lane j */
+        t = (int)(it.y & ((1u << 27) - 1));
+        tn = edge_testnum(qs, qe, (long long)it.x, offset, sc.ndof, dq);
+        const float c1 = (float)t / (float)(tn - 1), c2 = 1.0f - c1;
+        if (lane < sc.ndof)
+            x = c1 * qs[(long long)it.x + offset * lane] + c2 * qe[(long long)it.x + offset * lane];
+    }
+    const int code = warp_check64(sc, W.F, W.L, W.cen, W.queue, x, (int)(range & 0xffffu), (int)(range >> 16));
+    if (lane == 0) {
+        ++checks;
+        flips += ((code != 0) != ((int)(it.y >> 27) - 1 != 0));
+        recheck_store(kind, it, code, t, tn, policy, res, key);
+    }
+}
+
 __global__ void __launch_bounds__(RECHECK_THREADS) k_recheck(DevScene sc, int kind, const float* __restrict__ q,
                                                              const float* __restrict__ qs,
                                                              const float* __restrict__ qe, long long offset,
@@ -1317,12 +1436,20 @@ __global__ void __launch_bounds__(RECHECK_THREADS) k_recheck(DevScene sc, int ki
                                                              unsigned* __restrict__ key, const BandQueue bq,
                                                              Control* ctl)
 {
+    __shared__ Warp64 W[RECHECK_THREADS / 32];
     unsigned cnt = ctl->qcount;
     if (cnt > bq.cap) cnt = bq.cap;
     unsigned long long checks = 0, flips = 0;
-    for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < cnt; idx += gridDim.x * blockDim.x)
-        recheck_item(sc, kind, bq.items[idx], q, qs, qe, offset, dq, policy, res, key, checks, flips,
-                     bq.pair_range ? bq.pair_range[idx] : 0xffff0000u);
+    const unsigned warps = gridDim.x * (RECHECK_THREADS / 32), warp = threadIdx.x >> 5;
+    if (recheck_by_warp(cnt, warps, sc.npairs)) {
+        for (unsigned idx = warp * gridDim.x + blockIdx.x; idx < cnt; idx += warps)
+            recheck_item_warp(sc, kind, bq.items[idx], q, qs, qe, offset, dq, policy, res, key, checks, flips,
+                              bq.pair_range ? bq.pair_range[idx] : 0xffff0000u, W[warp]);
+    } else {
+        for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < cnt; idx += gridDim.x * blockDim.x)
+            recheck_item(sc, kind, bq.items[idx], q, qs, qe, offset, dq, policy, res, key, checks, flips,
+                         bq.pair_range ? bq.pair_range[idx] : 0xffff0000u);
+    }
     if (checks) atomicAdd(&ctl->band_checks, checks);
     if (flips) atomicAdd(&ctl->band_flips, flips);
 }
@@ -1404,78 +1531,6 @@ struct SmallShared {
     unsigned beaten;
     unsigned full, checks, flips;
 };
-
-/* check_config64 by a warp, joint j's value in lane j: joint trigonometry a
- * lane per joint, the frame products an entry per lane, the pairs of the
- * range over the lanes, those that no certificate settles queued (64
- * entries) and tested 32 at a time.  Same operations as check_config64, same
- * code. */
-__device__ __forceinline__ int warp_check64(const DevScene& sc, Frame<double>* F, Frame<double>* L, double* cen,
-                                            unsigned* queue, float q, int j_start, int j_end)
-{
-    const int lane = threadIdx.x & 31;
-    if (j_end > sc.npairs) j_end = sc.npairs;
-    if (lane < sc.ndof) {
-        float th = sc.q0[lane], d = sc.d0[lane];
-        if (sc.types[lane] == 0) th = q;
-        else d = q;
-        double cq, sq, ca, sa;
-        PF64::trig(th, cq, sq);
-        PF64::trig_alpha(sc, lane, ca, sa);
-        dh_frame<PF64>(L[lane], cq, sq, ca, sa, (double)sc.a[lane], (double)d);
-    }
-    if (lane < 12) F[0].m[lane] = lane % 4 == 0 && lane < 9 ? 1.0 : (lane == 3 || lane == 7 || lane == 10 ? -0.0 : 0.0);
-    __syncwarp();
-    const int c = lane / 3, r = lane - 3 * c;
-#pragma unroll 1
-    for (int i = 0; i < sc.ndof; ++i) {
-        if (lane < 12) {
-            const double* T = F[i].m;
-            const double* u = L[i].m + 3 * c;
-            double o = T[r] * u[0] + T[3 + r] * u[1] + T[6 + r] * u[2];
-            if (c == 3) o = o + T[9 + r];
-            F[i + 1].m[lane] = o;
-        }
-        __syncwarp();
-    }
-    if (lane < sc.nslots) {
-        const float4 b = sc.tab[sc.slot_block[lane]];
-        const V3<double> w = xform<double>(F[sc.slot_sys[lane]], (double)b.x, (double)b.y, (double)b.z);
-        cen[3 * lane] = w.x; cen[3 * lane + 1] = w.y; cen[3 * lane + 2] = w.z;
-    }
-    __syncwarp();
-    int code = 0, n = 0;
-#pragma unroll 1
-    for (int j0 = j_start; j0 < j_end || n > 0; j0 += 32) {
-        const int j = j0 + lane;
-        bool open = false;
-        if (j < j_end) open = !pair_certified64(sc, sc.tab, sc.pairs[j], sc.pairs_b[j], F, cen, j);
-        const unsigned m = __ballot_sync(FULL_MASK, open);
-        if (open) queue[n + __popc(m & ((1u << lane) - 1u))] = (unsigned)j;
-        n += __popc(m);
-        __syncwarp();
-        if (n < 32 && j0 + 32 < j_end) continue;
-        /* the first 32 open pairs side by side, in order */
-        int rr = 0;
-        if (lane < n) {
-            const int4 pr = sc.pairs[queue[lane]];
-            double mg;
-            rr = pair_test<PF64>(sc, sc.tab, pr, F[pr.z], F[pr.w], &mg);
-        }
-        const unsigned hit = __ballot_sync(FULL_MASK, rr != 0);
-        if (hit) {
-            code = __shfl_sync(FULL_MASK, rr, __ffs(hit) - 1);
-            break;
-        }
-        const unsigned mv = lane + 32 < n ? queue[32 + lane] : 0u;
-        __syncwarp();
-        if (lane + 32 < n) queue[lane] = mv;
-        n = n > 32 ? n - 32 : 0;
-        __syncwarp();
-    }
-    __syncwarp();
-    return code;
-}
 
 /* What B.cut holds of a lane's collision outside the band at pair j. */
 enum SmallCut { CUT_NONE, CUT_LANE, CUT_PAIR };
@@ -2259,6 +2314,17 @@ __global__ void __launch_bounds__(RECHECK_THREADS) k_recheck_multi(BatchView B, 
     unsigned cnt = ctl->qcount;
     if (cnt > bq.cap) cnt = bq.cap;
     unsigned long long checks = 0, flips = 0;
+    __shared__ Warp64 W[RECHECK_THREADS / 32];
+    const unsigned warps = gridDim.x * (RECHECK_THREADS / 32), warp = threadIdx.x >> 5;
+    if (recheck_by_warp(cnt, warps, 0)) {   /* the problems' pair lists differ: as for a short one */
+        for (unsigned idx = warp * gridDim.x + blockIdx.x; idx < cnt; idx += warps) {
+            const uint2 it = bq.items[idx];
+            const DevScene& sc = B.scenes[problem_of(B, (long long)it.x)];
+            recheck_item_warp(sc, kind, it, q, qs, qe, offset, sc.dq, policy, res, key, checks, flips,
+                              bq.pair_range ? bq.pair_range[idx] : 0xffff0000u, W[warp]);
+        }
+        cnt = 0;
+    }
     for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < cnt; idx += gridDim.x * blockDim.x) {
         const uint2 it = bq.items[idx];
         const DevScene& sc = B.scenes[problem_of(B, (long long)it.x)];

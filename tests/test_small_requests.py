@@ -115,3 +115,24 @@ def test_requests_in_flight_together():
     for (r, res), w in zip(reversed(reqs), reversed(want)):
         cs.indicator2_async_wait(r)
         np.testing.assert_array_equal(res, w)
+
+
+@pytest.mark.parametrize("kind,n", [("box4", 300), ("box4", 120000), ("hull6", 2000), ("wall7", 17000)])
+def test_large_path_rechecks_by_warp_and_by_thread_equal_the_oracle(kind, n):
+    """The large path's FP64 recheck takes a warp per item for few items and
+    a thread per item for many (a wide band makes many)."""
+    sc = SCENES[kind]()
+    q = scenes.uniform_configs(sc, n, 15)
+    for band in (1e-5, 2e-2):
+        cs = space(sc, 0.02, GPRM_MODE_FP64_BAND)
+        cs.set_band(band)
+        cs.profile_enable(True)
+        got = cs.check_configs(q)
+        m = min(n, 3000)
+        want, _, inb = O.Oracle(sc).check_configs(q[:m], O.FP32_BAND | O.DEVICE_TRIG, band=band)
+        np.testing.assert_array_equal(got[:m], want)
+        if m == n:
+            assert cs.stats()["band_rechecks"] == int(inb.sum())
+        small = space(sc, 0.02, GPRM_MODE_FP64_BAND)
+        small.set_band(band)
+        np.testing.assert_array_equal(small.check_configs(q[:m]), want)
