@@ -436,6 +436,8 @@ int build_space(const gprm_scene_desc* d, float dq, int nbuf, gprm_space** out)
         return fail(nullptr, GPRM_ERR_SCENE, "ndof %d outside 1..%d", d->ndof, GPRM_MAX_DOF);
     if (d->num_polytopes < 1) return fail(nullptr, GPRM_ERR_SCENE, "N<=0");
     if (d->num_pairs < 0) return fail(nullptr, GPRM_ERR_SCENE, "M<0");
+    /* the kernels pack a pair's index into 27 bits */
+    if (d->num_pairs >= (1 << 27)) return fail(nullptr, GPRM_ERR_SCENE, "M>=2^27");
     if (!d->dh_a || !d->dh_alpha || !d->dh_q || !d->dh_d || !d->dh_types || !d->mins || !d->maxs ||
         !d->poly_n || !d->poly_m || !d->vertices || !d->dsp || !d->cnt || !d->dest || !d->sys ||
         (d->num_pairs > 0 && (!d->pair_from || !d->pair_to)))
@@ -768,24 +770,26 @@ int event_pair(gprm_space* h, std::vector<cudaEvent_t>& pool, size_t& used, cuda
 }
 
 /* Whether a request of n items goes through the small-request kernels.
- * Measured on one B200, host buffers in and out, us a call, large path
- * against small (box: 67 pairs, hull: 394, wall: 4117):
- *   configurations  exact arithmetic  box        hull       wall
+ * Measured on one B200, host buffers in and out, exact arithmetic, us a
+ * call, large path against small (box: 67 pairs, hull: 394, wall: 4117):
+ *   configurations                    box        hull       wall
  *     n = 1                           68 / 27    104 / 43   219 / 54
- *     n = 592                         167 / 73   377 / 99   1992 / 162
- *     n = 16384                       243 / 112  600 / 209  2536 / 603
+ *     n = 592                         182 / 73   346 / 106  1502 / 201
+ *     n = 4096                        211 / 82   379 / 140  1661 / 545
+ *     n = 32768                       270 / 156  502 / 366  2053 / 1232
  *   edges (0.25 rad on average)
  *     n = 32                          123 / 84   196 / 130  322 / 256
  *     n = 592                         193 / 105  335 / 257  532 / 332
  *     n = 1024                        194 / 125  283 / 372  847 / 785
  *     n = 4096                        239 / 281  425 / 615  2493 / 1154
- * A configuration's block has as much to do as its lanes' share of a warp
- * elsewhere, so the small path holds far up; above 16384 the persistent
- * kernels, which keep the FP64 rechecks apart, catch up on the smaller
- * scenes.  An edge's block costs four warps for one: it pays while every
- * block is resident at once, and beyond that only on large pair lists,
- * where four warps share the sweep stage. */
-constexpr int SMALL_CONFIGS = 16384;
+ * A warp of the large vertex kernel takes its 32 configurations through the
+ * sweep stage one after the other, so its launch lasts that long however
+ * few there are; a small request's block shares them over four warps.  At
+ * 2^20 configurations the large kernel does three times the small one's
+ * rate (hull).  An edge's block costs four warps for one: it pays while
+ * every block is resident at once, and beyond that only on large pair
+ * lists, where four warps share the sweep stage. */
+constexpr int SMALL_CONFIGS = 32768;
 constexpr int SMALL_EDGE_WAVES = 16, SMALL_EDGE_PAIRS = 2048;
 bool small_request(const gprm_space* h, int kind, long long n)
 {

@@ -360,9 +360,9 @@ int gprm_batch_create(gprm_space* const* spaces, int count, gprm_batch** out)
             BATCH_TRY(b, dev_malloc((void**)&b->d_total, sizeof(Control)));
             BATCH_TRY(b, dev_malloc((void**)&b->d_scratch_total, sizeof(Control)));
             BATCH_TRY(b, cudaMemset(b->d_total, 0, sizeof(Control)));
-            BatchView v = view_of(b, 1);
-            BATCH_TRY(b, configure_batch_launch(v, 1, 128, &b->cfg[1]));
-            BATCH_TRY(b, configure_batch_launch(v, 0, 128, &b->cfg[0]));
+            /* the two kinds' shared areas differ */
+            BATCH_TRY(b, configure_batch_launch(view_of(b, 1), 1, 128, &b->cfg[1]));
+            BATCH_TRY(b, configure_batch_launch(view_of(b, 0), 0, 128, &b->cfg[0]));
             return GPRM_OK;
         }()))
         return bad(rc);

@@ -946,10 +946,10 @@ __device__ __forceinline__ void forward_kinematics_fast(const DevScene& sc, cons
  * ball goes to cen[(slot*3 + c) * 32], the world position of the slot
  * polytope's vertex 0 to cen[((nslots + slot)*3 + c) * 32] (both with FMA:
  * they only feed the certificates, whose slack covers their rounding).
- * joint(i): the lane's value of joint i.  One loop body for every joint (the
+ * SLOTS: whether to write them.  joint(i): the lane's value of joint i.  One loop body for every joint (the
  * kernels wait on instruction fetches), its slot's table entries loaded
  * before the trigonometry. */
-template <bool FAST, class Joint>
+template <bool FAST, bool SLOTS, class Joint>
 __device__ __forceinline__ void forward_kinematics_smem(const DevScene& sc, const float4* __restrict__ tab,
                                                         Joint joint, float* out, float* cen)
 {
@@ -959,7 +959,7 @@ __device__ __forceinline__ void forward_kinematics_smem(const DevScene& sc, cons
     int slot = 0;
 #pragma unroll 1
     for (int i = 0; i < sc.ndof; ++i) {
-        bool has = slot < sc.nslots && sc.slot_sys[slot] == i + 1;
+        bool has = SLOTS && slot < sc.nslots && sc.slot_sys[slot] == i + 1;
         float4 b = make_float4(0.0f, 0.0f, 0.0f, 0.0f), v = b;
         if (has) {
             const float4* blk = tab + sc.slot_block[slot];

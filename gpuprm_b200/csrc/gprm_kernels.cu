@@ -64,27 +64,29 @@ struct SceneView {
     const float4* scan_b;
     float* frames;   /* this lane's frames (lane-interleaved, stride 32) */
     float* cen;      /* this lane's slot ball centres, then the slots' world vertex 0 */
-    float4* sweep;   /* the warp's per-slot sweep balls (GPRM_MAX_SLOTS) */
-    unsigned* defer; /* vertex checks: the warp's deferred-test queue (64) and batch results (32 + 32);
-                        edge checks: the pairs of the sweep group left open (one bit each) */
+    float4* sweep;   /* the warp's per-slot sweep balls */
+    unsigned* bits;  /* the pairs of the sweep group left open (one bit each) */
 };
 
-/* The warp's sweep area: the last SWEEP_LANE_FLOATS entries of its block. */
+/* The warp's sweep area: after the frames in a vertex kernel
+ * (the start of its VertexArea), the last SWEEP_LANE_FLOATS entries of the
+ * block in an edge kernel. */
 template <bool VERTEX>
 __device__ __forceinline__ float4* sweep_area(const DevScene& sc, float* lane_frames)
 {
     const int lane = threadIdx.x & 31;
-    return reinterpret_cast<float4*>(lane_frames - lane + (lane_floats(sc, VERTEX) - SWEEP_LANE_FLOATS) * 32);
+    const size_t at = VERTEX ? (size_t)sc.ndof * 12 : lane_floats(sc, false) - SWEEP_LANE_FLOATS;
+    return reinterpret_cast<float4*>(lane_frames - lane + at * 32);
 }
 
-/* The warp's area before the sweep area: the deferred tests of a vertex
- * kernel, the open pairs of an edge kernel. */
+/* The open bits of the warp's sweep stage: before the sweep area in an edge
+ * kernel, after the VertexArea in a vertex kernel. */
 template <bool VERTEX>
-__device__ __forceinline__ unsigned* defer_area(const DevScene& sc, float* lane_frames)
+__device__ __forceinline__ unsigned* open_area(const DevScene& sc, float* lane_frames)
 {
     const int lane = threadIdx.x & 31;
-    return reinterpret_cast<unsigned*>(lane_frames - lane +
-                                       ((size_t)sc.ndof * 12 + (size_t)sc.nslots * 6) * 32);
+    const size_t at = (size_t)sc.ndof * 12 + (VERTEX ? (size_t)VERTEX_LANE_FLOATS : (size_t)sc.nslots * 6);
+    return reinterpret_cast<unsigned*>(lane_frames - lane + at * 32);
 }
 
 /* Copies the scene into shared memory (SMEM) and returns the pointers the
@@ -130,7 +132,7 @@ __device__ __forceinline__ SceneView stage_scene(const DevScene& sc, unsigned ch
     s.frames = reinterpret_cast<float*>(smem + off) + (size_t)warp * lane_floats(sc, VERTEX) * 32 + lane;
     s.cen = s.frames + (size_t)sc.ndof * 12 * 32;
     s.sweep = sweep_area<VERTEX>(sc, s.frames);
-    s.defer = defer_area<VERTEX>(sc, s.frames);
+    s.bits = open_area<VERTEX>(sc, s.frames);
     __syncthreads();
     return s;
 }
@@ -211,6 +213,21 @@ struct PairCounts {
     unsigned long long cert, full;
 };
 
+/* The MUFU's reciprocal square root and reciprocal, denormals as zero (no
+ * scaling around them). */
+__device__ __forceinline__ float rsqrt_fast(float x)
+{
+    float r;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rcp_fast(float x)
+{
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
 /* The direction test of pair_certified_dir for every lane of the warp at
  * once.  Each polytope's ball centre lies in a ball over the lanes, and so
  * does its vertex 0 (the slot's sweep balls; radius 0 for a polytope of
@@ -230,11 +247,11 @@ __device__ __forceinline__ bool swept_direction(float eps_dir, float thr_dir, fl
 {
     const float n2 = __fmaf_rn(sx, sx, __fmaf_rn(sy, sy, sz * sz));
     const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
-    const float sn = n2 * rsqrtf(n2), dn = d2 * rsqrtf(d2);   /* NaN for 0: not settled */
+    const float sn = n2 * rsqrt_fast(n2), dn = d2 * rsqrt_fast(d2);   /* NaN for 0: not settled */
     const float N = __fmaf_rn(sx, dx, __fmaf_rn(sy, dy, sz * dz)) * (1.0f - 1e-5f) -
                     __fmaf_rn(sn, rc, __fmaf_rn(rv, dn, rv * rc)) * (1.0f + 1e-5f);
     const float slo = sn * (1.0f - 1e-5f) - rv * (1.0f + 1e-5f), sup = (sn + rv) * (1.0f + 1e-5f);
-    const float err = (dn + rc + R) * (__fdividef(eps_dir, slo) + 1e-6f) * (1.0f + 2e-5f);
+    const float err = (dn + rc + R) * __fmaf_rn(eps_dir, rcp_fast(slo), 1e-6f) * (1.0f + 2e-5f);
     return N > 0.0f && slo > 1e-3f && N * (1.0f - 1e-5f) > sup * (__fmaf_rn(R, 1.0f + 1e-5f, err) + thr_dir);
 }
 
@@ -253,22 +270,38 @@ __device__ __forceinline__ bool swept_near(float4 o, float4 m, float root, float
 
 /* A sweep entry (r: swp, v: swb) against the warp's sweep balls: true when
  * neither the distance nor the direction settles its pair for every lane.
- * Branch-free, so that two entries go side by side. */
-__device__ __forceinline__ bool swept_open(const float4* sweep, bool dir_on, float eps_dir, float thr_dir, float4 r,
-                                           float4 v)
+ * Branch-free, so that two entries go side by side.  POINT: the balls have
+ * radius 0 (one configuration), and the direction test is that of
+ * lane_certified with a margin for the approximate roots. */
+template <bool POINT>
+__device__ __forceinline__ bool swept_open(const float4* sweep, const float4* v0, bool dir_on, float eps_dir,
+                                           float thr_dir, float4 r, float4 v)
 {
     const int w = __float_as_int(r.w);
     const int a = w & 15, b = (w >> 4) & 15;   /* a: a moving polytope's slot; b != a: the other's */
-    const float4* v0 = sweep + (dir_on ? SWEEP_V0_SLOTS : 0);
     float4 o = make_float4(r.x, r.y, r.z, 0.0f), u = make_float4(v.x, v.y, v.z, 0.0f);
     if (b != a) { o = sweep[b]; u = v0[b]; }
     const float root = __int_as_float(w | 255);   /* the slot bits round it up */
-    float dx, dy, dz, rc;
-    const bool near = swept_near(o, sweep[a], root, dx, dy, dz, rc);
     const float4 m = v0[a];
-    const bool settled = dir_on && swept_direction(eps_dir, thr_dir, u.x - m.x, u.y - m.y, u.z - m.z, u.w + m.w, dx,
-                                                   dy, dz, rc, v.w);
-    return near && !settled && !(root < 0.0f);
+    if constexpr (POINT) {
+        const float4 c = sweep[a];
+        const float dx = o.x - c.x, dy = o.y - c.y, dz = o.z - c.z;
+        const float sx = u.x - m.x, sy = u.y - m.y, sz = u.z - m.z;
+        const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
+        const float n2 = __fmaf_rn(sx, sx, __fmaf_rn(sy, sy, sz * sz));
+        const float inv = rsqrt_fast(n2);
+        const float G = __fmaf_rn(sx, dx, __fmaf_rn(sy, dy, sz * dz)) * inv;
+        const float err = __fmaf_rn(d2, rsqrt_fast(d2), v.w) * __fmaf_rn(eps_dir, inv, 1e-6f);
+        const bool settled = d2 * (1.0f - 2e-6f) > root * root ||
+                             (n2 > 1.00001e-6f && G * (1.0f - 1e-5f) > __fmaf_rn(v.w + err, 1.0f + 2e-5f, thr_dir));
+        return !settled && !(root < 0.0f);
+    } else {
+        float dx, dy, dz, rc;
+        const bool near = swept_near(o, sweep[a], root, dx, dy, dz, rc);
+        const bool settled = dir_on && swept_direction(eps_dir, thr_dir, u.x - m.x, u.y - m.y, u.z - m.z, u.w + m.w, dx,
+                                                       dy, dz, rc, v.w);
+        return near && !settled && !(root < 0.0f);
+    }
 }
 
 __device__ __forceinline__ void sweep_mark(const int* swj, unsigned* bits, int g, int i, bool open)
@@ -283,9 +316,11 @@ __device__ __forceinline__ void sweep_mark(const int* swj, unsigned* bits, int g
  * warp's sweep balls: a pair whose ball centres are farther apart in every
  * lane than rho_P + rho_Q + sqrt(T2) is settled for all lanes at once (each
  * lane's exact distance then exceeds sqrt(T2)); else the direction test is
- * bounded over all lanes at once (swept_direction).  Sets in S.defer the
+ * bounded over all lanes at once (swept_direction).  Sets in S.bits the
  * bits of the pairs left for the lanes' own tests (bit j - g *
- * SWEEP_GROUP); share: the leaves of every 32 that this warp goes through.
+ * SWEEP_GROUP); share: the leaves of every 32 that this warp goes through;
+ * POINT: see swept_open; dir_on, v0_at: whether, and from where, the sweep area holds balls of the
+ * slots' vertex 0.
  *
  * Two levels: lane l tests leaf l of the next 32 (32 pairs of one slot whose
  * static partners lie close together) by its ball, then the warp goes
@@ -297,16 +332,17 @@ __device__ __forceinline__ void sweep_mark(const int* swj, unsigned* bits, int g
  * wall scene (129 chunks of 32 pairs; 70,001 edges 27.7 -> 15.9 ms with the
  * leaves); on 64 obstacles (two leaves a slot) the leaf level costs what it
  * saves (62.1 -> 61.7 ms). */
-__device__ __forceinline__ void sweep_leaves(const DevScene& sc, const SceneView& S, int g, unsigned share)
+template <bool POINT>
+__device__ __forceinline__ void sweep_leaves(const DevScene& sc, const SceneView& S, int g, unsigned share, bool dir_on,
+                                             int v0_at)
 {
     const int lane = threadIdx.x & 31;
     /* the descriptor's fields in registers: a batch keeps it in shared
        memory, where the bits are set */
-    const bool dir_on = sc.nslots <= SWEEP_V0_SLOTS;
     const float eps_dir = sc.eps_dir, thr_dir = sc.thr_dir;
-    const float4 *swl = sc.swl, *swp = sc.swp, *swb = sc.swb, *sweep = S.sweep;
+    const float4 *swl = sc.swl, *swp = sc.swp, *swb = sc.swb, *sweep = S.sweep, *v0 = S.sweep + (dir_on ? v0_at : 0);
     const int* swj = sc.swj;
-    unsigned* bits = S.defer;
+    unsigned* bits = S.bits;
     const int end = sc.swg[g + 1];
 #pragma unroll 1
     for (int l0 = sc.swg[g]; l0 < end; l0 += 32) {
@@ -329,8 +365,8 @@ __device__ __forceinline__ void sweep_leaves(const DevScene& sc, const SceneView
 #pragma unroll 1
         for (;;) {
             const float4 ra = swp[ia], va = swb[ia], rb = swp[ib], vb = swb[ib];
-            const bool oa = swept_open(sweep, dir_on, eps_dir, thr_dir, ra, va);
-            const bool ob = swept_open(sweep, dir_on, eps_dir, thr_dir, rb, vb);
+            const bool oa = swept_open<POINT>(sweep, v0, dir_on, eps_dir, thr_dir, ra, va);
+            const bool ob = swept_open<POINT>(sweep, v0, dir_on, eps_dir, thr_dir, rb, vb);
             sweep_mark(swj, bits, g, ia, oa);
             sweep_mark(swj, bits, g, ib, ob);
             if (!left) break;
@@ -344,34 +380,108 @@ __device__ __forceinline__ void sweep_leaves(const DevScene& sc, const SceneView
 
 __device__ __forceinline__ void sweep_stage(const DevScene& sc, const SceneView& S, int g, int words)
 {
-    for (int w = threadIdx.x & 31; w < words; w += 32) S.defer[w] = 0u;
+    for (int w = threadIdx.x & 31; w < words; w += 32) S.bits[w] = 0u;
     __syncwarp();
-    sweep_leaves(sc, S, g, FULL_MASK);
+    sweep_leaves<false>(sc, S, g, FULL_MASK, sc.nslots <= SWEEP_V0_SLOTS, SWEEP_V0_SLOTS);
     __syncwarp();
+}
+
+/* The certificates of a pair for one configuration, given the world ball
+ * centres p, q and vertices 0 a, b of its polytopes (T2, R: of the pair; c:
+ * its scan_c; frames: the configuration's): the ball-distance and direction
+ * tests of pair_certified without a branch between them, then, where both
+ * miss, its box test. */
+__device__ __forceinline__ bool points_certified(const DevScene& sc, const float* frames, int4 c, float T2, float R,
+                                                 V3<float> p, V3<float> q, V3<float> a, V3<float> b)
+{
+    const float dx = q.x - p.x, dy = q.y - p.y, dz = q.z - p.z;
+    const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
+    float sx = b.x - a.x, sy = b.y - a.y, sz = b.z - a.z;
+    const float n2 = __fmaf_rn(sx, sx, __fmaf_rn(sy, sy, sz * sz));
+    const float inv = rsqrtf(n2);
+    const float G = __fmaf_rn(sx, dx, __fmaf_rn(sy, dy, sz * dz)) * inv - R;
+    /* |D| from above: d2 * rsqrt(d2) is within 3 ulp of |D| (rsqrtf <= 2
+       ulp), the factor covers it; d2 = 0 gives NaN, which fails the tests */
+    const float dn = d2 * rsqrtf(d2) * (1.0f + 2e-6f);
+    /* direction error <= eps_dir*inv (+ rsqrt and rounding, 1e-6) */
+    const float err = (dn + R) * __fmaf_rn(sc.eps_dir, inv, 1e-6f);
+    const bool dir = n2 > 1e-6f;   /* |s| < 1e-3: leave it to the test */
+    if (d2 > T2 || (dir && G - err > sc.thr_dir)) return true;
+    if (!dir) return false;
+    sx = sx * inv; sy = sy * inv; sz = sz * inv;
+    const float hp = box_support(sc.box + 3 * c.y, frames, SCAN_SYS_P(c.x), sx, sy, sz);
+    const float hq = box_support(sc.box + 3 * c.z, frames, SCAN_SYS_Q(c.x), sx, sy, sz);
+    const float Gb = __fmaf_rn(sx, dx, __fmaf_rn(sy, dy, sz * dz)) - (hp + hq) * (1.0f + 1e-5f);
+    return Gb - err > sc.thr_dir;
+}
+
+/* points_certified for the lane whose slots and frames S holds: the moving
+ * polytopes' points from the slots (written by the FK pass), a static one's
+ * from the records f and b.  A pair that is not SCAN_USABLE is never
+ * certified here (no slot, or two static polytopes whose certificate failed
+ * when the tables were uploaded). */
+__device__ __forceinline__ bool lane_certified(const DevScene& sc, const SceneView& S, int4 c, float4 f, float4 b)
+{
+    if (c.w != SCAN_USABLE) return false;
+    const float* v0w = S.cen + sc.nslots * 3 * 32;
+    V3<float> P = {f.x, f.y, f.z}, Q = P, A = {b.x, b.y, b.z}, B = A;
+    const int sp = SCAN_SLOT_P(c.x), sq = SCAN_SLOT_Q(c.x);
+    if (sp >= 0) {
+        const float* u = S.cen + sp * 3 * 32;
+        const float* v = v0w + sp * 3 * 32;
+        P.x = u[0]; P.y = u[32]; P.z = u[64];
+        A.x = v[0]; A.y = v[32]; A.z = v[64];
+    }
+    if (sq >= 0) {
+        const float* u = S.cen + sq * 3 * 32;
+        const float* v = v0w + sq * 3 * 32;
+        Q.x = u[0]; Q.y = u[32]; Q.z = u[64];
+        B.x = v[0]; B.y = v[32]; B.z = v[64];
+    }
+    return points_certified(sc, S.frames, c, f.w, b.w, P, Q, A, B);
+}
+
+/* Point x of frame f (1..ndof) of a configuration, with the FMA chain of the
+ * slot points. */
+__device__ __forceinline__ V3<float> frame_point(const float* frames, int f, float4 x)
+{
+    const float* T = frames + (f - 1) * 12 * 32;
+    V3<float> o;
+    o.x = __fmaf_rn(T[0], x.x, __fmaf_rn(T[3 * 32], x.y, __fmaf_rn(T[6 * 32], x.z, T[9 * 32])));
+    o.y = __fmaf_rn(T[32], x.x, __fmaf_rn(T[4 * 32], x.y, __fmaf_rn(T[7 * 32], x.z, T[10 * 32])));
+    o.z = __fmaf_rn(T[2 * 32], x.x, __fmaf_rn(T[5 * 32], x.y, __fmaf_rn(T[8 * 32], x.z, T[11 * 32])));
+    return o;
+}
+
+/* points_certified of pair j from the frames alone (a vertex check keeps no
+ * slot points). */
+__device__ __forceinline__ bool frames_certified(const DevScene& sc, const SceneView& S, const float* frames, int j)
+{
+    const int4 c = S.scan_c[j];
+    if (c.w != SCAN_USABLE) return false;
+    const int4 pr = S.pairs[j];
+    const float4 p = S.tab[pr.x], a = S.tab[pr.x + 1], q = S.tab[pr.y], b = S.tab[pr.y + 1];
+    V3<float> P = {p.x, p.y, p.z}, A = {a.x, a.y, a.z}, Q = {q.x, q.y, q.z}, B = {b.x, b.y, b.z};
+    if (pr.z) { P = frame_point(frames, pr.z, p); A = frame_point(frames, pr.z, a); }
+    if (pr.w) { Q = frame_point(frames, pr.w, q); B = frame_point(frames, pr.w, b); }
+    return points_certified(sc, frames, c, S.far[j].w, S.scan_b[j].w, P, Q, A, B);
 }
 
 /* This lane's certificates of the pairs j0 + k, k in cand (warp-uniform),
  * all order-free (a certified pair is free with its margin above the band,
- * so it changes neither a code nor a band decision): the ball-distance and
- * direction tests of pair_certified without a branch between them, then, on
- * the lanes both miss, its box test.  The moving polytopes' ball centres and
- * vertices 0 come from the lane's slots (written by the FK pass), a static
- * one's from far and scan_b.  A pair that is not SCAN_USABLE here is never
- * certified (no slot, or two static polytopes whose certificate failed when
- * the tables were uploaded).  Returns the pairs that need the exact test
- * (bit k).
+ * so it changes neither a code nor a band decision).  Returns the pairs that
+ * need the exact test (bit k).
  *
  * One copy of the code and the next pair's records loaded ahead, rather than
  * two pairs side by side with every case inlined for each: the edge kernel
- * waits on instruction fetches more than on anything else (2.6 of 9.5 warp
- * cycles per instruction before). */
+ * waited on instruction fetches more than on anything else (2.6 of 9.5 warp
+ * cycles per instruction; 2.5 M roadmap edges 86.7 -> 64.3 ms). */
 __device__ __forceinline__ unsigned lane_scan(const DevScene& sc, const SceneView& S, int j0, unsigned cand,
                                               PairCounts& pc)
 {
     if (!cand) return 0u;
-    unsigned need = 0, done = cand;
-    const float* cen = S.cen;
-    const float* v0w = cen + sc.nslots * 3 * 32;
+    const unsigned all = cand;
+    unsigned need = 0;
     int k = __ffs(cand) - 1;
     int4 c = S.scan_c[j0 + k];
     float4 f = S.far[j0 + k], b = S.scan_b[j0 + k];
@@ -381,65 +491,12 @@ __device__ __forceinline__ unsigned lane_scan(const DevScene& sc, const SceneVie
         const int kn = cand ? __ffs(cand) - 1 : k;
         const int4 cn = S.scan_c[j0 + kn];
         const float4 fn = S.far[j0 + kn], bn = S.scan_b[j0 + kn];
-        bool ok = false;
-        if (c.w == SCAN_USABLE) {
-            float px = f.x, py = f.y, pz = f.z, qx = f.x, qy = f.y, qz = f.z;
-            float ax = b.x, ay = b.y, az = b.z, bx = b.x, by = b.y, bz = b.z;
-            const int sp = SCAN_SLOT_P(c.x), sq = SCAN_SLOT_Q(c.x);
-            if (sp >= 0) {
-                const float* u = cen + sp * 3 * 32;
-                const float* v = v0w + sp * 3 * 32;
-                px = u[0]; py = u[32]; pz = u[64];
-                ax = v[0]; ay = v[32]; az = v[64];
-            }
-            if (sq >= 0) {
-                const float* u = cen + sq * 3 * 32;
-                const float* v = v0w + sq * 3 * 32;
-                qx = u[0]; qy = u[32]; qz = u[64];
-                bx = v[0]; by = v[32]; bz = v[64];
-            }
-            const float dx = qx - px, dy = qy - py, dz = qz - pz;
-            const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
-            float sx = bx - ax, sy = by - ay, sz = bz - az;
-            const float n2 = __fmaf_rn(sx, sx, __fmaf_rn(sy, sy, sz * sz));
-            const float inv = rsqrtf(n2);
-            const float G = __fmaf_rn(sx, dx, __fmaf_rn(sy, dy, sz * dz)) * inv - b.w;
-            /* |D| from above: d2 * rsqrt(d2) is within 3 ulp of |D| (rsqrtf
-               <= 2 ulp), the factor covers it; d2 = 0 gives NaN, which fails
-               the tests */
-            const float dn = d2 * rsqrtf(d2) * (1.0f + 2e-6f);
-            /* direction error <= eps_dir*inv (+ rsqrt and rounding, 1e-6) */
-            const float err = (dn + b.w) * __fmaf_rn(sc.eps_dir, inv, 1e-6f);
-            const bool dir = n2 > 1e-6f;   /* |s| < 1e-3: leave it to the test */
-            ok = d2 > f.w || (dir && G - err > sc.thr_dir);
-            if (!ok && dir) {
-                sx = sx * inv; sy = sy * inv; sz = sz * inv;
-                const float hp = box_support(sc.box + 3 * c.y, S.frames, SCAN_SYS_P(c.x), sx, sy, sz);
-                const float hq = box_support(sc.box + 3 * c.z, S.frames, SCAN_SYS_Q(c.x), sx, sy, sz);
-                const float Gb = __fmaf_rn(sx, dx, __fmaf_rn(sy, dy, sz * dz)) - (hp + hq) * (1.0f + 1e-5f);
-                ok = Gb - err > sc.thr_dir;
-            }
-        }
-        if (!ok) need |= 1u << k;
+        if (!lane_certified(sc, S, c, f, b)) need |= 1u << k;
         if (!cand) break;
         k = kn; c = cn; f = fn; b = bn;
     }
-    pc.cert += (unsigned)__popc(done & ~need);
+    pc.cert += (unsigned)__popc(all & ~need);
     return need;
-}
-
-/* lane_scan over the chunk j0 .. j0+jn-1 (jn <= 32) of a vertex check, whose
- * lanes hold unrelated configurations: every pair but those settled for
- * every configuration (SCAN_SETTLED).  0 for an inactive lane; every lane
- * of the warp must call it (it votes). */
-__device__ __forceinline__ unsigned config_scan(const DevScene& sc, const SceneView& S, int j0, int jn, bool active,
-                                                PairCounts& pc)
-{
-    const int lane = threadIdx.x & 31;
-    const unsigned cand = __ballot_sync(FULL_MASK, lane < jn && S.scan_c[j0 + lane].w != SCAN_SETTLED);
-    if (!active) return 0u;
-    pc.cert += (unsigned)(jn - __popc(cand));
-    return lane_scan(sc, S, j0, cand, pc);
 }
 
 /* The exact test of pair j for this lane (its certificates failed): the pair's code, and its margin in *margin. */
@@ -468,10 +525,10 @@ __device__ __forceinline__ int eval_pair(const DevScene& sc, const SceneView& S,
 
 /* Forward kinematics of a lane into its shared-memory frames, in the
  * arithmetic of the kernel variant. */
-template <bool FAST, class Joint>
+template <bool FAST, bool SLOTS = true, class Joint>
 __device__ __forceinline__ void lane_fk(const DevScene& sc, const SceneView& S, Joint joint)
 {
-    forward_kinematics_smem<FAST>(sc, S.tab, joint, S.frames, S.cen);
+    forward_kinematics_smem<FAST, SLOTS>(sc, S.tab, joint, S.frames, S.cen);
 }
 
 __device__ __forceinline__ void flush_counts(PairCounts pc, Control* ctl)
@@ -484,119 +541,6 @@ __device__ __forceinline__ void flush_counts(PairCounts pc, Control* ctl)
         if (pc.cert) atomicAdd(&ctl->certified, pc.cert);
         if (pc.full) atomicAdd(&ctl->full_tests, pc.full);
     }
-}
-
-/* ------------------------------------------------------------------ */
-/* deferred exact pair tests                                            */
-/* ------------------------------------------------------------------ */
-/*
- * Within a chunk of 32 pairs, the pairs a lane must test exactly are not run
- * where they are found (where most of the warp would idle) but queued as
- * items (owner lane, pair - j0) in the warp's shared area; every 32 items
- * the whole warp runs one each on its owner's frames.  Items reach the
- * queue in pair order, so each owner applies its results in pair order:
- * the first colliding pair decides its code (later items are ignored) and
- * the free ones before it feed its minimum margin, exactly as the
- * sequential loop.  first_k records the chunk index of that first
- * collision (DEFER_NONE: none in this chunk).
- *
- * Vertex checks use it: their lanes hold unrelated configurations, so the
- * pairs left to test differ from lane to lane (measured on hull6 with 2^20
- * samples: 11.0 -> 8.6 ms).  The lanes of an edge check hold neighbouring
- * steps of one edge, which mostly need the same pairs; there the queue
- * costs more than it saves (357 -> 436 ms) and the sequential loop stays.
- */
-constexpr int DEFER_NONE = 32;
-
-struct LaneState {
-    int code;
-    float mdec, mmin;
-    bool active;
-    int first_k;
-    int jrec, jlast;   /* first and last pair decided within the band (collision or margin < band) */
-};
-
-__device__ __forceinline__ void defer_push(unsigned* q, int& n, bool want, int k)
-{
-    const int lane = threadIdx.x & 31;
-    const unsigned m = __ballot_sync(FULL_MASK, want);
-    if (want) q[n + __popc(m & ((1u << lane) - 1u))] = (unsigned)lane | ((unsigned)k << 5);
-    n += __popc(m);
-}
-
-/* Runs the first cnt (<= 32) queued items, one per lane, and lets every
- * owner apply its results; the remaining items move to the front. */
-template <bool FAST>
-__device__ __forceinline__ void defer_run(const DevScene& sc, const SceneView& S, int j0, int& n, int cnt,
-                                          LaneState& st, PairCounts& pc, float band)
-{
-    const int lane = threadIdx.x & 31;
-    unsigned* q = S.defer;
-    int* rcode = reinterpret_cast<int*>(q + 64);
-    float* rm = reinterpret_cast<float*>(q + 96);
-    __syncwarp();
-    int c = 0;
-    float m = 0.0f;
-    if (lane < cnt) {
-        const unsigned it = q[lane];
-        const int owner = (int)(it & 31u);
-        const int jj = j0 + (int)(it >> 5);
-        const int4 pr = S.pairs[jj];
-        Frame<float> tp, tq;
-        pair_frames(S.frames - lane + owner, pr, tp, tq);
-        if constexpr (FAST) c = pair_test_fast(sc, S.tab, pr, sc.ppoly[jj], tp, tq, &m);
-        else c = pair_test<PF32>(sc, S.tab, pr, tp, tq, &m);
-        ++pc.full;
-    }
-    rcode[lane] = c;
-    rm[lane] = m;
-    __syncwarp();
-#pragma unroll 1
-    for (int t = 0; t < cnt; ++t) {
-        const unsigned it = q[t];
-        if ((int)(it & 31u) == lane && st.first_k == DEFER_NONE) {
-            const int ct = rcode[t];
-            const int jj = j0 + (int)(it >> 5);
-            if (ct != 0) {
-                st.code = ct;
-                st.mdec = rm[t];
-                st.first_k = (int)(it >> 5);
-                st.active = false;
-                st.jrec = min(st.jrec, jj);
-            } else {
-                st.mmin = min_nan(st.mmin, rm[t]);
-                if (!(rm[t] >= band)) {
-                    st.jrec = min(st.jrec, jj);
-                    st.jlast = max(st.jlast, jj);
-                }
-            }
-        }
-    }
-    const int rest = n - cnt;
-    __syncwarp();
-    const unsigned mv = lane < rest ? q[cnt + lane] : 0u;
-    __syncwarp();
-    if (lane < rest) q[lane] = mv;
-    n = rest;
-    __syncwarp();
-}
-
-/* One chunk's ordered pass with deferral: the pairs whose certificates
- * failed (need, from cert_scan) are queued in pair order. */
-template <bool FAST>
-__device__ __forceinline__ void defer_chunk(const DevScene& sc, const SceneView& S, int j0, unsigned need,
-                                            unsigned todo, LaneState& st, PairCounts& pc, float band)
-{
-    int n = 0;
-    st.first_k = DEFER_NONE;
-    while (todo) {
-        const int k = __ffs(todo) - 1;
-        todo &= todo - 1u;
-        const bool full = st.active && ((need >> k) & 1u);
-        defer_push(S.defer, n, full, k);
-        if (n >= 32) defer_run<FAST>(sc, S, j0, n, 32, st, pc, band);
-    }
-    while (n > 0) defer_run<FAST>(sc, S, j0, n, n < 32 ? n : 32, st, pc, band);
 }
 
 /* Appends the items of the lanes with `want` set, one atomic per warp;
@@ -644,7 +588,45 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long x)
 /* vertex checks                                                        */
 /* ------------------------------------------------------------------ */
 
-/* Configurations i0 .. i0+count-1 (count <= 32), one per lane. */
+/* The warp's shared area of a vertex kernel (VERTEX_LANE_FLOATS per lane):
+ * the balls of the configuration in the sweep stage, the queue of (lane |
+ * pair << 5) items that it leaves open, per configuration the pairs that
+ * need the exact test (count of them; those that found no room start at
+ * pair `resume`), the first colliding pair (pair << 5 | code + 1 | 16 if
+ * inside the band) and the first and last free one inside the band.  The
+ * open bits of the sweep stage follow. */
+constexpr int VERTEX_TESTS = 12;
+struct VertexArea {
+    float4 balls[2 * GPRM_MAX_SLOTS];
+    unsigned open[64];
+    unsigned test[VERTEX_TESTS][32];
+    int count[32];
+    unsigned resume[32];
+    unsigned jkey[32], jfirst[32];
+    int jlast[32];
+};
+static_assert(sizeof(VertexArea) == VERTEX_LANE_FLOATS * 32 * sizeof(float), "vertex area");
+constexpr unsigned JKEY_NONE = 0xffffffffu;
+constexpr unsigned PAIR_NONE = 0x7fffffffu;
+
+/* Configurations i0 .. i0+count-1 (count <= 32), one per lane.
+ *
+ * Lanes hold unrelated configurations, so what one needs another does not.
+ * FK runs a lane per configuration; then the configurations go through the
+ * sweep stage one after the other, a lane per pair, with balls of radius 0
+ * (whole leaves of far obstacles drop out at once); the pairs that leaves
+ * open, of whichever configurations, go 32 at a time through their
+ * certificates (frames_certified), and what those leave is listed per
+ * configuration in pair order.  The exact tests follow in rounds: every
+ * configuration without a collision gives its next tests, one while 32 take
+ * part, more as fewer do, so that a colliding configuration runs few tests
+ * behind the one that decides it (without that, 15 tests a configuration
+ * instead of 4 on the wall scene, the larger part of the kernel).  Lists
+ * that overflow resume with another sweep.
+ * With every pair's certificates evaluated per lane in pair order this
+ * kernel took 5.3 ms for 2^20 hull6 configurations and 7.4 ms for 100,003 of
+ * the wall scene (exact), nearly all of it in those tests; slot points are
+ * not kept, which leaves shared memory for 16 warps per SM. */
 template <bool FAST>
 __device__ __forceinline__ void check_config_chunk(const DevScene& sc, const SceneView& S, const float* __restrict__ q,
                                                    long long offset, long long i0, int count, int* __restrict__ res,
@@ -652,40 +634,190 @@ __device__ __forceinline__ void check_config_chunk(const DevScene& sc, const Sce
                                                    Control* ctl, PairCounts& pc, unsigned long long& exec)
 {
     const int lane = threadIdx.x & 31;
+    VertexArea& A = *reinterpret_cast<VertexArea*>(S.sweep);
     const long long i = i0 + lane;
     const bool valid = lane < count;
-    int code = 0;
     bool active = valid;
     if (valid) {
         /* check_boundaries(q) (robotconfigspace.cpp:795-802) */
 #pragma unroll 1
         for (int j = 0; j < sc.ndof; ++j) {
             const float x = q[i + offset * j];
-            if (x < sc.mins[j] || x > sc.maxs[j]) { code = 1; active = false; }
+            if (x < sc.mins[j] || x > sc.maxs[j]) active = false;
         }
     }
-    if (active) lane_fk<FAST>(sc, S, [&](int j) { return q[i + offset * j]; });
-    LaneState st{code, 0.0f, PF32::inf(), active, DEFER_NONE, 0x7fffffff, -1};
-    /* pairs in chunks of 32: the order-free certificate scan, then the
-       pairs left for the exact test in the reference's order, their exact
-       tests deferred and run by the whole warp */
-#pragma unroll 1
-    for (int j0 = 0; j0 < sc.npairs; j0 += 32) {
-        if (!__any_sync(FULL_MASK, st.active)) break;
-        const int jn = min(32, sc.npairs - j0);
-        const unsigned need = config_scan(sc, S, j0, jn, st.active, pc);
-        const unsigned todo = __reduce_or_sync(FULL_MASK, need);
-        defer_chunk<FAST>(sc, S, j0, need, todo, st, pc, band);
+    if (active) lane_fk<FAST, false>(sc, S, [&](int j) { return q[i + offset * j]; });
+    /* this lane's sweep ball: slot `lane`'s ball centre, or slot lane - 16's vertex 0 */
+    const int slot = lane & (GPRM_MAX_SLOTS - 1);
+    float4 point = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    int frame = 1;
+    if (slot < sc.nslots) {
+        point = S.tab[sc.slot_block[slot] + (lane >= GPRM_MAX_SLOTS)];
+        frame = sc.slot_sys[slot];
     }
-    code = st.code;
-    const float mmin = st.mmin, mdec = st.mdec;
+    A.jkey[lane] = JKEY_NONE;
+    A.jfirst[lane] = PAIR_NONE;
+    A.jlast[lane] = -1;
+    unsigned todo = __ballot_sync(FULL_MASK, active);   /* configurations to sweep */
+    if (lane == 0) pc.cert += (unsigned long long)sc.npairs * (unsigned)__popc(todo);
+    unsigned from = 0u;                                 /* this lane's configuration: from this pair on */
+#pragma unroll 1
+    while (todo) {
+        A.count[lane] = 0;
+        A.resume[lane] = PAIR_NONE;
+        /* the sweep in progress: configuration c, its next group of pairs
+           g0, the next word row of the group's open bits, this lane's word */
+        int c = 0, g0 = sc.npairs, row = 0, rows = 0, base = 0;
+        unsigned word = 0u;
+        int n = 0;                                      /* items in the open queue */
+        bool more = true;
+#pragma unroll 1
+        while (more || n > 0) {
+            while (n < 32 && more) {
+                const unsigned m = __ballot_sync(FULL_MASK, word != 0u);
+                if (m) {
+                    /* in pair order: the whole row where it fits, else its
+                       next word */
+                    int at = __popc(word);
+#pragma unroll
+                    for (int d = 1; d < 32; d <<= 1) {
+                        const int y = __shfl_up_sync(FULL_MASK, at, d);
+                        if (lane >= d) at += y;
+                    }
+                    const int total = __shfl_sync(FULL_MASK, at, 31);
+                    const bool fits = n + total <= 64;
+                    const int l = fits ? 31 : __ffs(m) - 1;         /* words up to lane l */
+                    const int pushed = __shfl_sync(FULL_MASK, at, l);
+                    if (lane <= l) {
+                        at += n - __popc(word);
+                        for (; word; word &= word - 1u)
+                            A.open[at++] = (unsigned)c | ((unsigned)(base + __ffs(word) - 1) << 5);
+                    }
+                    n += pushed;
+                } else if (row < rows) {
+                    const int w = row * 32 + lane;
+                    base = g0 - SWEEP_GROUP + w * 32;
+                    word = base < min(sc.npairs, g0) ? S.bits[w] : 0u;
+                    ++row;
+                    /* a resumed configuration: the pairs from there on */
+                    const unsigned lo = __shfl_sync(FULL_MASK, from, c);
+                    if (lo > (unsigned)base) word = lo >= (unsigned)base + 32u ? 0u : word & (FULL_MASK << (lo & 31u));
+                } else if (g0 < sc.npairs) {
+                    const int words = (min(sc.npairs - g0, SWEEP_GROUP) + 31) >> 5;
+                    __syncwarp();
+                    for (int w = lane; w < words; w += 32) S.bits[w] = 0u;
+                    __syncwarp();
+                    sweep_leaves<true>(sc, S, g0 / SWEEP_GROUP, FULL_MASK, true, GPRM_MAX_SLOTS);
+                    __syncwarp();
+                    row = 0;
+                    rows = (words + 31) >> 5;
+                    g0 += SWEEP_GROUP;
+                } else if (todo) {
+                    c = __ffs(todo) - 1;
+                    todo &= todo - 1u;
+                    __syncwarp();
+                    if (slot < sc.nslots) {
+                        const V3<float> w = frame_point(S.frames - lane + c, frame, point);
+                        A.balls[lane] = make_float4(w.x, w.y, w.z, 0.0f);
+                    }
+                    __syncwarp();
+                    g0 = row = rows = 0;
+                } else {
+                    more = false;
+                }
+            }
+            __syncwarp();
+            /* certificates of the first 32 open pairs; those left join their
+               configurations' lists in order */
+            unsigned own = 32u, j = 0u;
+            bool need = false;
+            if (lane < n) {
+                own = A.open[lane] & 31u;
+                j = A.open[lane] >> 5;
+                need = !frames_certified(sc, S, S.frames - lane + own, (int)j);
+            }
+            const unsigned same = __match_any_sync(FULL_MASK, need ? own : 32u);
+            if (need) {
+                const int at = A.count[own] + __popc(same & ((1u << lane) - 1u));
+                if (at < VERTEX_TESTS) A.test[at][own] = j;
+                else atomicMin(&A.resume[own], j);
+            }
+            __syncwarp();
+            if (need && (same >> lane) == 1u)   /* the last of its configuration */
+                A.count[own] = min(A.count[own] + __popc(same), VERTEX_TESTS);
+            const int left = n > 32 ? n - 32 : 0;       /* at most 31 */
+            const unsigned mv = lane < left ? A.open[32 + lane] : 0u;
+            __syncwarp();
+            if (lane < left) A.open[lane] = mv;
+            n = left;
+            __syncwarp();
+        }
+        /* the exact tests in rounds */
+        const int tests = A.count[lane];
+        int done = 0;
+#pragma unroll 1
+        for (;;) {
+            const bool open = done < tests && A.jkey[lane] == JKEY_NONE;
+            const unsigned m = __ballot_sync(FULL_MASK, open);
+            if (!m) break;
+            const int per = 32 / __popc(m);             /* tests each gives */
+            __syncwarp();
+            A.open[lane] = PAIR_NONE;
+            __syncwarp();
+            if (open) {
+                const int at = __popc(m & ((1u << lane) - 1u)) * per;
+                for (int k = 0; k < per && done + k < tests; ++k)
+                    A.open[at + k] = (unsigned)lane | (A.test[done + k][lane] << 5);
+            }
+            done += per;
+            __syncwarp();
+            const unsigned it = A.open[lane];
+            if (it != PAIR_NONE) {
+                const int own = (int)(it & 31u), j = (int)(it >> 5);
+                const int4 pr = S.pairs[j];
+                Frame<float> tp, tq;
+                pair_frames(S.frames - lane + own, pr, tp, tq);
+                float mg;
+                int code;
+                if constexpr (FAST) code = pair_test_fast(sc, S.tab, pr, sc.ppoly[j], tp, tq, &mg);
+                else code = pair_test<PF32>(sc, S.tab, pr, tp, tq, &mg);
+                ++pc.full;
+                --pc.cert;
+                if (code != 0) {
+                    const unsigned inb = band_on && in_band(code, mg, band) ? 16u : 0u;
+                    atomicMin(&A.jkey[own], ((unsigned)j << 5) | inb | (unsigned)(code + 1));
+                } else if (!(mg >= band)) {
+                    atomicMin(&A.jfirst[own], (unsigned)j);
+                    atomicMax(&A.jlast[own], j);
+                }
+            }
+            __syncwarp();
+        }
+        from = A.resume[lane];
+        todo = __ballot_sync(FULL_MASK, from != PAIR_NONE && A.jkey[lane] == JKEY_NONE);
+        __syncwarp();
+    }
+    int code = valid && !active ? 1 : 0;
+    bool want = false;
+    int jrec = 0x7fffffff, jlast = -1;
+    if (active) {
+        const unsigned jk = A.jkey[lane], jf = A.jfirst[lane];
+        jrec = (int)min(jf, jk >> 5);
+        if (jk != JKEY_NONE) {
+            code = (int)(jk & 15u) - 1;
+            want = (jk & 16u) != 0u;
+        } else {
+            want = band_on && jf != PAIR_NONE;
+            jlast = A.jlast[lane];
+        }
+    }
     if (valid) {
-        exec += (code != 1);
+        exec += active;
         res[i] = code;
     }
-    bool want = valid && band_on && code != 1 && in_band(code, code == 0 ? mmin : mdec, band);
-    warp_append(want, make_uint2((unsigned)i, (unsigned)(code + 1) << 27),
-                recheck_range(code, st.jrec, st.jlast, sc.npairs), bq, ctl);
+    warp_append(want, make_uint2((unsigned)i, (unsigned)(code + 1) << 27), recheck_range(code, jrec, jlast, sc.npairs),
+                bq, ctl);
+    __syncwarp();
 }
 
 template <bool SMEM, bool FAST>
@@ -821,7 +953,7 @@ __device__ __forceinline__ void check_edge(const DevScene& sc, const SceneView& 
             if (g0 % SWEEP_GROUP == 0)
                 sweep_stage(sc, S, g0 / SWEEP_GROUP, (min(sc.npairs - g0, SWEEP_GROUP) + 31) >> 5);
             const int wi = ((g0 % SWEEP_GROUP) >> 5) + lane;
-            const unsigned open = g0 + 32 * lane < gend ? S.defer[wi] : 0u;
+            const unsigned open = g0 + 32 * lane < gend ? S.bits[wi] : 0u;
             unsigned left = __ballot_sync(FULL_MASK, open != 0u);
             int pos = g0;   /* pairs before it are counted */
             while (left) {
@@ -1592,13 +1724,13 @@ __device__ __forceinline__ void small_pairs(const DevScene& sc, const SceneView&
 #pragma unroll 1
     for (int g0 = 0; g0 < sc.npairs; g0 += SWEEP_GROUP) {
         const int words = (min(sc.npairs - g0, SWEEP_GROUP) + 31) >> 5;
-        for (int w = threadIdx.x; w < words; w += SMALL_WARPS * 32) S.defer[w] = 0u;
+        for (int w = threadIdx.x; w < words; w += SMALL_WARPS * 32) S.bits[w] = 0u;
         __syncthreads();
-        sweep_leaves(sc, S, g0 / SWEEP_GROUP, 0x11111111u << warp);
+        sweep_leaves<false>(sc, S, g0 / SWEEP_GROUP, 0x11111111u << warp, sc.nslots <= SWEEP_V0_SLOTS, SWEEP_V0_SLOTS);
         __syncthreads();
 #pragma unroll 1
         for (int w = warp; w < words; w += SMALL_WARPS) {
-            const unsigned cand = S.defer[w];
+            const unsigned cand = S.bits[w];
             if (!cand) continue;
             const int j0 = g0 + 32 * w;
             bool scan = mine && ((unsigned)j0 << 8) <= *(volatile unsigned*)&B.jkey[lane];
@@ -1635,7 +1767,7 @@ __device__ __forceinline__ SceneView small_view(const DevScene& sc, unsigned cha
     S.frames = reinterpret_cast<float*>(smem) + (threadIdx.x & 31);
     S.cen = S.frames + (size_t)sc.ndof * 12 * 32;
     S.sweep = sweep_area<false>(sc, S.frames);
-    S.defer = defer_area<false>(sc, S.frames);
+    S.bits = open_area<false>(sc, S.frames);
     return S;
 }
 
@@ -2244,7 +2376,7 @@ __device__ __forceinline__ void switch_scene(const BatchView& B, int p, DevScene
     S.frames = frames;
     S.cen = frames + (size_t)wsc->ndof * 12 * 32;
     S.sweep = sweep_area<VERTEX>(*wsc, frames);
-    S.defer = defer_area<VERTEX>(*wsc, frames);
+    S.bits = open_area<VERTEX>(*wsc, frames);
 }
 
 template <bool FAST>

@@ -117,7 +117,7 @@ def test_requests_in_flight_together():
         np.testing.assert_array_equal(res, w)
 
 
-@pytest.mark.parametrize("kind,n", [("box4", 300), ("box4", 120000), ("hull6", 2000), ("wall7", 17000)])
+@pytest.mark.parametrize("kind,n", [("box4", 300), ("box4", 120000), ("hull6", 2000), ("wall7", 40000)])
 def test_large_path_rechecks_by_warp_and_by_thread_equal_the_oracle(kind, n):
     """The large path's FP64 recheck takes a warp per item for few items and
     a thread per item for many (a wide band makes many)."""
