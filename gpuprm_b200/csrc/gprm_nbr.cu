@@ -16,12 +16,11 @@
  *            the lower index.  Nodes are bucketed into a uniform grid over
  *            all joints (counting sort by cell); a query scans the
  *            3^ndof cells around its own and keeps a sorted top-k
- *            (a thread per query for the nodes themselves, a warp per query
- *            for outside queries); a
+ *            (a warp per query); a
  *            result is accepted only when its k-th distance is below the
  *            distance to the scanned block's boundary (with slack for float
- *            rounding), otherwise the query is redone over the 5^ndof block
- *            by a block of threads, and if that block's test fails too, by a
+ *            rounding), otherwise the query is redone over the 5^ndof block,
+ *            and if that block's test fails too, by a
  *            block that scans every node.  The result is therefore the exact
  *            top-k.
  *
@@ -33,6 +32,7 @@
 #include <stdarg.h>
 #include <stdio.h>
 
+#include <algorithm>
 #include <string>
 #include <vector>
 
@@ -43,6 +43,10 @@ namespace {
 constexpr int NBR_MAX_GRID = GPRM_MAX_DOF;
 constexpr int NBR_MAX_K = 32;
 constexpr int NBR_MAX_CELLS = 1 << 21;
+/* cell size over the estimated distance of the 16th neighbour: smaller cells
+ * hold fewer nodes out of reach, but more queries outgrow their 3^ndof block
+ * (480,001 6-D nodes, k = 10: 3.5 ms at 1.1, 4.5 at 1.0, 8.3 at 0.9) */
+constexpr double KNN_CELL = 1.1;
 
 struct GridView {
     int ndof, G, n;
@@ -289,60 +293,243 @@ __device__ __forceinline__ bool knn_exact(const GridView& g, bool finite, int le
     return finite && len == k && (!isfinite(gs) || (gs > 0.0f && kth < gs * gs * 0.99999f));
 }
 
-/* Thread per query: the node at sorted position t (queries are the nodes;
- * neighbouring threads hold neighbouring nodes). */
-__global__ void k_knn_grid(GridView g, int m, int k, int* out_idx, float* out_dist, int* redo, int* nredo)
+/* A lower bound of the squared distance to a node in a cell whose coordinate
+ * range starts `gap` beyond q: shortened by the rounding of the cell
+ * assignment and of the nodes' computed distances, so that a node whose cell
+ * is skipped for it could not have entered the list. */
+__device__ __forceinline__ float gap2(const GridView& g, float gap)
 {
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < m; t += gridDim.x * blockDim.x) {
-        float qv[GPRM_MAX_DOF];
+    const float d = fmaxf(gap - g.slack, 0.0f);
+    return d * d * 0.99998f;
+}
+
+/* gap2 of coordinate v of joint d to the cells with coordinate c (the edge
+ * cells hold every node beyond the grid as well). */
+__device__ __forceinline__ float cell_gap2(const GridView& g, float v, int d, int c)
+{
+    const float below = c > 0 ? (g.lo[d] + (float)c * g.cell) - v : 0.0f;
+    const float above = c < g.nc[d] - 1 ? v - (g.lo[d] + (float)(c + 1) * g.cell) : 0.0f;
+    return gap2(g, fmaxf(below, above));
+}
+
+template <int N> struct Pow3 { static constexpr int value = 3 * Pow3<N - 1>::value; };
+template <> struct Pow3<0> { static constexpr int value = 1; };
+
+/* A warp's candidates of k_knn_grid. */
+constexpr int KNN_CAND = 128;
+struct KnnWarp {
+    float s[KNN_CAND];
+    int id[KNN_CAND];
+};
+
+/* Keeps the k smallest of the warp's n candidates (n <= KNN_CAND), sorted by
+ * (distance, index): k rounds of a warp minimum over four candidates a
+ * lane.  Squared distances are not negative, so their bits order like
+ * them. */
+__device__ __forceinline__ void knn_select(KnnWarp& W, int& n, int k)
+{
+    const int lane = threadIdx.x & 31;
+    unsigned s[4];
+    int id[4];
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int c = lane + 32 * u;
+        s[u] = c < n ? __float_as_uint(W.s[c]) : 0xffffffffu;
+        id[u] = c < n ? W.id[c] : 0x7fffffff;
+    }
+    __syncwarp();
+    if (k > n) k = n;
+    n = k;
+#pragma unroll 1
+    for (int r = 0; r < k; ++r) {
+        const unsigned m = __reduce_min_sync(0xffffffffu, min(min(s[0], s[1]), min(s[2], s[3])));
+        int mine = 0x7fffffff;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) mine = s[u] == m ? min(mine, id[u]) : mine;
+        const int best = __reduce_min_sync(0xffffffffu, mine);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) s[u] = s[u] == m && id[u] == best ? 0xffffffffu : s[u];
+        if (lane == 0) {
+            W.s[r] = __uint_as_float(m);
+            W.id[r] = best;
+        }
+    }
+    __syncwarp();
+}
+
+/* The nodes of the lanes' rows [b, e) (sorted positions; e = b: none), one
+ * after the other over the lanes: those within `reach` of q (not the node at
+ * position self_at or of index self_id) join the warp's n candidates, cut
+ * back to the k best, with the bound they give, when the buffer fills. */
+template <int DIM>
+__device__ __forceinline__ void knn_scan(const GridView& g, KnnWarp& W, const float* qv, int b, int e, int self_at,
+                                         int self_id, int k, int& n, float& reach)
+{
+    const int lane = threadIdx.x & 31;
+    int upto = e - b;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, upto, d);
+        if (lane >= d) upto += y;
+    }
+    const int total = __shfl_sync(0xffffffffu, upto, 31);
+    const int shift = b - (upto - (e - b));         /* node = its number + its row's shift */
+#pragma unroll 1
+    for (int f0 = 0; f0 < total; f0 += 32) {
+        const int f = f0 + lane;
+        int row = 0;                                /* the first row with upto > f */
+#pragma unroll
+        for (int d = 16; d >= 1; d >>= 1) {
+            const int y = __shfl_sync(0xffffffffu, upto, row + d - 1);
+            if (y <= f) row += d;
+        }
+        const int p = f + __shfl_sync(0xffffffffu, shift, row & 31);
+        bool hit = false;
+        float s = 0.0f;
+        int id = 0;
+        if (f < total) {
+#pragma unroll
+            for (int j = 0; j < DIM; ++j) {
+                const float d = g.xs[p + (long long)g.n * j] - qv[j];
+                s = s + d * d;
+            }
+            if (s != s) s = INFINITY;               /* NaN sorts last */
+            hit = s <= reach && p != self_at;
+            if (hit) {
+                id = g.id[p];
+                hit = id != self_id;
+            }
+        }
+        const unsigned hm = __ballot_sync(0xffffffffu, hit);
+        if (hm) {
+            if (n > KNN_CAND - 32) {
+                knn_select(W, n, k);
+                if (n == k) reach = fminf(reach, W.s[k - 1]);
+            }
+            if (hit) {
+                const int at = n + __popc(hm & ((1u << lane) - 1u));
+                W.s[at] = s;
+                W.id[at] = id;
+            }
+            n += __popc(hm);
+        }
+    }
+}
+
+/* A warp per query, the node at sorted position t (queries are the nodes;
+ * neighbouring warps hold neighbouring nodes).  Of the 3^DIM cells around
+ * the query's, in rows of three along joint 0, first the own row and those
+ * one cell away in one other joint are read: the k-th distance so far is
+ * then a bound within which few of the other rows lie (the ball of the k-th
+ * distance holds k of the block's about 3000 nodes).  A lane per row adds up
+ * the gaps to its cells; the rows in reach are read eight at a time, four
+ * lanes a row.  Nodes within the bound are collected and cut back to the k
+ * best when the buffer fills.  A query that the block cannot settle leaves
+ * its k-th squared distance in its last output slot for k_knn_wide.
+ * 480,001 6-D nodes, k = 10: 7.1 ms with a thread per query reading every
+ * cell, 4.5 ms with a thread per query and the bound (10 of 32 lanes
+ * active), 3.7 ms
+ * with four lanes a row. */
+template <int DIM>
+__global__ void __launch_bounds__(256) k_knn_grid(GridView g, int m, int k, int* out_idx, float* out_dist, int* redo,
+                                                  int* nredo)
+{
+    constexpr int ROWS = Pow3<DIM - 1>::value;
+    __shared__ unsigned short digits[ROWS];      /* per row two bits a joint: own, below, above; few moves first */
+    __shared__ int slot[8];
+    __shared__ KnnWarp ws[8];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x < 8) slot[threadIdx.x] = 0;
+    __syncthreads();
+    for (int pass = 0; pass < 2; ++pass) {
+        for (int r = threadIdx.x; r < ROWS; r += blockDim.x) {
+            int rest = r, moved = 0, dg = 0;
+            for (int d = 0; d < DIM - 1; ++d) {
+                const int c = rest % 3;
+                rest /= 3;
+                moved += c != 0;
+                dg |= c << (2 * d);
+            }
+            const int at = atomicAdd(&slot[moved], 1);
+            if (pass == 1) digits[at] = (unsigned short)dg;
+        }
+        __syncthreads();
+        if (pass == 0 && threadIdx.x == 0) {
+            int sum = 0;
+            for (int c = 0; c < 8; ++c) {
+                const int n = slot[c];
+                slot[c] = sum;
+                sum += n;
+            }
+        }
+        __syncthreads();
+    }
+    KnnWarp& W = ws[warp];
+    for (int t = blockIdx.x * 8 + warp; t < m; t += gridDim.x * 8) {
+        float qv[DIM];
         const int qid = g.id[t];
-        for (int j = 0; j < g.ndof; ++j) qv[j] = g.xs[t + (long long)g.n * j];
-        float ts[NBR_MAX_K];
-        int ti[NBR_MAX_K];
-        int len = 0;
-        TopkBound bound{INFINITY, 0x7fffffff};
+#pragma unroll
+        for (int j = 0; j < DIM; ++j) qv[j] = g.xs[t + (long long)g.n * j];
         int lo[NBR_MAX_GRID], hi[NBR_MAX_GRID];
         float guard;
         const bool finite = query_block(g, qv, lo, hi, &guard);
-        const int rows = block_rows(g, lo, hi);
-        for (int r = 0; r < rows; ++r) {
-            int b, e;
-            block_row_range(g, lo, hi, r, &b, &e);
-            int p = b;
-            for (; p + 4 <= e; p += 4) {
-                float s4[4];
-                dist2_4(g.xs, g.n, p, qv, g.ndof, s4);
+        float below[DIM], above[DIM];            /* squared gaps, INFINITY: no such cell */
+        int stride[DIM], own = 0, cells = 1;
 #pragma unroll
-                for (int u = 0; u < 4; ++u) {
-                    float sd = s4[u];
-                    if (p + u == t) continue;      /* the query itself */
-                    if (sd != sd) sd = INFINITY;   /* NaN sorts last */
-                    if (sd > bound.s) continue;    /* cannot enter the list */
-                    const int nid = g.id[p + u];
-                    if (!less_pair(sd, nid, bound.s, bound.i)) continue;
-                    topk_insert(ts, ti, len, k, sd, nid);
-                    topk_bound(ts, ti, len, k, bound);
+        for (int d = 0; d < DIM; ++d) {
+            const int c = cell_coord(qv[d], g.lo[d], g.inv_cell, g.nc[d]);
+            own += c * cells;
+            stride[d] = cells;
+            cells *= g.nc[d];
+            below[d] = c > lo[d] ? gap2(g, qv[d] - (g.lo[d] + (float)c * g.cell)) : INFINITY;
+            above[d] = c < hi[d] ? gap2(g, (g.lo[d] + (float)(c + 1) * g.cell) - qv[d]) : INFINITY;
+        }
+        int n = 0;
+        float reach = INFINITY;                  /* nodes beyond it cannot enter the list */
+        const int first = 2 * DIM - 1;
+#pragma unroll 1
+        for (int r0 = 0; r0 < ROWS; r0 += r0 == 0 ? first : 32) {
+            const int r1 = r0 == 0 ? (first < 32 ? first : 32) : min(ROWS, r0 + 32);
+            const int r = r0 + lane;
+            bool open = false;
+            int b = 0, e = 0;
+            if (r < r1) {
+                const unsigned dg = digits[r];
+                float gap = 0.0f;
+                int cell = own;
+#pragma unroll
+                for (int d = 1; d < DIM; ++d) {
+                    const unsigned c = (dg >> (2 * (d - 1))) & 3u;
+                    gap = c == 0u ? gap : gap + (c == 1u ? below[d] : above[d]);
+                    cell += c == 0u ? 0 : c == 1u ? -stride[d] : stride[d];
+                }
+                open = gap <= reach && gap != INFINITY;
+                if (open) {
+                    b = g.start[cell - (below[0] != INFINITY && gap + below[0] <= reach)];
+                    e = g.start[cell + 1 + (above[0] != INFINITY && gap + above[0] <= reach)];
+                    open = e > b;
                 }
             }
-            for (; p < e; ++p) {
-                if (p == t) continue;
-                float sd = dist2(g.xs, g.n, p, qv, g.ndof);
-                if (sd != sd) sd = INFINITY;
-                if (sd > bound.s) continue;
-                const int nid = g.id[p];
-                if (!less_pair(sd, nid, bound.s, bound.i)) continue;
-                topk_insert(ts, ti, len, k, sd, nid);
-                topk_bound(ts, ti, len, k, bound);
+            knn_scan<DIM>(g, W, qv, open ? b : 0, open ? e : 0, t, -1, k, n, reach);
+            if (n > k) {
+                /* a tighter bound for the rows to come */
+                knn_select(W, n, k);
+                reach = W.s[k - 1];
             }
         }
-        if (knn_exact(g, finite, len, k, len ? ts[len - 1] : INFINITY, guard)) {
-            for (int r = 0; r < k; ++r) {
-                out_idx[(long long)qid * k + r] = ti[r];
-                out_dist[(long long)qid * k + r] = sqrtf(ts[r]);
+        knn_select(W, n, k);
+        const float kth = n ? W.s[n - 1] : INFINITY;
+        if (knn_exact(g, finite, n, k, kth, guard)) {
+            if (lane < k) {
+                out_idx[(long long)qid * k + lane] = W.id[lane];
+                out_dist[(long long)qid * k + lane] = sqrtf(W.s[lane]);
             }
-        } else {
+        } else if (lane == 0) {
+            out_dist[(long long)qid * k + k - 1] = finite && n == k ? kth : INFINITY;
             redo[atomicAdd(nredo, 1)] = qid;
         }
+        __syncwarp();
     }
 }
 
@@ -415,78 +602,81 @@ __global__ void k_knn_grid_warp(GridView g, const float* __restrict__ q, int m, 
                 out_dist[(long long)t * k + lane] = sqrtf(my_s);
             }
         } else if (lane == 0) {
+            out_dist[(long long)t * k + k - 1] = finite && found == k ? kth : INFINITY;
             redo[atomicAdd(nredo, 1)] = t;
         }
     }
 }
 
-/* Second try for the queries the 3^ndof block could not settle: one block
- * of threads per query scans the 5^ndof block around it (its rows split
- * over the threads, each keeping its own top-k, merged as in k_knn_full)
- * and applies the same exactness test with that block's guard; a query it
- * cannot settle either goes to the full scan (redo2). */
+/* Second try for the queries the 3^ndof block could not settle: a warp per
+ * query goes through the 5^ndof block around it and applies the same
+ * exactness test with that block's guard; a query it cannot settle either
+ * goes to the full scan (redo2).  The k-th squared distance over the 3^ndof
+ * block, left in the query's last output slot, bounds the true one from the
+ * start: few of the block's rows are in its reach.  (A block of threads per
+ * query that read every row took 3.6 ms for 6,600 of 480,001 6-D queries,
+ * with the bound 0.8 ms.) */
+template <int DIM>
 __global__ void __launch_bounds__(256) k_knn_wide(GridView g, const float* __restrict__ q, long long qstride, int k,
                                                   int exclude_self, const int* __restrict__ redo,
                                                   const int* __restrict__ nredo, int* redo2, int* nredo2,
                                                   int* out_idx, float* out_dist)
 {
-    __shared__ float ms[8 * NBR_MAX_K];
-    __shared__ int mi[8 * NBR_MAX_K];
+    constexpr int SPAN = 5;
+    __shared__ KnnWarp ws[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    KnnWarp& W = ws[warp];
     const int cnt = *nredo;
-    for (int w = blockIdx.x; w < cnt; w += gridDim.x) {
+    for (int w = blockIdx.x * 8 + warp; w < cnt; w += gridDim.x * 8) {
         const int qid = redo[w];
-        float qv[GPRM_MAX_DOF];
-        for (int j = 0; j < g.ndof; ++j) qv[j] = q[qid + qstride * j];
-        float ts[NBR_MAX_K];
-        int ti[NBR_MAX_K];
-        int len = 0;
-        TopkBound bound{INFINITY, 0x7fffffff};
+        float qv[DIM];
+#pragma unroll
+        for (int j = 0; j < DIM; ++j) qv[j] = q[qid + qstride * j];
         int lo[NBR_MAX_GRID], hi[NBR_MAX_GRID];
         float guard;
-        const bool finite = query_block(g, qv, lo, hi, &guard, 2);
-        const int rows = block_rows(g, lo, hi);
-        for (int r = threadIdx.x; r < rows; r += blockDim.x) {
-            int b, e;
-            block_row_range(g, lo, hi, r, &b, &e);
-            for (int p = b; p < e; ++p) {
-                const int nid = g.id[p];
-                if (exclude_self && nid == qid) continue;
-                float sd = dist2(g.xs, g.n, p, qv, g.ndof);
-                if (sd != sd) sd = INFINITY;
-                if (!less_pair(sd, nid, bound.s, bound.i)) continue;
-                topk_insert(ts, ti, len, k, sd, nid);
-                topk_bound(ts, ti, len, k, bound);
-            }
-        }
-        float my_s, kth;
-        int my_i, found;
-        warp_topk_merge(ts, ti, len, k, &my_s, &my_i, &kth, &found);
-        if (lane < k) {
-            ms[warp * k + lane] = my_s;
-            mi[warp * k + lane] = my_i < 0 ? 0x7fffffff : my_i;
-        }
-        __syncthreads();
-        if (warp == 0) {
-            len = 0;
-            bound = TopkBound{INFINITY, 0x7fffffff};
-            for (int e = lane; e < 8 * k; e += 32) {
-                if (mi[e] == 0x7fffffff) continue;
-                if (!less_pair(ms[e], mi[e], bound.s, bound.i)) continue;
-                topk_insert(ts, ti, len, k, ms[e], mi[e]);
-                topk_bound(ts, ti, len, k, bound);
-            }
-            warp_topk_merge(ts, ti, len, k, &my_s, &my_i, &kth, &found);
-            if (knn_exact(g, finite, found, k, kth, guard)) {
-                if (lane < k) {
-                    out_idx[(long long)qid * k + lane] = my_i;
-                    out_dist[(long long)qid * k + lane] = sqrtf(my_s);
+        const bool finite = query_block(g, qv, lo, hi, &guard, SPAN / 2);
+        float reach = out_dist[(long long)qid * k + k - 1];
+        const int self = exclude_self ? qid : -1;
+        int n = 0, rows = 1;
+#pragma unroll
+        for (int d = 1; d < DIM; ++d) rows *= hi[d] - lo[d] + 1;
+#pragma unroll 1
+        for (int r0 = 0; r0 < rows; r0 += 32) {
+            const int r = r0 + lane;
+            int b = 0, e = 0;
+            if (r < rows) {
+                float gap = 0.0f;
+                int rest = r, cell = 0, cells = g.nc[0];
+#pragma unroll
+                for (int d = 1; d < DIM; ++d) {
+                    const int span = hi[d] - lo[d] + 1;
+                    const int c = lo[d] + rest % span;
+                    rest /= span;
+                    gap = gap + cell_gap2(g, qv[d], d, c);
+                    cell += c * cells;
+                    cells *= g.nc[d];
                 }
-            } else if (lane == 0) {
-                redo2[atomicAdd(nredo2, 1)] = qid;
+                if (gap <= reach) {
+                    int c0 = lo[0], c1 = hi[0];
+                    while (c0 < c1 && gap + cell_gap2(g, qv[0], 0, c0) > reach) ++c0;
+                    while (c1 > c0 && gap + cell_gap2(g, qv[0], 0, c1) > reach) --c1;
+                    b = g.start[cell + c0];
+                    e = g.start[cell + c1 + 1];
+                }
             }
+            if (__any_sync(0xffffffffu, e > b)) knn_scan<DIM>(g, W, qv, b, e, -1, self, k, n, reach);
         }
-        __syncthreads();
+        knn_select(W, n, k);
+        const float kth = n ? W.s[n - 1] : INFINITY;
+        if (knn_exact(g, finite, n, k, kth, guard)) {
+            if (lane < k) {
+                out_idx[(long long)qid * k + lane] = W.id[lane];
+                out_dist[(long long)qid * k + lane] = sqrtf(W.s[lane]);
+            }
+        } else if (lane == 0) {
+            redo2[atomicAdd(nredo2, 1)] = qid;
+        }
+        __syncwarp();
     }
 }
 
@@ -699,7 +889,7 @@ int gprm_nbr_build(gprm_nbr* h, const float* x, int n, int stride, float cell, v
     double c = cell;
     if (!(c > 0.0)) {
         const double unit = pow(M_PI, nd / 2.0) / tgamma(nd / 2.0 + 1.0);
-        c = 1.1 * pow(16.0 * vol / ((n > 0 ? n : 1) * unit), 1.0 / nd);
+        c = KNN_CELL * pow(16.0 * vol / ((n > 0 ? n : 1) * unit), 1.0 / nd);
     }
     long long ncells = 1;
     for (int d = 0; d < G; ++d) {
@@ -782,9 +972,14 @@ int gprm_nbr_knn(gprm_nbr* h, const float* q, int m, int qstride, int k, int que
     if ((rc = grow(h, &h->redo2, h->cap_redo2, (size_t)m))) return rc;
     NBR_TRY(h, cudaMemsetAsync(h->nredo, 0, 2 * sizeof(int), st));
     if (queries_are_nodes) {
-        const int threads = 128;
-        const int blocks = (int)((m + threads - 1) / threads);
-        k_knn_grid<<<blocks, threads, 0, st>>>(h->g, m, k, idx, dist, h->redo, h->nredo);
+        const int blocks = (int)std::min<long long>(((long long)m + 7) / 8, (long long)h->sms * 16);
+        switch (h->ndof) {
+#define GPRM_KNN_GRID(D)                                                                             \
+        case D: k_knn_grid<D><<<blocks, 256, 0, st>>>(h->g, m, k, idx, dist, h->redo, h->nredo); break
+        GPRM_KNN_GRID(1); GPRM_KNN_GRID(2); GPRM_KNN_GRID(3); GPRM_KNN_GRID(4);
+        GPRM_KNN_GRID(5); GPRM_KNN_GRID(6); GPRM_KNN_GRID(7);
+#undef GPRM_KNN_GRID
+        }
     } else {
         const int wpb = 8;
         const long long wblocks = ((long long)m + wpb - 1) / wpb;
@@ -792,8 +987,14 @@ int gprm_nbr_knn(gprm_nbr* h, const float* q, int m, int qstride, int k, int que
         k_knn_grid_warp<<<blocks, 32 * wpb, 0, st>>>(h->g, q, m, qstride, k, idx, dist, h->redo, h->nredo);
     }
     NBR_TRY(h, cudaGetLastError());
-    k_knn_wide<<<h->sms * 8, 256, 0, st>>>(h->g, q, qstride, k, queries_are_nodes ? 1 : 0, h->redo, h->nredo,
-                                           h->redo2, h->nredo + 1, idx, dist);
+    switch (h->ndof) {
+#define GPRM_KNN_WIDE(D)                                                                                           \
+    case D: k_knn_wide<D><<<h->sms * 8, 256, 0, st>>>(h->g, q, qstride, k, queries_are_nodes ? 1 : 0, h->redo, h->nredo, \
+                                                      h->redo2, h->nredo + 1, idx, dist); break
+        GPRM_KNN_WIDE(1); GPRM_KNN_WIDE(2); GPRM_KNN_WIDE(3); GPRM_KNN_WIDE(4);
+        GPRM_KNN_WIDE(5); GPRM_KNN_WIDE(6); GPRM_KNN_WIDE(7);
+#undef GPRM_KNN_WIDE
+    }
     NBR_TRY(h, cudaGetLastError());
     k_knn_full<<<h->sms * 8, 256, 0, st>>>(h->x, h->n, h->xstride, q, qstride, h->ndof, k, queries_are_nodes ? 1 : 0,
                                            h->redo2, h->nredo + 1, idx, dist);
