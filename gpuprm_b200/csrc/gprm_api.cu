@@ -425,6 +425,8 @@ int upload_certificates(gprm_space* h)
         CUDA_TRY(h, cudaMemcpy((void*)s.swj, L.pair.data(), L.pair.size() * 4, cudaMemcpyHostToDevice));
     }
     CUDA_TRY(h, cudaMemcpy((void*)s.swg, L.group.data(), L.group.size() * 4, cudaMemcpyHostToDevice));
+    /* the checks run on streams that do not wait for these copies */
+    CUDA_TRY(h, cudaStreamSynchronize(cudaStreamLegacy));
     return GPRM_OK;
 }
 
@@ -1175,6 +1177,7 @@ int gprm_init(gprm_space* h, int rank, int size)
     CUDA_TRY(h, plan_launch(s, 0, 128, &h->cfg_e));
     CUDA_TRY(h, dev_malloc((void**)&h->d_total, sizeof(Control)));
     CUDA_TRY(h, cudaMemset(h->d_total, 0, sizeof(Control)));
+    CUDA_TRY(h, cudaStreamSynchronize(cudaStreamLegacy));
     memset(&h->host_stats, 0, sizeof(h->host_stats));
     h->inited = true;
     return GPRM_OK;
@@ -1418,8 +1421,8 @@ int gprm_debug_fk(gprm_space* h, const float* q, float* out)
     float* d = nullptr;
     size_t nf = (size_t)(h->ndof + 1) * 12;
     CUDA_TRY(h, dev_malloc((void**)&d, (nf + 8) * sizeof(float)));
-    cudaMemcpy(d + nf, q, h->ndof * sizeof(float), cudaMemcpyHostToDevice);
-    cudaError_t e = launch_fk_probe(h->dsc, d + nf, d, h->stream);
+    cudaError_t e = cudaMemcpyAsync(d + nf, q, h->ndof * sizeof(float), cudaMemcpyHostToDevice, h->stream);
+    if (e == cudaSuccess) e = launch_fk_probe(h->dsc, d + nf, d, h->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
     if (e == cudaSuccess) e = cudaMemcpy(out, d, nf * sizeof(float), cudaMemcpyDeviceToHost);
     cudaFree(d);

@@ -298,6 +298,8 @@ int build_work(gprm_batch* b, int vertex_kernel, long long solo_min)
             BATCH_TRY(b, cudaMemcpy(L.d_wprob, wprob.data(), sizeof(int) * L.K, cudaMemcpyHostToDevice));
         }
     }
+    /* the checks run on streams that do not wait for these copies */
+    BATCH_TRY(b, cudaStreamSynchronize(cudaStreamLegacy));
     return GPRM_OK;
 }
 
@@ -360,6 +362,7 @@ int gprm_batch_create(gprm_space* const* spaces, int count, gprm_batch** out)
             BATCH_TRY(b, dev_malloc((void**)&b->d_total, sizeof(Control)));
             BATCH_TRY(b, dev_malloc((void**)&b->d_scratch_total, sizeof(Control)));
             BATCH_TRY(b, cudaMemset(b->d_total, 0, sizeof(Control)));
+            BATCH_TRY(b, cudaStreamSynchronize(cudaStreamLegacy));
             /* the two kinds' shared areas differ */
             BATCH_TRY(b, configure_batch_launch(view_of(b, 1), 1, 128, &b->cfg[1]));
             BATCH_TRY(b, configure_batch_launch(view_of(b, 0), 0, 128, &b->cfg[0]));

@@ -1832,6 +1832,7 @@ int tc_setup(gprm_mlp* h)
     if (h->dev_err) return GPRM_OK;
     MLP_TRY(h, cudaMalloc((void**)&h->dev_err, sizeof(unsigned)));
     MLP_TRY(h, cudaMemset(h->dev_err, 0, sizeof(unsigned)));
+    MLP_TRY(h, cudaStreamSynchronize(cudaStreamLegacy));   /* the kernels run on other streams */
     int dev = 0;
     MLP_TRY(h, cudaGetDevice(&dev));
     MLP_TRY(h, cudaDeviceGetAttribute(&h->sms, cudaDevAttrMultiProcessorCount, dev));
@@ -2017,7 +2018,10 @@ int gprm_mlp_set_params(gprm_mlp* h, const float* in)
 {
     if (!h || !in) return GPRM_ERR_ARG;
     MLP_TRY(h, cudaStreamSynchronize(h->st));
-    MLP_TRY(h, cudaMemcpy(h->w, in, h->nparam * sizeof(float), cudaMemcpyHostToDevice));
+    /* on the handle's stream: a copy from pageable memory on the default
+       stream may still be under way when it returns, and this stream does
+       not wait for that one */
+    MLP_TRY(h, cudaMemcpyAsync(h->w, in, h->nparam * sizeof(float), cudaMemcpyHostToDevice, h->st));
     k_to_bf16<<<256, 256, 0, h->st>>>(h->nparam, h->w, h->bf_map, h->wbf);
     MLP_TRY(h, cudaStreamSynchronize(h->st));
     return GPRM_OK;
@@ -2155,7 +2159,10 @@ int gprm_mlp_set_wait_budget(gprm_mlp* h, long long cycles)
     if (!h || cycles < 0) return GPRM_ERR_ARG;
     MLP_TRY(h, cudaDeviceSynchronize());
     h->wait_cycles = cycles;
-    if (h->dev_err) MLP_TRY(h, cudaMemset(h->dev_err, 0, sizeof(unsigned)));
+    if (h->dev_err) {
+        MLP_TRY(h, cudaMemsetAsync(h->dev_err, 0, sizeof(unsigned), h->st));
+        MLP_TRY(h, cudaStreamSynchronize(h->st));
+    }
     return GPRM_OK;
 }
 
