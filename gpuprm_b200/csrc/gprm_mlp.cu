@@ -23,6 +23,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <string>
 #include <vector>
 
@@ -283,6 +284,7 @@ __global__ void k_out(int n, const __nv_bfloat16* __restrict__ H, const __nv_bfl
     const long long io = idx_off ? *idx_off : 0;
     const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
     const int nw = (gridDim.x * blockDim.x) >> 5;
+    float lsum = 0.0f;
     for (int r = warp; r < n; r += nw) {
         float s = 0.0f;
         for (int k = lane; k < HID; k += 32)
@@ -296,22 +298,46 @@ __global__ void k_out(int n, const __nv_bfloat16* __restrict__ H, const __nv_bfl
                 const float yy = y[yidx ? yidx[io + r] : r];
                 /* BCE with logits, stable form */
                 const float l = fmaxf(logit, 0.0f) - logit * yy + log1pf(expf(-fabsf(logit)));
-                atomicAdd(loss, l * inv_b);
+                lsum += l * inv_b;
                 dlogit[r] = (pr - yy) * inv_b;
             }
         }
     }
+    /* one atomic per block: one per row queued 4096 of them on a word */
+    __shared__ float ls[32];
+    if (!y) return;
+    if (lane == 0) ls[threadIdx.x >> 5] = lsum;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < (int)(blockDim.x >> 5); ++w) lsum += ls[w];
+        atomicAdd(loss, lsum);
+    }
+}
+
+/* Bias corrections of Adam step t. */
+__device__ __forceinline__ void adam_corrections(double t, float* corr)
+{
+    corr[0] = (float)(1.0 - pow(0.9, t));
+    corr[1] = (float)(1.0 - pow(0.999, t));
 }
 
 /* output-layer backward: dZ4 = (dlogit w5) * gelu'(Z4), and per block the
  * partial sums of dw5 = H4^T dlogit (part[b][0..HID)) and db5 = sum dlogit
  * (part[b][HID]) over the rows r = b (mod gridDim.x); the partials are
  * added in block order afterwards, so the gradients do not depend on
- * scheduling. */
+ * scheduling.  ctl (training, or null): moves on to the next step, (offset
+ * of the step's rows in the shuffled order, Adam steps); every reader of
+ * this step's offset has finished, Adam comes after.  corr (or null): gets
+ * that step's Adam corrections. */
 __global__ void k_out_back(int n, const __nv_bfloat16* __restrict__ H, const float* __restrict__ Z,
                            const __nv_bfloat16* __restrict__ w5, const float* __restrict__ dlogit,
-                           float* __restrict__ part, __nv_bfloat16* __restrict__ dZ)
+                           float* __restrict__ part, __nv_bfloat16* __restrict__ dZ, long long* ctl, float* corr)
 {
+    if (ctl && blockIdx.x == 0 && threadIdx.x == 0) {
+        ctl[0] += n;
+        ctl[1] += 1;
+        if (corr) adam_corrections((double)ctl[1], corr);
+    }
     /* column k = threadIdx.x (HID threads) */
     const int k = threadIdx.x;
     float acc = 0.0f, accb = 0.0f;
@@ -347,15 +373,26 @@ __global__ void k_reduce_parts(int parts, int cols, const float* __restrict__ pa
 }
 
 /* Adam on the FP32 master parameters, refreshing their BF16 copies.
- * bf_map[i] = index into the bf16 array or -1. */
-__global__ void k_adam(long long n, float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
-                       float* __restrict__ v, const int* __restrict__ bf_map, __nv_bfloat16* __restrict__ wbf,
-                       float lr, float b1, float b2, float eps, const long long* __restrict__ t_base, long long t_step)
+ * bf_map[i] = index into the bf16 array or -1.  The bias corrections (two
+ * FP64 powers) are those of step t, or were left in corr by a kernel beside
+ * the backward GEMMs: per parameter they were most of the kernel (7.6 us for
+ * 203,000 parameters; once per block 6.1).  w1p, wt (or null): the
+ * training GEMMs' copies of the weights (k_tc_weights), o1 .. the hidden
+ * layers' offsets in wbf. */
+__global__ void __launch_bounds__(256) k_adam(long long n, float* __restrict__ w, const float* __restrict__ g,
+                                              float* __restrict__ m, float* __restrict__ v,
+                                              const int* __restrict__ bf_map, __nv_bfloat16* __restrict__ wbf, float lr,
+                                              float b1, float b2, float eps, long long t,
+                                              const float* __restrict__ corr, __nv_bfloat16* __restrict__ w1p,
+                                              __nv_bfloat16* __restrict__ wt, long long o1)
 {
-    /* step t = (*t_base) + t_step: read on the device so that one captured
-       training epoch serves every epoch */
-    const double t = (double)((t_base ? *t_base : 0) + t_step);
-    const float c1 = (float)(1.0 - pow(0.9, t)), c2 = (float)(1.0 - pow(0.999, t));
+    __shared__ float own[2];
+    if (!corr) {
+        if (threadIdx.x == 0) adam_corrections((double)t, own);
+        __syncthreads();
+        corr = own;
+    }
+    const float c1 = corr[0], c2 = corr[1];
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n;
          i += (long long)gridDim.x * blockDim.x) {
         const float gi = g[i];
@@ -366,7 +403,18 @@ __global__ void k_adam(long long n, float* __restrict__ w, const float* __restri
         const float wi = w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
         w[i] = wi;
         const int b = bf_map[i];
-        if (b >= 0) wbf[b] = __float2bfloat16(wi);
+        if (b < 0) continue;
+        const __nv_bfloat16 x = __float2bfloat16(wi);
+        wbf[b] = x;
+        if (!wt) continue;
+        /* the layers follow one another in wbf: W1 [HID x IN_PAD], then
+           three [HID x HID], then the output row */
+        if (b < o1) {
+            w1p[(b / IN_PAD) * 64 + b % IN_PAD] = x;
+        } else {
+            const long long u = b - o1, l = u / (HID * HID), r = u % (HID * HID);
+            if (l < NLAYER - 1) wt[l * HID * HID + (r % HID) * HID + r / HID] = x;
+        }
     }
 }
 
@@ -1333,11 +1381,14 @@ k_tc_gemm(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUte
  * b < cparts of cpart[b][o]; then, with opart, (HID + 1) x 32 threads:
  * go[c] = sum over b < oparts of opart[b][c] (the output layer's k_out_back
  * partials); both a warp per column in a fixed order.  rows * kin is a
- * multiple of 32, so every warp lies in one segment. */
+ * multiple of 32, so every warp lies in one segment.  corr (training): gets
+ * the Adam corrections of the step in ctl, ahead of k_adam. */
 __global__ void k_reduce_w(int splits, int rows, int ldw, int kin, const float* __restrict__ ws, float* __restrict__ gw,
                            int cparts, const float* __restrict__ cpart, float* __restrict__ gb,
-                           int oparts, const float* __restrict__ opart, float* __restrict__ go)
+                           int oparts, const float* __restrict__ opart, float* __restrict__ go,
+                           const long long* __restrict__ ctl, float* __restrict__ corr)
 {
+    if (corr && blockIdx.x == 0 && threadIdx.x == 0) adam_corrections((double)ctl[1], corr);
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t < rows * kin) {
         const int o = t / kin, i = t % kin;
@@ -1428,26 +1479,37 @@ __global__ void k_tc_weights(const __nv_bfloat16* __restrict__ wbf, long long o0
 }
 
 /* Features padded to 64 columns (the tensor-core K step): row i of X64 =
- * sin/cos of configuration idx[i] (or i), zeros beyond 2 ndof. */
-__global__ void k_features64(const float* __restrict__ q, long long offset, int ndof, int n,
-                             const int* __restrict__ idx, const long long* __restrict__ idx_off,
-                             __nv_bfloat16* __restrict__ X)
+ * sin/cos of configuration idx[i] (or i), zeros beyond 2 ndof.  Eight
+ * threads a row, one joint and one 16-byte store each (a thread per row left
+ * 16 blocks for a batch of 4096: 7.5 us). */
+static_assert(IN_PAD == 16, "eight joints a row");
+__global__ void __launch_bounds__(256) k_features64(const float* __restrict__ q, long long offset, int ndof, int n,
+                                                    const int* __restrict__ idx, const long long* __restrict__ idx_off,
+                                                    __nv_bfloat16* __restrict__ X)
 {
     const long long io = idx_off ? *idx_off : 0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const long long src = idx ? idx[io + i] : i;
-        uint32_t x[32];
-#pragma unroll
-        for (int j = 0; j < 32; ++j) x[j] = 0u;
-#pragma unroll
-        for (int j = 0; j < IN_PAD / 2; ++j) {
-            float sv = 0.0f, cv = 0.0f;
-            if (j < ndof) sincosf(q[src + offset * j], &sv, &cv);
-            x[j] = pack_bf16(j < ndof ? sv : 0.0f, j < ndof ? cv : 0.0f);
+    const int j = threadIdx.x & 7;
+    const long long rows = ((long long)n + 31) / 32 * 32;     /* whole blocks: the row's threads stay together */
+    for (long long i = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 3; i < rows;
+         i += (gridDim.x * (long long)blockDim.x) >> 3) {
+        uint32_t x = 0u;
+        if (i < n && j < ndof) {
+            const long long src = idx ? idx[io + i] : i;
+            float sv, cv;
+            sincosf(q[src + offset * j], &sv, &cv);
+            x = pack_bf16(sv, cv);
+        } else {
+            x = pack_bf16(0.0f, 0.0f);
         }
-        uint4* row = reinterpret_cast<uint4*>(X + (size_t)i * 64);
-#pragma unroll
-        for (int c = 0; c < 8; ++c) row[c] = make_uint4(x[4 * c], x[4 * c + 1], x[4 * c + 2], x[4 * c + 3]);
+        /* thread c < 2 of the row gathers joints 4c .. 4c + 3 */
+        const int c4 = (j & 1) * 4;
+        uint4 v;
+        v.x = __shfl_sync(0xffffffffu, x, c4, 8);
+        v.y = __shfl_sync(0xffffffffu, x, c4 + 1, 8);
+        v.z = __shfl_sync(0xffffffffu, x, c4 + 2, 8);
+        v.w = __shfl_sync(0xffffffffu, x, c4 + 3, 8);
+        if (j >= 2) v = make_uint4(0u, 0u, 0u, 0u);
+        if (i < n) reinterpret_cast<uint4*>(X + (size_t)i * 64)[j] = v;
     }
 }
 
@@ -1460,6 +1522,7 @@ __global__ void k_features64(const float* __restrict__ q, long long offset, int 
 struct gprm_mlp {
     int ndof = 6;
     int max_batch = 0;
+    bool weights_kept = false;    /* capturing training steps: Adam keeps the GEMMs' copies of the weights */
     /* parameter vector (fp32 master): W1[HID x IN_PAD] b1 W2 b2 W3 b3 W4 b4 w5[HID] b5[1] */
     long long nparam = 0;
     long long offW[NLAYER + 1], offB[NLAYER + 1];
@@ -1473,8 +1536,8 @@ struct gprm_mlp {
     __nv_bfloat16* H[NLAYER] = {nullptr};
     float* Z[NLAYER] = {nullptr};
     __nv_bfloat16* dZ[NLAYER] = {nullptr};
-    float *p = nullptr, *dlogit = nullptr, *loss = nullptr, *ybatch = nullptr;
-    int* idx = nullptr;
+    float *p = nullptr, *dlogit = nullptr, *loss = nullptr;
+    void* batch_mem = nullptr;          /* the buffers of alloc_batch */
     long long adam_t = 0;
     cudaStream_t st = nullptr;
     /* inference on the tensor-core layers (k_mlp_tc) */
@@ -1487,7 +1550,7 @@ struct gprm_mlp {
     __nv_bfloat16* X64 = nullptr;       /* features padded to 64 columns [rows x 64] */
     /* the weight-gradient chain of each layer (transposes, split-K GEMM,
        ordered reduction) has its own buffers, so that the chains of
-       different layers can run side by side on st_w */
+       different layers run side by side, each on its own stream st_w[l] */
     __nv_bfloat16 *Ta = nullptr, *Tb = nullptr;   /* transposes [NLAYER][256 x ldT] */
     int ldT = 0;
     __nv_bfloat16* w1p = nullptr;       /* W1 padded [256 x 64] */
@@ -1495,13 +1558,13 @@ struct gprm_mlp {
     float* ws = nullptr;                /* split-K partials [NLAYER][TG_MAX_SPLITS x 256 x 256] */
     float* cpart = nullptr;             /* bias-gradient partials [NLAYER][cparts x 256] */
     size_t cparts = 0;
-    cudaStream_t st_w = nullptr;        /* weight-gradient chains */
+    cudaStream_t st_w[NLAYER] = {};     /* weight-gradient chains */
     cudaEvent_t ev_dz[NLAYER] = {};     /* dZ_l written (on st) */
-    cudaEvent_t ev_w = nullptr;         /* every chain done (on st_w) */
+    cudaEvent_t ev_w[NLAYER] = {};      /* layer l's chain done (on st_w[l]) */
     float* opart = nullptr;             /* output-layer gradient partials [1024 x 257] */
     int tc_n = -1;                      /* batch the tensor maps were made for */
     int tc_attr = 0;
-    long long* d_ctl = nullptr;         /* training epoch: [row offset into perm, Adam step before it] */
+    long long* d_ctl = nullptr;         /* training: [the step's row offset into perm, Adam steps, two floats: its corrections] */
     const long long* idx_off = nullptr; /* set while a training epoch is captured */
     CUtensorMap m_x64, m_h[NLAYER - 1], m_dz[NLAYER], m_w1p, m_w[NLAYER - 1], m_wt[NLAYER - 1], m_ta[NLAYER],
         m_tb256[NLAYER], m_tb64;
@@ -1531,39 +1594,48 @@ int mfail(gprm_mlp* h, int code, const char* msg, cudaError_t e = cudaSuccess)
 int alloc_batch(gprm_mlp* h, int rows)
 {
     if (rows <= h->max_batch) return GPRM_OK;
-    cudaFree(h->X);
-    for (int l = 0; l < NLAYER; ++l) { cudaFree(h->H[l]); cudaFree(h->Z[l]); cudaFree(h->dZ[l]); }
-    cudaFree(h->p); cudaFree(h->dlogit); cudaFree(h->ybatch); cudaFree(h->idx);
-    size_t R = (size_t)rows;
-    MLP_TRY(h, cudaMalloc((void**)&h->X, R * IN_PAD * sizeof(__nv_bfloat16)));
-    for (int l = 0; l < NLAYER; ++l) {
-        MLP_TRY(h, cudaMalloc((void**)&h->H[l], R * HID * sizeof(__nv_bfloat16)));
-        MLP_TRY(h, cudaMalloc((void**)&h->Z[l], R * HID * sizeof(float)));
-        MLP_TRY(h, cudaMalloc((void**)&h->dZ[l], R * HID * sizeof(__nv_bfloat16)));
-    }
-    MLP_TRY(h, cudaMalloc((void**)&h->p, R * sizeof(float)));
-    MLP_TRY(h, cudaMalloc((void**)&h->dlogit, R * sizeof(float)));
-    MLP_TRY(h, cudaMalloc((void**)&h->ybatch, R * sizeof(float)));
-    MLP_TRY(h, cudaMalloc((void**)&h->idx, R * sizeof(int)));
-    cudaFree(h->X64); cudaFree(h->Ta); cudaFree(h->Tb); cudaFree(h->cpart);
-    h->cpart = nullptr;
-    const size_t cparts = std::max<size_t>(1024, (R + 31) / 32);
-    h->cparts = cparts;
-    MLP_TRY(h, cudaMalloc((void**)&h->cpart, (size_t)NLAYER * cparts * HID * sizeof(float)));
-    if (!h->opart) MLP_TRY(h, cudaMalloc((void**)&h->opart, (size_t)1024 * (HID + 1) * sizeof(float)));
+    cudaFree(h->batch_mem);
+    h->batch_mem = nullptr;
+    h->max_batch = 0;
+    const size_t R = (size_t)rows;
+    h->cparts = std::max<size_t>(1024, (R + 31) / 32);
     h->ldT = (rows + 63) / 64 * 64;
-    MLP_TRY(h, cudaMalloc((void**)&h->X64, R * 64 * sizeof(__nv_bfloat16)));
-    MLP_TRY(h, cudaMalloc((void**)&h->Ta, (size_t)NLAYER * HID * h->ldT * sizeof(__nv_bfloat16)));
-    MLP_TRY(h, cudaMalloc((void**)&h->Tb, (size_t)NLAYER * HID * h->ldT * sizeof(__nv_bfloat16)));
-    if (!h->w1p) {
-        MLP_TRY(h, cudaMalloc((void**)&h->w1p, (size_t)HID * 64 * sizeof(__nv_bfloat16)));
-        MLP_TRY(h, cudaMalloc((void**)&h->wt, (size_t)(NLAYER - 1) * HID * HID * sizeof(__nv_bfloat16)));
-        MLP_TRY(h, cudaMalloc((void**)&h->ws, (size_t)NLAYER * TG_MAX_SPLITS * HID * HID * sizeof(float)));
+    /* every batch buffer in one allocation (two dozen of them took 6 ms of a
+       short training, and as long again to free); first the sizes, then the
+       pointers */
+    size_t off = 0;
+    char* base = nullptr;
+    for (int pass = 0; pass < 2; ++pass) {
+        off = 0;
+        auto take = [&](auto** p, size_t count) {
+            if (base) *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(base + off);
+            off += (count * sizeof(**p) + 255) & ~(size_t)255;
+        };
+        take(&h->X, R * IN_PAD);
+        for (int l = 0; l < NLAYER; ++l) {
+            take(&h->H[l], R * HID);
+            take(&h->Z[l], R * HID);
+            take(&h->dZ[l], R * HID);
+        }
+        take(&h->p, R);
+        take(&h->dlogit, R);
+        take(&h->cpart, (size_t)NLAYER * h->cparts * HID);
+        take(&h->opart, (size_t)1024 * (HID + 1));
+        take(&h->X64, R * 64);
+        take(&h->Ta, (size_t)NLAYER * HID * h->ldT);
+        take(&h->Tb, (size_t)NLAYER * HID * h->ldT);
+        take(&h->w1p, (size_t)HID * 64);
+        take(&h->wt, (size_t)(NLAYER - 1) * HID * HID);
+        take(&h->ws, (size_t)NLAYER * TG_MAX_SPLITS * HID * HID);
+        if (pass == 0) {
+            MLP_TRY(h, cudaMalloc(&h->batch_mem, off));
+            base = static_cast<char*>(h->batch_mem);
+        }
     }
-    if (!h->st_w) {
-        MLP_TRY(h, cudaStreamCreateWithFlags(&h->st_w, cudaStreamNonBlocking));
-        for (int l = 0; l < NLAYER; ++l) MLP_TRY(h, cudaEventCreateWithFlags(&h->ev_dz[l], cudaEventDisableTiming));
-        MLP_TRY(h, cudaEventCreateWithFlags(&h->ev_w, cudaEventDisableTiming));
+    for (int l = 0; l < NLAYER && !h->st_w[l]; ++l) {
+        MLP_TRY(h, cudaStreamCreateWithFlags(&h->st_w[l], cudaStreamNonBlocking));
+        MLP_TRY(h, cudaEventCreateWithFlags(&h->ev_dz[l], cudaEventDisableTiming));
+        MLP_TRY(h, cudaEventCreateWithFlags(&h->ev_w[l], cudaEventDisableTiming));
     }
     h->tc_n = -1;
     h->max_batch = rows;
@@ -1640,14 +1712,20 @@ int tc_maps(gprm_mlp* h, int n)
     return GPRM_OK;
 }
 
+/* The training GEMMs' copies of the weights, from the BF16 ones. */
+void tc_weights(gprm_mlp* h, cudaStream_t st)
+{
+    const int items = HID * 64 + (NLAYER - 1) * HID * HID;
+    k_tc_weights<<<(items + 255) / 256, 256, 0, st>>>(h->wbf, h->offWbf[0], h->offWbf[1], h->offWbf[2],
+                                                      h->offWbf[3], h->w1p, h->wt);
+}
+
 /* Forward through the tensor-core GEMMs on rows featurised in h->X64. */
 int forward_tc(gprm_mlp* h, int n, float* p, const float* y, const int* yidx, float inv_b, cudaStream_t st)
 {
     int rc = tc_setup(h);
     if (rc || (rc = tc_maps(h, n))) return rc;
-    const int items = HID * 64 + (NLAYER - 1) * HID * HID;
-    k_tc_weights<<<(items + 255) / 256, 256, 0, st>>>(h->wbf, h->offWbf[0], h->offWbf[1], h->offWbf[2],
-                                                      h->offWbf[3], h->w1p, h->wt);
+    if (!h->weights_kept) tc_weights(h, st);
     const dim3 grid(HID / TG_BN_LAYER, (n + TC_ROWS - 1) / TC_ROWS, 1);
     for (int l = 0; l < NLAYER; ++l) {
         TgArgs a{};
@@ -1672,7 +1750,7 @@ int backward_tc(gprm_mlp* h, int n, cudaStream_t st)
        ordered reductions of k_reduce_w), so h->g needs no clearing */
     int blocks = n < 1024 ? n : 1024;
     k_out_back<<<blocks, HID, 0, st>>>(n, h->H[NLAYER - 1], h->Z[NLAYER - 1], h->wbf + h->offWbf[NLAYER], h->dlogit,
-                                       h->opart, h->dZ[NLAYER - 1]);
+                                       h->opart, h->dZ[NLAYER - 1], h->idx_off ? h->d_ctl : nullptr, nullptr);
     /* weight gradients: K = n split over CTAs, partials reduced in split
        order (128 rows per split: 512-row splits made the step 1.4x slower,
        the GEMM's longer K loop costing more than the partials it saves) */
@@ -1683,9 +1761,12 @@ int backward_tc(gprm_mlp* h, int n, cudaStream_t st)
     const dim3 tblock(32, 8);
     /* layer l's weight gradients (transposes, split-K GEMM, ordered
        reduction) depend only on dZ_l and the forward activations: they run
-       on st_w, in their own buffers, while st carries the chain of backward
+       on st_w[l], in their own buffers, while st carries the chain of backward
        GEMMs dZ_l -> dZ_{l-1}; st waits for all of them at the end (a fork
-       and join that a captured graph keeps as dependencies) */
+       and join that a captured graph keeps as dependencies).  The layers'
+       chains are short kernels, 20 us a layer: one behind the other on one
+       stream they were 82 of a step's 128 us, and ended 50 us after the
+       backward GEMMs. */
     MLP_TRY(h, cudaEventRecord(h->ev_dz[NLAYER - 1], st));
     for (int l = NLAYER - 1; l >= 0; --l) {
         const int kin = l == 0 ? IN_PAD : HID, kin_p = l == 0 ? 64 : HID;
@@ -1693,26 +1774,31 @@ int backward_tc(gprm_mlp* h, int n, cudaStream_t st)
         __nv_bfloat16* Tb = h->Tb + (size_t)l * HID * h->ldT;
         float* ws = h->ws + (size_t)l * TG_MAX_SPLITS * HID * HID;
         float* cpart = h->cpart + (size_t)l * h->cparts * HID;
-        MLP_TRY(h, cudaStreamWaitEvent(h->st_w, h->ev_dz[l], 0));
+        cudaStream_t sw = h->st_w[l];
+        MLP_TRY(h, cudaStreamWaitEvent(sw, h->ev_dz[l], 0));
         /* dW_l = dZ_l^T H_{l-1}: A = dZ_l^T [256 x n], B = H_{l-1}^T [kin_p x n] */
-        k_transpose2_bf16<<<dim3(HID / 32 + kin_p / 32, (n + 31) / 32), tblock, 0, h->st_w>>>(
+        k_transpose2_bf16<<<dim3(HID / 32 + kin_p / 32, (n + 31) / 32), tblock, 0, sw>>>(
             n, HID / 32, HID, h->dZ[l], HID, Ta, cpart, kin_p, l == 0 ? h->X64 : h->H[l - 1], kin_p, Tb, h->ldT);
         TgArgs a{};
         a.M = HID; a.N = kin_p; a.K = n; a.kps = kps; a.ws = ws; a.ldc = kin_p; a.err = h->dev_err; a.wait_cycles = wait_budget(h);
         if (l == 0)
-            k_tc_gemm<TG_WPART, 64><<<dim3(1, HID / TC_ROWS, splits), TG_THREADS, TgSmem<64>::BYTES, h->st_w>>>(
+            k_tc_gemm<TG_WPART, 64><<<dim3(1, HID / TC_ROWS, splits), TG_THREADS, TgSmem<64>::BYTES, sw>>>(
                 h->m_ta[0], h->m_tb64, a);
         else
-            k_tc_gemm<TG_WPART, HID><<<dim3(1, HID / TC_ROWS, splits), TG_THREADS, TgSmem<HID>::BYTES, h->st_w>>>(
+            k_tc_gemm<TG_WPART, HID><<<dim3(1, HID / TC_ROWS, splits), TG_THREADS, TgSmem<HID>::BYTES, sw>>>(
                 h->m_ta[l], h->m_tb256[l], a);
         /* weights, this layer's biases (column sums of dZ_l from the transpose)
            and, with the last layer, the output layer's partials */
         const bool out_l = l == NLAYER - 1;
         const int red_threads = HID * kin + HID * 32 + (out_l ? (HID + 1) * 32 : 0);   /* segments of whole warps */
-        k_reduce_w<<<(red_threads + 255) / 256, 256, 0, h->st_w>>>(splits, HID, kin_p, kin, ws, h->g + h->offW[l],
+        k_reduce_w<<<(red_threads + 255) / 256, 256, 0, sw>>>(splits, HID, kin_p, kin, ws, h->g + h->offW[l],
                                                                    (n + 31) / 32, cpart, h->g + h->offB[l],
                                                                    out_l ? blocks : 0, out_l ? h->opart : nullptr,
-                                                                   h->g + h->offW[NLAYER]);
+                                                                   h->g + h->offW[NLAYER], h->d_ctl,
+                                                                   out_l && h->idx_off
+                                                                       ? reinterpret_cast<float*>(h->d_ctl + 2)
+                                                                       : nullptr);
+        MLP_TRY(h, cudaEventRecord(h->ev_w[l], sw));
         if (l > 0) {
             /* dZ_{l-1} = (dZ_l W_l) * gelu'(Z_{l-1}): A = dZ_l [n x 256], B = W_l^T [256 x 256] */
             TgArgs d{};
@@ -1725,8 +1811,7 @@ int backward_tc(gprm_mlp* h, int n, cudaStream_t st)
             MLP_TRY(h, cudaEventRecord(h->ev_dz[l - 1], st));
         }
     }
-    MLP_TRY(h, cudaEventRecord(h->ev_w, h->st_w));
-    MLP_TRY(h, cudaStreamWaitEvent(st, h->ev_w, 0));
+    for (int l = 0; l < NLAYER; ++l) MLP_TRY(h, cudaStreamWaitEvent(st, h->ev_w[l], 0));
     MLP_TRY(h, cudaGetLastError());
     return GPRM_OK;
 }
@@ -1735,7 +1820,7 @@ int backward_tc(gprm_mlp* h, int n, cudaStream_t st)
 void features(gprm_mlp* h, const float* q, int offset, int n, const int* idx, cudaStream_t st)
 {
     if (h->train_path == GPRM_MLP_TRAIN_TCGEN05)
-        k_features64<<<(n + 255) / 256, 256, 0, st>>>(q, offset, h->ndof, n, idx, h->idx_off, h->X64);
+        k_features64<<<(n + 31) / 32, 256, 0, st>>>(q, offset, h->ndof, n, idx, h->idx_off, h->X64);
     else
         k_features<<<(n + 255) / 256, 256, 0, st>>>(q, offset, h->ndof, n, idx, h->idx_off, h->X);
 }
@@ -1773,7 +1858,8 @@ int backward(gprm_mlp* h, int n, cudaStream_t st)
     MLP_TRY(h, cudaMemsetAsync(h->g, 0, (size_t)h->nparam * sizeof(float), st));
     int blocks = n < 1024 ? n : 1024;
     k_out_back<<<blocks, HID, 0, st>>>(n, h->H[NLAYER - 1], h->Z[NLAYER - 1], h->wbf + h->offWbf[NLAYER], h->dlogit,
-                                       h->opart, h->dZ[NLAYER - 1]);
+                                       h->opart, h->dZ[NLAYER - 1], h->idx_off ? h->d_ctl : nullptr,
+                                       h->idx_off ? reinterpret_cast<float*>(h->d_ctl + 2) : nullptr);
     k_reduce_parts<<<(HID + 1 + 255) / 256, 256, 0, st>>>(blocks, HID + 1, h->opart, h->g + h->offW[NLAYER]);
     for (int l = NLAYER - 1; l >= 0; --l) {
         const int kin = l == 0 ? IN_PAD : HID;
@@ -1799,11 +1885,12 @@ int backward(gprm_mlp* h, int n, cudaStream_t st)
     return GPRM_OK;
 }
 
-/* One Adam step: step number (*t_base) + t_step (t_base null: t_step). */
-int adam_at(gprm_mlp* h, float lr, const long long* t_base, long long t_step, cudaStream_t st)
+/* One Adam step: step t, or with corr its corrections on the device. */
+int adam_at(gprm_mlp* h, float lr, long long t, const float* corr, cudaStream_t st)
 {
     k_adam<<<1024, 256, 0, st>>>(h->nparam, h->w, h->g, h->m, h->v, h->bf_map, h->wbf, lr, 0.9f, 0.999f, 1e-8f,
-                                 t_base, t_step);
+                                 t, corr, h->weights_kept ? h->w1p : nullptr, h->weights_kept ? h->wt : nullptr,
+                                 h->offWbf[1]);
     MLP_TRY(h, cudaGetLastError());
     return GPRM_OK;
 }
@@ -1811,7 +1898,7 @@ int adam_at(gprm_mlp* h, float lr, const long long* t_base, long long t_step, cu
 int adam(gprm_mlp* h, float lr, cudaStream_t st)
 {
     h->adam_t += 1;
-    return adam_at(h, lr, nullptr, h->adam_t, st);
+    return adam_at(h, lr, h->adam_t, nullptr, st);
 }
 
 /* deterministic uniform init in [-1/sqrt(in), 1/sqrt(in)] (Linear's default
@@ -1984,20 +2071,17 @@ void gprm_mlp_destroy(gprm_mlp* h)
     if (!h) return;
     if (h->st) cudaStreamSynchronize(h->st);
     cudaFree(h->w); cudaFree(h->g); cudaFree(h->m); cudaFree(h->v); cudaFree(h->bf_map); cudaFree(h->wbf);
-    cudaFree(h->loss); cudaFree(h->X);
-    for (int l = 0; l < NLAYER; ++l) { cudaFree(h->H[l]); cudaFree(h->Z[l]); cudaFree(h->dZ[l]); }
-    cudaFree(h->p); cudaFree(h->dlogit); cudaFree(h->ybatch); cudaFree(h->idx);
+    cudaFree(h->loss); cudaFree(h->batch_mem);
     cudaFree(h->Ha); cudaFree(h->Hb); cudaFree(h->dev_err); cudaFree(h->wtc);
-    cudaFree(h->X64); cudaFree(h->Ta); cudaFree(h->Tb); cudaFree(h->w1p); cudaFree(h->wt); cudaFree(h->ws);
-    cudaFree(h->cpart); cudaFree(h->opart);
     cudaFree(h->d_ctl);
-    if (h->st_w) {
-        cudaStreamSynchronize(h->st_w);
-        cudaStreamDestroy(h->st_w);
-    }
-    for (int l = 0; l < NLAYER; ++l)
+    for (int l = 0; l < NLAYER; ++l) {
+        if (h->st_w[l]) {
+            cudaStreamSynchronize(h->st_w[l]);
+            cudaStreamDestroy(h->st_w[l]);
+        }
         if (h->ev_dz[l]) cudaEventDestroy(h->ev_dz[l]);
-    if (h->ev_w) cudaEventDestroy(h->ev_w);
+        if (h->ev_w[l]) cudaEventDestroy(h->ev_w[l]);
+    }
     if (h->st) cudaStreamDestroy(h->st);
     delete h;
 }
@@ -2079,7 +2163,7 @@ int gprm_mlp_adam_step(gprm_mlp* h, float lr)
  * `epochs` passes in shuffled order (perm: device array of epochs*n
  * indices, each epoch a permutation), batches of `batch`, Adam at `lr`.
  * Every step runs features, forward, loss, backward and Adam on the
- * device; each epoch's launches are captured into one CUDA graph.
+ * device, from a CUDA graph of a few steps.
  * losses[epoch] gets the mean batch loss of each epoch (host array). */
 int gprm_mlp_train(gprm_mlp* h, const float* q, const float* y, int n, int offset, const int* perm, int epochs,
                    int batch, float lr, float* losses)
@@ -2092,31 +2176,40 @@ int gprm_mlp_train(gprm_mlp* h, const float* q, const float* y, int n, int offse
     if (h->train_path == GPRM_MLP_TRAIN_TCGEN05 && ((rc = tc_setup(h)) || (rc = tc_maps(h, batch)))) return rc;
     const int steps = n / batch;
     std::vector<float> ep_loss(epochs, 0.0f);
-    if (!h->d_ctl) MLP_TRY(h, cudaMalloc((void**)&h->d_ctl, 2 * sizeof(long long)));
-    /* one epoch's launches are captured once into a graph; each epoch sets
-       its offset into perm and its first Adam step in device memory */
+    if (!h->d_ctl) MLP_TRY(h, cudaMalloc((void**)&h->d_ctl, 3 * sizeof(long long)));
+    /* a few steps' launches are captured once into a graph, which every epoch
+       replays; an epoch sets its offset into perm and the Adam steps so far
+       in device memory, each step moves both on (k_out_back).  A whole epoch
+       in one graph cost more host time to capture and instantiate (64 steps,
+       1,600 kernels: 15 ms) than its steps took to run (9 ms); a launch per
+       `unroll` steps keeps ahead of them easily. */
+    int unroll = steps < 8 ? steps : 8;
+    while (steps % unroll) --unroll;
+    const bool tc = h->train_path == GPRM_MLP_TRAIN_TCGEN05;
+    if (tc) tc_weights(h, h->st);
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     MLP_TRY(h, cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
     int crc = GPRM_OK;
     h->idx_off = h->d_ctl;
-    cudaMemsetAsync(h->loss, 0, sizeof(float), h->st);
-    for (int s = 0; s < steps && !crc; ++s) {
-        const int* idx = perm + (size_t)s * batch;
-        features(h, q, offset, batch, idx, h->st);
-        if (!crc) crc = forward(h, batch, h->p, y, idx, 1.0f / batch, h->st);
+    h->weights_kept = tc;
+    for (int s = 0; s < unroll && !crc; ++s) {
+        features(h, q, offset, batch, perm, h->st);
+        if (!crc) crc = forward(h, batch, h->p, y, perm, 1.0f / batch, h->st);
         if (!crc) crc = backward(h, batch, h->st);
-        if (!crc) crc = adam_at(h, lr, h->d_ctl + 1, s + 1, h->st);
+        if (!crc) crc = adam_at(h, lr, 0, reinterpret_cast<float*>(h->d_ctl + 2), h->st);
     }
     h->idx_off = nullptr;
+    h->weights_kept = false;
     cudaError_t ce = cudaStreamEndCapture(h->st, &graph);
     if (crc) { if (graph) cudaGraphDestroy(graph); return crc; }
-    if (ce != cudaSuccess) return mfail(h, GPRM_ERR_CUDA, "capturing the training epoch", ce);
+    if (ce != cudaSuccess) return mfail(h, GPRM_ERR_CUDA, "capturing the training steps", ce);
     ce = cudaGraphInstantiate(&exec, graph, 0);
     for (int e = 0; e < epochs && ce == cudaSuccess; ++e) {
         const long long ctl[2] = {(long long)e * n, h->adam_t};
         ce = cudaMemcpyAsync(h->d_ctl, ctl, sizeof(ctl), cudaMemcpyHostToDevice, h->st);
-        if (ce == cudaSuccess) ce = cudaGraphLaunch(exec, h->st);
+        if (ce == cudaSuccess) ce = cudaMemsetAsync(h->loss, 0, sizeof(float), h->st);
+        for (int s = 0; s < steps && ce == cudaSuccess; s += unroll) ce = cudaGraphLaunch(exec, h->st);
         float l = 0;
         if (ce == cudaSuccess) ce = cudaMemcpyAsync(&l, h->loss, sizeof(float), cudaMemcpyDeviceToHost, h->st);
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(h->st);
