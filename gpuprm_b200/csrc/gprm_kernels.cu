@@ -2164,11 +2164,14 @@ cudaError_t configure_launch(const DevScene& sc, int vertex_kernel, int threads,
 cudaError_t plan_launch(const DevScene& sc, int vertex_kernel, int threads, LaunchCfg* cfg)
 {
     /* default: the variant with the most resident warps, the scene in shared
-       memory on ties (the autotuner times the candidates instead) */
+       memory on ties (the autotuner times the candidates instead).  The
+       small blocks are for scenes whose frames leave room for some more
+       warps than whole blocks of four: 7 joints hold 12 warps in blocks of
+       128 and 13 in blocks of 32 (70,001 wall edges 14.19 -> 13.62 ms). */
     LaunchCfg best{};
     int best_w = -1;
-    const int cand_threads[4] = {threads, 256, 384, 512};
-    for (int ci = 0; ci < 4; ++ci)
+    const int cand_threads[6] = {threads, 256, 384, 512, 64, 32};
+    for (int ci = 0; ci < 6; ++ci)
         for (int sm = 1; sm >= 0; --sm) {
             LaunchCfg c{};
             if (configure_launch(sc, vertex_kernel, cand_threads[ci], sm, &c) != cudaSuccess) {
