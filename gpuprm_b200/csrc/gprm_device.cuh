@@ -942,16 +942,15 @@ __device__ __forceinline__ void forward_kinematics_fast(const DevScene& sc, cons
  * (FAST: fast_link; else the reference's operations as in
  * forward_kinematics): frames 1..ndof go to a lane-interleaved
  * shared-memory array, entry e of frame f at out[((f-1)*12 + e) * 32] (out
- * already offset by the lane).  The world centre of every slot's bounding
- * ball goes to cen[(slot*3 + c) * 32], the world position of the slot
- * polytope's vertex 0 to cen[((nslots + slot)*3 + c) * 32] (both with FMA:
- * they only feed the certificates, whose slack covers their rounding).
- * SLOTS: whether to write them.  joint(i): the lane's value of joint i.  One loop body for every joint (the
- * kernels wait on instruction fetches), its slot's table entries loaded
- * before the trigonometry. */
-template <bool FAST, bool SLOTS, class Joint>
+ * already offset by the lane).  SLOTS: point(slot, u, w) gets the world
+ * centre u of every slot's bounding ball and the world position w of the
+ * slot polytope's vertex 0 (both with FMA: they only feed the certificates,
+ * whose slack covers their rounding).  joint(i): the lane's value of joint
+ * i.  One loop body for every joint (the kernels wait on instruction
+ * fetches), its slot's table entries loaded before the trigonometry. */
+template <bool FAST, bool SLOTS, class Joint, class Point>
 __device__ __forceinline__ void forward_kinematics_smem(const DevScene& sc, const float4* __restrict__ tab,
-                                                        Joint joint, float* out, float* cen)
+                                                        Joint joint, float* out, Point point)
 {
     Frame<float> T;
     identity_frame(T);
@@ -994,13 +993,13 @@ __device__ __forceinline__ void forward_kinematics_smem(const DevScene& sc, cons
         for (int e = 0; e < 12; ++e) fr[e * 32] = O.m[e];
 #pragma unroll 1
         while (has) {
-            float* u = cen + slot * 3 * 32;
-            float* w = u + sc.nslots * 3 * 32;
+            float u[3], w[3];
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-                u[c * 32] = __fmaf_rn(O.m[c], b.x, __fmaf_rn(O.m[3 + c], b.y, __fmaf_rn(O.m[6 + c], b.z, O.m[9 + c])));
-                w[c * 32] = __fmaf_rn(O.m[c], v.x, __fmaf_rn(O.m[3 + c], v.y, __fmaf_rn(O.m[6 + c], v.z, O.m[9 + c])));
+                u[c] = __fmaf_rn(O.m[c], b.x, __fmaf_rn(O.m[3 + c], b.y, __fmaf_rn(O.m[6 + c], b.z, O.m[9 + c])));
+                w[c] = __fmaf_rn(O.m[c], v.x, __fmaf_rn(O.m[3 + c], v.y, __fmaf_rn(O.m[6 + c], v.z, O.m[9 + c])));
             }
+            point(slot, u, w);
             ++slot;
             has = slot < sc.nslots && sc.slot_sys[slot] == i + 1;
             if (has) {

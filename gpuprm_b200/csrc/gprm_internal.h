@@ -106,13 +106,11 @@ cudaError_t launch_recheck_multi(const BatchView& B, int blocks, int kind, const
                                  BandQueue bq, Control* ctl, cudaStream_t st);
 
 /* Per-lane shared floats of a warp's block: frames 1..ndof (12 floats each),
- * lane-interleaved.  Edge kernels: the world ball centres of the slots (3
- * floats each) and the world vertex 0 of the slots' polytopes (3 floats
- * each), lane-interleaved; then, together for the warp, one float per lane
- * and 1024 pairs of a sweep group, the bits of the pairs that the sweep
- * stage leaves open, and SWEEP_LANE_FLOATS per lane, the per-slot sweep
- * balls (GPRM_MAX_SLOTS float4).  Vertex kernels: VERTEX_LANE_FLOATS per
- * lane, the warp's VertexArea, then the open bits. */
+ * lane-interleaved.  Edge kernels: then, together for the warp, one float
+ * per lane and 1024 pairs of a sweep group, the bits of the pairs that the
+ * sweep stage leaves open, and SWEEP_LANE_FLOATS per lane, the per-slot
+ * sweep balls (GPRM_MAX_SLOTS float4).  Vertex kernels: VERTEX_LANE_FLOATS
+ * per lane, the warp's VertexArea, then the open bits. */
 #define SWEEP_LANE_FLOATS 2
 static_assert(SWEEP_LANE_FLOATS * 32 >= GPRM_MAX_SLOTS * 4, "sweep area too small");
 #define VERTEX_LANE_FLOATS 23
@@ -124,7 +122,7 @@ __host__ __device__ __forceinline__ int open_lane_floats(const DevScene& sc)
 __host__ __device__ __forceinline__ size_t lane_floats(const DevScene& sc, bool vertex_kernel)
 {
     return (size_t)sc.ndof * 12 + open_lane_floats(sc) +
-           (vertex_kernel ? VERTEX_LANE_FLOATS : (size_t)sc.nslots * 6 + SWEEP_LANE_FLOATS);
+           (vertex_kernel ? VERTEX_LANE_FLOATS : SWEEP_LANE_FLOATS);
 }
 
 /* Scene bytes when staged in shared memory; per-lane frame bytes of a block. */

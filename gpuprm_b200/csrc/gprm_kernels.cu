@@ -63,7 +63,6 @@ struct SceneView {
     const int4* scan_c;
     const float4* scan_b;
     float* frames;   /* this lane's frames (lane-interleaved, stride 32) */
-    float* cen;      /* this lane's slot ball centres, then the slots' world vertex 0 */
     float4* sweep;   /* the warp's per-slot sweep balls */
     unsigned* bits;  /* the pairs of the sweep group left open (one bit each) */
 };
@@ -85,7 +84,7 @@ template <bool VERTEX>
 __device__ __forceinline__ unsigned* open_area(const DevScene& sc, float* lane_frames)
 {
     const int lane = threadIdx.x & 31;
-    const size_t at = (size_t)sc.ndof * 12 + (VERTEX ? (size_t)VERTEX_LANE_FLOATS : (size_t)sc.nslots * 6);
+    const size_t at = (size_t)sc.ndof * 12 + (VERTEX ? (size_t)VERTEX_LANE_FLOATS : 0);
     return reinterpret_cast<unsigned*>(lane_frames - lane + at * 32);
 }
 
@@ -130,81 +129,27 @@ __device__ __forceinline__ SceneView stage_scene(const DevScene& sc, unsigned ch
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     s.frames = reinterpret_cast<float*>(smem + off) + (size_t)warp * lane_floats(sc, VERTEX) * 32 + lane;
-    s.cen = s.frames + (size_t)sc.ndof * 12 * 32;
     s.sweep = sweep_area<VERTEX>(sc, s.frames);
     s.bits = open_area<VERTEX>(sc, s.frames);
     __syncthreads();
     return s;
 }
 
-/* min / max of three, NaN if any is NaN */
-__device__ __forceinline__ float min3_nan(float a, float b, float c)
-{
-    float d;
-    asm("min.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
-}
-__device__ __forceinline__ float max3_nan(float a, float b, float c)
-{
-    float d;
-    asm("max.NaN.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
-    return d;
-}
-
-/* Per slot, a ball holding that slot's ball centre in every lane (every
- * lane's frames are current): centre m = the midpoint of the lanes'
- * bounding box, radius rho >= max |c_lane - m| (the box half-diagonal from
- * m, rounded up).  A non-finite centre makes rho infinite, which disables
- * the sweep tests for the slot.  sweep[slot] bounds the slots' ball
- * centres; with at most SWEEP_V0_SLOTS slots, sweep[SWEEP_V0_SLOTS + slot]
- * bounds the slots' vertex 0 the same way, for the swept direction test.
- *
- * A row of 32 lane values per coordinate (6 rows a slot): lane r reduces
- * row r on its own, eight 16-byte loads whose order is rotated by the lane
- * (the rows alias in the banks), two three-input min/max a load; the three
- * rows of a point then meet by shuffles.  One lane per point, one value at
- * a time with 12 lanes on the same bank, took 5,800 cycles of a hull6 round
- * (8 %); this takes about a third. */
+/* Slots whose vertex 0 has a sweep ball too (the swept direction test). */
 constexpr int SWEEP_V0_SLOTS = GPRM_MAX_SLOTS / 2;
-__device__ __forceinline__ void sweep_bounds(const DevScene& sc, const SceneView& S)
+
+/* One sweep ball: centre at lane mid's point, radius over the lanes'
+ * points.  Lane p keeps the squared radius as bits (NaN, which is larger
+ * than any number's bits, if a point is not finite). */
+__device__ __forceinline__ void sweep_ball(float4* sweep, int mid, int p, const float* u, unsigned& r2)
 {
     const int lane = threadIdx.x & 31;
-    __syncwarp();   /* the lanes' centres are written */
-    const int n3 = sc.nslots * 3;
-    const int rows = sc.nslots <= SWEEP_V0_SLOTS ? 2 * n3 : n3;
-    const float* base = S.cen - lane;   /* row r: base[r * 32 ..] */
-    float* out = reinterpret_cast<float*>(S.sweep);
-#pragma unroll 1
-    for (int r0 = 0; r0 < rows; r0 += 30) {       /* whole points per pass */
-        const int r = r0 + lane;
-        const bool mine = lane < 30 && r < rows;
-        const float4* row = reinterpret_cast<const float4*>(base + (mine ? r : 0) * 32);
-        float4 v = row[lane & 7];
-        float lo = min3_nan(v.x, v.y, v.z), hi = max3_nan(v.x, v.y, v.z);
-        lo = min3_nan(lo, v.w, v.w);
-        hi = max3_nan(hi, v.w, v.w);
-#pragma unroll
-        for (int i = 1; i < 8; ++i) {
-            v = row[(lane + i) & 7];
-            lo = min3_nan(min3_nan(lo, v.x, v.y), v.z, v.w);
-            hi = max3_nan(max3_nan(hi, v.x, v.y), v.z, v.w);
-        }
-        const float mid = 0.5f * (lo + hi);
-        const float e = fmaxf(hi - mid, mid - lo);
-        const float bad = mid - mid + (hi - lo) * 0.0f;      /* NaN unless both ends are finite */
-        const float e2 = __fmaf_rn(e, e, bad);
-        const float s2 = e2 + __shfl_down_sync(FULL_MASK, e2, 1) + __shfl_down_sync(FULL_MASK, e2, 2);
-        if (mine) {
-            const int pt = r / 3, c = r - 3 * pt;
-            float* o = out + 4 * (pt < sc.nslots ? pt : SWEEP_V0_SLOTS + pt - sc.nslots);
-            o[c] = mid;
-            if (c == 0) {
-                const float rho = __fsqrt_ru(s2) * (1.0f + 5e-6f) + 1e-30f;
-                o[3] = rho < PF32::inf() ? rho : PF32::inf();
-            }
-        }
-    }
-    __syncwarp();
+    const float dx = u[0] - __shfl_sync(FULL_MASK, u[0], mid);
+    const float dy = u[1] - __shfl_sync(FULL_MASK, u[1], mid);
+    const float dz = u[2] - __shfl_sync(FULL_MASK, u[2], mid);
+    const unsigned m = __reduce_max_sync(FULL_MASK, __float_as_uint(__fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz))));
+    if (lane == p) r2 = m;
+    if (lane == mid) sweep[p] = make_float4(u[0], u[1], u[2], 0.0f);
 }
 
 /* Counts of how pair tests were settled: by a certificate (a lane's own
@@ -415,32 +360,6 @@ __device__ __forceinline__ bool points_certified(const DevScene& sc, const float
     return Gb - err > sc.thr_dir;
 }
 
-/* points_certified for the lane whose slots and frames S holds: the moving
- * polytopes' points from the slots (written by the FK pass), a static one's
- * from the records f and b.  A pair that is not SCAN_USABLE is never
- * certified here (no slot, or two static polytopes whose certificate failed
- * when the tables were uploaded). */
-__device__ __forceinline__ bool lane_certified(const DevScene& sc, const SceneView& S, int4 c, float4 f, float4 b)
-{
-    if (c.w != SCAN_USABLE) return false;
-    const float* v0w = S.cen + sc.nslots * 3 * 32;
-    V3<float> P = {f.x, f.y, f.z}, Q = P, A = {b.x, b.y, b.z}, B = A;
-    const int sp = SCAN_SLOT_P(c.x), sq = SCAN_SLOT_Q(c.x);
-    if (sp >= 0) {
-        const float* u = S.cen + sp * 3 * 32;
-        const float* v = v0w + sp * 3 * 32;
-        P.x = u[0]; P.y = u[32]; P.z = u[64];
-        A.x = v[0]; A.y = v[32]; A.z = v[64];
-    }
-    if (sq >= 0) {
-        const float* u = S.cen + sq * 3 * 32;
-        const float* v = v0w + sq * 3 * 32;
-        Q.x = u[0]; Q.y = u[32]; Q.z = u[64];
-        B.x = v[0]; B.y = v[32]; B.z = v[64];
-    }
-    return points_certified(sc, S.frames, c, f.w, b.w, P, Q, A, B);
-}
-
 /* Point x of frame f (1..ndof) of a configuration, with the FMA chain of the
  * slot points. */
 __device__ __forceinline__ V3<float> frame_point(const float* frames, int f, float4 x)
@@ -451,6 +370,32 @@ __device__ __forceinline__ V3<float> frame_point(const float* frames, int f, flo
     o.y = __fmaf_rn(T[32], x.x, __fmaf_rn(T[4 * 32], x.y, __fmaf_rn(T[7 * 32], x.z, T[10 * 32])));
     o.z = __fmaf_rn(T[2 * 32], x.x, __fmaf_rn(T[5 * 32], x.y, __fmaf_rn(T[8 * 32], x.z, T[11 * 32])));
     return o;
+}
+
+/* World ball centre and vertex 0 of a slot's polytope (in frame f) for this
+ * lane, as the FK pass had them. */
+__device__ __forceinline__ void slot_points(const DevScene& sc, const SceneView& S, int slot, int f, V3<float>& p,
+                                            V3<float>& a)
+{
+    const float4* blk = S.tab + sc.slot_block[slot];
+    const float4 x = blk[0], v = blk[1];
+    p = frame_point(S.frames, f, x);
+    a = frame_point(S.frames, f, v);
+}
+
+/* points_certified for the lane whose slots and frames S holds: the moving
+ * polytopes' points from the slots (written by the FK pass), a static one's
+ * from the records f and b.  A pair that is not SCAN_USABLE is never
+ * certified here (no slot, or two static polytopes whose certificate failed
+ * when the tables were uploaded). */
+__device__ __forceinline__ bool lane_certified(const DevScene& sc, const SceneView& S, int4 c, float4 f, float4 b)
+{
+    if (c.w != SCAN_USABLE) return false;
+    V3<float> P = {f.x, f.y, f.z}, Q = P, A = {b.x, b.y, b.z}, B = A;
+    const int sp = SCAN_SLOT_P(c.x), sq = SCAN_SLOT_Q(c.x);
+    if (sp >= 0) slot_points(sc, S, sp, SCAN_SYS_P(c.x), P, A);
+    if (sq >= 0) slot_points(sc, S, sq, SCAN_SYS_Q(c.x), Q, B);
+    return points_certified(sc, S.frames, c, f.w, b.w, P, Q, A, B);
 }
 
 /* points_certified of pair j from the frames alone (a vertex check keeps no
@@ -524,11 +469,39 @@ __device__ __forceinline__ int eval_pair(const DevScene& sc, const SceneView& S,
 }
 
 /* Forward kinematics of a lane into its shared-memory frames, in the
- * arithmetic of the kernel variant. */
+ * arithmetic of the kernel variant, and (SLOTS) the warp's sweep balls:
+ * sweep[slot] holds the slot's ball centre in every lane; with at most
+ * SWEEP_V0_SLOTS slots, sweep[SWEEP_V0_SLOTS + slot] the slots' vertex 0,
+ * for the swept direction test.  Centred at lane mid's points (of an edge's
+ * round the middle step: its steps lie on a path), radius the largest
+ * distance from there, rounded up; a non-finite point makes it infinite,
+ * which disables the sweep tests for the slot.
+ *
+ * Nothing else of the points is kept: lane_scan takes them from the frames
+ * again.  With 6 floats a slot and lane in shared memory (and the balls
+ * from the rows' extremes) the 6-joint edge kernel left 28 KB to L1 and one
+ * of 7 joints ran 13 warps an SM; now 92 KB and 16 warps (2.5 M hull6 edges
+ * 59.9 -> 57.3 ms, 70,001 wall edges 13.6 -> 12.3, a mixed batch 26.8 -> 22.7;
+ * the exact arithmetic on hull6 16.9 -> 17.4).  The extremes by
+ * warp reductions instead (6 a point) took 1,900 cycles of a round more. */
 template <bool FAST, bool SLOTS = true, class Joint>
-__device__ __forceinline__ void lane_fk(const DevScene& sc, const SceneView& S, Joint joint)
+__device__ __forceinline__ void lane_fk(const DevScene& sc, const SceneView& S, Joint joint, int mid = 0)
 {
-    forward_kinematics_smem<FAST, SLOTS>(sc, S.tab, joint, S.frames, S.cen);
+    const bool v0 = sc.nslots <= SWEEP_V0_SLOTS;
+    unsigned r2 = 0u;
+    forward_kinematics_smem<FAST, SLOTS>(sc, S.tab, joint, S.frames, [&](int slot, const float* u, const float* w) {
+        sweep_ball(S.sweep, mid, slot, u, r2);
+        if (v0) sweep_ball(S.sweep, mid, SWEEP_V0_SLOTS + slot, w, r2);
+    });
+    if constexpr (SLOTS) {
+        __syncwarp();
+        const int lane = threadIdx.x & 31;
+        if (lane < GPRM_MAX_SLOTS) {
+            const float rho = __fsqrt_ru(__uint_as_float(r2)) * (1.0f + 5e-6f) + 1e-30f;
+            S.sweep[lane].w = rho < PF32::inf() ? rho : PF32::inf();
+        }
+        __syncwarp();
+    }
 }
 
 __device__ __forceinline__ void flush_counts(PairCounts pc, Control* ctl)
@@ -820,8 +793,12 @@ __device__ __forceinline__ void check_config_chunk(const DevScene& sc, const Sce
     __syncwarp();
 }
 
+/* 112 registers: 18 warps an SM where shared memory allows them (vertices of
+ * hull6 3.56 -> 3.40 ms, of the 7-DOF wall 3.25 -> 3.21; 96 registers spill:
+ * 3.55 and 3.48; the edge kernel is slower with 112 or 96: 57.9 -> 59.1 and
+ * 59.9 ms). */
 template <bool SMEM, bool FAST>
-__global__ void GPRM_BOUNDS k_check_configs(DevScene sc, const float* __restrict__ q,
+__global__ void __maxnreg__(112) k_check_configs(DevScene sc, const float* __restrict__ q,
                                             long long n, long long offset,
                                             int* __restrict__ res, int band_on, float band,
                                             BandQueue bq,
@@ -929,12 +906,11 @@ __device__ __forceinline__ void check_edge(const DevScene& sc, const SceneView& 
         }
         /* the step's configuration as edge_step_config */
         const float c1 = (float)t / (float)(tn - 1), c2 = 1.0f - c1;
+        const unsigned valid_mask = __ballot_sync(FULL_MASK, valid);
         lane_fk<FAST>(sc, S, [&](int j) {
             return c1 * __shfl_sync(FULL_MASK, ends, j) + c2 * __shfl_sync(FULL_MASK, ends, 16 + j);
-        });
-        const unsigned valid_mask = __ballot_sync(FULL_MASK, valid);
+        }, __popc(valid_mask) >> 1);
         if (lane == 0) exec += __popc(valid_mask);
-        sweep_bounds(sc, S);
         bool active = valid;
         int code = 0;
         float mmin = PF32::inf(), mdec = 0.0f;
@@ -1765,7 +1741,6 @@ __device__ __forceinline__ SceneView small_view(const DevScene& sc, unsigned cha
     S.tab = sc.tab; S.pairs = sc.pairs; S.pairs_b = sc.pairs_b;
     S.far = sc.far; S.scan_c = sc.scan_c; S.scan_b = sc.scan_b;
     S.frames = reinterpret_cast<float*>(smem) + (threadIdx.x & 31);
-    S.cen = S.frames + (size_t)sc.ndof * 12 * 32;
     S.sweep = sweep_area<false>(sc, S.frames);
     S.bits = open_area<false>(sc, S.frames);
     return S;
@@ -1815,9 +1790,8 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_configs_small(DevScene 
         if (warp == 0) {
             /* the other lanes repeat a valid one, so that the sweep balls hold no more */
             const int src = in ? lane : __ffs(valid) - 1;
-            lane_fk<FAST>(sc, S, [&](int j) { return B.q[j][src]; });
-            sweep_bounds(sc, S);
-        }
+            lane_fk<FAST>(sc, S, [&](int j) { return B.q[j][src]; }, __ffs(valid) - 1);
+            }
         small_pairs<FAST, CUT_NONE>(sc, S, B, valid, false, band_on, band);
         if (in) {
             const unsigned jk = B.jkey[lane];
@@ -1921,9 +1895,8 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_edges_small(DevScene sc
         if (warp == 0) {
             lane_fk<FAST>(sc, S, [&](int j) {
                 return c1 * __shfl_sync(FULL_MASK, ends, j) + c2 * __shfl_sync(FULL_MASK, ends, 16 + j);
-            });
-            sweep_bounds(sc, S);
-        }
+            }, __popc(valid) >> 1);
+            }
         exec += (unsigned)__popc(valid);
         /* settle the round as check_edge does; where the collision that the
            tests were cut by turned out to be decided by an earlier pair
@@ -2377,7 +2350,6 @@ __device__ __forceinline__ void switch_scene(const BatchView& B, int p, DevScene
     S.scan_c = wsc->scan_c;
     S.scan_b = wsc->scan_b;
     S.frames = frames;
-    S.cen = frames + (size_t)wsc->ndof * 12 * 32;
     S.sweep = sweep_area<VERTEX>(*wsc, frames);
     S.bits = open_area<VERTEX>(*wsc, frames);
 }
