@@ -138,18 +138,38 @@ __device__ __forceinline__ SceneView stage_scene(const DevScene& sc, unsigned ch
 /* Slots whose vertex 0 has a sweep ball too (the swept direction test). */
 constexpr int SWEEP_V0_SLOTS = GPRM_MAX_SLOTS / 2;
 
-/* One sweep ball: centre at lane mid's point, radius over the lanes'
- * points.  Lane p keeps the squared radius as bits (NaN, which is larger
- * than any number's bits, if a point is not finite). */
+/* Warp-wide minimum and maximum, NaN if any lane's value is. */
+__device__ __forceinline__ float warp_min_nan(float a)
+{
+    float d;
+    asm volatile("redux.sync.min.NaN.f32 %0, %1, 0xffffffff;" : "=f"(d) : "f"(a));
+    return d;
+}
+__device__ __forceinline__ float warp_max_nan(float a)
+{
+    float d;
+    asm volatile("redux.sync.max.NaN.f32 %0, %1, 0xffffffff;" : "=f"(d) : "f"(a));
+    return d;
+}
+
+/* One sweep ball: PATH: centre at lane mid's point, else the midpoint of the
+ * lanes' bounding box, radius over the lanes' points.  Lane p keeps the
+ * squared radius as bits (NaN, which is larger than any number's bits, if a
+ * point is not finite). */
+template <bool PATH>
 __device__ __forceinline__ void sweep_ball(float4* sweep, int mid, int p, const float* u, unsigned& r2)
 {
     const int lane = threadIdx.x & 31;
-    const float dx = u[0] - __shfl_sync(FULL_MASK, u[0], mid);
-    const float dy = u[1] - __shfl_sync(FULL_MASK, u[1], mid);
-    const float dz = u[2] - __shfl_sync(FULL_MASK, u[2], mid);
-    const unsigned m = __reduce_max_sync(FULL_MASK, __float_as_uint(__fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz))));
-    if (lane == p) r2 = m;
-    if (lane == mid) sweep[p] = make_float4(u[0], u[1], u[2], 0.0f);
+    float m[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+        m[c] = PATH ? __shfl_sync(FULL_MASK, u[c], mid) : 0.5f * (warp_min_nan(u[c]) + warp_max_nan(u[c]));
+    const float dx = u[0] - m[0], dy = u[1] - m[1], dz = u[2] - m[2];
+    const unsigned r = __reduce_max_sync(FULL_MASK, __float_as_uint(__fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz))));
+    if (lane == p) {
+        r2 = r;
+        sweep[p] = make_float4(m[0], m[1], m[2], 0.0f);
+    }
 }
 
 /* Counts of how pair tests were settled: by a certificate (a lane's own
@@ -472,10 +492,13 @@ __device__ __forceinline__ int eval_pair(const DevScene& sc, const SceneView& S,
  * arithmetic of the kernel variant, and (SLOTS) the warp's sweep balls:
  * sweep[slot] holds the slot's ball centre in every lane; with at most
  * SWEEP_V0_SLOTS slots, sweep[SWEEP_V0_SLOTS + slot] the slots' vertex 0,
- * for the swept direction test.  Centred at lane mid's points (of an edge's
- * round the middle step: its steps lie on a path), radius the largest
- * distance from there, rounded up; a non-finite point makes it infinite,
- * which disables the sweep tests for the slot.
+ * for the swept direction test.  PATH: centred at lane mid's points (of an
+ * edge's round the middle step: its steps lie on a path); else at the
+ * middle of the points' bounding box (configurations that lie anywhere:
+ * 4,096 of wall7 620 us with a configuration as the centre, 597 so; 543 when
+ * the points were kept in shared memory, which the edges paid for).  Radius
+ * the largest distance from there, rounded up; a non-finite point makes it
+ * infinite, which disables the sweep tests for the slot.
  *
  * Nothing else of the points is kept: lane_scan takes them from the frames
  * again.  With 6 floats a slot and lane in shared memory (and the balls
@@ -484,14 +507,14 @@ __device__ __forceinline__ int eval_pair(const DevScene& sc, const SceneView& S,
  * 59.9 -> 57.3 ms, 70,001 wall edges 13.6 -> 12.3, a mixed batch 26.8 -> 22.7;
  * the exact arithmetic on hull6 16.9 -> 17.4).  The extremes by
  * warp reductions instead (6 a point) took 1,900 cycles of a round more. */
-template <bool FAST, bool SLOTS = true, class Joint>
+template <bool FAST, bool SLOTS = true, bool PATH = true, class Joint>
 __device__ __forceinline__ void lane_fk(const DevScene& sc, const SceneView& S, Joint joint, int mid = 0)
 {
     const bool v0 = sc.nslots <= SWEEP_V0_SLOTS;
     unsigned r2 = 0u;
     forward_kinematics_smem<FAST, SLOTS>(sc, S.tab, joint, S.frames, [&](int slot, const float* u, const float* w) {
-        sweep_ball(S.sweep, mid, slot, u, r2);
-        if (v0) sweep_ball(S.sweep, mid, SWEEP_V0_SLOTS + slot, w, r2);
+        sweep_ball<PATH>(S.sweep, mid, slot, u, r2);
+        if (v0) sweep_ball<PATH>(S.sweep, mid, SWEEP_V0_SLOTS + slot, w, r2);
     });
     if constexpr (SLOTS) {
         __syncwarp();
@@ -1790,7 +1813,7 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_configs_small(DevScene 
         if (warp == 0) {
             /* the other lanes repeat a valid one, so that the sweep balls hold no more */
             const int src = in ? lane : __ffs(valid) - 1;
-            lane_fk<FAST>(sc, S, [&](int j) { return B.q[j][src]; }, __ffs(valid) - 1);
+            lane_fk<FAST, true, false>(sc, S, [&](int j) { return B.q[j][src]; });
             }
         small_pairs<FAST, CUT_NONE>(sc, S, B, valid, false, band_on, band);
         if (in) {
