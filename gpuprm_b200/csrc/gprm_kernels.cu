@@ -6,22 +6,25 @@
  * over indicator(q) (robotconfigspace.cpp:313-346, prmsolver.cpp:2611).
  *
  * Work mapping (persistent grid, warps take work from a device counter):
- *   vertex checks  a warp takes 32 configurations, one per lane; every lane
- *                  runs FK and then the reference's pair loop with its own
- *                  early exit, lanes stepping through the pairs together.
+ *   vertex checks  a warp takes 32 configurations: FK a lane each, then one
+ *                  configuration after the other swept with a lane per pair,
+ *                  and the pairs left tested 32 at a time whoever they belong
+ *                  to, applied per configuration in pair order.
  *   edge checks    a warp takes one edge; its lanes hold 32 steps of that
  *                  edge (coarse-to-fine: round r, lane i -> step i*R + r with
  *                  R = ceil(testnum/32); or descending steps when every step's
- *                  code is wanted) and step through the pairs together.  Nearby
- *                  steps take nearly the same path through the algorithm, so
- *                  the lanes stay converged, and one warp vote after each pair
- *                  ends the edge at its first colliding step.
+ *                  code is wanted).  A sweep stage settles most pairs for all
+ *                  lanes at once, the lanes step through the rest together,
+ *                  and one warp vote after each exact test ends the edge at
+ *                  its first colliding step.
+ *   small requests a block of four warps per configuration or edge, its FP64
+ *                  checks included, in one launch.
  * The scene (vertices with packed adjacency, neighbour bytes, pair table)
- * is copied into shared memory per block when it fits.
+ * can be copied into shared memory per block where it fits.
  *
  * FP64 band: a check whose FP32 result is decided within the band (or by
  * the iteration cap) is appended to a queue; k_recheck recomputes it in
- * FP64, thread per item, and its verdict replaces the FP32 one.
+ * FP64, a thread or a warp per item, and its verdict replaces the FP32 one.
  */
 #include "gprm_internal.h"
 
