@@ -864,8 +864,7 @@ int enqueue_part(gprm_space* h, Request& r, int kind, const float* a, const floa
     if (h->debug_qcap && h->debug_qcap < bq.cap) bq.cap = h->debug_qcap;
     bq.n = n;
     bq.ovf = nullptr;
-    /* pair indices fit 16 bits on every scene the library builds; a larger
-       pair list rechecks every pair */
+    /* a pair list whose indices do not fit 16 bits rechecks every pair */
     bq.pair_range = h->dsc.npairs <= 65535 ? r.d_qpair : nullptr;
     if (band_on && r.d_ovf) {
         /* every part's keys start at its first item (key = d_key + c0) */

@@ -1513,16 +1513,28 @@ __device__ __forceinline__ bool recheck_by_warp(unsigned items, unsigned warps, 
 }
 constexpr int RECHECK_THREADS = 128;
 
+/* The pairs [lo, hi) of queue item idx: as recorded, else all of them (a
+ * pair list whose indices do not fit a recorded range). */
+struct PairSpan {
+    int lo, hi;
+};
+__device__ __forceinline__ PairSpan recheck_span(const BandQueue& bq, unsigned idx, int npairs)
+{
+    if (!bq.pair_range) return {0, npairs};
+    const unsigned range = bq.pair_range[idx];
+    return {(int)(range & 0xffffu), (int)(range >> 16)};
+}
+
 __device__ __forceinline__ void recheck_item(const DevScene& sc, int kind, uint2 it, const float* __restrict__ q,
                                              const float* __restrict__ qs, const float* __restrict__ qe,
                                              long long offset, float dq, int policy, int* __restrict__ res,
                                              unsigned* __restrict__ key, unsigned long long& checks,
-                                             unsigned long long& flips, unsigned range)
+                                             unsigned long long& flips, PairSpan span)
 {
     float qi[GPRM_MAX_FRAMES];
     int t, tn;
     recheck_config(sc, kind, it, q, qs, qe, offset, dq, qi, t, tn);
-    const int code = check_config64(sc, qi, (int)(range & 0xffffu), (int)(range >> 16));
+    const int code = check_config64(sc, qi, span.lo, span.hi);
     ++checks;
     flips += ((code != 0) != ((int)(it.y >> 27) - 1 != 0));
     recheck_store(kind, it, code, t, tn, policy, res, key);
@@ -1540,7 +1552,7 @@ __device__ __forceinline__ void recheck_item_warp(const DevScene& sc, int kind, 
                                                   const float* __restrict__ qs, const float* __restrict__ qe,
                                                   long long offset, float dq, int policy, int* __restrict__ res,
                                                   unsigned* __restrict__ key, unsigned long long& checks,
-                                                  unsigned long long& flips, unsigned range, Warp64& W)
+                                                  unsigned long long& flips, PairSpan span, Warp64& W)
 {
     const int lane = threadIdx.x & 31;
     int t = 0, tn = 0;
@@ -1555,7 +1567,7 @@ __device__ __forceinline__ void recheck_item_warp(const DevScene& sc, int kind, 
         if (lane < sc.ndof)
             x = c1 * qs[(long long)it.x + offset * lane] + c2 * qe[(long long)it.x + offset * lane];
     }
-    const int code = warp_check64(sc, W.F, W.L, W.cen, W.queue, x, (int)(range & 0xffffu), (int)(range >> 16));
+    const int code = warp_check64(sc, W.F, W.L, W.cen, W.queue, x, span.lo, span.hi);
     if (lane == 0) {
         ++checks;
         flips += ((code != 0) != ((int)(it.y >> 27) - 1 != 0));
@@ -1578,11 +1590,11 @@ __global__ void __launch_bounds__(RECHECK_THREADS) k_recheck(DevScene sc, int ki
     if (recheck_by_warp(cnt, warps, sc.npairs)) {
         for (unsigned idx = warp * gridDim.x + blockIdx.x; idx < cnt; idx += warps)
             recheck_item_warp(sc, kind, bq.items[idx], q, qs, qe, offset, dq, policy, res, key, checks, flips,
-                              bq.pair_range ? bq.pair_range[idx] : 0xffff0000u, W[warp]);
+                              recheck_span(bq, idx, sc.npairs), W[warp]);
     } else {
         for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < cnt; idx += gridDim.x * blockDim.x)
             recheck_item(sc, kind, bq.items[idx], q, qs, qe, offset, dq, policy, res, key, checks, flips,
-                         bq.pair_range ? bq.pair_range[idx] : 0xffff0000u);
+                         recheck_span(bq, idx, sc.npairs));
     }
     if (checks) atomicAdd(&ctl->band_checks, checks);
     if (flips) atomicAdd(&ctl->band_flips, flips);
@@ -2454,7 +2466,7 @@ __global__ void __launch_bounds__(RECHECK_THREADS) k_recheck_multi(BatchView B, 
             const uint2 it = bq.items[idx];
             const DevScene& sc = B.scenes[problem_of(B, (long long)it.x)];
             recheck_item_warp(sc, kind, it, q, qs, qe, offset, sc.dq, policy, res, key, checks, flips,
-                              bq.pair_range ? bq.pair_range[idx] : 0xffff0000u, W[warp]);
+                              recheck_span(bq, idx, sc.npairs), W[warp]);
         }
         cnt = 0;
     }
@@ -2462,7 +2474,7 @@ __global__ void __launch_bounds__(RECHECK_THREADS) k_recheck_multi(BatchView B, 
         const uint2 it = bq.items[idx];
         const DevScene& sc = B.scenes[problem_of(B, (long long)it.x)];
         recheck_item(sc, kind, it, q, qs, qe, offset, sc.dq, policy, res, key, checks, flips,
-                     bq.pair_range ? bq.pair_range[idx] : 0xffff0000u);
+                     recheck_span(bq, idx, sc.npairs));
     }
     if (checks) atomicAdd(&ctl->band_checks, checks);
     if (flips) atomicAdd(&ctl->band_flips, flips);
