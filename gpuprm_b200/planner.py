@@ -472,13 +472,23 @@ def lazy_prm(cs, scene, starts, goals, n_samples, k=10, seed=0, mlp=None, prune=
                        "pruned": pruned, **({"phases_ms": ph.t} if profile else {})})
 
 
+# samples without a free one after which make_queries gives the scene up (a
+# free share of 1e-6 is missed with probability e^-16)
+QUERY_DRAWS = 1 << 24
+
+
 def make_queries(cs, scene, n_queries, seed):
-    """Seeded start/goal pairs among exactly checked free configurations."""
+    """Seeded start/goal pairs among exactly checked free configurations.
+    ValueError for a scene without free ones: as many draws in a row as hold
+    QUERY_DRAWS configurations, all colliding."""
     need = 2 * n_queries
-    got, s = [], 0
+    got, s, empty = [], 0, 0
     while sum(len(g) for g in got) < need:
         q = scenes.uniform_configs(scene, 4 * need, seed + 424242 + s)
         got.append(q[cs.check_configs(q) == 0])
+        empty = 0 if len(got[-1]) else empty + len(q)
+        if empty >= QUERY_DRAWS:
+            raise ValueError(f"no free configuration among {empty} uniform samples of the scene")
         s += 1
     allq = np.concatenate(got)[:need]
     return allq[:n_queries].copy(), allq[n_queries:].copy()
