@@ -415,6 +415,8 @@ int upload_certificates(gprm_space* h)
         CUDA_TRY(h, launch_static_pairs(s, cudaStreamLegacy));   /* after the copies, on their stream */
         CUDA_TRY(h, cudaMemcpy(settled.data(), s.scan_c, pb, cudaMemcpyDeviceToHost));
     }
+    h->general_pairs = 0;
+    for (const int4& c : settled) h->general_pairs += c.w == SCAN_GENERAL;
     SweepLists L;
     build_sweep(h, settled, L);
     if (L.leaf.size() > sweep_leaf_cap(h)) return fail(h, GPRM_ERR_STATE, "sweep lists exceed their buffer");
@@ -823,6 +825,19 @@ int enqueue_small(gprm_space* h, Request& r, int kind, const float* a, const flo
     return GPRM_OK;
 }
 
+/* Whether vertex checks of every size take a block per 32 configurations
+ * (k_configs_small): with pairs that no certificate can settle (links past
+ * GPRM_MAX_SLOTS) nearly every configuration fills its list of the large
+ * kernel's exact tests several times, each time after another sweep, while
+ * the blocks queue the tests as they come.  200,000 configurations, exact
+ * (fast) arithmetic: 21 moving links on 261 pairs 12.0 (11.7) ms in the
+ * large kernel, 3.2 (2.3) so; on 1,395 pairs 59 (56) ms, 7.4 (5.3). */
+constexpr int GENERAL_PAIRS = 12;
+bool vertices_by_block(const gprm_space* h)
+{
+    return h->small_smem && !h->profiling && !h->debug_qcap && h->npairs <= 65535 && h->general_pairs > GENERAL_PAIRS;
+}
+
 /* Enqueues one request on stream `st` with device inputs/outputs.
  * kind 0: q -> res.  kind 1: (qs, qe) -> res. */
 int enqueue_part(gprm_space* h, Request& r, int kind, const float* a, const float* b, int* res, long long n,
@@ -855,6 +870,12 @@ int enqueue_part(gprm_space* h, Request& r, int kind, const float* a, const floa
 {
     const int band_on = (h->mode & GPRM_MODE_FP64_BAND) != 0;
     CUDA_TRY(h, cudaMemsetAsync(ctl, 0, sizeof(Control), st));
+    if (kind == 0 && vertices_by_block(h)) {
+        CUDA_TRY(h, launch_configs_small(h->dsc, h->small_smem, a, (int)n, offset, 32, res, band_on, h->band, ctl, st));
+        CUDA_TRY(h, launch_accumulate(ctl, h->d_total, st));
+        h->host_stats.launches += 2;
+        return GPRM_OK;
+    }
     int recheck_blocks = h->sms * 4;
     /* the FP64 queue and, after the items' own region of the request
        (2 words per item from the part's first item), its overflow record */

@@ -110,6 +110,7 @@ struct gprm_space {
     void* d_scene = nullptr;
     gprm::DevScene dsc;
     gprm::LaunchCfg cfg_v, cfg_e;
+    int general_pairs = 0;        /* pairs that no certificate can settle (SCAN_GENERAL) */
     size_t small_smem = 0;        /* shared bytes of a small request's block (0: not available) */
 
     int mode = GPRM_MODE_FP64_BAND;

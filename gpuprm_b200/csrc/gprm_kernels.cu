@@ -620,8 +620,13 @@ constexpr unsigned PAIR_NONE = 0x7fffffffu;
  * configuration without a collision gives its next tests, one while 32 take
  * part, more as fewer do, so that a colliding configuration runs few tests
  * behind the one that decides it (without that, 15 tests a configuration
- * instead of 4 on the wall scene, the larger part of the kernel).  Lists
- * that overflow resume with another sweep.
+ * instead of 4 on the wall scene, the larger part of the kernel).  A
+ * configuration whose list is full leaves its other pairs to another sweep,
+ * which resumes with them; those pairs are not looked at before.  50,000
+ * configurations with a NaN joint, whose pairs all stay open, took 15 ms on
+ * 5,410 pairs with all their certificates evaluated in every sweep, 2.4 ms
+ * with that, 0.7 ms with their sweep left out (usual ones 2.5 ms); 100,003
+ * of the wall scene 3.20 -> 2.81 ms.
  * With every pair's certificates evaluated per lane in pair order this
  * kernel took 5.3 ms for 2^20 hull6 configurations and 7.4 ms for 100,003 of
  * the wall scene (exact), nearly all of it in those tests; slot points are
@@ -645,7 +650,14 @@ __device__ __forceinline__ void check_config_chunk(const DevScene& sc, const Sce
             if (x < sc.mins[j] || x > sc.maxs[j]) active = false;
         }
     }
-    if (active) lane_fk<FAST, false>(sc, S, [&](int j) { return q[i + offset * j]; });
+    bool finite = true;
+    if (active) {
+        lane_fk<FAST, false>(sc, S, [&](int j) { return q[i + offset * j]; });
+        const float* T = S.frames + (sc.ndof - 1) * 12 * 32;
+        finite = T[9 * 32] - T[9 * 32] == 0.0f && T[0] - T[0] == 0.0f;
+    }
+    /* a joint that is no number: no pair can be settled, the sweep is left out */
+    const unsigned wild = __ballot_sync(FULL_MASK, !finite);
     /* this lane's sweep ball: slot `lane`'s ball centre, or slot lane - 16's vertex 0 */
     const int slot = lane & (GPRM_MAX_SLOTS - 1);
     float4 point = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -703,10 +715,14 @@ __device__ __forceinline__ void check_config_chunk(const DevScene& sc, const Sce
                     if (lo > (unsigned)base) word = lo >= (unsigned)base + 32u ? 0u : word & (FULL_MASK << (lo & 31u));
                 } else if (g0 < sc.npairs) {
                     const int words = (min(sc.npairs - g0, SWEEP_GROUP) + 31) >> 5;
+                    const bool sweep = !((wild >> c) & 1u);
                     __syncwarp();
-                    for (int w = lane; w < words; w += 32) S.bits[w] = 0u;
+                    for (int w = lane; w < words; w += 32) {
+                        const int left = sc.npairs - g0 - 32 * w;
+                        S.bits[w] = sweep ? 0u : left >= 32 ? FULL_MASK : (1u << left) - 1u;
+                    }
                     __syncwarp();
-                    sweep_leaves<true>(sc, S, g0 / SWEEP_GROUP, FULL_MASK, true, GPRM_MAX_SLOTS);
+                    if (sweep) sweep_leaves<true>(sc, S, g0 / SWEEP_GROUP, FULL_MASK, true, GPRM_MAX_SLOTS);
                     __syncwarp();
                     row = 0;
                     rows = (words + 31) >> 5;
@@ -720,7 +736,9 @@ __device__ __forceinline__ void check_config_chunk(const DevScene& sc, const Sce
                         A.balls[lane] = make_float4(w.x, w.y, w.z, 0.0f);
                     }
                     __syncwarp();
-                    g0 = row = rows = 0;
+                    /* a resumed configuration: from the group of its pair on */
+                    g0 = (int)(__shfl_sync(FULL_MASK, from, c) / SWEEP_GROUP) * SWEEP_GROUP;
+                    row = rows = 0;
                 } else {
                     more = false;
                 }
@@ -750,6 +768,17 @@ __device__ __forceinline__ void check_config_chunk(const DevScene& sc, const Sce
             if (lane < left) A.open[lane] = mv;
             n = left;
             __syncwarp();
+            if (more && A.count[c] == VERTEX_TESTS) {
+                /* the list of the configuration in the sweep is full: its
+                   pairs that are not queued wait for another sweep */
+                const unsigned m = __ballot_sync(FULL_MASK, word != 0u);
+                int next = row < rows ? g0 - SWEEP_GROUP + row * 1024 : g0;
+                if (m) next = __shfl_sync(FULL_MASK, base + __ffs(word) - 1, __ffs(m) - 1);
+                if (lane == 0 && next < sc.npairs) atomicMin(&A.resume[c], (unsigned)next);
+                word = 0u;
+                row = rows;
+                g0 = sc.npairs;
+            }
         }
         /* the exact tests in rounds */
         const int tests = A.count[lane];
@@ -819,12 +848,11 @@ __device__ __forceinline__ void check_config_chunk(const DevScene& sc, const Sce
     __syncwarp();
 }
 
-/* 112 registers: 18 warps an SM where shared memory allows them (vertices of
- * hull6 3.56 -> 3.40 ms, of the 7-DOF wall 3.25 -> 3.21; 96 registers spill:
- * 3.55 and 3.48; the edge kernel is slower with 112 or 96: 57.9 -> 59.1 and
- * 59.9 ms). */
+/* 120 registers, without spills: 16 warps an SM (vertices of hull6 and of the
+ * 7-DOF wall 3.41 and 2.80 ms; 112 and 18 warps 3.43 and 2.80).  The
+ * edge kernel is slower with fewer than 128 (112: 57.9 -> 59.1 ms, 96: 59.9). */
 template <bool SMEM, bool FAST>
-__global__ void __maxnreg__(112) k_check_configs(DevScene sc, const float* __restrict__ q,
+__global__ void __maxnreg__(120) k_check_configs(DevScene sc, const float* __restrict__ q,
                                             long long n, long long offset,
                                             int* __restrict__ res, int band_on, float band,
                                             BandQueue bq,
@@ -2319,7 +2347,7 @@ cudaError_t configure_small(const DevScene& sc, size_t* bytes)
 cudaError_t launch_configs_small(const DevScene& sc, size_t smem, const float* q, int n, long long offset, int per,
                                  int* res, int band_on, float band, Control* total, cudaStream_t st)
 {
-    const int blocks = (n + per - 1) / per;
+    const int blocks = (int)(((long long)n + per - 1) / per);
     if (sc.fast)
         k_configs_small<true><<<blocks, SMALL_WARPS * 32, smem, st>>>(sc, q, n, offset, per, res, band_on, band, total);
     else
