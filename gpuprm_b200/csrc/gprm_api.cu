@@ -773,6 +773,14 @@ int event_pair(gprm_space* h, std::vector<cudaEvent_t>& pool, size_t& used, cuda
     return GPRM_OK;
 }
 
+/* Whether requests of the kind may take the kernels with a block per
+ * configuration or edge.  The queue-capacity hook, the per-kernel profile
+ * and a launch shape that the caller has set belong to the others. */
+bool block_kernels(const gprm_space* h, int kind)
+{
+    return h->small_smem && !h->profiling && !h->debug_qcap && h->npairs <= 65535 && !h->shape_set[kind];
+}
+
 /* Whether a request of n items goes through the small-request kernels.
  * Measured on one B200, host buffers in and out, exact arithmetic, us a
  * call, large path against small (box: 67 pairs, hull: 394, wall: 4117):
@@ -797,10 +805,11 @@ constexpr int SMALL_CONFIGS = 32768;
 constexpr int SMALL_EDGE_WAVES = 16, SMALL_EDGE_PAIRS = 2048;
 bool small_request(const gprm_space* h, int kind, long long n)
 {
-    /* the queue-capacity hook and the per-kernel profile belong to the large path */
-    if (!h->small_smem || h->profiling || h->debug_qcap || h->npairs > 65535 || n < 1) return false;
+    if (!block_kernels(h, kind) || n < 1) return false;
     const int wave = h->sms * 4;     /* resident blocks */
     if (kind == 0) return n <= SMALL_CONFIGS;
+    /* edges that the caller has not split, or in segments of its own choice */
+    if (n > h->split_max || h->split_rounds != SPLIT_ROUNDS) return false;
     return n <= wave || (n <= (long long)wave * SMALL_EDGE_WAVES && h->npairs >= SMALL_EDGE_PAIRS);
 }
 
@@ -835,7 +844,7 @@ int enqueue_small(gprm_space* h, Request& r, int kind, const float* a, const flo
 constexpr int GENERAL_PAIRS = 12;
 bool vertices_by_block(const gprm_space* h)
 {
-    return h->small_smem && !h->profiling && !h->debug_qcap && h->npairs <= 65535 && h->general_pairs > GENERAL_PAIRS;
+    return block_kernels(h, 0) && h->general_pairs > GENERAL_PAIRS;
 }
 
 /* Enqueues one request on stream `st` with device inputs/outputs.
@@ -1497,6 +1506,7 @@ int gprm_set_launch_shape(gprm_space* h, int vertex_kernel, int threads, int sce
                     threads, scene_in_smem, cudaGetErrorString(e));
     }
     (vertex_kernel ? h->cfg_v : h->cfg_e) = c;
+    h->shape_set[vertex_kernel ? 0 : 1] = true;
     return GPRM_OK;
 }
 

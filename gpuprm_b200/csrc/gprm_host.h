@@ -27,6 +27,9 @@ cudaError_t dev_malloc(void** p, size_t bytes);
  * previous one */
 constexpr int HOST_PARTS = 4;
 
+/* default rounds of 32 steps per segment of a split edge */
+constexpr int SPLIT_ROUNDS = 2;
+
 struct Request {
     cudaStream_t st = nullptr;
     Control* ctl = nullptr;       /* device, HOST_PARTS blocks (one per part) */
@@ -116,7 +119,8 @@ struct gprm_space {
     int mode = GPRM_MODE_FP64_BAND;
     int policy = GPRM_EDGES_ALL_STEPS;
     int split_max = 16384;        /* edge batches up to this size split long edges */
-    int split_rounds = 2;         /* rounds of 32 steps per segment */
+    int split_rounds = gprm::SPLIT_ROUNDS;  /* rounds of 32 steps per segment */
+    bool shape_set[2] = {false, false};     /* per kind (0 vertices, 1 edges): gprm_set_launch was called */
     float band = 1e-5f;
     unsigned debug_qcap = 0;      /* test hook: FP64 queue capacity cap (0 = none) */
     double qdens_edges = 0.0;     /* most FP64 queue items per edge seen in a call (sizes later queues) */

@@ -164,8 +164,12 @@ int gprm_set_edge_policy(gprm_space* h, int policy);
  * several warps, one per segment of about seg_rounds x 32 steps, so that a
  * small batch of long edges (lazy planning rounds, query attachment, path
  * verification) keeps the GPU busy; larger batches give each edge one
- * warp.  The codes do not depend on it.  No reference counterpart (the
- * reference runs one CUDA thread per edge step, robotconfigspace.cpp:362-595). */
+ * warp.  With the default seg_rounds the smallest of the batches that
+ * max_edges covers (how many edges depends on the pair list and the
+ * policy) give every edge blocks of four warps instead, in one launch that
+ * includes the FP64 checks.  The codes do not depend on any of it.  No
+ * reference counterpart (the reference runs one CUDA thread per edge step,
+ * robotconfigspace.cpp:362-595). */
 int gprm_set_edge_split(gprm_space* h, int max_edges, int seg_rounds);
 /* FP64 band half-width in metres (default 1e-5). */
 int gprm_set_band(gprm_space* h, float band_m);
@@ -527,7 +531,11 @@ int gprm_device_sm_count(const gprm_space* h);
  * 0: edge checks): threads per block (a multiple of 32, <= 512) and
  * whether the scene table is copied into shared memory (1) or read through
  * L1 (0).  Fails without changing anything if the shape does not fit.
- * gprm_init picks the shape with the most resident warps. */
+ * gprm_init picks the shape with the most resident warps.  Setting one takes
+ * every later request of the kind through these kernels; before, small
+ * requests (and vertex checks of robots with more moving links than the
+ * kernels track) take a block of four warps per configuration, per 32 of
+ * them or per edge, whose shape is fixed. */
 int gprm_set_launch(gprm_space* h, int vertex_kernel, int threads, int scene_in_smem);
 /* The same with at most blocks_per_sm resident blocks per SM (0 = as many
  * as fit): the kernel's shared-memory carveout is then set, before each
@@ -542,7 +550,10 @@ int gprm_get_launch(const gprm_space* h, int vertex_kernel, int* threads, int* s
 /* Kernel timing: while enabled, every request records CUDA events around
  * its FP32 check kernel and its FP64 recheck kernel on the stream they run
  * on; gprm_profile_read synchronises the device and returns the summed
- * durations (ms) and the number of timed FP32 launches since enabling. */
+ * durations (ms) and the number of timed FP32 launches since enabling.
+ * While enabled, requests of every size run these two kernels: the ones
+ * with a block per configuration or edge, which small requests take
+ * otherwise, check in FP32 and FP64 in one launch. */
 int gprm_profile_enable(gprm_space* h, int on);
 int gprm_profile_read(gprm_space* h, double* fp32_ms, double* fp64_ms, int64_t* fp32_launches);
 
