@@ -674,6 +674,7 @@ void release_request(Request& r)
     cudaFree(r.d_queue);
     cudaFree(r.d_qpair);
     cudaFree(r.d_ovf);
+    cudaFree(r.d_small);
     cudaFreeHost(r.ctl_host);
     cudaFreeHost(r.h_qwant);
     if (r.ev_q) cudaEventDestroy(r.ev_q);
@@ -690,6 +691,9 @@ void note_queue_demand(gprm_space* h, unsigned items, long long m)
     const double d = (double)items / (double)m;
     if (d > h->qdens_edges) h->qdens_edges = d;
 }
+
+/* Resident blocks of the small-request kernels. */
+int small_wave(const gprm_space* h) { return h->sms * 4; }
 
 /* Grows the buffers of `r` to hold `n` items of `kind`; the stream and
  * the control block are created on first use.  with_host: pinned staging. */
@@ -711,6 +715,18 @@ int ensure_request(gprm_space* h, Request& r, int kind, size_t n, bool with_host
             CUDA_TRY(h, dev_malloc((void**)&r.d_seg, edge_seg_words((long long)cap) * sizeof(unsigned)));
             r.cap_seg = cap;
         }
+    }
+    /* keys and counts of the edges that several blocks of a small request
+       share: zeroed once, every launch leaves them so */
+    if (kind == 1 && h->small_smem && !r.d_small) {
+        unsigned* p = nullptr;
+        const size_t bytes = 2 * (size_t)small_wave(h) * sizeof(unsigned);
+        CUDA_TRY(h, dev_malloc((void**)&p, bytes));
+        cudaError_t e = cudaMemset(p, 0, bytes);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);   /* other streams do not wait for it */
+        if (e != cudaSuccess) cudaFree(p);
+        CUDA_TRY(h, e);
+        r.d_small = p;
     }
     /* the demand of the last device-pointer edge call, once it has finished */
     if (r.q_pending) {
@@ -782,52 +798,87 @@ bool block_kernels(const gprm_space* h, int kind)
 }
 
 /* Whether a request of n items goes through the small-request kernels.
- * Measured on one B200, host buffers in and out, exact arithmetic, us a
- * call, large path against small (box: 67 pairs, hull: 394, wall: 4117):
- *   configurations                    box        hull       wall
- *     n = 1                           68 / 27    104 / 43   219 / 54
- *     n = 592                         182 / 73   346 / 106  1502 / 201
- *     n = 4096                        211 / 82   379 / 140  1661 / 545
- *     n = 32768                       270 / 156  502 / 366  2053 / 1232
- *   edges (0.25 rad on average)
- *     n = 32                          123 / 84   196 / 130  322 / 256
- *     n = 592                         193 / 105  335 / 257  532 / 332
- *     n = 1024                        194 / 125  283 / 372  847 / 785
- *     n = 4096                        239 / 281  425 / 615  2493 / 1154
+ * Measured on one B200, us a call, large path against small (box: 67 pairs,
+ * hull: 394, wall: 4117):
+ *   configurations       box             hull            wall
+ *   exact, host buffers
+ *     n = 1              68 / 26         82 / 40         93 / 51
+ *     n = 592            188 / 69        340 / 102       1495 / 199
+ *     n = 4096           221 / 80        381 / 143       1658 / 596
+ *     n = 32768          276 / 157       506 / 386       2073 / 1350
+ *   fast, device buffers
+ *     n = 592            153 / 42        272 / 71        1312 / 156
+ *     n = 32768          189 / 89        339 / 260       1733 / 1140
  * A warp of the large vertex kernel takes its 32 configurations through the
  * sweep stage one after the other, so its launch lasts that long however
  * few there are; a small request's block shares them over four warps.  At
  * 2^20 configurations the large kernel does three times the small one's
- * rate (hull).  An edge's block costs four warps for one: it pays while
- * every block is resident at once, and beyond that only on large pair
- * lists, where four warps share the sweep stage. */
+ * rate (hull).
+ *   edges of 0.25 | 2 | up to 9 rad on average, fast, device buffers, three
+ *   scenes each
+ *   all steps            box                     hull                    wall
+ *     n = 20             77/51 107/133 112/103   104/92 136/172 144/151  332/183 422/238 434/295
+ *     n = 74             81/59 107/66 110/106    119/99 159/164 166/248  537/322 611/277 636/493
+ *     n = 148            86/77 105/95 120/168    126/96 162/291 175/288  449/301 635/540 686/717
+ *     n = 592            100/79 125/143 126/202  148/221 192/319 285/434 617/652 641/702 1009/848
+ *     n = 4000                                                           811/1197 1968/2328
+ *   early exit
+ *     n = 74             81/58 99/60 101/65      133/103 199/111 249/126 464/203 1149/341 1068/606
+ *     n = 592            89/55 120/113 135/121   158/174 276/206 342/232 622/366 1918/786 2213/821
+ *     n = 4000                                                           869/902 3866/5450
+ * A block costs four warps for one.  It pays while there are few edges, on
+ * a long pair list, where the four share the sweep stage, as long as every
+ * edge has a block at once; on short lists (below SHORT_PAIRS) as long,
+ * because the large path's launches take longer than the checks; between
+ * them only for the fewest edges, but with early exit as long as on the
+ * others: there one step's collision cuts the other steps' tests short,
+ * which a warp an edge gains little from.  (149 and 789 pairs behave as the
+ * hull, 1621 as the wall.) */
 constexpr int SMALL_CONFIGS = 32768;
-constexpr int SMALL_EDGE_WAVES = 16, SMALL_EDGE_PAIRS = 2048;
+constexpr int SHORT_PAIRS = 128, LONG_PAIRS = 1536;
+int small_edges(const gprm_space* h)
+{
+    const bool all = h->policy != GPRM_EDGES_EARLY_EXIT;
+    return all && h->npairs >= SHORT_PAIRS && h->npairs < LONG_PAIRS ? small_wave(h) / 8 : small_wave(h);
+}
+
+/* Blocks per edge of a small request; those past an edge's rounds of 32
+ * steps return at once.  With all steps the rounds go from the end that
+ * decides, and a block that runs ahead is often for nothing: up to four,
+ * and two waves of them.  With early exit every round of a free edge has to
+ * be run: 8, or 16 on long lists.  A batch that leaves SMs idle has up to
+ * 16 either way.  One block an edge from half a wave on (the 2- and 9-rad
+ * edges above, n = 592, early exit): hull 206 -> 597, 232 -> 612; wall 786 ->
+ * 4591, 821 -> 5920 us. */
+int small_segs(const gprm_space* h, int n)
+{
+    const bool all = h->policy != GPRM_EDGES_EARLY_EXIT;
+    const int most = all ? 4 : h->npairs < LONG_PAIRS ? 8 : 16, blocks = all ? 2 * small_wave(h) : INT_MAX;
+    int segs = 1;
+    while (segs < 16 && ((2 * segs <= most && 2 * segs * n <= blocks) || 2 * segs * n <= h->sms)) segs *= 2;
+    return segs;
+}
+
 bool small_request(const gprm_space* h, int kind, long long n)
 {
     if (!block_kernels(h, kind) || n < 1) return false;
-    const int wave = h->sms * 4;     /* resident blocks */
     if (kind == 0) return n <= SMALL_CONFIGS;
     /* edges that the caller has not split, or in segments of its own choice */
     if (n > h->split_max || h->split_rounds != SPLIT_ROUNDS) return false;
-    return n <= wave || (n <= (long long)wave * SMALL_EDGE_WAVES && h->npairs >= SMALL_EDGE_PAIRS);
+    return n <= small_edges(h);
 }
 
-/* Enqueues a small request: one launch (after zeroing the keys of edges
- * that several blocks share).  status: pinned word for a rejected edge. */
+/* Enqueues a small request: one launch.  status: pinned word for a rejected edge. */
 int enqueue_small(gprm_space* h, Request& r, int kind, const float* a, const float* b, int* res, int n, long long offset,
                   cudaStream_t st, unsigned* status)
 {
     const int band_on = (h->mode & GPRM_MODE_FP64_BAND) != 0;
-    const int wave = h->sms * 4;     /* resident blocks */
+    const int wave = small_wave(h);
     if (kind == 0) {
         const int per = n <= wave ? 1 : std::min(32, (n + wave - 1) / wave);
         CUDA_TRY(h, launch_configs_small(h->dsc, h->small_smem, a, n, offset, per, res, band_on, h->band, h->d_total, st));
     } else {
-        int segs = 1;
-        while (segs < 16 && 2 * segs * n <= wave) segs *= 2;
-        if (segs > 1) CUDA_TRY(h, cudaMemsetAsync(r.d_ovf, 0, 2 * (size_t)n * sizeof(unsigned), st));
-        CUDA_TRY(h, launch_edges_small(h->dsc, h->small_smem, a, b, n, offset, h->dq, h->policy, segs, res, r.d_ovf,
+        CUDA_TRY(h, launch_edges_small(h->dsc, h->small_smem, a, b, n, offset, h->dq, h->policy, small_segs(h, n), res, r.d_small,
                                        band_on, h->band, h->d_total, status, st));
     }
     h->host_stats.launches += 1;

@@ -44,6 +44,7 @@ struct Request {
     size_t cap_seg = 0;           /* edges d_seg serves */
     uint2* d_queue = nullptr;
     unsigned* d_qpair = nullptr;  /* pair range of each queue item's recheck (BandQueue) */
+    unsigned* d_small = nullptr;  /* small edge requests: 2 words per edge, zero between launches */
     unsigned* d_ovf = nullptr;    /* overflow record of the FP64 queue: 2 words per item (BandQueue) */
     float* h_a = nullptr;         /* pinned staging */
     float* h_b = nullptr;

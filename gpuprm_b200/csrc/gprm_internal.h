@@ -164,8 +164,8 @@ cudaError_t launch_check_edges(const DevScene& sc, const LaunchCfg& cfg, const f
 /* Small requests in one launch each (k_configs_small, k_edges_small):
  * checks, FP64 rechecks, results and counters (added to `total`).  Inputs,
  * results and status may be pinned host memory.  per: configurations per
- * block (1..32); segs: blocks per edge, with scratch = 2 n zeroed words when
- * it is above 1.  smem: configure_small's bytes, not 0. */
+ * block (1..32); segs: blocks per edge, with scratch = 2 n zeroed words,
+ * which the launch leaves zeroed, when it is above 1.  smem: configure_small's bytes, not 0. */
 cudaError_t configure_small(const DevScene& sc, size_t* bytes);
 cudaError_t launch_configs_small(const DevScene& sc, size_t smem, const float* q, int n, long long offset, int per,
                                  int* res, int band_on, float band, Control* total, cudaStream_t st);

@@ -1899,7 +1899,8 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_configs_small(DevScene 
 
 /* Edges: block (e, s) of n * segs checks rounds s, s + segs, ... of edge e.
  * With segs > 1 scratch (2 n zeroed words) holds the edges' merged keys and
- * counts their finished blocks, the last of which writes the code.  status:
+ * counts their finished blocks, the last of which writes the code and leaves
+ * the words zeroed (a memset before each launch took 4 us).  status:
  * gets GPRM_DEVFLAG_BAD_EDGE for a non-finite or oversized edge (or null). */
 template <int POLICY, bool FAST>
 __global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_edges_small(DevScene sc, const float* __restrict__ qs,
@@ -1913,7 +1914,7 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_edges_small(DevScene sc
     __shared__ SmallShared B;
     const SceneView S = small_view(sc, smem);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int e = blockIdx.x / segs, s = blockIdx.x - e * segs;
+    const int s = blockIdx.x / n, e = blockIdx.x - s * n;   /* the edges' first rounds first */
     constexpr unsigned NONE = POLICY == EDGE_EARLY_EXIT ? 0xffffffffu : 0u;
     float ends = 0.0f;
     if ((lane & 15) < sc.ndof) ends = (lane < 16 ? qs : qe)[e + offset * (lane & 15)];
@@ -1927,6 +1928,8 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_edges_small(DevScene sc
     const float x = __fsqrt_rn(norm) / dq;
     const int tn = x < 1.0e8f ? (int)x + 1 : -1;
     const int R = (tn + 31) >> 5;      /* no round for a rejected edge */
+    if (s > 0 && s >= R) return;
+    const int parts = min(segs, max(R, 1));   /* blocks that share the edge */
     if (threadIdx.x == 0) {
         B.key = NONE;
         B.full = B.checks = B.flips = 0u;
@@ -1934,7 +1937,7 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_edges_small(DevScene sc
     unsigned exec = 0;
 #pragma unroll 1
     for (int r = s; r < R; r += segs) {
-        if (segs > 1) {
+        if (parts > 1) {
             /* a decision that no step of this round or a later one improves on */
             if (threadIdx.x == 0) {
                 unsigned kv = *(volatile unsigned*)&scratch[e];
@@ -2021,15 +2024,16 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_edges_small(DevScene sc
     if (threadIdx.x != 0) return;
     unsigned key = B.key;
     bool write = true;
-    if (segs > 1) {
+    if (parts > 1) {
         /* zeroed words: the larger is the better for both policies */
         if (key != NONE) atomicMax(&scratch[e], POLICY == EDGE_EARLY_EXIT ? ~key : key);
         __threadfence();
-        write = atomicAdd(&scratch[n + e], 1u) == (unsigned)segs - 1u;
+        write = atomicAdd(&scratch[n + e], 1u) == (unsigned)parts - 1u;
         if (write) {
             __threadfence();
             key = *(volatile unsigned*)&scratch[e];
             if (POLICY == EDGE_EARLY_EXIT) key = ~key;
+            scratch[e] = scratch[n + e] = 0u;   /* for the next launch */
         }
     }
     if (write) res[e] = key == NONE ? 0 : (int)(key & 15u) - 1;
