@@ -756,8 +756,12 @@ __device__ __forceinline__ void check_config_chunk(const DevScene& sc, const Sce
             const unsigned same = __match_any_sync(FULL_MASK, need ? own : 32u);
             if (need) {
                 const int at = A.count[own] + __popc(same & ((1u << lane) - 1u));
-                if (at < VERTEX_TESTS) A.test[at][own] = j;
-                else atomicMin(&A.resume[own], j);
+                if (at < VERTEX_TESTS) {
+                    A.test[at][own] = j;
+                    --pc.cert;
+                } else {
+                    atomicMin(&A.resume[own], j);
+                }
             }
             __syncwarp();
             if (need && (same >> lane) == 1u)   /* the last of its configuration */
@@ -810,7 +814,6 @@ __device__ __forceinline__ void check_config_chunk(const DevScene& sc, const Sce
                 if constexpr (FAST) code = pair_test_fast(sc, S.tab, pr, sc.ppoly[j], tp, tq, &mg);
                 else code = pair_test<PF32>(sc, S.tab, pr, tp, tq, &mg);
                 ++pc.full;
-                --pc.cert;
                 if (code != 0) {
                     const unsigned inb = band_on && in_band(code, mg, band) ? 16u : 0u;
                     atomicMin(&A.jkey[own], ((unsigned)j << 5) | inb | (unsigned)(code + 1));
@@ -822,7 +825,9 @@ __device__ __forceinline__ void check_config_chunk(const DevScene& sc, const Sce
             __syncwarp();
         }
         from = A.resume[lane];
-        todo = __ballot_sync(FULL_MASK, from != PAIR_NONE && A.jkey[lane] == JKEY_NONE);
+        const bool again = from != PAIR_NONE && A.jkey[lane] == JKEY_NONE;
+        if (from != PAIR_NONE && !again) pc.cert -= sc.npairs - from;   /* not looked at */
+        todo = __ballot_sync(FULL_MASK, again);
         __syncwarp();
     }
     int code = valid && !active ? 1 : 0;
@@ -1704,6 +1709,7 @@ struct SmallShared {
     unsigned key;                 /* the edge's merged key (all steps: max, early exit: min) */
     unsigned beaten;
     unsigned full, checks, flips;
+    unsigned long long cert;      /* pairs settled by a certificate */
 };
 
 /* What B.cut holds of a lane's collision outside the band at pair j. */
@@ -1762,6 +1768,7 @@ __device__ __forceinline__ void small_pairs(const DevScene& sc, const SceneView&
     const bool mine = (valid >> lane) & 1u;
     unsigned* q = B.queue[warp];
     PairCounts pc = {0, 0};
+    unsigned open = 0;            /* pairs that the sweep leaves to this warp */
     int n = 0;
 #pragma unroll 1
     for (int g0 = 0; g0 < sc.npairs; g0 += SWEEP_GROUP) {
@@ -1774,6 +1781,7 @@ __device__ __forceinline__ void small_pairs(const DevScene& sc, const SceneView&
         for (int w = warp; w < words; w += SMALL_WARPS) {
             const unsigned cand = S.bits[w];
             if (!cand) continue;
+            open += (unsigned)__popc(cand);
             const int j0 = g0 + 32 * w;
             bool scan = mine && ((unsigned)j0 << 8) <= *(volatile unsigned*)&B.jkey[lane];
             if (CUT != CUT_NONE && cutting) scan = scan && small_cut<CUT>(lane, j0) <= *(volatile unsigned*)&B.cut;
@@ -1797,6 +1805,11 @@ __device__ __forceinline__ void small_pairs(const DevScene& sc, const SceneView&
         __syncthreads();
     }
     if (n > 0) small_run<FAST, CUT>(sc, S, B, q, n, cutting, band_on, band);
+    const unsigned settled = __reduce_add_sync(FULL_MASK, (unsigned)pc.cert);
+    if (lane == 0) {
+        const long long left = (long long)(warp == 0 ? sc.npairs : 0) - open;
+        atomicAdd(&B.cert, settled + (unsigned long long)(left * __popc(valid)));
+    }
     __syncthreads();
 }
 
@@ -1835,7 +1848,10 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_configs_small(DevScene 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int i0 = blockIdx.x * per, count = min(per, n - i0);
     small_reset(B);
-    if (threadIdx.x == 0) B.full = B.checks = B.flips = 0u;
+    if (threadIdx.x == 0) {
+        B.full = B.checks = B.flips = 0u;
+        B.cert = 0ull;
+    }
     for (int t = threadIdx.x; t < sc.ndof * 32; t += blockDim.x) {
         const int j = t >> 5, i = t & 31;
         if (i < count) B.q[j][i] = q[i0 + i + offset * j];
@@ -1890,7 +1906,7 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_configs_small(DevScene 
     if (threadIdx.x == 0) {
         const unsigned done = (unsigned)__popc(valid);
         atomicAdd(&total->configs_exec, (unsigned long long)done);
-        atomicAdd(&total->certified, (unsigned long long)done * (unsigned)sc.npairs - B.full);
+        atomicAdd(&total->certified, B.cert);
         if (B.full) atomicAdd(&total->full_tests, (unsigned long long)B.full);
         if (B.checks) atomicAdd(&total->band_checks, (unsigned long long)B.checks);
         if (B.flips) atomicAdd(&total->band_flips, (unsigned long long)B.flips);
@@ -1933,6 +1949,7 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_edges_small(DevScene sc
     if (threadIdx.x == 0) {
         B.key = NONE;
         B.full = B.checks = B.flips = 0u;
+        B.cert = 0ull;
     }
     unsigned exec = 0;
 #pragma unroll 1
@@ -2046,7 +2063,7 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_edges_small(DevScene sc
     }
     if (exec) {
         atomicAdd(&total->steps_exec, (unsigned long long)exec);
-        atomicAdd(&total->certified, (unsigned long long)exec * (unsigned)sc.npairs - B.full);
+        atomicAdd(&total->certified, B.cert);
     }
     if (B.full) atomicAdd(&total->full_tests, (unsigned long long)B.full);
     if (B.checks) atomicAdd(&total->band_checks, (unsigned long long)B.checks);
