@@ -1709,7 +1709,7 @@ struct SmallShared {
     unsigned key;                 /* the edge's merged key (all steps: max, early exit: min) */
     unsigned beaten;
     unsigned full, checks, flips;
-    unsigned long long cert;      /* pairs settled by a certificate */
+    unsigned open;                /* pairs of the round that no certificate settles or that are left out */
 };
 
 /* What B.cut holds of a lane's collision outside the band at pair j. */
@@ -1758,17 +1758,19 @@ __device__ __forceinline__ void small_run(const DevScene& sc, const SceneView& S
 }
 
 /* Certificates and exact tests of one round for the lanes of `valid` (their
- * frames in S, ready to read by the block): fills jkey, jfirst and jlast.
- * Every thread of the block calls it; ends with a block barrier. */
+ * frames in S, ready to read by the block): fills jkey, jfirst and jlast,
+ * adds the pairs that certificates settle to total's.  Every thread of the
+ * block calls it; ends with a block barrier.  (The count is kept in shared
+ * memory: a register for it through the tests took 500 edges of the box
+ * scene from 100 to 104 us.) */
 template <bool FAST, int CUT>
 __device__ __forceinline__ void small_pairs(const DevScene& sc, const SceneView& S, SmallShared& B, unsigned valid,
-                                            bool cutting, int band_on, float band)
+                                            bool cutting, int band_on, float band, Control* total)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool mine = (valid >> lane) & 1u;
     unsigned* q = B.queue[warp];
     PairCounts pc = {0, 0};
-    unsigned open = 0;            /* pairs that the sweep leaves to this warp */
     int n = 0;
 #pragma unroll 1
     for (int g0 = 0; g0 < sc.npairs; g0 += SWEEP_GROUP) {
@@ -1781,11 +1783,12 @@ __device__ __forceinline__ void small_pairs(const DevScene& sc, const SceneView&
         for (int w = warp; w < words; w += SMALL_WARPS) {
             const unsigned cand = S.bits[w];
             if (!cand) continue;
-            open += (unsigned)__popc(cand);
             const int j0 = g0 + 32 * w;
             bool scan = mine && ((unsigned)j0 << 8) <= *(volatile unsigned*)&B.jkey[lane];
             if (CUT != CUT_NONE && cutting) scan = scan && small_cut<CUT>(lane, j0) <= *(volatile unsigned*)&B.cut;
             const unsigned need = scan ? lane_scan(sc, S, j0, cand, pc) : 0u;
+            const unsigned open = __reduce_add_sync(FULL_MASK, mine ? __popc(scan ? need : cand) : 0);
+            if (lane == 0) atomicAdd(&B.open, open);
             unsigned todo = __reduce_or_sync(FULL_MASK, need);
             while (todo) {
                 const int k = __ffs(todo) - 1;
@@ -1805,12 +1808,11 @@ __device__ __forceinline__ void small_pairs(const DevScene& sc, const SceneView&
         __syncthreads();
     }
     if (n > 0) small_run<FAST, CUT>(sc, S, B, q, n, cutting, band_on, band);
-    const unsigned settled = __reduce_add_sync(FULL_MASK, (unsigned)pc.cert);
-    if (lane == 0) {
-        const long long left = (long long)(warp == 0 ? sc.npairs : 0) - open;
-        atomicAdd(&B.cert, settled + (unsigned long long)(left * __popc(valid)));
-    }
     __syncthreads();
+    if (threadIdx.x == 0) {
+        atomicAdd(&total->certified, (unsigned long long)sc.npairs * (unsigned)__popc(valid) - B.open);
+        B.open = 0u;
+    }
 }
 
 /* The view of the block's one set of frames for this thread's lane. */
@@ -1848,10 +1850,7 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_configs_small(DevScene 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int i0 = blockIdx.x * per, count = min(per, n - i0);
     small_reset(B);
-    if (threadIdx.x == 0) {
-        B.full = B.checks = B.flips = 0u;
-        B.cert = 0ull;
-    }
+    if (threadIdx.x == 0) B.full = B.checks = B.flips = B.open = 0u;
     for (int t = threadIdx.x; t < sc.ndof * 32; t += blockDim.x) {
         const int j = t >> 5, i = t & 31;
         if (i < count) B.q[j][i] = q[i0 + i + offset * j];
@@ -1874,7 +1873,7 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_configs_small(DevScene 
             const int src = in ? lane : __ffs(valid) - 1;
             lane_fk<FAST, true, false>(sc, S, [&](int j) { return B.q[j][src]; });
             }
-        small_pairs<FAST, CUT_NONE>(sc, S, B, valid, false, band_on, band);
+        small_pairs<FAST, CUT_NONE>(sc, S, B, valid, false, band_on, band, total);
         if (in) {
             const unsigned jk = B.jkey[lane];
             if (jk != 0xffffffffu) {
@@ -1906,7 +1905,6 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_configs_small(DevScene 
     if (threadIdx.x == 0) {
         const unsigned done = (unsigned)__popc(valid);
         atomicAdd(&total->configs_exec, (unsigned long long)done);
-        atomicAdd(&total->certified, B.cert);
         if (B.full) atomicAdd(&total->full_tests, (unsigned long long)B.full);
         if (B.checks) atomicAdd(&total->band_checks, (unsigned long long)B.checks);
         if (B.flips) atomicAdd(&total->band_flips, (unsigned long long)B.flips);
@@ -1948,8 +1946,7 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_edges_small(DevScene sc
     const int parts = min(segs, max(R, 1));   /* blocks that share the edge */
     if (threadIdx.x == 0) {
         B.key = NONE;
-        B.full = B.checks = B.flips = 0u;
-        B.cert = 0ull;
+        B.full = B.checks = B.flips = B.open = 0u;
     }
     unsigned exec = 0;
 #pragma unroll 1
@@ -1993,7 +1990,8 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_edges_small(DevScene sc
 #pragma unroll 1
         for (bool cutting = true;; cutting = false) {
             small_reset(B);
-            small_pairs<FAST, POLICY == EDGE_EARLY_EXIT ? CUT_PAIR : CUT_LANE>(sc, S, B, valid, cutting, band_on, band);
+            small_pairs<FAST, POLICY == EDGE_EARLY_EXIT ? CUT_PAIR : CUT_LANE>(sc, S, B, valid, cutting, band_on, band,
+                                                                              total);
             jk = B.jkey[lane];
             code = jk == 0xffffffffu ? 0 : (int)(jk & 15u) - 1;
             oob = in && code != 0 && !(jk & 16u);
@@ -2061,10 +2059,7 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_edges_small(DevScene sc
             if (status) *status = GPRM_DEVFLAG_BAD_EDGE;
         }
     }
-    if (exec) {
-        atomicAdd(&total->steps_exec, (unsigned long long)exec);
-        atomicAdd(&total->certified, B.cert);
-    }
+    if (exec) atomicAdd(&total->steps_exec, (unsigned long long)exec);
     if (B.full) atomicAdd(&total->full_tests, (unsigned long long)B.full);
     if (B.checks) atomicAdd(&total->band_checks, (unsigned long long)B.checks);
     if (B.flips) atomicAdd(&total->band_flips, (unsigned long long)B.flips);
