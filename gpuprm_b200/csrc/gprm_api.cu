@@ -847,15 +847,18 @@ int small_edges(const gprm_space* h)
  * decides, and a block that runs ahead is often for nothing: up to four,
  * and two waves of them.  With early exit every round of a free edge has to
  * be run: 8, or 16 on long lists.  A batch that leaves SMs idle has up to
- * 16 either way.  One block an edge from half a wave on (the 2- and 9-rad
+ * 16 either way.  No more than the longest edge's rounds, where the caller
+ * knows them (host buffers, which every block reads its edge from: 592
+ * one-round edges of the box, early exit, 82 us; with 8 blocks each 112).
+ * One block an edge from half a wave on (the 2- and 9-rad
  * edges above, n = 592, early exit): hull 206 -> 597, 232 -> 612; wall 786 ->
  * 4591, 821 -> 5920 us. */
-int small_segs(const gprm_space* h, int n)
+int small_segs(const gprm_space* h, int n, int rounds)
 {
     const bool all = h->policy != GPRM_EDGES_EARLY_EXIT;
     const int most = all ? 4 : h->npairs < LONG_PAIRS ? 8 : 16, blocks = all ? 2 * small_wave(h) : INT_MAX;
     int segs = 1;
-    while (segs < 16 && ((2 * segs <= most && 2 * segs * n <= blocks) || 2 * segs * n <= h->sms)) segs *= 2;
+    while (segs < 16 && segs < rounds && ((2 * segs <= most && 2 * segs * n <= blocks) || 2 * segs * n <= h->sms)) segs *= 2;
     return segs;
 }
 
@@ -868,9 +871,28 @@ bool small_request(const gprm_space* h, int kind, long long n)
     return n <= small_edges(h);
 }
 
-/* Enqueues a small request: one launch.  status: pinned word for a rejected edge. */
+/* Rounds of 32 steps of the longest of n edges in host buffers (row stride
+ * n), not less than the kernels take. */
+int longest_rounds(const gprm_space* h, const float* a, const float* b, int n)
+{
+    float most = 0;
+    for (int i0 = 0; i0 < n; i0 += 256) {
+        const int m = std::min(256, n - i0);
+        float s[256] = {0};
+        for (int j = 0; j < h->ndof; ++j) {
+            const float *x = a + i0 + (size_t)n * j, *y = b + i0 + (size_t)n * j;
+            for (int i = 0; i < m; ++i) s[i] += (y[i] - x[i]) * (y[i] - x[i]);
+        }
+        for (int i = 0; i < m; ++i) most = s[i] > most ? s[i] : most;
+    }
+    const double steps = sqrt((double)most) * (1 + 1e-5) / h->dq + 1;
+    return steps < 1e8 ? (int)(steps / 32) + 1 : INT_MAX;
+}
+
+/* Enqueues a small request: one launch.  status: pinned word for a rejected
+ * edge.  rounds: of the longest edge, INT_MAX where that is not known. */
 int enqueue_small(gprm_space* h, Request& r, int kind, const float* a, const float* b, int* res, int n, long long offset,
-                  cudaStream_t st, unsigned* status)
+                  cudaStream_t st, unsigned* status, int rounds)
 {
     const int band_on = (h->mode & GPRM_MODE_FP64_BAND) != 0;
     const int wave = small_wave(h);
@@ -878,8 +900,8 @@ int enqueue_small(gprm_space* h, Request& r, int kind, const float* a, const flo
         const int per = n <= wave ? 1 : std::min(32, (n + wave - 1) / wave);
         CUDA_TRY(h, launch_configs_small(h->dsc, h->small_smem, a, n, offset, per, res, band_on, h->band, h->d_total, st));
     } else {
-        CUDA_TRY(h, launch_edges_small(h->dsc, h->small_smem, a, b, n, offset, h->dq, h->policy, small_segs(h, n), res, r.d_small,
-                                       band_on, h->band, h->d_total, status, st));
+        CUDA_TRY(h, launch_edges_small(h->dsc, h->small_smem, a, b, n, offset, h->dq, h->policy, small_segs(h, n, rounds), res,
+                                       r.d_small, band_on, h->band, h->d_total, status, st));
     }
     h->host_stats.launches += 1;
     return GPRM_OK;
@@ -906,7 +928,7 @@ int enqueue_part(gprm_space* h, Request& r, int kind, const float* a, const floa
 int enqueue(gprm_space* h, Request& r, int kind, const float* a, const float* b, int* res, long long n,
             long long offset, cudaStream_t st)
 {
-    if (small_request(h, kind, n)) return enqueue_small(h, r, kind, a, b, res, (int)n, offset, st, nullptr);
+    if (small_request(h, kind, n)) return enqueue_small(h, r, kind, a, b, res, (int)n, offset, st, nullptr, INT_MAX);
     int rc = enqueue_part(h, r, kind, a, b, res, n, offset, st, r.ctl, r.d_key);
     if (rc || kind != 1 || !(h->mode & GPRM_MODE_FP64_BAND) || r.q_pending) return rc;
     /* read the queue demand back for the next call's sizing, unless the
@@ -1025,7 +1047,8 @@ int submit_host(gprm_space* h, int kind, const float* a, const float* b, int* re
         }
         r.parts = 1;
         r.ctl_host[0].flags = 0;
-        rc = enqueue_small(h, r, kind, r.h_a, r.h_b, r.h_res, n, n, r.st, &r.ctl_host[0].flags);
+        rc = enqueue_small(h, r, kind, r.h_a, r.h_b, r.h_res, n, n, r.st, &r.ctl_host[0].flags,
+                           kind == 1 ? longest_rounds(h, r.h_a, r.h_b, n) : INT_MAX);
         if (rc) return rc;
     }
     /* parts: the host copies part p into pinned staging while the device
