@@ -889,20 +889,27 @@ int longest_rounds(const gprm_space* h, const float* a, const float* b, int n)
     return steps < 1e8 ? (int)(steps / 32) + 1 : INT_MAX;
 }
 
+/* Enqueues n vertex checks with a block per configuration or per up to 32 of
+ * them: one launch, which adds its counters to `total`. */
+int enqueue_vertices(gprm_space* h, const float* q, int* res, int n, long long offset, cudaStream_t st, Control* total)
+{
+    const int wave = small_wave(h);
+    const int per = n <= wave ? 1 : (int)std::min(32ll, ((long long)n + wave - 1) / wave);
+    CUDA_TRY(h, launch_configs_small(h->dsc, h->small_smem, q, n, offset, per, res, (h->mode & GPRM_MODE_FP64_BAND) != 0,
+                                     h->band, total, st));
+    h->host_stats.launches += 1;
+    return GPRM_OK;
+}
+
 /* Enqueues a small request: one launch.  status: pinned word for a rejected
  * edge.  rounds: of the longest edge, INT_MAX where that is not known. */
 int enqueue_small(gprm_space* h, Request& r, int kind, const float* a, const float* b, int* res, int n, long long offset,
                   cudaStream_t st, unsigned* status, int rounds)
 {
-    const int band_on = (h->mode & GPRM_MODE_FP64_BAND) != 0;
-    const int wave = small_wave(h);
-    if (kind == 0) {
-        const int per = n <= wave ? 1 : std::min(32, (n + wave - 1) / wave);
-        CUDA_TRY(h, launch_configs_small(h->dsc, h->small_smem, a, n, offset, per, res, band_on, h->band, h->d_total, st));
-    } else {
-        CUDA_TRY(h, launch_edges_small(h->dsc, h->small_smem, a, b, n, offset, h->dq, h->policy, small_segs(h, n, rounds), res,
-                                       r.d_small, band_on, h->band, h->d_total, status, st));
-    }
+    if (kind == 0) return enqueue_vertices(h, a, res, n, offset, st, h->d_total);
+    CUDA_TRY(h, launch_edges_small(h->dsc, h->small_smem, a, b, n, offset, h->dq, h->policy, small_segs(h, n, rounds),
+                                   res, r.d_small, (h->mode & GPRM_MODE_FP64_BAND) != 0, h->band, h->d_total, status,
+                                   st));
     h->host_stats.launches += 1;
     return GPRM_OK;
 }
@@ -953,9 +960,10 @@ int enqueue_part(gprm_space* h, Request& r, int kind, const float* a, const floa
     const int band_on = (h->mode & GPRM_MODE_FP64_BAND) != 0;
     CUDA_TRY(h, cudaMemsetAsync(ctl, 0, sizeof(Control), st));
     if (kind == 0 && vertices_by_block(h)) {
-        CUDA_TRY(h, launch_configs_small(h->dsc, h->small_smem, a, (int)n, offset, 32, res, band_on, h->band, ctl, st));
+        const int rc = enqueue_vertices(h, a, res, (int)n, offset, st, ctl);
+        if (rc) return rc;
         CUDA_TRY(h, launch_accumulate(ctl, h->d_total, st));
-        h->host_stats.launches += 2;
+        h->host_stats.launches += 1;
         return GPRM_OK;
     }
     int recheck_blocks = h->sms * 4;
@@ -1701,6 +1709,13 @@ extern "C" int gprm_indicator_batch_device_noalloc(gprm_space* h, const float* q
     unsigned char* base = nullptr;
     rc = noalloc_scratch(h, &base);
     if (rc) return rc;
+    /* the requests that take a block per configuration (or 32) need no
+       scratch: 32 configurations of the box scene (fast) took 90 us in the
+       large kernel (67 before it swept them one after the other), 18 so */
+    if (small_request(h, 0, n) || vertices_by_block(h)) {
+        h->host_stats.vertex_checks += n;
+        return enqueue_vertices(h, q, res, n, offset, (cudaStream_t)stream, h->d_total);
+    }
     Control* ctl = (Control*)base;
     /* one queue entry per configuration: the queue cannot overflow */
     BandQueue bq;

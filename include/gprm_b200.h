@@ -312,7 +312,10 @@ int gprm_mlp_set_wait_budget(gprm_mlp* h, long long cycles);
  * calls that overlap on the GPU (other streams, other handles, other host
  * threads) race and must be serialised by the caller.  q and res are
  * device pointers as in gprm_indicator_batch_device; `stream` NULL is the
- * legacy default stream.  Nothing is allocated by this call. */
+ * legacy default stream.  Nothing is allocated by this call.  Calls that
+ * gprm_indicator_batch_device checks with a block per configuration or per
+ * 32 of them (up to 32768 configurations, see gprm_set_launch) do so here
+ * too. */
 #define GPRM_NOALLOC_MAX_CONFIGS 65536
 int gprm_indicator_batch_device_noalloc(gprm_space* h, const float* q, int* res, int n, int offset,
                                         void* stream);
