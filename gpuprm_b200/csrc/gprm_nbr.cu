@@ -43,6 +43,7 @@ namespace {
 constexpr int NBR_MAX_GRID = GPRM_MAX_DOF;
 constexpr int NBR_MAX_K = 32;
 constexpr int NBR_MAX_CELLS = 1 << 21;
+constexpr int NBR_MAX_JOINT_CELLS = 1 << 17;   /* the slack for rounding is then 0.13 of a cell */
 /* cell size over the estimated distance of the 16th neighbour: smaller cells
  * hold fewer nodes out of reach, but more queries outgrow their 3^ndof block
  * (480,001 6-D nodes, k = 10: 3.5 ms at 1.1, 4.5 at 1.0, 8.3 at 0.9) */
@@ -640,7 +641,7 @@ __global__ void k_knn_grid_warp(GridView g, const float* __restrict__ q, int m, 
 }
 
 /* Second try for the queries the 3^ndof block could not settle: a warp per
- * query goes through the 5^ndof block around it and applies the same
+ * query goes through the 5^ndof (1-D: 17) block around it and applies the same
  * exactness test with that block's guard; a query it cannot settle either
  * goes to the full scan (redo2).  The k-th squared distance over the 3^ndof
  * block, left in the query's last output slot, bounds the true one from the
@@ -653,7 +654,7 @@ __global__ void __launch_bounds__(256) k_knn_wide(GridView g, const float* __res
                                                   const int* __restrict__ nredo, int* redo2, int* nredo2,
                                                   int* out_idx, float* out_dist)
 {
-    constexpr int SPAN = 5;
+    constexpr int SPAN = DIM == 1 ? 17 : 5;   /* 1-D: 44 nodes in five cells, too few for k = 32 */
     __shared__ KnnWarp ws[8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     KnnWarp& W = ws[warp];
@@ -922,26 +923,23 @@ int gprm_nbr_build(gprm_nbr* h, const float* x, int n, int stride, float cell, v
         const double unit = pow(M_PI, nd / 2.0) / tgamma(nd / 2.0 + 1.0);
         c = KNN_CELL * pow(16.0 * vol / ((n > 0 ? n : 1) * unit), 1.0 / nd);
     }
-    long long ncells = 1;
-    for (int d = 0; d < G; ++d) {
-        const double e = (n > 0 && mm[2 * d + 1] > mm[2 * d]) ? (double)mm[2 * d + 1] - mm[2 * d] : 0.0;
-        long long k = (long long)ceil(e / c);
-        if (k < 1) k = 1;
-        if (k > 1024) k = 1024;
-        g.nc[d] = (int)k;
-        g.lo[d] = n > 0 ? mm[2 * d] : 0.0f;
-        ncells *= k;
-    }
-    while (ncells > NBR_MAX_CELLS) {   /* coarsen until the grid fits */
-        c *= 1.25;
-        ncells = 1;
+    /* the whole range in cells of that size, coarsened until the grid fits
+       (at most 1024 cells in a joint and the nodes beyond in the last one:
+       91 % of 200,000 1-D nodes, 72 ms for their neighbours, 0.1 ms so) */
+    double cells, most;
+    for (;; c *= 1.25) {
+        cells = most = 1.0;
         for (int d = 0; d < G; ++d) {
-            const double e = (double)mm[2 * d + 1] - mm[2 * d];
-            long long k = (long long)ceil(e / c);
-            g.nc[d] = (int)(k < 1 ? 1 : k);
-            ncells *= g.nc[d];
+            const double e = (n > 0 && mm[2 * d + 1] > mm[2 * d]) ? (double)mm[2 * d + 1] - mm[2 * d] : 0.0;
+            const double k = fmin(fmax(ceil(e / c), 1.0), NBR_MAX_CELLS);
+            g.nc[d] = (int)k;
+            g.lo[d] = n > 0 ? mm[2 * d] : 0.0f;
+            cells *= k;
+            most = fmax(most, k);
         }
+        if (cells <= NBR_MAX_CELLS && most <= NBR_MAX_JOINT_CELLS) break;
     }
+    const long long ncells = (long long)cells;
     g.cell = (float)c;
     g.inv_cell = (float)(1.0 / c);
     /* slack of the exactness test: rounding of the cell assignment and of
