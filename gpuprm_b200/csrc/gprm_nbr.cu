@@ -344,6 +344,70 @@ __device__ __forceinline__ float cell_gap2(const GridView& g, float v, int d, in
     return gap2(g, fmaxf(below, above));
 }
 
+/* A thread per query, the node at sorted position t, over every cell around
+ * its own (queries and nodes in the same order: neighbouring threads read
+ * the same cells).  In up to three joints those are few cells, and a warp
+ * that shares them among its lanes mostly idles; with many nodes and a short
+ * list the threads are faster.  Uniform nodes, us, warp against thread:
+ *            65,536 nodes             200,000                  1,000,000
+ *   joints   k = 1    4       10      k = 1    4       10      k = 1     4        10
+ *   1        53/25    69/34   103/52  118/32   167/53  270/110 506/71    754/164  1291/402
+ *   2        69/34    83/51   119/86  163/48   209/80  309/193 726/138   961/264  1460/622
+ *   3        91/57    111/88  159/151 225/94   285/150 428/345 1040/336  1337/549 2048/1199
+ * (30,000 nodes, k = 10: 60/47, 68/78, 86/133; 30,000 crowded ones take a
+ * thread twice as long as a warp.) */
+constexpr int KNN_THREAD_DIM = 3, KNN_THREAD_K = 10, KNN_THREAD_NODES = 1 << 16;
+template <int DIM>
+__global__ void __launch_bounds__(128) k_knn_grid_thread(GridView g, int m, int k, int* out_idx, float* out_dist,
+                                                         int* redo, int* nredo)
+{
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < m; t += gridDim.x * blockDim.x) {
+        float qv[DIM];
+        const int qid = g.id[t];
+#pragma unroll
+        for (int j = 0; j < DIM; ++j) qv[j] = g.xs[t + (long long)g.n * j];
+        float ts[KNN_THREAD_K];
+        int ti[KNN_THREAD_K];
+        int len = 0;
+        TopkBound bound{INFINITY, 0x7fffffff};
+        int lo[NBR_MAX_GRID], hi[NBR_MAX_GRID];
+        float guard;
+        const bool finite = query_block(g, qv, lo, hi, &guard);
+        const int rows = block_rows(g, lo, hi);
+        for (int r = 0; r < rows; ++r) {
+            int b, e;
+            block_row_range(g, lo, hi, r, &b, &e);
+            for (int p = b; p < e; p += 4) {
+                float s[4];
+                if (p + 4 <= e) {
+                    dist2_4(g.xs, g.n, p, qv, DIM, s);
+                } else {
+                    for (int u = 0; u < 4; ++u) s[u] = p + u < e ? dist2(g.xs, g.n, p + u, qv, DIM) : 0.0f;
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const float sd = s[u] == s[u] ? s[u] : INFINITY;     /* NaN sorts last */
+                    if (p + u >= e || p + u == t || sd > bound.s) continue;
+                    const int id = g.id[p + u];
+                    if (!less_pair(sd, id, bound.s, bound.i)) continue;
+                    topk_insert(ts, ti, len, k, sd, id);
+                    topk_bound(ts, ti, len, k, bound);
+                }
+            }
+        }
+        const float kth = len ? ts[len - 1] : INFINITY;
+        if (knn_exact(g, finite, len, k, kth, guard)) {
+            for (int r = 0; r < k; ++r) {
+                out_idx[(long long)qid * k + r] = ti[r];
+                out_dist[(long long)qid * k + r] = sqrtf(ts[r]);
+            }
+        } else {
+            out_dist[(long long)qid * k + k - 1] = finite && len == k ? kth : INFINITY;
+            redo[atomicAdd(nredo, 1)] = qid;
+        }
+    }
+}
+
 template <int N> struct Pow3 { static constexpr int value = 3 * Pow3<N - 1>::value; };
 template <> struct Pow3<0> { static constexpr int value = 1; };
 
@@ -1002,7 +1066,13 @@ int gprm_nbr_knn(gprm_nbr* h, const float* q, int m, int qstride, int k, int que
     NBR_TRY(h, cudaMemsetAsync(h->nredo, 0, 2 * sizeof(int), st));
     if (queries_are_nodes) {
         const int blocks = (int)std::min<long long>(((long long)m + 7) / 8, (long long)h->sms * 16);
-        switch (h->ndof) {
+        const int tblocks = (int)(((long long)m + 127) / 128);
+        const bool by_thread = h->ndof <= KNN_THREAD_DIM && k <= KNN_THREAD_K && m >= KNN_THREAD_NODES;
+        switch (by_thread ? -h->ndof : h->ndof) {
+#define GPRM_KNN_THREAD(D)                                                                                    \
+        case -D: k_knn_grid_thread<D><<<tblocks, 128, 0, st>>>(h->g, m, k, idx, dist, h->redo, h->nredo); break
+        GPRM_KNN_THREAD(1); GPRM_KNN_THREAD(2); GPRM_KNN_THREAD(3);
+#undef GPRM_KNN_THREAD
 #define GPRM_KNN_GRID(D)                                                                             \
         case D: k_knn_grid<D><<<blocks, 256, 0, st>>>(h->g, m, k, idx, dist, h->redo, h->nredo); break
         GPRM_KNN_GRID(1); GPRM_KNN_GRID(2); GPRM_KNN_GRID(3); GPRM_KNN_GRID(4);
