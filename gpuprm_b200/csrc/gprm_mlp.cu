@@ -1901,6 +1901,13 @@ int adam(gprm_mlp* h, float lr, cudaStream_t st)
     return adam_at(h, lr, h->adam_t, nullptr, st);
 }
 
+/* Trainings of so few steps launch them directly: capturing and instantiating
+ * the graph costs 0.6 ms for a step and 2 ms for eight, with a stream per
+ * layer more than with one (batches of 4096, us, graph against direct: 1
+ * step 827 / 284, 8 2789 / 1203, 16 3735 / 2228, 2 x 16 5557 / 4332, 31 4207 /
+ * 4133, 128 16166 / 16673). */
+constexpr long long TRAIN_DIRECT_STEPS = 32;
+
 /* deterministic uniform init in [-1/sqrt(in), 1/sqrt(in)] (Linear's default
  * range) from a 64-bit LCG */
 double lcg_uniform(uint64_t& s)
@@ -2163,7 +2170,7 @@ int gprm_mlp_adam_step(gprm_mlp* h, float lr)
  * `epochs` passes in shuffled order (perm: device array of epochs*n
  * indices, each epoch a permutation), batches of `batch`, Adam at `lr`.
  * Every step runs features, forward, loss, backward and Adam on the
- * device, from a CUDA graph of a few steps.
+ * device, from a CUDA graph of a few steps (short trainings without one).
  * losses[epoch] gets the mean batch loss of each epoch (host array). */
 int gprm_mlp_train(gprm_mlp* h, const float* q, const float* y, int n, int offset, const int* perm, int epochs,
                    int batch, float lr, float* losses)
@@ -2187,29 +2194,40 @@ int gprm_mlp_train(gprm_mlp* h, const float* q, const float* y, int n, int offse
     while (steps % unroll) --unroll;
     const bool tc = h->train_path == GPRM_MLP_TRAIN_TCGEN05;
     if (tc) tc_weights(h, h->st);
+    /* the launches of `count` steps */
+    auto enqueue_steps = [&](int count) {
+        int r = GPRM_OK;
+        h->idx_off = h->d_ctl;
+        h->weights_kept = tc;
+        for (int s = 0; s < count && !r; ++s) {
+            features(h, q, offset, batch, perm, h->st);
+            if (!r) r = forward(h, batch, h->p, y, perm, 1.0f / batch, h->st);
+            if (!r) r = backward(h, batch, h->st);
+            if (!r) r = adam_at(h, lr, 0, reinterpret_cast<float*>(h->d_ctl + 2), h->st);
+        }
+        h->idx_off = nullptr;
+        h->weights_kept = false;
+        return r;
+    };
+    const bool direct = (long long)epochs * steps <= TRAIN_DIRECT_STEPS;
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
-    MLP_TRY(h, cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
+    cudaError_t ce = cudaSuccess;
     int crc = GPRM_OK;
-    h->idx_off = h->d_ctl;
-    h->weights_kept = tc;
-    for (int s = 0; s < unroll && !crc; ++s) {
-        features(h, q, offset, batch, perm, h->st);
-        if (!crc) crc = forward(h, batch, h->p, y, perm, 1.0f / batch, h->st);
-        if (!crc) crc = backward(h, batch, h->st);
-        if (!crc) crc = adam_at(h, lr, 0, reinterpret_cast<float*>(h->d_ctl + 2), h->st);
+    if (!direct) {
+        MLP_TRY(h, cudaStreamBeginCapture(h->st, cudaStreamCaptureModeThreadLocal));
+        crc = enqueue_steps(unroll);
+        ce = cudaStreamEndCapture(h->st, &graph);
+        if (crc) { if (graph) cudaGraphDestroy(graph); return crc; }
+        if (ce != cudaSuccess) return mfail(h, GPRM_ERR_CUDA, "capturing the training steps", ce);
+        ce = cudaGraphInstantiate(&exec, graph, 0);
     }
-    h->idx_off = nullptr;
-    h->weights_kept = false;
-    cudaError_t ce = cudaStreamEndCapture(h->st, &graph);
-    if (crc) { if (graph) cudaGraphDestroy(graph); return crc; }
-    if (ce != cudaSuccess) return mfail(h, GPRM_ERR_CUDA, "capturing the training steps", ce);
-    ce = cudaGraphInstantiate(&exec, graph, 0);
-    for (int e = 0; e < epochs && ce == cudaSuccess; ++e) {
+    for (int e = 0; e < epochs && ce == cudaSuccess && !crc; ++e) {
         const long long ctl[2] = {(long long)e * n, h->adam_t};
         ce = cudaMemcpyAsync(h->d_ctl, ctl, sizeof(ctl), cudaMemcpyHostToDevice, h->st);
         if (ce == cudaSuccess) ce = cudaMemsetAsync(h->loss, 0, sizeof(float), h->st);
-        for (int s = 0; s < steps && ce == cudaSuccess; s += unroll) ce = cudaGraphLaunch(exec, h->st);
+        if (direct && ce == cudaSuccess) crc = enqueue_steps(steps);
+        for (int s = 0; !direct && s < steps && ce == cudaSuccess; s += unroll) ce = cudaGraphLaunch(exec, h->st);
         float l = 0;
         if (ce == cudaSuccess) ce = cudaMemcpyAsync(&l, h->loss, sizeof(float), cudaMemcpyDeviceToHost, h->st);
         if (ce == cudaSuccess) ce = cudaStreamSynchronize(h->st);
@@ -2217,7 +2235,8 @@ int gprm_mlp_train(gprm_mlp* h, const float* q, const float* y, int n, int offse
         h->adam_t += steps;
     }
     if (exec) cudaGraphExecDestroy(exec);
-    cudaGraphDestroy(graph);
+    if (graph) cudaGraphDestroy(graph);
+    if (crc) return crc;
     if (ce != cudaSuccess) return mfail(h, GPRM_ERR_CUDA, "running the training epochs", ce);
     if (losses) memcpy(losses, ep_loss.data(), epochs * sizeof(float));
     if (h->dev_err) {
