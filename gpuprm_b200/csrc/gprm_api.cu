@@ -96,7 +96,7 @@ float float_ceil(double x)
     return f;
 }
 
-/* Certificate thresholds (see pair_certified in gprm_device.cuh).
+/* Certificate thresholds (see gprm_device.cuh).
  * eps_pos bounds, per coordinate, both the rounding of the reference's
  * world vertices (float transforms) and of the kernel's FMA ball centres;
  * radii are inflated by 2*eps_pos and by 1e-5 relative for the deviation

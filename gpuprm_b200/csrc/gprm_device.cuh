@@ -22,7 +22,7 @@
  *   int4   pairs[M]         (blockA, blockB, sysA, sysB) in the reference's
  *                           pair order (CRS by `from`)
  *   float4 pairs_b[M]       (R = rA + rB, T2, slotA, slotB) for the
- *                           separation certificates (see pair_certified)
+ *                           separation certificates (see points_certified)
  * A polytope in frame 0 (the world) is used untransformed: the reference
  * multiplies it by trafos[0], whose entries are exactly 1 and +-0, which
  * changes at most the sign of a zero coordinate; no comparison or nonzero
@@ -93,7 +93,7 @@ struct DevScene {
     /* certificates: a pair whose guaranteed separation along the first
        search direction exceeds thr_dir is reported free without the test;
        eps_dir bounds the direction error of the approximate first direction
-       times its distance (see pair_certified) */
+       times its distance (see points_certified) */
     float thr_dir, eps_dir;
     /* box certificate: per polytope 3 records (unit axis in its frame, half
        extent about the ball centre, inflated); per pair the two polytopes */
@@ -481,7 +481,8 @@ __device__ __forceinline__ int pair_test(const DevScene& sc, const float4* __res
     return -1;
 }
 
-/* Separation certificate for pair `pr` (FP32 kernels).
+/* Separation certificates of a pair (points_certified, lane by lane or for a
+ * whole warp in the sweep stage; pair_certified64).
  *
  * Balls: every world vertex the reference computes for polytope X lies in
  * the ball (c_X, r_X) (radii are inflated on the host by the rounding of
@@ -499,6 +500,10 @@ __device__ __forceinline__ int pair_test(const DevScene& sc, const float4* __res
  *   direction  S0 from vertex 0 of each polytope (FMA, rsqrt); its error
  *              against the reference's S0 is at most eps_dir/|s| (s the
  *              vertex-0 offset), charged against G with |D| + R.
+ *   box        the direction test with each polytope's support along S0
+ *              taken from its bounding box instead of its ball (every
+ *              vertex v of X has <S0, v - c_X> <= sum_a e_a |<a_a, R_X^T
+ *              S0>|), tighter for elongated links and flat obstacles.
  * NaN never passes (every test is a '>' comparison). */
 /* Support of polytope box B (3 records) along u, u in world coordinates;
  * frame f (0: world) rotates the box: its local direction is R^T u. */
@@ -521,67 +526,6 @@ __device__ __forceinline__ float box_support(const float4* __restrict__ B, const
         h = __fmaf_rn(b.w, fabsf(__fmaf_rn(b.x, lx, __fmaf_rn(b.y, ly, b.z * lz))), h);
     }
     return h;
-}
-
-/* The direction and box tests of pair_certified, for a pair whose distance
- * test failed: D = c_Q - c_P and d2 = |D|^2 as that test computed them.
- * The world vertex 0 of a moving polytope comes from its slot (written by
- * the FK pass with the FMA chain T*v0; cen points at the slot ball
- * centres, the vertex-0 points follow them), that of a static polytope is
- * its body-frame vertex 0.  A moving polytope without a slot has R = T2 =
- * infinity: nothing can be certified. */
-__device__ __forceinline__ bool pair_certified_dir(const DevScene& sc, const float4* __restrict__ tab, int4 pr,
-                                                   float4 pb, const float* cen, const float* frames, int j,
-                                                   float dx, float dy, float dz, float d2)
-{
-    if (!(pb.x < PF32::inf())) return false;
-    const int sa = __float_as_int(pb.z), sb = __float_as_int(pb.w);
-    const float* v0w = cen + sc.nslots * 3 * 32;
-    float ax, ay, az, bx, by, bz;
-    if (sa >= 0) { ax = v0w[(sa * 3) * 32]; ay = v0w[(sa * 3 + 1) * 32]; az = v0w[(sa * 3 + 2) * 32]; }
-    else { const float4 v = tab[pr.x + 1]; ax = v.x; ay = v.y; az = v.z; }
-    if (sb >= 0) { bx = v0w[(sb * 3) * 32]; by = v0w[(sb * 3 + 1) * 32]; bz = v0w[(sb * 3 + 2) * 32]; }
-    else { const float4 v = tab[pr.y + 1]; bx = v.x; by = v.y; bz = v.z; }
-    const float sx = bx - ax, sy = by - ay, sz = bz - az;
-    const float n2 = __fmaf_rn(sx, sx, __fmaf_rn(sy, sy, sz * sz));
-    if (!(n2 > 1e-6f)) return false;           /* |s| < 1e-3: leave it to the test */
-    const float inv = rsqrtf(n2);
-    const float G = __fmaf_rn(sx, dx, __fmaf_rn(sy, dy, sz * dz)) * inv - pb.x;
-    /* |D| from above (d2 * rsqrt(d2) is within 3 ulp of it) */
-    const float dn = d2 * rsqrtf(d2) * (1.0f + 2e-6f);
-    /* direction error <= eps_dir*inv (+ rsqrt and rounding, 1e-6) */
-    const float err = (dn + pb.x) * __fmaf_rn(sc.eps_dir, inv, 1e-6f);
-    if (G - err > sc.thr_dir) return true;
-    /* box test: the same bound with each polytope's support along S taken
-       from its bounding box instead of its ball (every vertex v of X has
-       <S, v - c_X> <= sum_a e_a |<a_a, R_X^T S>|), tighter for elongated
-       links and flat obstacles */
-    if (!sc.box || !(pb.x < PF32::inf())) return false;
-    const int2 pp = sc.ppoly[j];
-    const float ux = sx * inv, uy = sy * inv, uz = sz * inv;
-    const float hp = box_support(sc.box + 3 * pp.x, frames, pr.z, ux, uy, uz);
-    const float hq = box_support(sc.box + 3 * pp.y, frames, pr.w, ux, uy, uz);
-    const float Gb = __fmaf_rn(ux, dx, __fmaf_rn(uy, dy, uz * dz)) - (hp + hq) * (1.0f + 1e-5f);
-    return Gb - err > sc.thr_dir;
-}
-
-__device__ __forceinline__ bool pair_certified(const DevScene& sc, const float4* __restrict__ tab,
-                                               int4 pr, float4 pb, const float* cen,
-                                               const float* frames, bool* used_dir, int j)
-{
-    *used_dir = false;
-    const int sa = __float_as_int(pb.z), sb = __float_as_int(pb.w);
-    float px, py, pz, qx, qy, qz;
-    if (sa >= 0) { px = cen[(sa * 3) * 32]; py = cen[(sa * 3 + 1) * 32]; pz = cen[(sa * 3 + 2) * 32]; }
-    else { float4 b = tab[pr.x]; px = b.x; py = b.y; pz = b.z; }
-    if (sb >= 0) { qx = cen[(sb * 3) * 32]; qy = cen[(sb * 3 + 1) * 32]; qz = cen[(sb * 3 + 2) * 32]; }
-    else { float4 b = tab[pr.y]; qx = b.x; qy = b.y; qz = b.z; }
-    const float dx = qx - px, dy = qy - py, dz = qz - pz;
-    const float d2 = __fmaf_rn(dx, dx, __fmaf_rn(dy, dy, dz * dz));
-    if (d2 > pb.y) return true;
-    /* direction test: approximate first direction from vertex 0 of each */
-    *used_dir = true;
-    return pair_certified_dir(sc, tab, pr, pb, cen, frames, j, dx, dy, dz, d2);
 }
 
 /* The same certificate for the FP64 recheck, in double from the FP64
@@ -638,7 +582,7 @@ __device__ __forceinline__ bool pair_certified64(const DevScene& sc, const float
     const double G = (sx * dx + sy * dy + sz * dz) * inv - (double)pb.x;
     const double err = (sqrt(d2) + (double)pb.x) * 1e-6;
     if (G - err > (double)sc.thr_dir) return true;
-    /* the box test of pair_certified_dir: each polytope's support along the
+    /* the box test: each polytope's support along the
        first direction bounded by its box about the ball centre (the box
        records are inflated for float rounding, which covers FP64 vertices
        too); a moving polytope without a slot has no usable centre */

@@ -49,8 +49,8 @@ namespace gprm {
 
 size_t scene_smem_bytes(const DevScene& sc)
 {
-    /* tab | pairs | pairs_b | far | scan_c | scan_b, padded to 16 bytes */
-    return ((size_t)sc.ntab * 16 + (size_t)sc.npairs * 80 + 15) & ~(size_t)15;
+    /* tab | pairs | far | scan_c | scan_b */
+    return (size_t)sc.ntab * 16 + (size_t)sc.npairs * 64;
 }
 
 size_t frame_smem_bytes(const DevScene& sc, int threads, bool vertex_kernel)
@@ -61,7 +61,6 @@ size_t frame_smem_bytes(const DevScene& sc, int threads, bool vertex_kernel)
 struct SceneView {
     const float4* tab;
     const int4* pairs;
-    const float4* pairs_b;
     const float4* far;
     const int4* scan_c;
     const float4* scan_b;
@@ -103,29 +102,25 @@ __device__ __forceinline__ SceneView stage_scene(const DevScene& sc, unsigned ch
         const size_t np = (size_t)sc.npairs;
         float4* t = reinterpret_cast<float4*>(smem);
         int4* p = reinterpret_cast<int4*>(smem + (size_t)sc.ntab * 16);
-        float4* pb = reinterpret_cast<float4*>(smem + (size_t)sc.ntab * 16 + np * 16);
-        float4* fr = reinterpret_cast<float4*>(smem + (size_t)sc.ntab * 16 + np * 32);
-        int4* scc = reinterpret_cast<int4*>(smem + (size_t)sc.ntab * 16 + np * 48);
-        float4* scb = reinterpret_cast<float4*>(smem + (size_t)sc.ntab * 16 + np * 64);
+        float4* fr = reinterpret_cast<float4*>(smem + (size_t)sc.ntab * 16 + np * 16);
+        int4* scc = reinterpret_cast<int4*>(smem + (size_t)sc.ntab * 16 + np * 32);
+        float4* scb = reinterpret_cast<float4*>(smem + (size_t)sc.ntab * 16 + np * 48);
         for (int i = threadIdx.x; i < sc.ntab; i += blockDim.x) t[i] = sc.tab[i];
         for (int i = threadIdx.x; i < sc.npairs; i += blockDim.x) {
             p[i] = sc.pairs[i];
-            pb[i] = sc.pairs_b[i];
             fr[i] = sc.far[i];
             scc[i] = sc.scan_c[i];
             scb[i] = sc.scan_b[i];
         }
         s.tab = t;
         s.pairs = p;
-        s.pairs_b = pb;
         s.far = fr;
         s.scan_c = scc;
         s.scan_b = scb;
-        off = ((size_t)sc.ntab * 16 + np * 80 + 15) & ~(size_t)15;   /* frames stay 16-byte aligned */
+        off = (size_t)sc.ntab * 16 + np * 64;
     } else {
         s.tab = sc.tab;
         s.pairs = sc.pairs;
-        s.pairs_b = sc.pairs_b;
         s.far = sc.far;
         s.scan_c = sc.scan_c;
         s.scan_b = sc.scan_b;
@@ -196,7 +191,7 @@ __device__ __forceinline__ float rcp_fast(float x)
     return r;
 }
 
-/* The direction test of pair_certified_dir for every lane of the warp at
+/* The direction test of points_certified for every lane of the warp at
  * once.  Each polytope's ball centre lies in a ball over the lanes, and so
  * does its vertex 0 (the slot's sweep balls; radius 0 for a polytope of
  * frame 0): s = the difference of the vertex-0 ball centres, D = that of
@@ -357,8 +352,8 @@ __device__ __forceinline__ void sweep_stage(const DevScene& sc, const SceneView&
 /* The certificates of a pair for one configuration, given the world ball
  * centres p, q and vertices 0 a, b of its polytopes (T2, R: of the pair; c:
  * its scan_c; frames: the configuration's): the ball-distance and direction
- * tests of pair_certified without a branch between them, then, where both
- * miss, its box test. */
+ * tests without a branch between them, then, where both miss, the box
+ * test. */
 __device__ __forceinline__ bool points_certified(const DevScene& sc, const float* frames, int4 c, float T2, float R,
                                                  V3<float> p, V3<float> q, V3<float> a, V3<float> b)
 {
@@ -406,9 +401,9 @@ __device__ __forceinline__ void slot_points(const DevScene& sc, const SceneView&
     a = frame_point(S.frames, f, v);
 }
 
-/* points_certified for the lane whose slots and frames S holds: the moving
- * polytopes' points from the slots (written by the FK pass), a static one's
- * from the records f and b.  A pair that is not SCAN_USABLE is never
+/* points_certified for the lane whose frames S holds: the moving polytopes'
+ * points from their frames (slot_points), a static one's from the records f
+ * and b.  A pair that is not SCAN_USABLE is never
  * certified here (no slot, or two static polytopes whose certificate failed
  * when the tables were uploaded). */
 __device__ __forceinline__ bool lane_certified(const DevScene& sc, const SceneView& S, int4 c, float4 f, float4 b)
@@ -1683,7 +1678,7 @@ __global__ void k_fk_probe(DevScene sc, const float* q, float* out)
  * GPU idles, the exact tests of a warp run one after the other, the FP64
  * recheck is a second launch in which one thread goes through a check's
  * pairs, and control words, keys and results pass through eight more stream
- * operations.  k_check_small runs the whole request in one launch: a block
+ * operations.  The kernels below run the whole request in one launch: a block
  * of four warps per configuration (up to 32 of them, one per lane, for
  * larger requests) or per edge, whose rounds of 32 steps `segs` blocks
  * share.  Per round warp 0 runs the forward kinematics and the sweep balls,
@@ -1819,7 +1814,7 @@ __device__ __forceinline__ void small_pairs(const DevScene& sc, const SceneView&
 __device__ __forceinline__ SceneView small_view(const DevScene& sc, unsigned char* smem)
 {
     SceneView S;
-    S.tab = sc.tab; S.pairs = sc.pairs; S.pairs_b = sc.pairs_b;
+    S.tab = sc.tab; S.pairs = sc.pairs;
     S.far = sc.far; S.scan_c = sc.scan_c; S.scan_b = sc.scan_b;
     S.frames = reinterpret_cast<float*>(smem) + (threadIdx.x & 31);
     S.sweep = sweep_area<false>(sc, S.frames);
@@ -2080,10 +2075,11 @@ __global__ void k_static_pairs(DevScene sc, int4* __restrict__ scan_c)
     const int4 c = scan_c[j];
     const int4 pr = sc.pairs[j];
     if (c.w == SCAN_USABLE || pr.z != 0 || pr.w != 0) return;
-    /* no slot and no frame is read: both polytopes are untransformed */
-    __shared__ float none[1];
-    bool used_dir;
-    if (pair_certified(sc, sc.tab, pr, sc.pairs_b[j], none, none, &used_dir, j)) scan_c[j].w = SCAN_SETTLED;
+    const float4 pb = sc.pairs_b[j];
+    const float4 p = sc.tab[pr.x], a = sc.tab[pr.x + 1], q = sc.tab[pr.y], b = sc.tab[pr.y + 1];
+    /* no frame is read: both polytopes are untransformed */
+    if (points_certified(sc, nullptr, c, pb.y, pb.x, {p.x, p.y, p.z}, {q.x, q.y, q.z}, {a.x, a.y, a.z}, {b.x, b.y, b.z}))
+        scan_c[j].w = SCAN_SETTLED;
 }
 
 /* ------------------------------------------------------------------ */
@@ -2219,14 +2215,13 @@ cudaError_t configure_launch(const DevScene& sc, int vertex_kernel, int threads,
 cudaError_t plan_launch(const DevScene& sc, int vertex_kernel, int threads, LaunchCfg* cfg)
 {
     /* default: the variant with the most resident warps, the scene in shared
-       memory on ties (the autotuner times the candidates instead).  The
-       small blocks are for scenes whose frames leave room for some more
-       warps than whole blocks of four: 7 joints hold 12 warps in blocks of
-       128 and 13 in blocks of 32 (70,001 wall edges 14.19 -> 13.62 ms). */
+       memory on ties (the autotuner times the candidates instead).  Blocks
+       smaller than four warps never hold more: without the slots' points 16
+       warps fit for seven joints too. */
     LaunchCfg best{};
     int best_w = -1;
-    const int cand_threads[6] = {threads, 256, 384, 512, 64, 32};
-    for (int ci = 0; ci < 6; ++ci)
+    const int cand_threads[4] = {threads, 256, 384, 512};
+    for (int ci = 0; ci < 4; ++ci)
         for (int sm = 1; sm >= 0; --sm) {
             LaunchCfg c{};
             if (configure_launch(sc, vertex_kernel, cand_threads[ci], sm, &c) != cudaSuccess) {
@@ -2427,7 +2422,6 @@ __device__ __forceinline__ void switch_scene(const BatchView& B, int p, DevScene
     __syncwarp();
     S.tab = wsc->tab;
     S.pairs = wsc->pairs;
-    S.pairs_b = wsc->pairs_b;
     S.far = wsc->far;
     S.scan_c = wsc->scan_c;
     S.scan_b = wsc->scan_b;
