@@ -85,8 +85,8 @@ extern "C" {
  * edge, since the steps after it cannot hold the last colliding one.  The
  * default: besides giving the reference's codes, its rounds of neighbouring
  * steps let the warp-wide sweep certificates settle more pairs, and it ran
- * faster than the early-exit order on every workload measured (headline
- * edges 198 vs 218 ms, 7-DOF wall edges 1.64 vs 1.91 s). */
+ * faster than the early-exit order on every large batch measured (headline
+ * edges 105 vs 142 ms, 7-DOF wall edges 0.22 vs 0.64 s). */
 #define GPRM_EDGES_ALL_STEPS  1
 
 /* ---- scene description --------------------------------------------- */
