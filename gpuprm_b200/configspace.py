@@ -213,7 +213,8 @@ class RobotConfigspace:
     def set_launch(self, vertex_kernel: bool, threads: int, scene_in_smem: bool, blocks_per_sm: int = 0) -> None:
         """Launch shape of the FP32 kernels: threads per block, scene table in
         shared memory or through L1, and at most blocks_per_sm resident
-        blocks per SM (0: as many as fit; fewer leave more L1)."""
+        blocks per SM (0: as many as fit; fewer leave more L1).  Every later
+        request of the kind takes them, small ones too."""
         _check(self.lib, self.h, self.lib.gprm_set_launch_shape(self.h, int(vertex_kernel), threads,
                                                                 int(scene_in_smem), int(blocks_per_sm)))
 

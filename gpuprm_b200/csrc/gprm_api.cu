@@ -902,14 +902,18 @@ int enqueue_vertices(gprm_space* h, const float* q, int* res, int n, long long o
 }
 
 /* Enqueues a small request: one launch.  status: pinned word for a rejected
- * edge.  rounds: of the longest edge, INT_MAX where that is not known. */
+ * edge.  rounds: of the longest edge, INT_MAX where that is not known.
+ * zeroed: r.d_small is as the last launch left it, as it is for a request
+ * with a stream of its own; calls on the caller's streams zero it first, so
+ * that two that overlap against the rule spoil each other only. */
 int enqueue_small(gprm_space* h, Request& r, int kind, const float* a, const float* b, int* res, int n, long long offset,
-                  cudaStream_t st, unsigned* status, int rounds)
+                  cudaStream_t st, unsigned* status, int rounds, bool zeroed)
 {
     if (kind == 0) return enqueue_vertices(h, a, res, n, offset, st, h->d_total);
-    CUDA_TRY(h, launch_edges_small(h->dsc, h->small_smem, a, b, n, offset, h->dq, h->policy, small_segs(h, n, rounds),
-                                   res, r.d_small, (h->mode & GPRM_MODE_FP64_BAND) != 0, h->band, h->d_total, status,
-                                   st));
+    const int segs = small_segs(h, n, rounds);
+    if (segs > 1 && !zeroed) CUDA_TRY(h, cudaMemsetAsync(r.d_small, 0, 2 * (size_t)n * sizeof(unsigned), st));
+    CUDA_TRY(h, launch_edges_small(h->dsc, h->small_smem, a, b, n, offset, h->dq, h->policy, segs, res, r.d_small,
+                                   (h->mode & GPRM_MODE_FP64_BAND) != 0, h->band, h->d_total, status, st));
     h->host_stats.launches += 1;
     return GPRM_OK;
 }
@@ -935,7 +939,7 @@ int enqueue_part(gprm_space* h, Request& r, int kind, const float* a, const floa
 int enqueue(gprm_space* h, Request& r, int kind, const float* a, const float* b, int* res, long long n,
             long long offset, cudaStream_t st)
 {
-    if (small_request(h, kind, n)) return enqueue_small(h, r, kind, a, b, res, (int)n, offset, st, nullptr, INT_MAX);
+    if (small_request(h, kind, n)) return enqueue_small(h, r, kind, a, b, res, (int)n, offset, st, nullptr, INT_MAX, false);
     int rc = enqueue_part(h, r, kind, a, b, res, n, offset, st, r.ctl, r.d_key);
     if (rc || kind != 1 || !(h->mode & GPRM_MODE_FP64_BAND) || r.q_pending) return rc;
     /* read the queue demand back for the next call's sizing, unless the
@@ -1056,7 +1060,7 @@ int submit_host(gprm_space* h, int kind, const float* a, const float* b, int* re
         r.parts = 1;
         r.ctl_host[0].flags = 0;
         rc = enqueue_small(h, r, kind, r.h_a, r.h_b, r.h_res, n, n, r.st, &r.ctl_host[0].flags,
-                           kind == 1 ? longest_rounds(h, r.h_a, r.h_b, n) : INT_MAX);
+                           kind == 1 ? longest_rounds(h, r.h_a, r.h_b, n) : INT_MAX, true);
         if (rc) return rc;
     }
     /* parts: the host copies part p into pinned staging while the device

@@ -1912,7 +1912,7 @@ __global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_configs_small(DevScene 
 /* Edges: block (e, s) of n * segs checks rounds s, s + segs, ... of edge e.
  * With segs > 1 scratch (2 n zeroed words) holds the edges' merged keys and
  * counts their finished blocks, the last of which writes the code and leaves
- * the words zeroed (a memset before each launch took 4 us).  status:
+ * the words zeroed (a memset before a launch takes 4 us).  status:
  * gets GPRM_DEVFLAG_BAD_EDGE for a non-finite or oversized edge (or null). */
 template <int POLICY, bool FAST>
 __global__ void __launch_bounds__(SMALL_WARPS * 32, 4) k_edges_small(DevScene sc, const float* __restrict__ qs,

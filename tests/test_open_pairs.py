@@ -50,6 +50,23 @@ def test_codes_equal_the_oracle(size, mode):
             np.testing.assert_array_equal(got, want)
 
 
+@pytest.mark.parametrize("size", [SIZES[3], (7, 2, 350, False, 0)])
+def test_lists_that_overflow_in_both_sweep_groups(size):
+    """A band of 10 to 40 cm leaves hundreds of pairs a configuration open."""
+    sc = make(*size)
+    assert sc.num_pairs > 4096
+    q = scenes.uniform_configs(sc, 200, 11)
+    for band in (0.1, 0.4):
+        want, _, inb = O.Oracle(sc).check_configs(q, O.FP32_BAND | O.DEVICE_TRIG, band=band)
+        for large in (True, False):
+            cs = space(sc, EXACT, large)
+            cs.set_band(band)
+            np.testing.assert_array_equal(cs.check_configs(q), want)
+            s = cs.stats()
+            assert s["band_rechecks"] == int(inb.sum())
+            assert s["pairs_tested"] > 13 * (want == 0).sum()
+
+
 @pytest.mark.parametrize("mode", [EXACT, FAST])
 def test_many_configurations_by_block_equal_the_large_kernel(mode):
     sc = make(*SIZES[0])
@@ -63,7 +80,7 @@ def test_many_configurations_by_block_equal_the_large_kernel(mode):
 def seconds(cs, q, res):
     import torch
     best = 1e9
-    for _ in range(4):
+    for _ in range(10):
         torch.cuda.synchronize()
         t = time.perf_counter()
         cs.check_configs_device(q, res)
