@@ -692,9 +692,6 @@ void note_queue_demand(gprm_space* h, unsigned items, long long m)
     if (d > h->qdens_edges) h->qdens_edges = d;
 }
 
-/* Resident blocks of the small-request kernels. */
-int small_wave(const gprm_space* h) { return h->sms * 4; }
-
 /* Grows the buffers of `r` to hold `n` items of `kind`; the stream and
  * the control block are created on first use.  with_host: pinned staging. */
 int ensure_request(gprm_space* h, Request& r, int kind, size_t n, bool with_host, bool own_stream)
@@ -720,7 +717,7 @@ int ensure_request(gprm_space* h, Request& r, int kind, size_t n, bool with_host
        share: zeroed once, every launch leaves them so */
     if (kind == 1 && h->small_smem && !r.d_small) {
         unsigned* p = nullptr;
-        const size_t bytes = 2 * (size_t)small_wave(h) * sizeof(unsigned);
+        const size_t bytes = 2 * (size_t)small_wave(h->sms) * sizeof(unsigned);
         CUDA_TRY(h, dev_malloc((void**)&p, bytes));
         cudaError_t e = cudaMemset(p, 0, bytes);
         if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);   /* other streams do not wait for it */
@@ -839,7 +836,7 @@ constexpr int SHORT_PAIRS = 128, LONG_PAIRS = 1536;
 int small_edges(const gprm_space* h)
 {
     const bool all = h->policy != GPRM_EDGES_EARLY_EXIT;
-    return all && h->npairs >= SHORT_PAIRS && h->npairs < LONG_PAIRS ? small_wave(h) / 8 : small_wave(h);
+    return all && h->npairs >= SHORT_PAIRS && h->npairs < LONG_PAIRS ? small_wave(h->sms) / 8 : small_wave(h->sms);
 }
 
 /* Blocks per edge of a small request; those past an edge's rounds of 32
@@ -856,7 +853,7 @@ int small_edges(const gprm_space* h)
 int small_segs(const gprm_space* h, int n, int rounds)
 {
     const bool all = h->policy != GPRM_EDGES_EARLY_EXIT;
-    const int most = all ? 4 : h->npairs < LONG_PAIRS ? 8 : 16, blocks = all ? 2 * small_wave(h) : INT_MAX;
+    const int most = all ? 4 : h->npairs < LONG_PAIRS ? 8 : 16, blocks = all ? 2 * small_wave(h->sms) : INT_MAX;
     int segs = 1;
     while (segs < 16 && segs < rounds && ((2 * segs <= most && 2 * segs * n <= blocks) || 2 * segs * n <= h->sms)) segs *= 2;
     return segs;
@@ -893,10 +890,8 @@ int longest_rounds(const gprm_space* h, const float* a, const float* b, int n)
  * them: one launch, which adds its counters to `total`. */
 int enqueue_vertices(gprm_space* h, const float* q, int* res, int n, long long offset, cudaStream_t st, Control* total)
 {
-    const int wave = small_wave(h);
-    const int per = n <= wave ? 1 : (int)std::min(32ll, ((long long)n + wave - 1) / wave);
-    CUDA_TRY(h, launch_configs_small(h->dsc, h->small_smem, q, n, offset, per, res, (h->mode & GPRM_MODE_FP64_BAND) != 0,
-                                     h->band, total, st));
+    CUDA_TRY(h, launch_configs_small(h->dsc, h->small_smem, q, n, offset, configs_per_block(h->sms, n), res,
+                                     (h->mode & GPRM_MODE_FP64_BAND) != 0, h->band, total, st));
     h->host_stats.launches += 1;
     return GPRM_OK;
 }
@@ -918,17 +913,10 @@ int enqueue_small(gprm_space* h, Request& r, int kind, const float* a, const flo
     return GPRM_OK;
 }
 
-/* Whether vertex checks of every size take a block per 32 configurations
- * (k_configs_small): with pairs that no certificate can settle (links past
- * GPRM_MAX_SLOTS) nearly every configuration fills its list of the large
- * kernel's exact tests several times, each time after another sweep, while
- * the blocks queue the tests as they come.  200,000 configurations, exact
- * (fast) arithmetic: 21 moving links on 261 pairs 12.0 (11.7) ms in the
- * large kernel, 3.2 (2.3) so; on 1,395 pairs 59 (56) ms, 7.4 (5.3). */
-constexpr int GENERAL_PAIRS = 12;
+/* space_by_block, for a request of the handle's own. */
 bool vertices_by_block(const gprm_space* h)
 {
-    return block_kernels(h, 0) && h->general_pairs > GENERAL_PAIRS;
+    return block_kernels(h, 0) && space_by_block(h);
 }
 
 /* Enqueues one request on stream `st` with device inputs/outputs.

@@ -44,6 +44,7 @@ struct Layout {
     /* problems checked by their own launches (at least solo_min items) and
        the edge ranges of the shared launch (BatchView) */
     std::vector<int> solo;
+    std::vector<int> by_block;       /* configurations: problems that take a block per 32 (space_by_block) */
     long long nwork_e = 0;
     int K = 0;
     long long* d_woffs = nullptr;
@@ -147,8 +148,9 @@ BatchView view_of(const gprm_batch* b, int vertex_kernel)
 
 /* The call sequence of one batched check on stream `st`: every solo
  * problem through the single-problem kernels (its own scene and launch
- * shape), then the other problems in one shared launch, each part with its
- * FP64 recheck and overflow pass.  Allocates nothing and never
+ * shape), problems whose configurations take blocks of their own, then the
+ * others in one shared launch, each part but the blocks with its FP64 recheck
+ * and overflow pass.  Allocates nothing and never
  * synchronises (capturable). */
 int enqueue_batch(gprm_batch* b, int vertex_kernel, const float* qa, const float* qb, int* res, long long stride,
                   const LaunchCfg& cfg, Control* total, cudaStream_t st)
@@ -193,6 +195,12 @@ int enqueue_batch(gprm_batch* b, int vertex_kernel, const float* qa, const float
         }
         BATCH_TRY(b, launch_accumulate(b->ctl, total, st));
     }
+    for (int p : L.by_block) {
+        const gprm_space* s = b->spaces[p];
+        const long long off = L.offs[p], n = L.offs[p + 1] - off;
+        BATCH_TRY(b, launch_configs_small(s->dsc, s->small_smem, qa + off, (int)n, stride, configs_per_block(b->sms, n),
+                                          res + off, band_on, b->band, total, st));
+    }
     if (v.nwork > 0) {
         BandQueue bq;
         bq.items = L.d_queue;
@@ -235,7 +243,7 @@ int launches_per_call(const gprm_batch* b, int vertex_kernel)
     const int band_on = (b->mode & GPRM_MODE_FP64_BAND) != 0;
     const int per_part = 2 + 2 * band_on;
     const long long shared = vertex_kernel ? L.nchunks : L.nwork_e;
-    return per_part * ((int)L.solo.size() + (shared > 0 ? 1 : 0)) + (vertex_kernel ? 0 : 1);
+    return per_part * ((int)L.solo.size() + (shared > 0 ? 1 : 0)) + (int)L.by_block.size() + (vertex_kernel ? 0 : 1);
 }
 
 /* The solo problems and the shared launch's work of layout L under the
@@ -255,10 +263,14 @@ int build_work(gprm_batch* b, int vertex_kernel, long long solo_min)
     L.nchunks = L.nwork_e = 0;
     L.K = 0;
     L.solo.clear();
+    L.by_block.clear();
     std::vector<char> own(S, 0);
     for (int p = 0; p < S; ++p) {
         const long long n = L.offs[p + 1] - L.offs[p];
-        if (solo_min >= 0 && n > 0 && n >= solo_min) {
+        if (vertex_kernel && n > 0 && space_by_block(b->spaces[p])) {
+            own[p] = 1;
+            L.by_block.push_back(p);
+        } else if (solo_min >= 0 && n > 0 && n >= solo_min) {
             own[p] = 1;
             L.solo.push_back(p);
         }

@@ -139,3 +139,30 @@ struct gprm_space {
 
     std::string err = "no error";
 };
+
+namespace gprm {
+
+/* Whether vertex checks of the space take a block per 32 configurations
+ * (k_configs_small) at every size: with pairs that no certificate can settle
+ * (links past GPRM_MAX_SLOTS) nearly every configuration fills its list of
+ * the large kernel's exact tests several times, each time after another
+ * sweep, while the blocks queue the tests as they come.  200,000
+ * configurations, exact (fast) arithmetic: 21 moving links on 261 pairs 12.0
+ * (11.7) ms in the large kernel, 3.2 (2.3) so; on 1,395 pairs 59 (56) ms, 7.4
+ * (5.3). */
+constexpr int GENERAL_PAIRS = 12;
+inline bool space_by_block(const gprm_space* h)
+{
+    return h->small_smem && h->npairs <= 65535 && h->general_pairs > GENERAL_PAIRS;
+}
+
+/* Resident blocks of the small-request kernels, and the configurations that
+ * each of them takes of n. */
+inline int small_wave(int sms) { return sms * 4; }
+inline int configs_per_block(int sms, long long n)
+{
+    const long long wave = small_wave(sms);
+    return n <= wave ? 1 : (int)((n + wave - 1) / wave < 32 ? (n + wave - 1) / wave : 32);
+}
+
+}  // namespace gprm

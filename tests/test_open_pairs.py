@@ -110,3 +110,49 @@ def test_links_without_a_slot_cost_in_proportion():
     res = torch.empty(n, dtype=torch.int32, device="cuda:0")
     few = seconds(cs, q[:, :m].contiguous(), res[:m])
     assert seconds(cs, q, res) < 2.0 * n / m * few     # 4.4 times in the large kernel
+
+
+@pytest.mark.parametrize("mode", [EXACT, FAST])
+def test_a_batch_with_links_without_a_slot(mode):
+    import torch
+    from gpuprm_b200.batch import CONFIGS, ProblemBatch, offsets_of
+    scs = [scenes.make_box4(2), make(*SIZES[0]), scenes.make_hull6(3), make(*SIZES[1])]
+    counts = [700, 900, 0, 40]
+    q = [scenes.uniform_configs(s, n, 12 + n) for s, n in zip(scs, counts)]
+    spaces = [space(s, mode) for s in scs]
+    want = np.concatenate([space(s, mode).check_configs(x) for s, x in zip(scs, q)])
+    offs = offsets_of(counts)
+    rows = np.zeros((7, int(offs[-1])), np.float32)
+    for x, o in zip(q, offs):
+        rows[:x.shape[1], o:o + len(x)] = x.T
+    t = torch.tensor(rows, device="cuda:0")
+    b = ProblemBatch(spaces)
+    b.set_layout(CONFIGS, offs)
+    for threshold in (-1, 0, 800):
+        b.set_solo_threshold(CONFIGS, threshold)
+        res = torch.full((int(offs[-1]),), -7, dtype=torch.int32, device="cuda:0")
+        s = b.stats()
+        b.check_configs_device(t, res)
+        torch.cuda.synchronize()
+        np.testing.assert_array_equal(res.cpu().numpy(), want)
+        e = b.stats()
+        assert e["vertex_checks"] - s["vertex_checks"] == len(want)
+        assert e["pairs_tested"] > s["pairs_tested"]
+    b.capture(CONFIGS, t, None, res)
+    res.fill_(-7)
+    b.replay(CONFIGS)
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(res.cpu().numpy(), want)
+
+
+def test_a_batch_of_links_without_a_slot_costs_no_more_than_its_problem():
+    import torch
+    from gpuprm_b200.batch import CONFIGS, ProblemBatch, offsets_of
+    sc = make(*SIZES[0])
+    n = 200000
+    q = torch.tensor(np.ascontiguousarray(scenes.uniform_configs(sc, n, 10).T), device="cuda:0")
+    res = torch.empty(n, dtype=torch.int32, device="cuda:0")
+    alone = seconds(space(sc, FAST), q, res)
+    b = ProblemBatch([space(sc, FAST)])
+    b.set_layout(CONFIGS, offsets_of([n]))
+    assert seconds(b, q, res) < 1.5 * alone          # 5 times in the shared launch
