@@ -818,16 +818,17 @@ bool block_kernels(const gprm_space* h, int kind)
  * hull: 394, wall: 4117):
  *   configurations       box             hull            wall
  *   exact, host buffers
- *     n = 1              68 / 26         82 / 40         93 / 51
- *     n = 592            188 / 69        340 / 102       1495 / 199
- *     n = 4096           221 / 80        381 / 143       1658 / 596
- *     n = 32768          276 / 157       506 / 386       2073 / 1350
+ *     n = 1              77 / 36         82 / 40         93 / 51
+ *     n = 592            146 / 81        340 / 102       1495 / 199
+ *     n = 4096           189 / 95        381 / 143       1658 / 596
+ *     n = 32768          288 / 241       506 / 386       2073 / 1350
  *   fast, device buffers
- *     n = 592            153 / 42        272 / 71        1312 / 156
- *     n = 32768          189 / 89        339 / 260       1733 / 1140
+ *     n = 592            118 / 59        272 / 71        1312 / 156
+ *     n = 32768          145 / 114       339 / 260       1733 / 1140
  * A warp of the large vertex kernel takes its 32 configurations through the
- * sweep stage one after the other, so its launch lasts that long however
- * few there are; a small request's block shares them over four warps.  At
+ * sweep stage one after the other (on short lists, the box's, each lane goes
+ * through its own pairs), so its launch lasts that long however few there
+ * are; a small request's block shares them over four warps.  At
  * 2^20 configurations the large kernel does three times the small one's
  * rate (hull).
  *   edges of 0.25 | 2 | up to 9 rad on average, fast, device buffers, three

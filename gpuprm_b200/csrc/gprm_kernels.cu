@@ -7,7 +7,8 @@
  *
  * Work mapping (persistent grid, warps take work from a device counter):
  *   vertex checks  a warp takes 32 configurations: FK a lane each, then one
- *                  configuration after the other swept with a lane per pair,
+ *                  configuration after the other swept with a lane per pair
+ *                  (on short pair lists each by its lane),
  *                  and the pairs left tested 32 at a time whoever they belong
  *                  to, applied per configuration in pair order.
  *   edge checks    a warp takes one edge; its lanes hold 32 steps of that
@@ -606,10 +607,54 @@ static_assert(sizeof(VertexArea) == VERTEX_LANE_FLOATS * 32 * sizeof(float), "ve
 constexpr unsigned JKEY_NONE = 0xffffffffu;
 constexpr unsigned PAIR_NONE = 0x7fffffffu;
 
+/* Whether the certificates of a vertex check go a lane per configuration
+ * through every pair (lane_list) instead of a configuration after the other
+ * with a lane per pair.  The sweep of one configuration costs about 1,000
+ * warp instructions however short its leaves are, a pair's certificates for
+ * 32 configurations about 60.  400,000 configurations, fast (exact), us a
+ * call, sweep against lanes: 67 pairs of the box scene 859/519 (925/612), 91
+ * pairs 659/419 (748/529), 131 911/718 (1084/923), 208 1297/1118 (1523/1392),
+ * 256 1298/1121 (1464/1307), 340 1741/1634 (2040/1928), 370 1889/1911
+ * (2305/2296), 412 2057/2069 (2477/2494); the same order at 40,000. */
+constexpr int LANE_LIST_PAIRS = 256;
+__device__ __forceinline__ bool lane_lists(const DevScene& sc) { return sc.npairs <= LANE_LIST_PAIRS; }
+
+/* The certificates of this lane's configuration (mine: it takes part) over
+ * the pairs from `from` on, in pair order; the pairs that they leave go on
+ * its list, those that find no room there wait from the first on. */
+__device__ __forceinline__ void lane_list(const DevScene& sc, const SceneView& S, VertexArea& A, bool mine,
+                                          unsigned from, PairCounts& pc)
+{
+    const int lane = threadIdx.x & 31;
+    int at = 0;
+    unsigned rest = PAIR_NONE;
+#pragma unroll 1
+    for (int j0 = 0; j0 < sc.npairs; j0 += 32) {
+        const unsigned cand = __ballot_sync(FULL_MASK, j0 + lane < sc.npairs && S.scan_c[j0 + lane].w != SCAN_SETTLED);
+        if (!mine || rest != PAIR_NONE || from >= (unsigned)j0 + 32u) continue;
+        PairCounts settled = {0, 0};                /* the caller counts what is left */
+        unsigned need = lane_scan(sc, S, j0, cand, settled);
+        if (from > (unsigned)j0) need &= FULL_MASK << (from & 31u);
+        for (; need; need &= need - 1u) {
+            const unsigned j = (unsigned)(j0 + __ffs(need) - 1);
+            if (at == VERTEX_TESTS) {
+                rest = j;
+                break;
+            }
+            A.test[at++][lane] = j;
+            --pc.cert;
+        }
+    }
+    A.count[lane] = at;
+    A.resume[lane] = rest;
+    __syncwarp();
+}
+
 /* Configurations i0 .. i0+count-1 (count <= 32), one per lane.
  *
  * Lanes hold unrelated configurations, so what one needs another does not.
- * FK runs a lane per configuration; then the configurations go through the
+ * FK runs a lane per configuration; then, but on short pair lists
+ * (lane_lists), the configurations go through the
  * sweep stage one after the other, a lane per pair, with balls of radius 0
  * (whole leaves of far obstacles drop out at once); the pairs that leaves
  * open, of whichever configurations, go 32 at a time through their
@@ -674,12 +719,14 @@ __device__ __forceinline__ void check_config_chunk(const DevScene& sc, const Sce
     while (todo) {
         A.count[lane] = 0;
         A.resume[lane] = PAIR_NONE;
+        const bool lanes = lane_lists(sc);
+        if (lanes) lane_list(sc, S, A, (todo >> lane) & 1u, from, pc);
         /* the sweep in progress: configuration c, its next group of pairs
            g0, the next word row of the group's open bits, this lane's word */
         int c = 0, g0 = sc.npairs, row = 0, rows = 0, base = 0;
         unsigned word = 0u;
         int n = 0;                                      /* items in the open queue */
-        bool more = true;
+        bool more = !lanes;
 #pragma unroll 1
         while (more || n > 0) {
             while (n < 32 && more) {
